@@ -232,6 +232,8 @@ struct Schedule {
   std::vector<int32_t> nlev;       // [n_dir]
   std::vector<int32_t> nslots;     // [n_dir]
   int max_slots = 0;
+  int base_slots = 0;              // rows alive at once when outputs are read back within their own level
+  int64_t n_cut = 0;               // cut periodic inflow faces of all directions
   int max_src = 0;                 // largest number of periodic source elements of one direction
   // periodic interface
   std::vector<int64_t> x_base;     // [n_dir+1] source-cell offsets
@@ -308,22 +310,26 @@ obte_status build_schedule(const obte_problem* prob, const obte_material* mat, S
 obte_status set_transmission(Schedule& s, const double* side_transmission);
 
 // Device copy of the schedule in precision Real.
-//   rec      packed per-item records (level order, all directions)
-//   klev_*   kernel level pointers: levels split into units of at most `cap` items
+//   blk      static data of the units (records, outputs), desc their descriptors, unit_base the first unit of
+//            each direction
 //   vals     per-sweep (DeltaT + h, perturbation - wall inflow) pairs, level order
+//   pfe      periodic bank rows (source slot, destination), xrow their per-sweep values by unit and chunk
 //   si/sr    side table of special elements (periodic inflow, wall/periodic/contact outputs)
 struct DevSchedule {
   bool ready = false;
-  int G = 1, KV = 4, mc = 0, mcp = 0, n_chunks = 0, zero_slot = 0, rows = 0;   // G lanes x KV MFPs per element, mcp per CTA
-  int emax = 0, unit_wo = 0, pf_pad = 0, unit_sx = 0;   // periodic bank rows, per-unit staging sizes
-  int nbuf = 2;                            // TMA pipeline depth
+  int mc = 0, n_chunks = 0;                // MFPs per CTA, chunks of them
+  int threads = 128;                       // per CTA
+  int prow0 = 0, emax = 0;                 // first periodic bank row of the ring, rows per bank
+  int nbuf = 2;                            // units staged at once
+  int stage0 = 0, stage = 0, val_off = 0, gain_off = 0;   // shared-memory stages (bytes)
+  int out0 = 0, out = 0;                   // output blocks in shared memory
   size_t smem = 0;
-  DevBuf rec, klev_ptr, klev_off, knlev, kwo, kpf, pf, sx, ksx, mfp, tco, sig, wo_wall, wo_geo, kcoef, scoef, hs, vals, cellmap,
-      Pq, si, sr, wo_off, spec;
+  int64_t n_units = 0, n_pf = 0, row_stride = 0;   // units, periodic bank rows, reals of one state's rows
+  DevBuf blk, desc, unit_base, pfe, xrow, mfp, tco, sig, kcoef, scoef, hs, vals, cellmap, Pq, si, sr, spec;
   DevBuf lpt;                              // launch order: CTAs of the directions with the most units first
-  // FP64 tables: 1 / (1 + mfp_m D) per (direction, chunk, position, MFP of the chunk), so that the FP64
+  // FP64 tables: mfp_m / (1 + mfp_m D) per (direction, chunk, position, MFP of the chunk), so that the FP64
   // sweep multiplies instead of dividing on GB300's narrow FP64 pipe (null when over its memory cap)
-  DevBuf rinv;
+  DevBuf gain;
   // deterministic reductions (OBTE_DETERMINISTIC=1): per-(direction, chunk) partials and per-position sums
   DevBuf det_d, det_j, det_w, det_k, det_s, det_S, det_SJ;
   // transmission plans: the special-entry index of each item (host), so that new transmissions rewrite
@@ -424,6 +430,7 @@ struct obte_plan_s {
   int sweep_n_cta = 0;
   int sweep_batch = 1;                    // with the map: that many state vectors, sweep_batch_stride apart
   int64_t sweep_batch_stride = 0;
+  void* sweep_batch_rows = nullptr;       // periodic inflow rows of the batch (sweep_batch x d32.row_stride floats)
   std::unique_ptr<obte::XPrec> xprec;     // periodic-inflow block preconditioner
   std::unique_ptr<obte::DsaOp> dsa;       // diffusion-synthetic acceleration (built on first use)
   // set-up of `dsa` for new transmissions, on a host thread beside the refresh of the tables (joined by

@@ -909,6 +909,7 @@ extern "C" obte_status obte_bte_solve(obte_plan plan, const obte_solve_opts* opt
       plan->sweep_n_cta = 0;
       plan->sweep_batch = 1;
       plan->sweep_batch_stride = 0;
+      plan->sweep_batch_rows = nullptr;
     } else {
       OBTE_TRY(xs);
     }

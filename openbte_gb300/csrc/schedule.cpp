@@ -406,9 +406,10 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
   }
 
   struct DirOut {
+    int64_t n_cut = 0;
     std::vector<int32_t> lev, x_cell, wo_wall;
     std::vector<double> kcoef, scoef;
-    int nslots = 0;
+    int nslots = 0, base_slots = 0;
     obte_status st = OBTE_OK;
     std::string err;
   };
@@ -531,19 +532,27 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
     }
 
     // slots: an element is alive from its level to the last level of its consumers; elements
-    // with per-MFP outputs (periodic source, wall re-emission, contact) hold a slot for their
-    // own level so their outputs can be read back after the MFP loop
+    // with per-MFP outputs (periodic source, wall re-emission, contact) hold a slot until the next level,
+    // during which the sweep reads their outputs back
+    std::vector<int32_t> alive(nl + 1, 0);
     for (int64_t e = 0; e < n; ++e) {
       int32_t lu = -1;
       for (int64_t k = out_ptr[e]; k < out_ptr[e + 1]; ++k) lu = std::max(lu, level[out_adj[k]]);
       const bool special = src_of[e] >= 0 || !wall_out[e].empty() || ck == OBTE_CONTACT_NANOWIRE ||
                            co_ptr[e] != co_ptr[e + 1];
-      if (special) lu = std::max(lu, level[e]);
+      // (rows alive at once if they were read back within their own level: the FP32 shape's rule)
+      const int32_t own = special ? std::max(lu, level[e]) : lu;
+      if (own >= 0) { ++alive[level[e]]; --alive[own + 1]; }
+      if (special) lu = std::max(lu, level[e] + 1);
       last_use[e] = lu;
       slot_of[e] = -1;
     }
+    for (int32_t L = 0, live = 0; L < nl; ++L) {
+      live += alive[L];
+      o.base_slots = std::max(o.base_slots, live);
+    }
     {
-      std::vector<std::vector<int32_t>> release(nl + 1);
+      std::vector<std::vector<int32_t>> release(nl + 2);
       std::vector<int32_t> free_slots;
       int32_t next = 0;
       int64_t p = 0;
@@ -580,7 +589,7 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
       for (int64_t t = in_ptr[e]; t < in_ptr[e + 1]; ++t) {
         const int32_t f = in_face[t];
         if (k >= nf) { o.st = OBTE_ERR_BAD_ARG; o.err = "more inflow faces than element sides"; return; }
-        if (f_cut[f]) s.in_idx[it * nf + k] = pack_item(ITEM_PERIODIC, src_of[f_nb[f]]);
+        if (f_cut[f]) { s.in_idx[it * nf + k] = pack_item(ITEM_PERIODIC, src_of[f_nb[f]]); ++o.n_cut; }
         else s.in_idx[it * nf + k] = pack_item(ITEM_CELL, slot_of[f_nb[f]]);
         s.in_coef[it * nf + k] = g[f] * f_t[f];
         if (keep_tf) {
@@ -679,6 +688,8 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
   s.kcoef.clear();
   s.scoef.clear();
   s.max_slots = s.max_src = s.max_wo = 0;
+  s.n_cut = 0;
+  s.base_slots = 0;
   std::vector<int32_t> wo_base(n_dir), ce_base(n_dir);
   for (int q = 0; q < n_dir; ++q) {
     DirOut& o = outs[q];
@@ -688,6 +699,8 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
     s.nlev[q] = (int32_t)o.lev.size() - 1;
     s.nslots[q] = o.nslots;
     s.max_slots = std::max(s.max_slots, o.nslots);
+    s.base_slots = std::max(s.base_slots, o.base_slots);
+    s.n_cut += o.n_cut;
     s.x_base[q + 1] = s.x_base[q] + (int64_t)o.x_cell.size();
     s.x_cell.insert(s.x_cell.end(), o.x_cell.begin(), o.x_cell.end());
     s.max_src = std::max(s.max_src, (int)o.x_cell.size());

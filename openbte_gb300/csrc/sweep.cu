@@ -1,40 +1,33 @@
 // Batched upwind transport sweep for sm_103a.
 //
-// One CTA = one direction q x one chunk of MCP mean free paths.  The CTA walks
-// the direction's elements level by level (longest-path layers of the upwind
-// DAG with periodic inflow cut, split into units of at most 128 elements);
-// within a unit every thread owns one element and loops over the chunk's MFPs:
+// One CTA = one direction q x one chunk of KV mean free paths.  The CTA walks the direction's elements level
+// by level (longest-path layers of the upwind DAG with periodic inflow cut, split into units); within a
+// unit every thread takes elements tid, tid + threads, ... and computes the chunk's MFPs of each:
 //
 //   T_mq[c] = (b[c] + L_m (p[c] - sum_in g_f T_up,m)) / (1 + L_m D_q[c])
 //
-// the row of A_mq T = B of openbte/bte.py:183-218 for an element whose upwind
-// neighbours are known; b = DeltaT + heat source, p = perturbation minus the
-// wall inflow g_w T_B (openbte/bte.py:200,211-214).
+// the row of A_mq T = B of openbte/bte.py:183-218 for an element whose upwind neighbours are known;
+// b = DeltaT + heat source, p = perturbation minus the wall inflow g_w T_B (openbte/bte.py:200,211-214).
 //
-// T_up lives in a ring of shared-memory rows, one per live upstream element
-// and one column per MFP (row-major by MFP).  Extra rows: a zero row for absent
-// faces, a trash row for elements nobody reads, and two banks of rows for the
-// inflow across cut periodic faces: while unit u runs, its threads load the
-// periodic source values unit u+1 reads from the state vector and store them
-// into bank (u+1) & 1, so inflow across a cut face is an ordinary row read and
-// the ring does not grow with the number of periodic sources (3D meshes have
-// thousands per direction).  The MFP loop is therefore branch-free; elements
-// with per-MFP outputs (periodic source, wall re-emission, contact) read their
-// T back from their row afterwards.
+// T_up lives in a ring of shared-memory rows, one per live upstream element and one column per MFP.  Extra
+// rows: a zero row for absent faces, a trash row for elements nobody reads, and one bank of rows per staged
+// unit for the inflow across cut periodic faces, so inflow across a cut face is an ordinary row read and
+// the ring does not grow with the number of periodic sources (3D meshes have thousands per direction).
+// The MFP loop is branch-free; per-MFP outputs (periodic source, wall re-emission, contact) are read back from
+// the ring while the next unit runs.
 //
-// Data movement per unit: the packed element records, the per-sweep values
-// (b, p), the wall re-emission weights of the unit's wall entries and the
-// periodic prefetch list of the next unit arrive in shared memory by TMA bulk
-// copies (cp.async.bulk + mbarrier) issued two units ahead.  T never goes to
-// HBM.  Reductions of
-// openbte/bte.py:222-243 are register accumulations over the MFP loop followed
-// by one FP64 atomic per element (DeltaT', T_B', J) or per MFP (K, S).
-// Every mbarrier wait is bounded; on timeout the CTA raises the device error
-// word, stops using the buffers, waits (bounded) for its copies in flight and
-// leaves at the next block-wide barrier.
+// Data movement: everything a unit reads arrives in its stage of shared memory by TMA bulk copies
+// (cp.async.bulk + mbarrier), `nbuf` units ahead: the unit's records, its list of outputs, its (b, p) values, its periodic inflow rows (gathered per sweep by
+// sweep_prep_kernel, already in the table's precision and row layout) and, in FP64, its rows of the gain
+// table.  The header carries the source addresses of the unit nbuf further, so the loop reads no global
+// metadata.  T never goes to HBM.  Reductions of openbte/bte.py:222-243 are register accumulations over the
+// MFPs followed by one FP64 atomic per element (DeltaT', T_B', J) or per MFP (K, S).
+// Every mbarrier wait is bounded; on timeout the thread raises the device error word and skips the unit,
+// and the CTA waits (bounded) for its copies in flight and leaves after the next block-wide barrier.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -45,15 +38,24 @@
 
 namespace obte {
 
-static constexpr int kUnit = 128;      // elements per level unit = threads per CTA
+static constexpr int kMaxThreads = 128;   // threads per CTA at most
+static constexpr int kBaseUnit = 128;     // elements per unit of the base layout
 
 // ---- packed element records -------------------------------------------------------
-// 32-bit words, ring rows in 16-bit halves:
-//   w0 cell | w1 so, s0 | w2 s1, s2 | w3 s3, sp | the reals c0 .. c(NF-1), D | padding to 16 B
-// so = output row, s* = inflow rows (s3 only for NF = 4), sp = 1 + index of the element's output entry
-// among its unit's entries (0: no per-MFP outputs).  Triangles: 32 B (FP32) / 48 B (FP64);
-// tetrahedra: 48 B / 64 B.  Output entries (int4: periodic source index xk, wall re-emission entries
-// (begin << 3 | count, begin relative to the direction), contact entry, 0) are a separate per-unit table.
+// 32-bit words, ring rows as 16-bit halves in units of 16 bytes (ring_field):
+//   w0 cell | w1 so, s0 | w2 s1, s2 | w3 s3, kc | the reals c0 .. c(NF-1), D | padding to 16 B
+// so = output row, s* = inflow rows (s3 only for NF = 4), kc = 1 + index of a contact element's entry in its
+// unit's list of wall / contact entries (0: no contact side), bit 15 set for a periodic source.  Triangles: 32 B (FP32) / 48 B (FP64); tetrahedra:
+// 48 B / 64 B.
+// A unit's static data: its record block (header, records), followed by its output block:
+//   header 0: elements | (values start one pair into their window) << 16, first position, periodic outputs |
+//             wall and contact outputs << 16, then of unit u + nbuf: bank rows | size of its output block << 16
+//   header 1: of unit u + nbuf: record block and value sources (16-byte units), their sizes (16-byte units,
+//             block | values << 16), its first bank row among all units' rows
+//   outputs:  periodic sources (int2: source slot, row; padded to 16 B), wall / contact entries (int4: row,
+//             count | first of the unit's wall entries << 3 | wall entries of the unit << 16, contact entry, first
+//             wall entry overall), wall entries (4 reals: area vector / volume, 1 / (-sum_mq min(sigma . w, 0))),
+//             their wall indices
 __host__ __device__ constexpr int rec_words(int real_bytes, int nf) {
   return ((4 + (nf + 1) * (real_bytes / 4)) + 3) & ~3;
 }
@@ -61,29 +63,38 @@ template <typename Real, int NF> struct Rec {
   static constexpr int CSTEP = sizeof(Real) / 4, COEF = 4, D = COEF + NF * CSTEP;
   static constexpr int W = rec_words(sizeof(Real), NF);
 };
+static constexpr int kHeader = 32;   // bytes
+
+// 16-bit row reference: byte offset of the row's first 16 bytes in the ring, over 16.  A lane reads a 32-byte
+// row as two 16-byte halves; eight lanes (128 bytes) are served per pass, and with the halves in plain
+// order all first halves would share 4 of the 8 16-byte bank groups.  Rows whose index has bit 2 set keep
+// their halves swapped, so eight consecutive rows' first halves cover all the banks (60k-triangle cell,
+// random row order: 9.0 -> 7.0 passes per 32-lane load; 3.6 would be conflict-free).
+__host__ __device__ constexpr int ring_field(int row, int row_bytes) {
+  return row_bytes == 32 ? 2 * row + ((row >> 2) & 1) : row;
+}
 
 // special-element table
 //   si: xk wout contact nwall w0 w1 w2 pad     (8 ints)
 //   sr: wc0 wc1 wc2 pad                          (4 reals)
 static constexpr int SI = 8, SR = 4;
 
-// Level units: each level of direction q split into runs of at most kUnit elements, and cut so that no
-// unit holds more than kUnitPf cut periodic inflow faces or kUnitSx output entries.  The per-unit
-// staging areas and the two periodic banks of the ring are sized by the largest unit; without the caps
-// the few units on the periodic boundaries (up to ~110 cut faces and outputs each on the 60k-triangle
-// cell) set them, and the extra ~5 KB cost a CTA per SM (4 instead of 5 at 8 MFPs per lane).  A cap only
-// applies when at most 1 % of the uncapped units exceed it: where most units are over it (the pixel
-// model, where every element has reflecting-wall outputs) it would split every unit and lengthen every
-// chain instead.
+// Level units: each level of direction q split into runs of at most `cap` elements, and cut so that no unit
+// holds more than kUnitPf cut periodic inflow faces or kUnitSx output entries.  The stages and the periodic
+// banks of the ring are sized by the largest unit; without the caps the few units on the periodic
+// boundaries (up to ~110 cut faces and outputs each on the 60k-triangle cell) set them, and the extra ~5 KB
+// cost a CTA per SM.  A cap only applies when at most 1 % of the uncapped units exceed it: where most units
+// are over it (the pixel model, where every element has reflecting-wall outputs) it would split every unit
+// in two and lengthen every chain instead.
 constexpr int kUnitPf = 48;
 constexpr int kUnitSx = 64;
 struct Units {
   std::vector<int32_t> ptr;   // per direction: n[q] + 1 positions (relative to the direction)
-  std::vector<int64_t> off;   // [n_dir] first entry of direction q in ptr (and in kpf, kwo)
+  std::vector<int64_t> off;   // [n_dir] first entry of direction q in ptr
   std::vector<int32_t> n;     // [n_dir] units of direction q
 };
 
-static void build_units_capped(const Schedule& s, int cap_pf, int cap_sx, Units& un, int64_t* over_pf,
+static void build_units_capped(const Schedule& s, int cap, int cap_pf, int cap_sx, Units& un, int64_t* over_pf,
                                int64_t* over_sx) {
   // directions in parallel into their own lists, concatenated in direction order
   std::vector<std::vector<int32_t>> per(s.n_dir);
@@ -107,7 +118,7 @@ static void build_units_capped(const Schedule& s, int cap_pf, int cap_sx, Units&
         for (int f = 0; f < s.nf; ++f)
           if ((int)((uint32_t)s.in_idx[it * s.nf + f] >> ITEM_SHIFT) == ITEM_PERIODIC) ++pf;
         const int sx = (s.xk[it] >= 0 || s.wout[it] != 0 || s.contact[it] >= 0) ? 1 : 0;
-        if (cnt > 0 && (cnt == kUnit || npf + pf > cap_pf || nsx + sx > cap_sx)) close(pos);
+        if (cnt > 0 && (cnt == cap || npf + pf > cap_pf || nsx + sx > cap_sx)) close(pos);
         ++cnt;
         npf += pf;
         nsx += sx;
@@ -130,128 +141,214 @@ static void build_units_capped(const Schedule& s, int cap_pf, int cap_sx, Units&
   if (over_sx) *over_sx = std::accumulate(osx.begin(), osx.end(), (int64_t)0);
 }
 
-static void build_units(const Schedule& s, Units& un) {
+static void build_units(const Schedule& s, int cap, Units& un) {
   constexpr int kNone = 1 << 30;
   int64_t over_pf = 0, over_sx = 0;
-  build_units_capped(s, kNone, kNone, un, &over_pf, &over_sx);
+  build_units_capped(s, cap, kNone, kNone, un, &over_pf, &over_sx);
   const int64_t units = (int64_t)un.ptr.size() - s.n_dir;
   const int cap_pf = over_pf * 100 <= units ? kUnitPf : kNone;
   const int cap_sx = over_sx * 100 <= units ? kUnitSx : kNone;
-  if (cap_pf != kNone || cap_sx != kNone) build_units_capped(s, cap_pf, cap_sx, un, nullptr, nullptr);
+  if (cap_pf != kNone || cap_sx != kNone) build_units_capped(s, cap, cap_pf, cap_sx, un, nullptr, nullptr);
+}
+// What the layout of the staged units has to hold.
+struct UnitStats {
+  int emax = 0;       // most cut inflow faces in one unit
+  int unit_wo = 0;    // most wall entries
+  int unit_sx = 0;    // most elements with outputs
+  int unit_el = 0;    // most elements
+  int unit_out = 0;   // largest output block
+  int units = 0;      // most units of one direction
+  bool bad_wo = false;
+};
+
+static inline bool has_outputs(const Schedule& s, size_t it) {
+  return s.xk[it] >= 0 || s.wout[it] != 0 || s.contact[it] >= 0;
+}
+static inline int cut_faces(const Schedule& s, size_t it) {
+  int c = 0;
+  for (int f = 0; f < s.nf; ++f) c += (int)((uint32_t)s.in_idx[it * s.nf + f] >> ITEM_SHIFT) == ITEM_PERIODIC;
+  return c;
+}
+
+// Output block of a unit: nx periodic sources, nw wall / contact entries, nwo wall entries.
+static inline int out_bytes(int nx, int nw, int nwo, int real_bytes) {
+  return ((nx * 8 + 15) & ~15) + nw * 16 + nwo * 4 * real_bytes + ((nwo * 4 + 15) & ~15);
+}
+
+// Counts of every unit (cut faces, wall entries, periodic outputs, wall / contact outputs), in parallel over
+// directions: cnt[4 u + k] for unit u of all directions in order (unit_base[q] + unit of the direction).
+static UnitStats count_units(const Schedule& s, const Units& un, int real_bytes, std::vector<int64_t>& unit_base,
+                             std::vector<int32_t>& cnt) {
+  unit_base.assign(s.n_dir + 1, 0);
+  for (int q = 0; q < s.n_dir; ++q) unit_base[q + 1] = unit_base[q] + un.n[q];
+  cnt.assign((size_t)unit_base[s.n_dir] * 4, 0);
+  std::vector<UnitStats> per(s.n_dir);
+  parallel_tasks(s.n_dir, [&](int64_t q) {
+    const int32_t* up = un.ptr.data() + un.off[q];
+    UnitStats& st = per[q];
+    st.units = un.n[q];
+    int64_t wo = 0;
+    for (int u = 0; u < un.n[q]; ++u) {
+      int npf = 0, nwo = 0, nsx = 0, nx = 0, nw = 0;
+      for (int32_t pos = up[u]; pos < up[u + 1]; ++pos) {
+        const size_t it = (size_t)q * s.n + pos;
+        npf += cut_faces(s, it);
+        nwo += s.wout[it] & 7;
+        nsx += has_outputs(s, it) ? 1 : 0;
+        nx += s.xk[it] >= 0 ? 1 : 0;
+        nw += s.wout[it] != 0 || s.contact[it] >= 0 ? 1 : 0;
+      }
+      int32_t* c = cnt.data() + 4 * (size_t)(unit_base[q] + u);
+      c[0] = npf; c[1] = nwo; c[2] = nx; c[3] = nw;
+      st.unit_out = std::max(st.unit_out, out_bytes(nx, nw, nwo, real_bytes));
+      wo += nwo;
+      st.emax = std::max(st.emax, npf);
+      st.unit_wo = std::max(st.unit_wo, nwo);
+      st.unit_sx = std::max(st.unit_sx, nsx);
+      st.unit_el = std::max(st.unit_el, (int)(up[u + 1] - up[u]));
+    }
+    st.bad_wo = wo != s.wo_off[q + 1] - s.wo_off[q];
+  });
+  UnitStats t;
+  for (const UnitStats& p : per) {
+    t.emax = std::max(t.emax, p.emax);
+    t.unit_wo = std::max(t.unit_wo, p.unit_wo);
+    t.unit_sx = std::max(t.unit_sx, p.unit_sx);
+    t.unit_el = std::max(t.unit_el, p.unit_el);
+    t.unit_out = std::max(t.unit_out, p.unit_out);
+    t.units = std::max(t.units, p.units);
+    t.bad_wo = t.bad_wo || p.bad_wo;
+  }
+  return t;
+}
+
+// ---- shared memory of a CTA (bytes) --------------------------------------------------
+//   [0, 64) mbarriers | [64, 68) first unit that timed out | [96, ...) sigma [3][KV], K, S accumulators [KV]
+//   | [kRingOff, ...) ring | nbuf stages of (record block | values | gain rows) | nbuf + 1 output blocks
+// (a unit's outputs are written while the next unit runs, so its output block outlives its stage)
+static constexpr int kMaxBuf = 8;
+static constexpr int kFailOff = 64, kSigOff = 96, kRingOff = 384;
+static_assert(kSigOff + 5 * 32 <= kRingOff, "sigma and accumulators of 32-byte rows");
+static constexpr size_t kSmemPerSM = 233472, kSmemPerCta = 1024;   // capacity, reserved per CTA
+
+struct Layout {
+  int KV = 0;         // MFPs per thread and per CTA
+  int threads = 0;
+  int nbuf = 2;
+  int emax = 0;       // rows of one periodic bank
+  int prow0 = 0;      // first bank row
+  int rows = 0;       // ring rows
+  int blk = 0, val = 0, gain = 0;   // bytes of a stage's parts
+  int out = 0;                      // bytes of an output block
+  size_t smem = 0;
+  int stage() const { return blk + val + gain; }
+};
+
+template <typename Real>
+static Layout make_layout(const Schedule& s, const UnitStats& st, const Layout& shape, int nbuf) {
+  Layout l = shape;
+  const int row_bytes = l.KV * (int)sizeof(Real), al = row_bytes == 32 ? 7 : 0;   // swapped halves: runs of 8 rows
+  const int over = std::max(st.unit_el, kMaxThreads);   // every thread reads a record, its own or a stale one
+  l.nbuf = nbuf;
+  l.emax = (st.emax + al) & ~al;
+  l.prow0 = (s.max_slots + 2 + al) & ~al;
+  l.rows = l.prow0 + nbuf * l.emax;
+  l.blk = kHeader + over * rec_words(sizeof(Real), s.nf) * 4;
+  l.val = ((over + 2) * 2 * (int)sizeof(Real) + 15) & ~15;
+  l.gain = sizeof(Real) == 8 ? over * row_bytes : 0;
+  l.out = st.unit_out;
+  l.smem = (size_t)kRingOff + (size_t)l.rows * row_bytes + (size_t)nbuf * l.stage() + (size_t)(nbuf + 1) * l.out;
+  return l;
+}
+
+// CTAs that share an SM: by shared memory and by registers (launch bounds of the kernel).
+template <typename Real>
+static int resident(const Layout& l) {
+  const int by_regs = (sizeof(Real) == 4 && l.KV == 8 ? 5 : 4) * kMaxThreads / l.threads;
+  return (int)std::min<size_t>((size_t)std::min(by_regs, 32), kSmemPerSM / (l.smem + kSmemPerCta));
 }
 
 struct Packed {
-  RawVec<int32_t> rec, cellmap, spec;   // one entry per item, every one written by pass 2
+  Layout lay;
+  RawVec<int32_t> blk;                  // static blocks of all units, direction by direction
+  RawVec<int32_t> cellmap, spec;        // one entry per item
   RawVec<double> P;
   std::vector<int32_t> si;
   std::vector<double> sr;
-  // periodic inflow prefetch: the source indices read by unit u (one entry per cut inflow face, in
-  // element then face order), each unit's list padded with -1 to a multiple of 4 ints; kpf[u] is the
-  // absolute start of unit u's list (n[q] + 1 entries per direction, indexed like Units::ptr)
-  std::vector<int32_t> pf, kpf;
-  std::vector<int32_t> sx, ksx;  // output entries (4 ints each) in sweep order; first entry of unit u
-  int unit_sx = 0;               // most output entries in one unit
-  std::vector<int32_t> kwo;   // first wall re-emission entry of unit u, relative to the direction
-  int emax = 0;               // most cut inflow faces in one unit
-  int pf_pad = 0;             // longest padded list
-  int unit_wo = 0;            // most wall re-emission entries in one unit
-  int rows = 0;               // ring rows
+  // 8 ints per unit: elements | odd << 16, first position, first bank row, bank rows | output block's size << 16;
+  // record block and value offsets (16-byte units), their sizes (block | values << 16), periodic outputs | wall
+  // and contact outputs << 16
+  std::vector<int32_t> desc;
+  std::vector<int32_t> pfe;             // 4 ints per bank row: source slot | swapped halves << 30, its row among
+                                        // chunk 0's rows of all units, rows of its unit, 0
+  int64_t n_pf = 0;
 };
 
-static int ring_rows(const Schedule& s, int emax) { return s.max_slots + 2 + 2 * emax; }
-
-// Ring rows: [0, S) slots, S zero row, S+1 trash row, then two banks of emax rows that alternate
-// by unit parity: the cut inflow values of unit u live in bank u & 1, written during unit u - 1
-// (at CTA start for unit 0) from the state vector.
 template <typename Real>
-static obte_status pack(const Schedule& s, const Units& un, Packed& pk) {
+static obte_status pack(const Schedule& s, const Units& un, const std::vector<int64_t>& unit_base,
+                        const std::vector<int32_t>& cnt, const Layout& lay, Packed& pk) {
   const int W = rec_words(sizeof(Real), s.nf);
-  constexpr int CSTEP = sizeof(Real) / 4, COEF = 4;
-  const int S = s.max_slots;
-  const int zero_row = S, trash_row = S + 1, prow0 = S + 2;
-  // pass 1: per-unit counts of cut inflow faces, wall re-emission entries and output entries, in parallel
-  // over directions; per-unit starts are running sums within the direction (kwo) or over the directions
-  // in order (kpf, ksx), so the direction totals are summed in order between the two parallel steps
-  pk.emax = pk.pf_pad = pk.unit_wo = pk.unit_sx = 0;
-  pk.kwo.assign(un.ptr.size(), 0);
-  pk.kpf.assign(un.ptr.size(), 0);
-  pk.ksx.assign(un.ptr.size(), 0);
-  std::vector<int64_t> pf_tot(s.n_dir + 1, 0), sx_tot(s.n_dir + 1, 0);
-  std::vector<int> emax_q(s.n_dir, 0), pfpad_q(s.n_dir, 0), uwo_q(s.n_dir, 0), usx_q(s.n_dir, 0);
-  std::vector<char> wo_bad(s.n_dir, 0);
-  parallel_tasks(s.n_dir, [&](int64_t qq) {
-    const int q = (int)qq;
-    const int32_t* up = un.ptr.data() + un.off[q];
-    int32_t wo_run = 0;
-    int64_t pf_run = 0, sx_run = 0;
-    for (int u = 0; u < un.n[q]; ++u) {
-      int cnt = 0, wcnt = 0, scnt = 0;
-      for (int32_t pos = up[u]; pos < up[u + 1]; ++pos) {
-        const size_t it = (size_t)q * s.n + pos;
-        for (int f = 0; f < s.nf; ++f)
-          if ((int)((uint32_t)s.in_idx[it * s.nf + f] >> ITEM_SHIFT) == ITEM_PERIODIC) ++cnt;
-        wcnt += s.wout[it] & 7;
-        scnt += (s.xk[it] >= 0 || s.wout[it] != 0 || s.contact[it] >= 0) ? 1 : 0;
-      }
-      const int padded = (cnt + 3) & ~3;
-      pk.kwo[un.off[q] + u] = wo_run;
-      pk.kpf[un.off[q] + u] = (int32_t)pf_run;   // relative here, made absolute below
-      pk.ksx[un.off[q] + u] = (int32_t)sx_run;
-      sx_run += scnt;
-      usx_q[q] = std::max(usx_q[q], scnt);
-      wo_run += wcnt;
-      pf_run += padded;
-      emax_q[q] = std::max(emax_q[q], cnt);
-      pfpad_q[q] = std::max(pfpad_q[q], padded);
-      uwo_q[q] = std::max(uwo_q[q], wcnt);
-    }
-    pk.kwo[un.off[q] + un.n[q]] = wo_run;
-    pk.kpf[un.off[q] + un.n[q]] = (int32_t)pf_run;
-    pk.ksx[un.off[q] + un.n[q]] = (int32_t)sx_run;
-    pf_tot[q + 1] = pf_run;
-    sx_tot[q + 1] = sx_run;
-    wo_bad[q] = wo_run != s.wo_off[q + 1] - s.wo_off[q];
-  });
-  for (int q = 0; q < s.n_dir; ++q) {
-    if (wo_bad[q]) {
-      set_error("wall re-emission entries are not in sweep order");
-      return OBTE_ERR_BAD_ARG;
-    }
-    pf_tot[q + 1] += pf_tot[q];
-    sx_tot[q + 1] += sx_tot[q];
-    pk.emax = std::max(pk.emax, emax_q[q]);
-    pk.pf_pad = std::max(pk.pf_pad, pfpad_q[q]);
-    pk.unit_wo = std::max(pk.unit_wo, uwo_q[q]);
-    pk.unit_sx = std::max(pk.unit_sx, usx_q[q]);
-  }
-  const int64_t n_pf = pf_tot[s.n_dir], n_sx = sx_tot[s.n_dir];
-  if (n_pf >= (int64_t)1 << 31 || n_sx >= (int64_t)1 << 31) {
-    set_error("too many periodic inflow faces or output entries"); return OBTE_ERR_UNSUPPORTED;
-  }
-  parallel_tasks(s.n_dir, [&](int64_t q) {
-    for (int u = 0; u <= un.n[q]; ++u) {
-      pk.kpf[un.off[q] + u] += (int32_t)pf_tot[q];
-      pk.ksx[un.off[q] + u] += (int32_t)sx_tot[q];
-    }
-  });
-  pk.sx.assign((size_t)std::max<int64_t>(n_sx, 1) * 4, 0);
-  pk.rows = ring_rows(s, pk.emax);
-  if (pk.rows >= 65535 || s.max_src >= (1 << 30)) {
+  constexpr int CSTEP = sizeof(Real) / 4, COEF = 4, VB = 2 * sizeof(Real);
+  const int row_bytes = lay.KV * (int)sizeof(Real);
+  const int n_chunks = (s.n_mfp + lay.KV - 1) / lay.KV;
+  auto field = [&](int row) { return ring_field(row, row_bytes); };
+  const int zero_row = s.max_slots, trash_row = s.max_slots + 1;
+  pk.lay = lay;
+  if (field(lay.rows) >= 65535 || s.x_base[s.n_dir] >= ((int64_t)1 << 30)) {
     set_error("sweep ring rows do not fit 16-bit indices");
     return OBTE_ERR_UNSUPPORTED;
   }
-  pk.pf.assign((size_t)n_pf, -1);
-  const size_t total = (size_t)s.n_dir * s.n;
-  pk.rec.resize(total * W);     // uninitialised: pass 2 writes every word of every record
+  const int64_t n_units = unit_base[s.n_dir];
+  // offsets of every unit: block, bank rows
+  std::vector<int64_t> boff(n_units + 1, 0), poff(n_units + 1, 0);
+  {
+    int64_t u = 0;
+    for (int q = 0; q < s.n_dir; ++q) {
+      const int32_t* up = un.ptr.data() + un.off[q];
+      for (int k = 0; k < un.n[q]; ++k, ++u) {
+        const int32_t* c = cnt.data() + 4 * (size_t)u;
+        boff[u + 1] = boff[u] + (kHeader + (int64_t)(up[k + 1] - up[k]) * W * 4 + out_bytes(c[2], c[3], c[1], sizeof(Real))) / 16;
+        poff[u + 1] = poff[u] + c[0];
+      }
+    }
+  }
+  pk.n_pf = poff[n_units];
+  const int64_t total = (int64_t)s.n_dir * s.n;
+  if (boff[n_units] >= ((int64_t)1 << 32) || pk.n_pf * n_chunks >= ((int64_t)1 << 31) ||
+      total / (16 / VB) >= ((int64_t)1 << 32)) {
+    set_error("sweep tables too large");
+    return OBTE_ERR_UNSUPPORTED;
+  }
+  pk.blk.resize((size_t)boff[n_units] * 4);   // uninitialised: every word is written below
+  pk.desc.assign((size_t)std::max<int64_t>(n_units, 1) * 8, 0);
+  pk.pfe.assign((size_t)std::max<int64_t>(pk.n_pf, 1) * 4, 0);
   pk.cellmap.resize(total);
   pk.spec.resize(total);
   pk.P.resize(total);
-  pk.si.clear();
-  pk.sr.clear();
-  // pass 2: records, in parallel over directions.  Elements with outputs or wall inflow get a "special"
-  // entry (si/sr); a first sweep counts them per direction so every direction writes its own range.
+  // descriptors
+  parallel_tasks(s.n_dir, [&](int64_t q) {
+    const int32_t* up = un.ptr.data() + un.off[q];
+    for (int k = 0; k < un.n[q]; ++k) {
+      const int64_t u = unit_base[q] + k;
+      const int64_t v0 = ((int64_t)q * s.n + up[k]) * VB, v1 = ((int64_t)q * s.n + up[k + 1]) * VB;
+      const int odd = (int)((v0 & 15) / VB);
+      int32_t* d = pk.desc.data() + 8 * (size_t)u;
+      d[0] = (up[k + 1] - up[k]) | (odd << 16);
+      d[1] = up[k];
+      d[2] = (int32_t)poff[u];
+      const int32_t* c = cnt.data() + 4 * (size_t)u;
+      const int out16 = out_bytes(c[2], c[3], c[1], sizeof(Real)) / 16;
+      d[3] = (int32_t)(poff[u + 1] - poff[u]) | (out16 << 16);
+      d[4] = (int32_t)(uint32_t)boff[u];
+      d[5] = (int32_t)(uint32_t)(v0 >> 4);
+      d[6] = (int32_t)((uint32_t)(boff[u + 1] - boff[u] - out16) | ((uint32_t)(((v1 + 15) >> 4) - (v0 >> 4)) << 16));
+      d[7] = c[2] | (c[3] << 16);
+    }
+  });
+  // special entries (elements with outputs or wall inflow): counted per direction, then every direction fills
+  // its own range
   auto is_special = [&](size_t it) {
-    if (s.xk[it] >= 0 || s.wout[it] != 0 || s.contact[it] >= 0) return true;
+    if (has_outputs(s, it)) return true;
     for (int f = 0; f < s.nf; ++f)
       if ((int)((uint32_t)s.in_idx[it * s.nf + f] >> ITEM_SHIFT) == ITEM_WALL) return true;
     return false;
@@ -270,25 +367,56 @@ static obte_status pack(const Schedule& s, const Units& un, Packed& pk) {
     const int q = (int)qq;
     int64_t nsp = spec_base[q];
     const int32_t* up = un.ptr.data() + un.off[q];
+    int32_t wo_run = s.wo_off[q];          // first wall entry of the unit
     for (int u = 0; u < un.n[q]; ++u) {
-      int ent = 0, sent = 0;
-      const int bank = prow0 + (u & 1) * pk.emax;
-      int32_t* plist = pk.pf.data() + pk.kpf[un.off[q] + u];
-      int32_t* slist = pk.sx.data() + (size_t)pk.ksx[un.off[q] + u] * 4;
+      const int64_t gu = unit_base[q] + u;
+      const int n_el = up[u + 1] - up[u], npf = cnt[4 * gu], nwo = cnt[4 * gu + 1], nx = cnt[4 * gu + 2],
+                nw = cnt[4 * gu + 3];
+      int32_t* base = pk.blk.data() + (size_t)boff[gu] * 4;
+      int32_t* recs = base + kHeader / 4;
+      int32_t* xo = recs + (size_t)n_el * W;
+      int32_t* wo = xo + (((size_t)nx * 2 + 3) & ~(size_t)3);
+      int32_t* wg = wo + (size_t)nw * 4;
+      if (nx & 1) xo[2 * nx] = xo[2 * nx + 1] = 0;
+      // header: this unit, and the source addresses of the unit nbuf further
+      const int32_t* own = pk.desc.data() + 8 * (size_t)gu;
+      base[0] = own[0];
+      base[1] = own[1];
+      base[2] = nx | (nw << 16);
+      std::fill(base + 3, base + 8, 0);
+      if (u + lay.nbuf < un.n[q]) {
+        const int32_t* f = pk.desc.data() + 8 * (size_t)(gu + lay.nbuf);
+        base[3] = f[3];
+        base[4] = f[4];
+        base[5] = f[5];
+        base[6] = f[6];
+        base[7] = f[2];
+      }
+      for (int e = 0; e < nwo; ++e) {      // wall geometry
+        const int32_t w = s.wo_wall[wo_run + e];
+        Real g[4] = {0, 0, 0, 0};
+        for (int k = 0; k < s.dim; ++k) g[k] = (Real)s.w_db[(size_t)w * s.dim + k];
+        g[3] = s.gbm_sum[w] != 0 ? (Real)(1.0 / (-s.gbm_sum[w])) : Real(0);
+        std::memcpy(wg + (size_t)e * 4 * CSTEP, g, sizeof(g));
+        wg[(size_t)nwo * 4 * CSTEP + e] = w;
+      }
+      for (int e = nwo; e & 3; ++e) wg[(size_t)nwo * 4 * CSTEP + e] = 0;
+      int ent = 0, nwl = 0;
+      const int bank = lay.prow0 + (u % lay.nbuf) * lay.emax;
       for (int32_t pos = up[u]; pos < up[u + 1]; ++pos) {
         const size_t it = (size_t)q * s.n + pos;
-        int32_t* r = pk.rec.data() + it * W;
-        const int32_t so = s.slot[it] >= 0 ? s.slot[it] : trash_row;
+        int32_t* r = recs + (size_t)(pos - up[u]) * W;
+        const int so = s.slot[it] >= 0 ? s.slot[it] : trash_row;
         r[0] = s.cell[it];
         pk.cellmap[it] = s.cell[it];
         pk.P[it] = s.P[it];
         int32_t si[SI] = {s.xk[it], s.wout[it], s.contact[it], 0, 0, 0, 0, 0};
         double sr[SR] = {0, 0, 0, 0};
-        const bool outputs = s.xk[it] >= 0 || s.wout[it] != 0 || s.contact[it] >= 0;
+        const bool outputs = has_outputs(s, it);
         if (outputs && s.slot[it] < 0) { dir_err[q] = 1; return; }
         bool special = outputs;
         double coef[4] = {0, 0, 0, 0};
-        int32_t row_in[4] = {zero_row, zero_row, zero_row, zero_row};
+        int row_in[4] = {zero_row, zero_row, zero_row, zero_row};
         int k = 0;
         for (int f = 0; f < s.nf; ++f) {
           const int32_t code = s.in_idx[it * s.nf + f];
@@ -299,8 +427,11 @@ static obte_status pack(const Schedule& s, const Units& un, Packed& pk) {
             if (kind == ITEM_CELL) {
               row_in[k] = idx;
             } else {
-              plist[ent] = idx;
               row_in[k] = bank + ent;
+              int32_t* pe = pk.pfe.data() + 4 * (size_t)(poff[gu] + ent);
+              pe[0] = (int32_t)(s.x_base[q] + idx) | ((row_bytes == 32 ? ((bank + ent) >> 2) & 1 : 0) << 30);
+              pe[1] = (int32_t)(poff[gu] * n_chunks + ent);
+              pe[2] = npf;
               ++ent;
             }
             coef[k] = g;
@@ -313,19 +444,23 @@ static obte_status pack(const Schedule& s, const Units& un, Packed& pk) {
             special = true;
           }
         }
-        int sp = 0;
-        if (outputs) {
-          // wall re-emission entries: begin relative to the direction's first entry
-          int32_t* e = slist + (size_t)sent * 4;
-          e[0] = s.xk[it];
-          e[1] = s.wout[it] ? (((s.wout[it] >> 3) - s.wo_off[q]) << 3) | (s.wout[it] & 7) : 0;
-          e[2] = s.contact[it];
-          e[3] = 0;
-          sp = ++sent;
+        if (s.xk[it] >= 0) {
+          xo[0] = (int32_t)(s.x_base[q] + s.xk[it]);
+          xo[1] = field(so) << 4;
+          xo += 2;
         }
-        r[1] = (so & 0xFFFF) | (row_in[0] << 16);
-        r[2] = (row_in[1] & 0xFFFF) | (row_in[2] << 16);
-        r[3] = (row_in[3] & 0xFFFF) | (sp << 16);
+        r[3] = field(row_in[3]) | (s.xk[it] >= 0 ? (int)0x80000000 : 0);
+        if (s.wout[it] != 0 || s.contact[it] >= 0) {
+          if (s.contact[it] >= 0) r[3] |= (nwl + 1) << 16;
+          ++nwl;
+          wo[0] = field(so) << 4;
+          wo[1] = (s.wout[it] ? (((s.wout[it] >> 3) - wo_run) << 3) | (s.wout[it] & 7) : 0) | (nwo << 16);
+          wo[2] = s.contact[it];
+          wo[3] = s.wout[it] >> 3;
+          wo += 4;
+        }
+        r[1] = field(so) | (field(row_in[0]) << 16);
+        r[2] = field(row_in[1]) | (field(row_in[2]) << 16);
         if (special) {
           pk.spec[it] = (int32_t)nsp;
           std::copy(si, si + SI, pk.si.begin() + (size_t)nsp * SI);
@@ -342,6 +477,7 @@ static obte_status pack(const Schedule& s, const Units& un, Packed& pk) {
         std::memcpy(&r[COEF + s.nf * CSTEP], &dv, sizeof(Real));
         for (int wd = COEF + (s.nf + 1) * CSTEP; wd < W; ++wd) r[wd] = 0;   // padding to 16 bytes
       }
+      wo_run += nwo;
     }
   });
   for (int q = 0; q < s.n_dir; ++q) {
@@ -355,7 +491,6 @@ static obte_status pack(const Schedule& s, const Units& un, Packed& pk) {
     pk.si.assign(SI, 0);
     pk.sr.assign(SR, 0.0);
   }
-  if (pk.pf.empty()) pk.pf.assign(4, -1);
   return OBTE_OK;
 }
 
@@ -401,117 +536,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity
     if (mbar_try_wait(bar, parity)) return true;
   return false;
 }
-
-// ---- per-sweep values: b = DeltaT + h, p = P - sum_walls g_w T_B ------------------
-template <typename Real>
-__global__ void sweep_values_kernel(const int32_t* __restrict__ cellmap, const double* __restrict__ Pq,
-                                    const int32_t* __restrict__ spec, const int32_t* __restrict__ si,
-                                    const Real* __restrict__ sr, const double* __restrict__ u_in, int64_t n,
-                                    const double* __restrict__ hs, int with_src, int64_t total, Real* __restrict__ vals) {
-  const double* TB = u_in + n;
-  for (int64_t it = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; it < total; it += (int64_t)gridDim.x * blockDim.x) {
-    const int c = cellmap[it];
-    double b = u_in[c];
-    double pp = 0;
-    if (with_src) {
-      if (hs) b += hs[c];
-      pp = Pq[it];
-    }
-    const int sp = spec[it];
-    if (sp >= 0) {
-      const int32_t* s = si + (int64_t)sp * SI;
-      const Real* r = sr + (int64_t)sp * SR;
-      for (int k = 0; k < s[3]; ++k) pp -= (double)r[k] * TB[s[4 + k]];
-    }
-    vals[2 * it] = (Real)b;
-    vals[2 * it + 1] = (Real)pp;
-  }
-}
-
-template <typename Real>
-struct SweepParams {
-  int64_t n;
-  int64_t nd;
-  int n_mfp, n_dir, ds, m_pad;
-  int n_chunks;            // chunks of MCP MFPs per direction
-  int rows;                // ring rows
-  int S;                   // slot rows before the zero/trash/periodic rows
-  int emax;                // rows per periodic bank
-  int unit_wo, pf_pad;     // staging sizes: wall entries and prefetch-list ints per unit
-  int nbuf;                // TMA pipeline depth (units staged at once)
-  const int32_t* __restrict__ rec;
-  const Real* __restrict__ vals;
-  const int32_t* __restrict__ lev_ptr;   // unit boundaries (n[q] + 1 per direction)
-  const int64_t* __restrict__ lev_off;
-  const int32_t* __restrict__ nlev;      // units per direction
-  const int32_t* __restrict__ kwo;       // first wall entry of each unit (relative to the direction)
-  const int32_t* __restrict__ kpf;       // start of each unit's prefetch list in pf
-  const int32_t* __restrict__ pf;        // periodic source index per cut inflow face (-1 = padding)
-  const int32_t* __restrict__ ksx;       // first output entry of each unit (absolute)
-  const int32_t* __restrict__ sx;        // output entries: xk, wall entries, contact, 0
-  int unit_sx;                           // most output entries in one unit
-  const int64_t* __restrict__ x_base;
-  const int32_t* __restrict__ wo_off;   // [n_dir+1] first wall-output entry of each direction
-  const int32_t* __restrict__ wo_wall;
-  const Real* __restrict__ mfp;    // [m_pad]
-  const Real* __restrict__ tco;    // [n_dir * m_pad]
-  const Real* __restrict__ sig;    // [n_dir * m_pad * ds]
-  const Real* __restrict__ wo_geo; // [wall entry][4]: wall area vector / volume (x, y, z), 1 / (-sum_mq min(sigma.w, 0))
-  const Real* __restrict__ kcoef;  // [n_ce * m_pad]
-  const Real* __restrict__ scoef;  // [n_ce]
-  const double* __restrict__ u_in;
-  double* __restrict__ u_out;
-  double* __restrict__ Jraw;
-  double* __restrict__ K;
-  double* __restrict__ S_out;
-  int* __restrict__ err;
-  const double* __restrict__ rinv;   // FP64: 1 / (1 + mfp D) [n_dir][n_chunks][n][MC], or null: divide
-  float* __restrict__ Xs;   // final pass only: per-ordinate temperatures [n_dir][n][n_mfp], or null
-  int xs_add;               // 1: add this pass's temperatures to Xs (the pass at a correction d)
-  double* __restrict__ Xd;  // the same in FP64 (FP64 sweeps of obte_bte_sweep_fields), or null
-  const int32_t* __restrict__ cta_map;   // CTA -> direction * n_chunks + chunk (a subset), or null: all
-  // batched subset sweeps (batch_stride > 0): CTA b runs entry b % n_cta_batch of cta_map on the state
-  // vectors u_in / u_out + (b / n_cta_batch) batch_stride.  The batch shares one set of staged values
-  // (computed from the first state), so its states must agree on DeltaT and T_B.
-  int n_cta_batch;
-  int64_t batch_stride;
-  // bounded-wait test (obte_bte_plan_test_wait_timeout): level unit whose bulk copy is not issued (-1: none)
-  // and the poll cap of the wait for a unit's copy (kWaitPolls normally)
-  int skip_unit;
-  int wait_limit;
-  // deterministic reductions (det != 0, full sweeps only): each (direction, chunk) CTA stores its partial sums
-  // instead of adding them atomically; fixed-order reduction kernels sum them afterwards
-  int det;
-  Real* __restrict__ dpart;   // [n_dir n_chunks][n] lattice-temperature partial of each sweep position
-  Real* __restrict__ jpart;   // [n_dir n_chunks][n][ds] flux partials (final pass)
-  Real* __restrict__ wpart;   // [n_chunks][n_wo] wall-output partials (wall-output entries of all directions)
-  Real* __restrict__ kpart;   // [n_ce][m_pad] kcoef T of each contact entry (final pass)
-  Real* __restrict__ spart;   // [n_ce][m_pad] scoef T
-  int64_t n_wo;
-};
-
-template <typename Real>
-__device__ __forceinline__ Real word_real(const int32_t* r, int word);
-template <>
-__device__ __forceinline__ float word_real<float>(const int32_t* r, int word) {
-  return __int_as_float(r[word]);
-}
-template <>
-__device__ __forceinline__ double word_real<double>(const int32_t* r, int word) {
-  return __hiloint2double(r[word + 1], r[word]);
-}
-
-// num / den.  FP32: hardware reciprocal.  FP64: an FP32 reciprocal seed r (relative error e <= 2^-21)
-// and one residual correction of the quotient (Markstein's method), t = num r, q = t + (num - den t) r,
-// with relative error e^2 <= 2^-42 (~2e-13): three FP64 operations instead of the five of a fully
-// refined reciprocal, on GB300's narrow FP64 pipe, which bounds the FP64 sweep.
-__device__ __forceinline__ float quot(float num, float den) { return num * __fdividef(1.0f, den); }
-__device__ __forceinline__ double quot(double num, double den) {
-  const double r = (double)__fdividef(1.0f, (float)den);
-  const double t = num * r;
-  return fma(fma(-den, t, num), r, t);
-}
-
 // ---- double-float arithmetic (the output pass of the FP32+refine solve) ----------------------------
 // A value is an unevaluated pair hi + lo of FP32 numbers (~44 significant bits), computed on the FP32 pipe
 // with error-free transformations: Knuth's two-sum, the FMA two-product (Dekker 1971; Ogita, Rump and
@@ -570,42 +594,170 @@ __device__ __forceinline__ double dpack_value(double x) { return (double)dpack_h
 __device__ __forceinline__ df2 dunpack2(double a, double b) {   // two packed pairs -> lanes x, y
   return {make_float2(dpack_hi(a), dpack_hi(b)), make_float2(dpack_lo(a), dpack_lo(b))};
 }
+// float -> double, exactly, on the integer pipe for normal numbers (GB300's FP64 pipe converts two lanes a
+// clock per SM; zeros, denormals, infinities and NaN take the conversion instruction)
+__device__ __forceinline__ double widen(float f) {
+  const unsigned b = __float_as_uint(f), e = b & 0x7f800000u;
+  if (e == 0u || e == 0x7f800000u) return (double)f;
+  return __hiloint2double((int)(((b & 0x7fffffffu) >> 3) + (896u << 20) | (b & 0x80000000u)), (int)(b << 29));
+}
+__device__ __forceinline__ double widen(double f) { return f; }
 
-// Shared memory layout (bytes):
-//   [0,64) mbarriers  [64,128) unused
-//   [128, ...) nbuf x records | nbuf x values | nbuf x wall weights | nbuf x prefetch lists | sig | K S | ring
-// nbuf = TMA pipeline depth: unit u + nbuf - 1 is issued while unit u runs (at most kMaxBuf mbarriers)
-static constexpr int kMaxBuf = 8;
-// 2 units staged: measured 2.19 ms per FP32 sweep on the 60k-triangle benchmark against 2.46 ms with 3
-// (the smaller staging area lets 6 instead of 5 CTAs share an SM); deeper pipelines were no faster.
-static constexpr int kDefaultBuf = 2;
+// ---- per-sweep inputs -------------------------------------------------------------------
+// One launch: the (b, p) values of every item, b = DeltaT + h, p = P - sum_walls g_w T_B; the periodic inflow
+// rows of every unit (one warp per row and state: coalesced reads of the source's MFPs, written chunk by
+// chunk in the table's precision and row layout, so that a unit's rows are one bulk copy); and zeros for the
+// sums the sweep adds to.
+template <typename Real>
+struct PrepParams {
+  const int32_t* __restrict__ cellmap;
+  const double* __restrict__ Pq;
+  const int32_t* __restrict__ spec;
+  const int32_t* __restrict__ si;
+  const Real* __restrict__ sr;
+  const double* __restrict__ hs;      // heat source, or null
+  const double* __restrict__ u_in;
+  int64_t n, nd, total;
+  int with_src;
+  Real* __restrict__ vals;
+  const int32_t* __restrict__ pfe;
+  int64_t n_pf;
+  int n_mfp, m_row;                    // MFPs, MFPs rounded up to whole chunks
+  int batch;
+  int64_t batch_stride;                // states of a batched sweep (rows only: they agree on DeltaT and T_B)
+  int64_t row_stride;                  // reals between two states' rows
+  Real* __restrict__ xrow;
+  double *zero0, *zero1;               // sums to clear
+  int64_t nz0, nz1;
+  int row_blocks;                      // blocks that gather rows (the others: values and zeros)
+};
+
+template <typename Real, int MC, bool DF>
+__global__ void __launch_bounds__(256) sweep_prep_kernel(const __grid_constant__ PrepParams<Real> p) {
+  if ((int)blockIdx.x < p.row_blocks) {
+    constexpr bool kWide = MC * sizeof(Real) == 32;
+    constexpr int U = 4;                 // loads in flight per lane
+    const double* __restrict__ X = p.u_in + p.n + p.nd;
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = (int64_t)p.row_blocks * (blockDim.x >> 5);
+    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < p.n_pf * p.batch; w += nw) {
+      const int64_t t = p.batch > 1 ? w / p.n_pf : 0;
+      const int4 e = reinterpret_cast<const int4*>(p.pfe)[w - t * p.n_pf];
+      const double* src = X + t * p.batch_stride + (int64_t)(e.x & 0x3fffffff) * p.n_mfp;
+      Real* dst = p.xrow + t * p.row_stride + (int64_t)e.y * MC;
+      const int flip = kWide && (e.x >> 30) ? MC / 2 : 0;
+      for (int m0 = lane; m0 < p.m_row; m0 += 32 * U) {
+        double v[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) v[k] = m0 + 32 * k < p.n_mfp ? src[m0 + 32 * k] : 0.0;
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+          const int m = m0 + 32 * k;
+          Real r = (Real)v[k];
+          if constexpr (DF) r = dpack_split((double)r);
+          if (m < p.m_row) dst[(int64_t)(m / MC) * e.z * MC + ((m % MC) ^ flip)] = r;
+        }
+      }
+    }
+    return;
+  }
+  const int64_t t0 = (int64_t)(blockIdx.x - p.row_blocks) * blockDim.x + threadIdx.x;
+  const int64_t stride = (int64_t)(gridDim.x - p.row_blocks) * blockDim.x;
+  const double* __restrict__ TB = p.u_in + p.n;
+  for (int64_t it = t0; it < p.total; it += stride) {
+    const int c = p.cellmap[it];
+    double b = p.u_in[c];
+    double pp = 0;
+    if (p.with_src) {
+      if (p.hs) b += p.hs[c];
+      pp = p.Pq[it];
+    }
+    const int sp = p.spec[it];
+    if (sp >= 0) {
+      const int32_t* s = p.si + (int64_t)sp * SI;
+      const Real* r = p.sr + (int64_t)sp * SR;
+      for (int k = 0; k < s[3]; ++k) pp -= (double)r[k] * TB[s[4 + k]];
+    }
+    p.vals[2 * it] = (Real)b;
+    p.vals[2 * it + 1] = (Real)pp;
+  }
+  for (int64_t i = t0; i < p.nz0; i += stride) p.zero0[i] = 0.0;
+  for (int64_t i = t0; i < p.nz1; i += stride) p.zero1[i] = 0.0;
+}
 
 template <typename Real>
-struct SmemLayout {
-  size_t rec, val, gg, pfl, sxo, rec_stride, val_stride, gg_stride, pf_stride, sx_stride, sig, kacc, sacc, ring,
-      total;
-  __host__ __device__ SmemLayout(int nf, int mcp, int rows, int unit_wo, int pf_pad, int unit_sx, int nbuf) {
-    const int W = rec_words(sizeof(Real), nf);
-    size_t o = 128;
-    rec_stride = (size_t)kUnit * W * 4;
-    val_stride = (size_t)(kUnit + 2) * 2 * sizeof(Real);
-    val_stride = (val_stride + 15) & ~(size_t)15;
-    gg_stride = (size_t)unit_wo * 4 * sizeof(Real);        // 4 Reals per wall entry (16-B multiple)
-    pf_stride = (size_t)pf_pad * 4;                        // pf_pad is a multiple of 4
-    sx_stride = (size_t)unit_sx * 16;                      // output entries, int4 each
-    rec = o; o += nbuf * rec_stride;
-    val = o; o += nbuf * val_stride;
-    gg = o; o += nbuf * gg_stride;
-    pfl = o; o += nbuf * pf_stride;
-    sxo = o; o += nbuf * sx_stride;
-    sig = o; o += (size_t)mcp * 3 * sizeof(Real);
-    kacc = o; o += (size_t)mcp * sizeof(Real);
-    sacc = o; o += (size_t)mcp * sizeof(Real);
-    o = (o + 15) & ~(size_t)15;
-    ring = o; o += (size_t)mcp * rows * sizeof(Real);
-    total = o;
-  }
+struct SweepParams {
+  int64_t n;
+  int64_t nd;
+  int n_mfp, n_dir, ds, m_pad;
+  int n_chunks;            // chunks of KV MFPs per direction
+  int zero_row, prow0;     // ring rows: zero row, first periodic bank row
+  int emax;                // rows per periodic bank
+  int nbuf;                // units staged at once
+  int stage0, stage, val_off, gain_off;   // first stage, bytes of a stage, its values and gain rows
+  int out0, out;           // first output block, bytes of one
+  const int32_t* __restrict__ blk;        // static blocks
+  const int32_t* __restrict__ desc;       // unit descriptors (8 ints), directions in order
+  const int64_t* __restrict__ unit_base;  // [n_dir + 1]
+  const Real* __restrict__ vals;
+  const Real* __restrict__ xrow;          // periodic inflow rows: [unit][chunk][row][KV]
+  const int64_t* __restrict__ x_base;
+  const Real* __restrict__ mfp;    // [m_pad]
+  const Real* __restrict__ tco;    // [n_dir * m_pad]
+  const Real* __restrict__ sig;    // [n_dir * m_pad * ds]
+  const Real* __restrict__ kcoef;  // [n_ce * m_pad]
+  const Real* __restrict__ scoef;  // [n_ce]
+  double* __restrict__ u_out;
+  double* __restrict__ Jraw;
+  double* __restrict__ K;
+  double* __restrict__ S_out;
+  int* __restrict__ err;
+  const double* __restrict__ gain;   // FP64: mfp / (1 + mfp D) [n_dir][n_chunks][n][KV], or null: divide
+  float* __restrict__ Xs;   // final pass only: per-ordinate temperatures [n_dir][n][n_mfp], or null
+  int xs_add;               // 1: add this pass's temperatures to Xs (the pass at a correction d)
+  double* __restrict__ Xd;  // the same in FP64 (FP64 sweeps of obte_bte_sweep_fields), or null
+  const int32_t* __restrict__ cta_map;   // CTA -> direction * n_chunks + chunk (a subset or launch order), or null
+  // batched subset sweeps (n_cta_batch > 0): CTA b runs entry b % n_cta_batch of cta_map on the state vector
+  // u_out + (b / n_cta_batch) batch_stride and the inflow rows xrow + (b / n_cta_batch) row_stride.  The batch
+  // shares one set of values (from the first state), so its states must agree on DeltaT and T_B.
+  int n_cta_batch;
+  int64_t batch_stride, row_stride;
+  // bounded-wait test (obte_bte_plan_test_wait_timeout): unit whose bulk copies are not issued (-1: none) and
+  // the poll cap of the wait for a unit's copies (kWaitPolls normally)
+  int skip_unit;
+  int wait_limit;
+  // deterministic reductions (det != 0, full sweeps only): each (direction, chunk) CTA stores its partial sums
+  // instead of adding them atomically; fixed-order reduction kernels sum them afterwards
+  int det;
+  Real* __restrict__ dpart;   // [n_dir n_chunks][n] lattice-temperature partial of each sweep position
+  Real* __restrict__ jpart;   // [n_dir n_chunks][n][ds] flux partials (final pass)
+  Real* __restrict__ wpart;   // [n_chunks][n_wo] wall-output partials (wall-output entries of all directions)
+  Real* __restrict__ kpart;   // [n_ce][m_pad] kcoef T of each contact entry (final pass)
+  Real* __restrict__ spart;   // [n_ce][m_pad] scoef T
+  int64_t n_wo;
 };
+
+template <typename Real>
+__device__ __forceinline__ Real word_real(const int32_t* r, int word);
+template <>
+__device__ __forceinline__ float word_real<float>(const int32_t* r, int word) {
+  return __int_as_float(r[word]);
+}
+template <>
+__device__ __forceinline__ double word_real<double>(const int32_t* r, int word) {
+  return __hiloint2double(r[word + 1], r[word]);
+}
+
+// num / den.  FP32: hardware reciprocal.  FP64: an FP32 reciprocal seed r (relative error e <= 2^-21)
+// and one residual correction of the quotient (Markstein's method), t = num r, q = t + (num - den t) r,
+// with relative error e^2 <= 2^-42 (~2e-13): three FP64 operations instead of the five of a fully
+// refined reciprocal, on GB300's narrow FP64 pipe, which bounds the FP64 sweep.
+__device__ __forceinline__ float quot(float num, float den) { return num * __fdividef(1.0f, den); }
+__device__ __forceinline__ double quot(double num, double den) {
+  const double r = (double)__fdividef(1.0f, (float)den);
+  const double t = num * r;
+  return fma(fma(-den, t, num), r, t);
+}
 
 // 16-byte vectors of the ring: 4 floats or 2 doubles per lane.
 template <typename Real> struct V16;
@@ -653,108 +805,141 @@ __device__ __forceinline__ void vstore(double* p, const double (&x)[K]) {
   for (int i = 0; i < K; i += 2) *reinterpret_cast<double2*>(p + i) = make_double2(x[i], x[i + 1]);
 }
 
-// Sum over the G lanes of an element group (aligned groups of G lanes inside a warp).
-template <int G, typename T>
-__device__ __forceinline__ T group_sum(T v, unsigned mask) {
+// Lane `lane`'s KV of a ring row's MC MFPs, by the row's byte offset: a 16-byte row, or a 32-byte row of which
+// bit 4 of the offset says which half comes first (the lane's offset in the row is added without carry).
+template <int MC, int KV, typename Real>
+__device__ __forceinline__ void row_load(const unsigned char* ring, unsigned off, int lane, Real (&x)[KV]) {
+  constexpr int H = 16 / (int)sizeof(Real);
+  static_assert(MC == H || MC == 2 * H, "one or two 16-byte vectors per row");
+  const unsigned o = MC == KV ? off : off ^ (unsigned)(lane * KV * (int)sizeof(Real));
+  if constexpr (KV <= H) {
+    vload(reinterpret_cast<const Real*>(ring + o), x);
+  } else {
+    Real a[H];
+    vload(reinterpret_cast<const Real*>(ring + o), a);
 #pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
-  return v;
+    for (int i = 0; i < H; ++i) x[i] = a[i];
+    vload(reinterpret_cast<const Real*>(ring + (o ^ 16u)), a);
+#pragma unroll
+    for (int i = 0; i < H; ++i) x[H + i] = a[i];
+  }
+}
+template <int MC, int KV, typename Real>
+__device__ __forceinline__ void row_store(unsigned char* ring, unsigned off, int lane, const Real (&x)[KV]) {
+  constexpr int H = 16 / (int)sizeof(Real);
+  const unsigned o = MC == KV ? off : off ^ (unsigned)(lane * KV * (int)sizeof(Real));
+  if constexpr (KV <= H) {
+    vstore(reinterpret_cast<Real*>(ring + o), x);
+  } else {
+    Real a[H];
+#pragma unroll
+    for (int i = 0; i < H; ++i) a[i] = x[i];
+    vstore(reinterpret_cast<Real*>(ring + o), a);
+#pragma unroll
+    for (int i = 0; i < H; ++i) a[i] = x[H + i];
+    vstore(reinterpret_cast<Real*>(ring + (o ^ 16u)), a);
+  }
 }
 
-// One CTA = direction q x a chunk of MC = G * KV mean free paths, 128 G threads (KV a multiple of the
-// 16-byte vector: 4 or 8 FP32, 2 or 4 FP64).  Every element of
-// a unit is owned by a group of G consecutive threads; lane l of the group computes the KV MFPs
-// [l KV, (l+1) KV) of the chunk.  The ring is [row][MC] (MFP fastest), so an upstream read is one
-// 16-byte shared load per lane and a group of 8 reads one full 128-byte row.
-// Resident CTAs per SM the register allocation is bounded for: 8 FP32 MFPs per lane would otherwise take
-// ~125 registers and hold an SM to 4 CTAs (a third wave of 32 CTAs on the 60k-triangle cell, 1,248 CTAs
-// over 608 slots); at 5 the 1,248 CTAs fit in two waves.  (Capping 4 FP32 MFPs per lane at 64 registers
-// made the 110k-tetrahedron sweep, held to 3 CTAs per SM by shared memory, 5 % slower.)
-template <typename Real, int G, int KV>
-struct SweepMinBlocks { static constexpr int v = (sizeof(Real) == 4 && G == 1 && KV == 8) ? 5 : 1; };
+// 1 / x for a normal x (the sweep's denominators are 1 + L D >= 1)
+__device__ __forceinline__ float rcp(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 
-// The thread that issues the bulk copies: lane 0 of the last warp.  Its elements are the last of a unit,
-// which most units do not have (median 88 of 128 elements on the 60k-triangle cell), so the issue work stays
-// off the warps that every unit keeps busy.
-template <int G>
-struct Issuer { static constexpr int tid = kUnit * G - 32; };
+// Wall re-emission of entry i of a unit's nw (wb: the entries, the wall geometry after them).
+// Re-emission weight max(sigma . w, 0) / (-sum min(sigma . w, 0)) from the staged wall geometry (bte.py:73-78),
+// wall by wall; the sum runs over the MFPs in order.
+template <typename Real, int MC, bool DF>
+__device__ __forceinline__ void wall_outputs(const SweepParams<Real>& p, const unsigned char* wb, int nw, int i,
+                                             const unsigned char* ring, const Real* s_sig, double* dT_out, int chunk) {
+  const int4 ent = reinterpret_cast<const int4*>(wb)[i];
+  Real T[MC];
+  row_load<MC, MC>(ring, (unsigned)ent.x, 0, T);
+  if constexpr (DF) {
+#pragma unroll
+    for (int j = 0; j < MC; ++j) T[j] = dpack_value(T[j]);
+  }
+  auto sigv = [&](Real x) -> Real {
+    if constexpr (DF) return dpack_value(x);
+    else return x;
+  };
+  const int wn = ent.y & 7;
+  const int first = (ent.y >> 3) & 0x1FFF;
+  const Real* gw = reinterpret_cast<const Real*>(wb + nw * 16);
+  const int* wall = reinterpret_cast<const int*>(gw + 4 * (int)((unsigned)ent.y >> 16)) + first;
+  gw += 4 * first;
+  for (int k = 0; k < wn; ++k, gw += 4) {
+    const Real g0 = gw[0], g1 = gw[1], g2 = gw[2], g3 = gw[3];
+    Real w = 0;
+#pragma unroll
+    for (int j = 0; j < MC; ++j) {
+      const Real a = sigv(s_sig[j]) * g0 + sigv(s_sig[MC + j]) * g1 + sigv(s_sig[2 * MC + j]) * g2;
+      w += (a > Real(0) ? a * g3 : Real(0)) * T[j];
+    }
+    if (p.det) p.wpart[(int64_t)chunk * p.n_wo + ent.w + k] = w;
+    else atomicAdd(&dT_out[p.n + wall[k]], widen(w));
+  }
+}
+
+// Resident CTAs per SM the register allocation is bounded for.
+template <typename Real, int KV>
+struct SweepMinBlocks { static constexpr int v = (sizeof(Real) == 4 && KV == 8) ? 5 : 4; };
 
 // DF (Real = double, FINAL only): the FP64 tables swept in double-float arithmetic (see df2).
-template <typename Real, int NF, int G, int KV, bool FINAL, bool DF = false>
-__global__ void __launch_bounds__(kUnit * G, SweepMinBlocks<Real, G, KV>::v) bte_sweep_kernel(const SweepParams<Real> p) {
+template <typename Real, int NF, int KV, bool FINAL, bool DF = false>
+__global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
+    bte_sweep_kernel(const __grid_constant__ SweepParams<Real> p) {
   static_assert(!DF || (sizeof(Real) == 8 && FINAL && KV % 2 == 0), "double-float sweeps: FP64 tables, output pass");
-  constexpr int RW = Rec<Real, NF>::W;           // record words
-  constexpr int MC = G * KV;                     // MFPs per CTA
-  constexpr int VB = 2 * sizeof(Real);           // bytes of one (b, p) pair
+  constexpr int MC = KV;
+  using RR = Rec<Real, NF>;
+  constexpr int RW = RR::W;                        // record words
+  constexpr int RB = RW * 4, ROWB = MC * (int)sizeof(Real), VB = 2 * (int)sizeof(Real);
+  constexpr bool kGain = sizeof(Real) == 8 && !DF;
   extern __shared__ __align__(128) unsigned char smem[];
-  const int rows = p.rows;
-  const int nbuf = p.nbuf;
-  const SmemLayout<Real> L(NF, MC, rows, p.unit_wo, p.pf_pad, p.unit_sx, nbuf);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
-  Real* s_k = reinterpret_cast<Real*>(smem + L.kacc);
-  Real* s_s = reinterpret_cast<Real*>(smem + L.sacc);
-  Real* ring = reinterpret_cast<Real*>(smem + L.ring);    // [rows][MC]
+  int* s_fail = reinterpret_cast<int*>(smem + kFailOff);
+  Real* s_sig = reinterpret_cast<Real*>(smem + kSigOff);    // [3][MC]
+  Real* s_k = s_sig + 3 * MC;
+  Real* s_s = s_k + MC;
+  unsigned char* ring = smem + kRingOff;
 
   int bid = (int)blockIdx.x;
-  int64_t boff = 0;
-  if (p.batch_stride > 0) {
-    const int bt = bid / p.n_cta_batch;
+  int bt = 0;
+  if (p.n_cta_batch > 0) {
+    bt = bid / p.n_cta_batch;
     bid -= bt * p.n_cta_batch;
-    boff = (int64_t)bt * p.batch_stride;
   }
   const int cta = p.cta_map ? p.cta_map[bid] : bid;
   const int q = cta / p.n_chunks;
   const int chunk = cta - q * p.n_chunks;
   const int m0 = chunk * MC;
   const int mc = min(MC, p.n_mfp - m0);
-  const int tid = threadIdx.x;
-  const int el = tid / G;                        // element of the unit owned by this group
-  const int lane = tid - el * G;
-  const int mo = lane * KV;                      // first MFP of this lane (within the chunk)
-  const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << ((tid & 31) & ~(G - 1)));
-  const int32_t* __restrict__ lev = p.lev_ptr + p.lev_off[q];
-  const int32_t* __restrict__ kwo = p.kwo + p.lev_off[q];
-  const int32_t* __restrict__ kpf = p.kpf + p.lev_off[q];
-  const int32_t* __restrict__ ksx = p.ksx + p.lev_off[q];
-  const int nlev = p.nlev[q];
-  const int32_t* __restrict__ rec_q = p.rec + (int64_t)q * p.n * RW;
-  // values: absolute byte offsets from the (256-B aligned) array base keep every TMA window 16-B aligned
-  const unsigned char* __restrict__ val_base = reinterpret_cast<const unsigned char*>(p.vals);
-  const int64_t val_q0 = (int64_t)q * p.n * VB;
-  const int64_t xq = p.x_base[q];
-  const int wo0 = p.wo_off[q];
-  const int nwo = p.wo_off[q + 1] - wo0;
-  // wall weights of this (direction, chunk): [entry][MC], entries in sweep order
-  const Real* __restrict__ gg_q = p.wo_geo + (int64_t)wo0 * 4;
-  const int prow0 = p.S + 2;
-  const double* __restrict__ X = p.u_in + boff + p.n + p.nd;
-  double* __restrict__ dT_out = p.u_out + boff;
-  double* __restrict__ TB_out = p.u_out + boff + p.n;
-  double* __restrict__ X_out = p.u_out + boff + p.n + p.nd;
+  const int tid = threadIdx.x, nthr = blockDim.x;
+  const int nbuf = p.nbuf;
+  const int64_t ub = p.unit_base[q];
+  const int nlev = (int)(p.unit_base[q + 1] - ub);
+  double* __restrict__ dT_out = p.u_out + bt * p.batch_stride;
+  const double* __restrict__ gain_qc =
+      kGain && p.gain ? p.gain + ((int64_t)q * p.n_chunks + chunk) * p.n * MC : nullptr;
 
-  // this lane's ordinate data in registers; padded MFPs get L = t = sigma = 0 (harmless T = b).
-  // sigma (wall re-emission and the final pass only) is read from shared memory: [MC][3]
+  // this chunk's ordinate data in registers; padded MFPs get L = t = sigma = 0 (harmless T = b).
+  // sigma (wall re-emission and the final pass only) is read from shared memory
   Real lam[KV], tt[KV];
 #pragma unroll
   for (int j = 0; j < KV; ++j) {
-    const bool ok = mo + j < mc;
-    const int64_t m = m0 + mo + j;
-    lam[j] = ok ? p.mfp[m] : Real(0);
-    tt[j] = ok ? p.tco[(int64_t)q * p.m_pad + m] : Real(0);
+    const bool ok = j < mc;
+    lam[j] = ok ? p.mfp[m0 + j] : Real(0);
+    tt[j] = ok ? p.tco[(int64_t)q * p.m_pad + m0 + j] : Real(0);
   }
-  Real* s_sig = reinterpret_cast<Real*>(smem + L.sig);
-  for (int i = tid; i < MC * 3; i += blockDim.x) {
-    const int jj = i / 3, d = i - 3 * jj;
-    const Real sv = (jj < mc && d < p.ds) ? p.sig[((int64_t)q * p.m_pad + m0 + jj) * p.ds + d] : Real(0);
+  for (int i = tid; i < MC * 3; i += nthr) {
+    const int d = i / MC, j = i - d * MC;
+    const Real sv = (j < mc && d < p.ds) ? p.sig[((int64_t)q * p.m_pad + m0 + j) * p.ds + d] : Real(0);
     if constexpr (DF) s_sig[i] = dpack_split(sv);   // packed hi / lo pairs
     else s_sig[i] = sv;
   }
-  // real value of a shared sigma entry (DF keeps them as packed pairs)
-  auto sigv = [&](Real x) -> Real {
-    if constexpr (DF) return dpack_value(x);
-    else return x;
-  };
-  // DF: this lane's MFPs and weights as pairs (lanes x, y = MFPs j, j + 1)
+  // DF: the MFPs and weights as pairs (lanes x, y = MFPs j, j + 1)
   df2 lam2[DF ? KV / 2 : 1], tt2[DF ? KV / 2 : 1];
   if constexpr (DF) {
 #pragma unroll
@@ -764,346 +949,342 @@ __global__ void __launch_bounds__(kUnit * G, SweepMinBlocks<Real, G, KV>::v) bte
       tt2[j / 2] = {make_float2(t0.x, t1.x), make_float2(t0.y, t1.y)};
     }
   }
-  if (FINAL)
-    for (int j = tid; j < MC; j += blockDim.x) { s_k[j] = 0; s_s[j] = 0; }
-  // ring: zero everything, then bank 0 holds the cut inflow values of unit 0
-  const int npf0 = nlev > 0 ? kpf[1] - kpf[0] : 0;
-  for (int i = tid; i < MC * rows; i += blockDim.x) {
-    const int row = i / MC, col = i - row * MC;
-    Real v = 0;
-    const int j = row - prow0;
-    if (j >= 0 && j < npf0 && col < mc) {
-      const int k = p.pf[kpf[0] + j];
-      if (k >= 0) v = (Real)X[(xq + k) * p.n_mfp + m0 + col];
-    }
-    if constexpr (DF) ring[i] = dpack_split(v);
-    else ring[i] = v;
+  for (int j = tid; j < MC; j += nthr) {
+    reinterpret_cast<Real*>(ring + (size_t)p.zero_row * ROWB)[j] = Real(0);
+    if (FINAL) { s_k[j] = 0; s_s[j] = 0; }
   }
   if (tid == 0) {
     for (int i = 0; i < nbuf; ++i) mbar_init(&bars[i], 1);
+    *s_fail = INT_MAX;
     fence_mbar_init();
   }
   __syncthreads();
 
-  // TMA of unit u into buffer bi: records [a, e), values [a, e) (16-B aligned window), the
-  // wall weights of the unit's wall entries and the prefetch list of unit u + 1
-  auto issue = [&](int u, int bi) {
-    if (u == p.skip_unit) return;   // test of the bounded wait: this unit's copy never arrives
-    const int a = lev[u], e = lev[u + 1];
-    const unsigned rbytes = (unsigned)(e - a) * RW * 4u;
-    const int64_t vb0 = (val_q0 + (int64_t)a * VB) & ~(int64_t)15;
-    const int64_t vb1 = (val_q0 + (int64_t)e * VB + 15) & ~(int64_t)15;
-    const unsigned vbytes = (unsigned)(vb1 - vb0);
-    const int w0 = kwo[u], w1 = kwo[u + 1];
-    const unsigned gbytes = (unsigned)(w1 - w0) * 4u * (unsigned)sizeof(Real);
-    const int f0 = u + 1 < nlev ? kpf[u + 1] : 0, f1 = u + 1 < nlev ? kpf[u + 2] : 0;
-    const unsigned pbytes = (unsigned)(f1 - f0) * 4u;
-    const int x0 = ksx[u], x1 = ksx[u + 1];
-    const unsigned sbytes = (unsigned)(x1 - x0) * 16u;
+  // Bulk copies of a unit into stage bi and output block oi: records, values, outputs, periodic inflow rows, gain
+  // rows.  blk16, val16 = record and value sources, size = their sizes in 16-byte units, prow = first bank row,
+  // np = bank rows | size of the output block << 16
+  auto issue = [&](int u, int bi, int oi, unsigned blk16, unsigned val16, unsigned size, int prow, unsigned np) {
+    if (u == p.skip_unit) return;   // test of the bounded wait: this unit's copies never arrive
+    const unsigned bb = (size & 0xFFFFu) << 4, vb = (size >> 16) << 4, ob = (np >> 16) << 4, npf = np & 0xFFFFu;
+    unsigned char* st = smem + p.stage0 + bi * p.stage;
+    const unsigned char* src = reinterpret_cast<const unsigned char*>(p.blk) + ((uint64_t)blk16 << 4);
     uint64_t* bar = &bars[bi];
+    unsigned gb = 0;
+    if constexpr (kGain) gb = gain_qc ? (vb / VB) * ROWB : 0u;     // FP64 values are 16 bytes: vb / 16 elements
     fence_proxy_async();
-    mbar_expect_tx(bar, rbytes + vbytes + gbytes + pbytes + sbytes);
-    tma_load_1d(smem + L.rec + bi * L.rec_stride, rec_q + (int64_t)a * RW, rbytes, bar);
-    tma_load_1d(smem + L.val + bi * L.val_stride, val_base + vb0, vbytes, bar);
-    if (gbytes) tma_load_1d(smem + L.gg + bi * L.gg_stride, gg_q + (int64_t)w0 * 4, gbytes, bar);
-    if (pbytes) tma_load_1d(smem + L.pfl + bi * L.pf_stride, p.pf + f0, pbytes, bar);
-    if (sbytes) tma_load_1d(smem + L.sxo + bi * L.sx_stride, p.sx + (int64_t)x0 * 4, sbytes, bar);
+    mbar_expect_tx(bar, bb + vb + ob + gb + npf * ROWB);
+    tma_load_1d(st, src, bb, bar);
+    tma_load_1d(st + p.val_off, reinterpret_cast<const unsigned char*>(p.vals) + ((uint64_t)val16 << 4), vb, bar);
+    if (ob) tma_load_1d(smem + p.out0 + oi * p.out, src + bb, ob, bar);
+    if (npf)
+      tma_load_1d(ring + (size_t)(p.prow0 + bi * p.emax) * ROWB,
+                  p.xrow + bt * p.row_stride + ((int64_t)prow * p.n_chunks + (int64_t)chunk * npf) * MC, npf * ROWB, bar);
+    if constexpr (kGain)
+      if (gb) tma_load_1d(st + p.gain_off, gain_qc + ((int64_t)val16 - (int64_t)q * p.n) * MC, gb, bar);
   };
-  constexpr int kIssuer = Issuer<G>::tid;
-  if (tid == kIssuer)
-    for (int u = 0; u < nbuf - 1 && u < nlev; ++u) issue(u, u);
+  // the issuing thread: lane 0 of the last warp, whose elements are the last of a unit
+  const int issuer = nthr - 32;
+  if (tid == issuer)
+    for (int u = 0; u < nbuf && u < nlev; ++u) {
+      const int4* d = reinterpret_cast<const int4*>(p.desc) + 2 * (ub + u);
+      const int4 a = __ldg(d), b = __ldg(d + 1);
+      issue(u, u, u, (unsigned)b.x, (unsigned)b.y, (unsigned)b.z, a.z, (unsigned)a.w);
+    }
 
-  // per-unit metadata, loaded one unit ahead so that its latency stays off the unit's critical path
-  int a = nlev > 0 ? lev[0] : 0, e = nlev > 0 ? lev[1] : 0;
-  int wu = kwo[0];
-  int kpf1 = nlev > 1 ? kpf[1] : 0, kpf2 = nlev > 1 ? kpf[2] : 0;
-  // the value window of a unit starts (q n + a) pairs into the array; FP32 pairs are 8 bytes, so the
-  // 16-byte aligned window starts one pair early when q n + a is odd (FP64 pairs are 16 bytes: never)
-  const int qn_odd = (int)(((int64_t)q * p.n) & 1);
-  // FP64 with the reciprocal table: this element's 1 / (1 + mfp D) for the current unit, and for the next
-  // unit loaded one unit ahead (a coalesced 16-byte global load per lane, off the unit's critical path)
-  constexpr bool kRinv = sizeof(Real) == 8 && !DF;
-  double rcur[KV], rnxt[KV];
-  const double* __restrict__ rinv_qc =
-      (kRinv && p.rinv) ? p.rinv + ((int64_t)q * p.n_chunks + chunk) * p.n * MC : nullptr;
-  if (rinv_qc && nlev > 0 && el < e - a) vload(rinv_qc + (int64_t)(a + el) * MC + mo, rcur);
-  int bi = 0;            // buffer of unit u (u mod nbuf)
-  unsigned phase = 0;    // parity of its mbarrier phase ((u / nbuf) & 1)
-  for (int u = 0; u < nlev; ++u) {
-    const int e_next = u + 2 <= nlev ? lev[u + 2] : 0;
-    const int wu_next = kwo[u + 1];
-    const int kpf3 = u + 3 <= nlev ? kpf[u + 3] : 0;
-    const int npf = u + 1 < nlev ? kpf2 - kpf1 : 0;   // padded length of unit u+1's list
-    const int prow_next = prow0 + ((u + 1) & 1) * p.emax;
-    if (rinv_qc && u + 1 < nlev && el < e_next - e) vload(rinv_qc + (int64_t)(e + el) * MC + mo, rnxt);
-    // buffer (u + nbuf - 1) mod nbuf was last read during unit u - 1, finished at the barrier below
-    if (tid == kIssuer && u + nbuf - 1 < nlev) issue(u + nbuf - 1, bi == 0 ? nbuf - 1 : bi - 1);
-    const bool ready = mbar_wait_bounded(&bars[bi], phase, p.wait_limit);
-    // the periodic prefetch runs on the high thread indices (list entry i on element kUnit - 1 - i), which
-    // most units leave without an element
-    const int pf_i = kUnit - 1 - el;
-    if (!ready) {
-      atomicOr(p.err, 1);
+  // record, value pair and gains of one element of a staged unit
+  int32_t r[RW];
+  Real bv, pw;
+  Real gn[kGain ? KV : 1];
+  auto fetch = [&](const unsigned char* st, int odd, int el) {
+    const int4* r4 = reinterpret_cast<const int4*>(st + kHeader + el * RB);
+#pragma unroll
+    for (int i = 0; i < RW / 4; ++i) {
+      const int4 x = r4[i];
+      r[4 * i] = x.x; r[4 * i + 1] = x.y; r[4 * i + 2] = x.z; r[4 * i + 3] = x.w;
+    }
+    const Real* v = reinterpret_cast<const Real*>(st + p.val_off) + 2 * (odd + el);
+    if constexpr (sizeof(Real) == 4) {
+      const float2 x = *reinterpret_cast<const float2*>(v);
+      bv = x.x; pw = x.y;
     } else {
-      // cut inflow values of unit u+1: loads issued now, stored into bank (u+1)&1 after the MFP loop
-      const int32_t* s_pf = reinterpret_cast<const int32_t*>(smem + L.pfl + bi * L.pf_stride);
-      const int pk = pf_i < npf ? s_pf[pf_i] : -1;
-      double xv[KV];
-      if (pk >= 0) {
-        const double* xs = X + (xq + pk) * p.n_mfp + m0 + mo;
-#pragma unroll
-        for (int j = 0; j < KV; ++j) xv[j] = mo + j < mc ? __ldg(xs + j) : 0.0;
+      const double2 x = *reinterpret_cast<const double2*>(v);
+      bv = x.x; pw = x.y;
+    }
+    if constexpr (kGain)
+      if (gain_qc) vload(reinterpret_cast<const double*>(st + p.gain_off) + el * KV, gn);
+  };
+
+  int bi = 0;            // stage of unit u (u mod nbuf)
+  int oi = 0;            // output block of unit u - 1 (mod nbuf + 1)
+  unsigned phase = 0;    // parity of its mbarrier phase ((u / nbuf) & 1)
+  const unsigned char* st = smem + p.stage0;
+  int4 hd = make_int4(0, 0, 0, 0);
+  // Per-MFP outputs of a finished unit, from its rows in the ring: one lane per (periodic source, MFP) from the
+  // last thread down, one lane per wall element from the warp before (the high threads have no
+  // element in most units).  Done while the next unit runs, off the chain from level to level; inside the
+  // element loop they would take ~150 instructions of every warp with one such element.
+  auto outputs = [&](const unsigned char* ob, int counts) {
+    const int nx = counts & 0xFFFF, nw = (int)((unsigned)counts >> 16);
+    for (int i = nthr - 1 - tid; i < nx * MC; i += nthr) {
+      const int k = i / MC, j = MC - 1 - (i - k * MC);      // consecutive lanes, consecutive MFPs
+      const int2 e = reinterpret_cast<const int2*>(ob)[k];
+      constexpr int H = 16 / (int)sizeof(Real);
+      const unsigned off = (unsigned)e.y ^ (j >= H ? 16u : 0u);
+      Real v = reinterpret_cast<const Real*>(ring + off)[j % H];
+      if constexpr (DF) v = dpack_value(v);
+      if (j < mc) dT_out[p.n + p.nd + (int64_t)e.x * p.n_mfp + m0 + j] = widen(v);
+    }
+    if (nw) {
+      const unsigned char* wb = ob + ((nx * 8 + 15) & ~15);
+      int i = nthr - 33 - tid;
+      if (i < 0) i += nthr;
+      for (; i < nw; i += nthr) {
+        wall_outputs<Real, MC, DF>(p, wb, nw, i, ring, s_sig, dT_out, chunk);
       }
-      if (el < e - a) {
-        // record: RW/4 vector loads (the G lanes of the group read the same record)
-        int32_t r[RW];
-        const int4* r4 = reinterpret_cast<const int4*>(smem + L.rec + bi * L.rec_stride) + el * (RW / 4);
+    }
+  };
+  // kappa and suppression sums of contact entry ce (final pass)
+  auto contact = [&](int ce, const Real* Tc) {
 #pragma unroll
-        for (int i = 0; i < RW / 4; ++i) {
-          const int4 x = r4[i];
-          r[4 * i] = x.x; r[4 * i + 1] = x.y; r[4 * i + 2] = x.z; r[4 * i + 3] = x.w;
+    for (int j = 0; j < KV; ++j) {
+      if (j < mc) {
+        const Real kv = p.kcoef[(int64_t)ce * p.m_pad + m0 + j] * Tc[j], sv = p.scoef[ce] * Tc[j];
+        if (p.det) {
+          p.kpart[(int64_t)ce * p.m_pad + m0 + j] = kv;
+          p.spart[(int64_t)ce * p.m_pad + m0 + j] = sv;
+        } else {
+          atomicAdd(&s_k[j], kv);
+          atomicAdd(&s_s[j], sv);
         }
-        const int voff = sizeof(Real) == 4 ? ((qn_odd + a) & 1) : 0;
-        const Real* v = reinterpret_cast<const Real*>(smem + L.val + bi * L.val_stride) + 2 * (voff + el);
-        const Real b = v[0], pw = v[1];
-        const int c = r[0];
-        const int so = r[1] & 0xFFFF, s0 = (int)((unsigned)r[1] >> 16);
-        const int s1 = r[2] & 0xFFFF, s2 = (int)((unsigned)r[2] >> 16);
-        const int s3 = r[3] & 0xFFFF, sp = (int)((unsigned)r[3] >> 16);
-        int xk = -1, wo = 0, ce = -1;
-        if (sp) {
-          const int4 ent = reinterpret_cast<const int4*>(smem + L.sxo + bi * L.sx_stride)[sp - 1];
-          xk = ent.x; wo = ent.y; ce = ent.z;
+      }
+    }
+  };
+  // wait for a unit's stage and read its header and this thread's first element; a thread whose wait gives up
+  // skips the unit and says so
+  auto arrive = [&](int u) {
+    if (mbar_wait_bounded(&bars[bi], phase, p.wait_limit)) {
+      hd = *reinterpret_cast<const int4*>(st);
+      fetch(st, hd.x >> 16, tid);
+    } else {
+      hd = make_int4(0, 0, 0, 0);
+      atomicOr(p.err, 1);
+      atomicMin(s_fail, u);
+    }
+  };
+  arrive(0);
+  __syncthreads();
+  int counts = 0;        // outputs of unit u - 1
+  for (int u = 0; u < nlev; ++u) {
+    // the first failed unit, written before the barrier above; later ones carry a larger number
+    const int fail = *(volatile int*)s_fail;
+    const int n_el = hd.x & 0xFFFF;
+    const int co = u == 0 ? 0 : oi == nbuf ? 0 : oi + 1;   // output block of this unit
+    int pend = -1;                                         // final pass: contact entry summed at the unit's end
+    Real Tp0[FINAL ? KV : 1];
+    int el = tid;
+    // read together: while the row loads are in flight the issuer refills the stage of unit u - 1
+    Real v0[KV], v1[KV], v2[KV], v3[NF > 3 ? KV : 1];
+    auto rows = [&]() {
+      row_load<MC, KV>(ring, ((unsigned)r[1] >> 12) & 0xFFFF0u, 0, v0);
+      row_load<MC, KV>(ring, ((unsigned)r[2] << 4) & 0xFFFF0u, 0, v1);
+      row_load<MC, KV>(ring, ((unsigned)r[2] >> 12) & 0xFFFF0u, 0, v2);
+      if constexpr (NF > 3) row_load<MC, KV>(ring, ((unsigned)r[3] << 4) & 0xFFFF0u, 0, v3);
+    };
+    if (el < n_el) rows();
+    if (fail <= u) {
+      // let the copies this CTA still has in flight land before leaving (bounded)
+      if (tid == issuer)
+        for (int w = u; w < nlev && w < (u ? u - 1 + nbuf : nbuf); ++w)
+          mbar_wait_bounded(&bars[w % nbuf], (unsigned)(w / nbuf) & 1u, p.wait_limit);
+      __syncthreads();
+      return;
+    }
+    if (tid == issuer && u > 0 && u - 1 + nbuf < nlev) {
+      const int pb = bi == 0 ? nbuf - 1 : bi - 1;
+      const int4* h = reinterpret_cast<const int4*>(smem + p.stage0 + pb * p.stage);
+      const int np = h[0].w;
+      const int4 d = h[1];
+      // unit u - 1 + nbuf takes the stage of unit u - 1, and the output block of unit u - 2
+      issue(u - 1 + nbuf, pb, oi == 0 ? nbuf : oi - 1, (unsigned)d.x, (unsigned)d.y, (unsigned)d.z, d.w, (unsigned)np);
+    }
+    while (el < n_el) {
+      const int c = r[0];
+      const unsigned so = ((unsigned)r[1] << 4) & 0xFFFF0u;
+      const Real b = bv;
+      const Real c0 = word_real<Real>(r, RR::COEF);
+      const Real c1 = word_real<Real>(r, RR::COEF + RR::CSTEP);
+      const Real c2 = word_real<Real>(r, RR::COEF + 2 * RR::CSTEP);
+      const Real c3 = NF > 3 ? word_real<Real>(r, RR::COEF + 3 * RR::CSTEP) : Real(0);
+      const Real D = word_real<Real>(r, RR::D);
+      Real T[KV];
+      Real dacc = 0, j0 = 0, j1 = 0, j2 = 0;
+      const Real* sg0 = s_sig;
+      const Real* sg1 = sg0 + MC;
+      const Real* sg2 = sg1 + MC;
+      if constexpr (DF) {
+        // output pass in double-float: the ring holds packed pairs, every product and sum is a pair
+        const df2 C0 = dbcast(c0), C1 = dbcast(c1), C2 = dbcast(c2), C3 = dbcast(c3), DD = dbcast(D);
+        const df2 BB = dbcast(b), PW = dbcast(pw);
+        const df2 ONE = {make_float2(1.0f, 1.0f), make_float2(0.0f, 0.0f)};
+        df2 da = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)}, ja = da, jb = da, jc = da;
+        Real Tp[KV];
+#pragma unroll
+        for (int j = 0; j < KV; j += 2) {
+          df2 sm = dmul2(C0, dunpack2(v0[j], v0[j + 1]));
+          sm = dadd2(sm, dmul2(C1, dunpack2(v1[j], v1[j + 1])));
+          sm = dadd2(sm, dmul2(C2, dunpack2(v2[j], v2[j + 1])));
+          if constexpr (NF > 3) sm = dadd2(sm, dmul2(C3, dunpack2(v3[j], v3[j + 1])));
+          const df2 LM = lam2[j / 2];
+          const df2 num = dadd2(BB, dmul2(LM, dadd2(PW, dneg2(sm))));   // b + L (pw - sm)
+          const df2 den = dadd2(ONE, dmul2(LM, DD));                    // 1 + L D
+          const df2 t2 = ddiv2(num, den);
+          Tp[j] = dpack(t2.h.x, t2.l.x);
+          Tp[j + 1] = dpack(t2.h.y, t2.l.y);
+          da = dadd2(da, dmul2(tt2[j / 2], t2));
+          ja = dadd2(ja, dmul2(dunpack2(sg0[j], sg0[j + 1]), t2));
+          jb = dadd2(jb, dmul2(dunpack2(sg1[j], sg1[j + 1]), t2));
+          if (p.ds > 2) jc = dadd2(jc, dmul2(dunpack2(sg2[j], sg2[j + 1]), t2));
         }
-        using RR = Rec<Real, NF>;
-        const Real c0 = word_real<Real>(r, RR::COEF);
-        const Real c1 = word_real<Real>(r, RR::COEF + RR::CSTEP);
-        const Real c2 = word_real<Real>(r, RR::COEF + 2 * RR::CSTEP);
-        const Real c3 = NF > 3 ? word_real<Real>(r, RR::COEF + 3 * RR::CSTEP) : Real(0);
-        const Real D = word_real<Real>(r, RR::D);
-        Real v0[KV], v1[KV], v2[KV], v3[KV];
-        vload(ring + s0 * MC + mo, v0);
-        vload(ring + s1 * MC + mo, v1);
-        vload(ring + s2 * MC + mo, v2);
-        if (NF > 3) vload(ring + s3 * MC + mo, v3);
-        Real T[KV];
-        Real dacc = 0, j0 = 0, j1 = 0, j2 = 0;
-        if constexpr (DF) {
-          // output pass in double-float: the ring holds packed pairs, every product and sum is a pair
-          const df2 C0 = dbcast(c0), C1 = dbcast(c1), C2 = dbcast(c2), C3 = dbcast(c3), DD = dbcast(D);
-          const df2 BB = dbcast(b), PW = dbcast(pw);
-          const df2 ONE = {make_float2(1.0f, 1.0f), make_float2(0.0f, 0.0f)};
-          df2 da = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)}, ja = da, jb = da, jc = da;
-          Real Tp[KV];
+        dacc = ((double)da.h.x + (double)da.h.y) + ((double)da.l.x + (double)da.l.y);
+        j0 = ((double)ja.h.x + (double)ja.h.y) + ((double)ja.l.x + (double)ja.l.y);
+        j1 = ((double)jb.h.x + (double)jb.h.y) + ((double)jb.l.x + (double)jb.l.y);
+        j2 = ((double)jc.h.x + (double)jc.h.y) + ((double)jc.l.x + (double)jc.l.y);
+        row_store<MC, KV>(ring, so, 0, Tp);
+        // real values for the stored fields and contact sums below
+        const bool need = p.Xs != nullptr || p.Xd != nullptr || (((unsigned)r[3] >> 16) & 0x7FFFu) != 0u;
 #pragma unroll
-          for (int j = 0; j < KV; j += 2) {
-            df2 sm = dmul2(C0, dunpack2(v0[j], v0[j + 1]));
-            sm = dadd2(sm, dmul2(C1, dunpack2(v1[j], v1[j + 1])));
-            sm = dadd2(sm, dmul2(C2, dunpack2(v2[j], v2[j + 1])));
-            if (NF > 3) sm = dadd2(sm, dmul2(C3, dunpack2(v3[j], v3[j + 1])));
-            const df2 LM = lam2[j / 2];
-            const df2 num = dadd2(BB, dmul2(LM, dadd2(PW, dneg2(sm))));   // b + L (pw - sm)
-            const df2 den = dadd2(ONE, dmul2(LM, DD));                    // 1 + L D
-            const df2 t2 = ddiv2(num, den);
-            Tp[j] = dpack(t2.h.x, t2.l.x);
-            Tp[j + 1] = dpack(t2.h.y, t2.l.y);
-            da = dadd2(da, dmul2(tt2[j / 2], t2));
-            const Real* sj = s_sig + (mo + j) * 3;   // packed sigma of MFPs j (sj[0..2]) and j + 1 (sj[3..5])
-            ja = dadd2(ja, dmul2(dunpack2(sj[0], sj[3]), t2));
-            jb = dadd2(jb, dmul2(dunpack2(sj[1], sj[4]), t2));
-            if (p.ds > 2) jc = dadd2(jc, dmul2(dunpack2(sj[2], sj[5]), t2));
+        for (int j = 0; j < KV; ++j) T[j] = need ? dpack_value(Tp[j]) : Real(0);
+      } else if constexpr (sizeof(Real) == 4) {
+        // FP32: the MFPs in pairs with Blackwell's packed FP32x2 arithmetic (one instruction per two MFPs;
+        // each lane of a packed operation rounds like the scalar one)
+        const float2 C0 = make_float2(c0, c0), C1 = make_float2(c1, c1), C2 = make_float2(c2, c2);
+        const float2 C3 = make_float2(c3, c3), DD = make_float2(D, D), BB = make_float2(b, b);
+        const float2 PW = make_float2(pw, pw), ONE = make_float2(1.0f, 1.0f), NEG = make_float2(-1.0f, -1.0f);
+#pragma unroll
+        for (int j = 0; j < KV; j += 2) {
+          float2 sm = __fmul2_rn(C0, make_float2(v0[j], v0[j + 1]));
+          sm = __ffma2_rn(C1, make_float2(v1[j], v1[j + 1]), sm);
+          sm = __ffma2_rn(C2, make_float2(v2[j], v2[j + 1]), sm);
+          if constexpr (NF > 3) sm = __ffma2_rn(C3, make_float2(v3[j], v3[j + 1]), sm);
+          const float2 lm = make_float2(lam[j], lam[j + 1]);
+          const float2 num = __ffma2_rn(lm, __ffma2_rn(NEG, sm, PW), BB);    // b + L (pw - sm)
+          const float2 den = __ffma2_rn(lm, DD, ONE);                        // 1 + L D
+          const float2 t2 = __fmul2_rn(num, make_float2(rcp(den.x), rcp(den.y)));
+          T[j] = t2.x;
+          T[j + 1] = t2.y;
+        }
+        row_store<MC, KV>(ring, so, 0, T);
+        // sum over the chunk's MFPs, even and odd ones apart, in MFP order
+        auto wsum = [&](auto weight) -> float {
+          float2 acc = make_float2(0.0f, 0.0f);
+#pragma unroll
+          for (int j = 0; j < KV; j += 2) acc = __ffma2_rn(weight(j), make_float2(T[j], T[j + 1]), acc);
+          return acc.x + acc.y;
+        };
+        dacc = wsum([&](int j) { return make_float2(tt[j], tt[j + 1]); });
+        if (FINAL) {
+          j0 = wsum([&](int j) { return make_float2(sg0[j], sg0[j + 1]); });
+          j1 = wsum([&](int j) { return make_float2(sg1[j], sg1[j + 1]); });
+          if (p.ds > 2) j2 = wsum([&](int j) { return make_float2(sg2[j], sg2[j + 1]); });
+        }
+      } else {
+        if (gain_qc) {
+          // T = b + G (p - D b - sum g T_up) with G = L / (1 + L D): five FP64 operations per unknown (four
+          // and the weighted sum) instead of the seven of the quotient form times the reciprocal
+          const Real y = fma(-D, b, pw);
+#pragma unroll
+          for (int j = 0; j < KV; ++j) {
+            Real z = fma(-c0, v0[j], y);
+            z = fma(-c1, v1[j], z);
+            z = fma(-c2, v2[j], z);
+            if constexpr (NF > 3) z = fma(-c3, v3[j], z);
+            T[j] = fma((Real)gn[kGain ? j : 0], z, b);
           }
-          dacc = ((double)da.h.x + (double)da.h.y) + ((double)da.l.x + (double)da.l.y);
-          j0 = ((double)ja.h.x + (double)ja.h.y) + ((double)ja.l.x + (double)ja.l.y);
-          j1 = ((double)jb.h.x + (double)jb.h.y) + ((double)jb.l.x + (double)jb.l.y);
-          j2 = ((double)jc.h.x + (double)jc.h.y) + ((double)jc.l.x + (double)jc.l.y);
-          vstore(ring + so * MC + mo, Tp);
-          // real values for the per-MFP outputs below (periodic outflow, walls, contact, stored fields)
-          const bool need = sp != 0 || p.Xs != nullptr || p.Xd != nullptr;
-#pragma unroll
-          for (int j = 0; j < KV; ++j) T[j] = need ? dpack_value(Tp[j]) : Real(0);
-        } else if constexpr (sizeof(Real) == 4 && KV % 2 == 0) {
-          // FP32: the MFPs in pairs with Blackwell's packed FP32x2 arithmetic (one instruction per two MFPs;
-          // each lane of a packed operation rounds like the scalar one)
-          const float2 C0 = make_float2(c0, c0), C1 = make_float2(c1, c1), C2 = make_float2(c2, c2);
-          const float2 C3 = make_float2(c3, c3), DD = make_float2(D, D), BB = make_float2(b, b);
-          const float2 PW = make_float2(pw, pw), ONE = make_float2(1.0f, 1.0f), NEG = make_float2(-1.0f, -1.0f);
-          float2 da = make_float2(0.0f, 0.0f), ja = da, jb = da, jc = da;
-#pragma unroll
-          for (int j = 0; j < KV; j += 2) {
-            float2 sm = __fmul2_rn(C0, make_float2(v0[j], v0[j + 1]));
-            sm = __ffma2_rn(C1, make_float2(v1[j], v1[j + 1]), sm);
-            sm = __ffma2_rn(C2, make_float2(v2[j], v2[j + 1]), sm);
-            if (NF > 3) sm = __ffma2_rn(C3, make_float2(v3[j], v3[j + 1]), sm);
-            const float2 lm = make_float2(lam[j], lam[j + 1]);
-            const float2 num = __ffma2_rn(lm, __ffma2_rn(NEG, sm, PW), BB);    // b + L (pw - sm)
-            const float2 den = __ffma2_rn(lm, DD, ONE);                        // 1 + L D
-            const float2 t2 = __fmul2_rn(num, make_float2(__fdividef(1.0f, den.x), __fdividef(1.0f, den.y)));
-            T[j] = t2.x;
-            T[j + 1] = t2.y;
-            da = __ffma2_rn(make_float2(tt[j], tt[j + 1]), t2, da);
-            if (FINAL) {
-              const Real* sj = s_sig + (mo + j) * 3;
-              ja = __ffma2_rn(make_float2(sj[0], sj[3]), t2, ja);
-              jb = __ffma2_rn(make_float2(sj[1], sj[4]), t2, jb);
-              if (p.ds > 2) jc = __ffma2_rn(make_float2(sj[2], sj[5]), t2, jc);
-            }
-          }
-          dacc = da.x + da.y;
-          j0 = ja.x + ja.y;
-          j1 = jb.x + jb.y;
-          j2 = jc.x + jc.y;
         } else {
 #pragma unroll
           for (int j = 0; j < KV; ++j) {
             Real sm = c0 * v0[j] + c1 * v1[j] + c2 * v2[j];
-            if (NF > 3) sm += c3 * v3[j];
-            if (kRinv && rinv_qc) T[j] = (Real)((b + lam[j] * (pw - sm)) * rcur[j]);
-            else T[j] = quot(b + lam[j] * (pw - sm), Real(1) + lam[j] * D);
-            dacc += tt[j] * T[j];
-            if (FINAL) {
-              const Real* sj = s_sig + (mo + j) * 3;
-              j0 += sj[0] * T[j];
-              j1 += sj[1] * T[j];
-              if (p.ds > 2) j2 += sj[2] * T[j];
-            }
+            if constexpr (NF > 3) sm += c3 * v3[j];
+            T[j] = quot(b + lam[j] * (pw - sm), Real(1) + lam[j] * D);
           }
         }
-        if constexpr (!DF) vstore(ring + so * MC + mo, T);
-        if (FINAL && p.Xs != nullptr) {
-#pragma unroll
-          for (int j = 0; j < KV; ++j)
-            if (mo + j < mc) {
-              float* xs = p.Xs + ((int64_t)q * p.n + c) * p.n_mfp + m0 + mo + j;
-              *xs = p.xs_add ? *xs + (float)T[j] : (float)T[j];
-            }
-        }
-        if (FINAL && p.Xd != nullptr) {
-#pragma unroll
-          for (int j = 0; j < KV; ++j)
-            if (mo + j < mc) p.Xd[((int64_t)q * p.n + c) * p.n_mfp + m0 + mo + j] = (double)T[j];
-        }
-        dacc = group_sum<G>(dacc, gmask);
-        if (lane == 0) {
-          if (p.det) p.dpart[(int64_t)cta * p.n + a + el] = dacc;
-          else atomicAdd(&dT_out[c], (double)dacc);
-        }
-        if (FINAL) {
-          j0 = group_sum<G>(j0, gmask);
-          j1 = group_sum<G>(j1, gmask);
-          j2 = group_sum<G>(j2, gmask);
-          if (lane == 0) {
-            if (p.det) {
-              Real* jp = p.jpart + ((int64_t)cta * p.n + a + el) * p.ds;
-              jp[0] = j0;
-              if (p.ds > 1) jp[1] = j1;
-              if (p.ds > 2) jp[2] = j2;
-            } else {
-              atomicAdd(&p.Jraw[(int64_t)c * p.ds], (double)j0);
-              if (p.ds > 1) atomicAdd(&p.Jraw[(int64_t)c * p.ds + 1], (double)j1);
-              if (p.ds > 2) atomicAdd(&p.Jraw[(int64_t)c * p.ds + 2], (double)j2);
-            }
-          }
-        }
-        // per-MFP outputs of special elements (the group is uniform in these conditions)
-        if (xk >= 0) {
-#pragma unroll
-          for (int j = 0; j < KV; ++j)
-            if (mo + j < mc) X_out[(xq + xk) * p.n_mfp + m0 + mo + j] = (double)T[j];
-        }
-        if (wo != 0) {
-          const int wb = wo >> 3, wn = wo & 7;
-          // re-emission weight max(sigma . w, 0) / (-sum min(sigma . w, 0)) from the staged wall geometry
-          // (bte.py:73-78); absent entries read the first entry (unused)
-          const Real* gw = reinterpret_cast<const Real*>(smem + L.gg + bi * L.gg_stride) + (size_t)(wb - wu) * 4;
-          const Real* gw1 = gw + (wn > 1 ? 4 : 0);
-          const Real* gw2 = gw + (wn > 2 ? 8 : 0);
-          Real w0 = 0, w1 = 0, w2 = 0;
-#pragma unroll
-          for (int j = 0; j < KV; ++j) {
-            const Real* sj = s_sig + (mo + j) * 3;
-            const Real s0r = sigv(sj[0]), s1r = sigv(sj[1]), s2r = sigv(sj[2]);
-            const Real a0 = s0r * gw[0] + s1r * gw[1] + s2r * gw[2];
-            const Real a1 = s0r * gw1[0] + s1r * gw1[1] + s2r * gw1[2];
-            const Real a2 = s0r * gw2[0] + s1r * gw2[1] + s2r * gw2[2];
-            w0 += (a0 > Real(0) ? a0 * gw[3] : Real(0)) * T[j];
-            w1 += (a1 > Real(0) ? a1 * gw1[3] : Real(0)) * T[j];
-            w2 += (a2 > Real(0) ? a2 * gw2[3] : Real(0)) * T[j];
-          }
-          w0 = group_sum<G>(w0, gmask);
-          if (wn > 1) w1 = group_sum<G>(w1, gmask);
-          if (wn > 2) w2 = group_sum<G>(w2, gmask);
-          if (lane == 0) {
-            if (p.det) {
-              Real* wp = p.wpart + (int64_t)chunk * p.n_wo + wo0 + wb;
-              wp[0] = w0;
-              if (wn > 1) wp[1] = w1;
-              if (wn > 2) wp[2] = w2;
-            } else {
-              atomicAdd(&TB_out[p.wo_wall[wo0 + wb]], (double)w0);
-              if (wn > 1) atomicAdd(&TB_out[p.wo_wall[wo0 + wb + 1]], (double)w1);
-              if (wn > 2) atomicAdd(&TB_out[p.wo_wall[wo0 + wb + 2]], (double)w2);
-            }
-          }
-        }
-        if (FINAL && ce >= 0) {
-#pragma unroll
-          for (int j = 0; j < KV; ++j) {
-            if (mo + j < mc) {
-              const Real kv = p.kcoef[(int64_t)ce * p.m_pad + m0 + mo + j] * T[j], sv = p.scoef[ce] * T[j];
-              if (p.det) {
-                p.kpart[(int64_t)ce * p.m_pad + m0 + mo + j] = kv;
-                p.spart[(int64_t)ce * p.m_pad + m0 + mo + j] = sv;
-              } else {
-                atomicAdd(&s_k[mo + j], kv);
-                atomicAdd(&s_s[mo + j], sv);
-              }
-            }
-          }
-        }
-      }
-      // bank (u+1)&1 was last read during unit u-1
-      if (pk >= 0) {
-        Real xr[KV];
 #pragma unroll
         for (int j = 0; j < KV; ++j) {
-          if constexpr (DF) xr[j] = dpack_split(xv[j]);
-          else xr[j] = (Real)xv[j];
-        }
-        vstore(ring + (prow_next + pf_i) * MC + mo, xr);
-      }
-      for (int i = pf_i + kUnit; i < npf; i += kUnit) {   // units with more than kUnit cut inflow faces
-        const int k = s_pf[i];
-        if (k < 0) continue;
-        const double* xs = X + (xq + k) * p.n_mfp + m0 + mo;
-        for (int j = 0; j < KV; ++j) {
-          const Real xval = mo + j < mc ? (Real)xs[j] : Real(0);
-          if constexpr (DF) ring[(size_t)(prow_next + i) * MC + mo + j] = dpack_split(xval);
-          else ring[(size_t)(prow_next + i) * MC + mo + j] = xval;
+          dacc += tt[j] * T[j];
+          if (FINAL) {
+            j0 += sg0[j] * T[j];
+            j1 += sg1[j] * T[j];
+            if (p.ds > 2) j2 += sg2[j] * T[j];
+          }
         }
       }
+      if constexpr (!DF && sizeof(Real) == 8) row_store<MC, KV>(ring, so, 0, T);
+      if (FINAL && p.Xs != nullptr) {
+#pragma unroll
+        for (int j = 0; j < KV; ++j)
+          if (j < mc) {
+            float* xs = p.Xs + ((int64_t)q * p.n + c) * p.n_mfp + m0 + j;
+            *xs = p.xs_add ? *xs + (float)T[j] : (float)T[j];
+          }
+      }
+      if (FINAL && p.Xd != nullptr) {
+#pragma unroll
+        for (int j = 0; j < KV; ++j)
+          if (j < mc) p.Xd[((int64_t)q * p.n + c) * p.n_mfp + m0 + j] = (double)T[j];
+      }
+      if (p.det) p.dpart[(int64_t)cta * p.n + hd.y + el] = dacc;
+      else atomicAdd(&dT_out[c], widen(dacc));
+      if (FINAL) {
+        if (p.det) {
+          Real* jp = p.jpart + ((int64_t)cta * p.n + hd.y + el) * p.ds;
+          jp[0] = j0;
+          if (p.ds > 1) jp[1] = j1;
+          if (p.ds > 2) jp[2] = j2;
+        } else {
+          atomicAdd(&p.Jraw[(int64_t)c * p.ds], widen(j0));
+          if (p.ds > 1) atomicAdd(&p.Jraw[(int64_t)c * p.ds + 1], widen(j1));
+          if (p.ds > 2) atomicAdd(&p.Jraw[(int64_t)c * p.ds + 2], widen(j2));
+        }
+      }
+      if (FINAL) {
+        // contact elements; those of a warp with a periodic source after the others of the unit (the sums are in
+        // the sweep's precision: this keeps their order, inflow side first)
+        const int kc = (int)((unsigned)r[3] >> 16);
+        const bool late = __any_sync(__activemask(), (kc & 0x8000) != 0);
+        if (pend >= 0) contact(pend, Tp0);
+        pend = -1;
+        if (kc & 0x7FFF) {
+          const int nx = hd.z & 0xFFFF;
+          const int ce = reinterpret_cast<const int4*>(smem + p.out0 + co * p.out + ((nx * 8 + 15) & ~15))[(kc & 0x7FFF) - 1].z;
+          if (late) {
+            pend = ce;
+#pragma unroll
+            for (int j = 0; j < KV; ++j) Tp0[FINAL ? j : 0] = T[j];
+          } else {
+            contact(ce, T);
+          }
+        }
+      }
+      el += nthr;
+      if (el < n_el) {           // units wider than the CTA
+        fetch(st, hd.x >> 16, el);
+        rows();
+      }
     }
-    // block barrier that also tells every thread whether any wait of this unit gave up
-    if (__syncthreads_or(ready ? 0 : 1)) {
-      // let the copies this CTA still has in flight land before leaving (bounded)
-      if (tid == kIssuer)
-        for (int w = u + 1; w < nlev && w < u + nbuf; ++w) mbar_wait_bounded(&bars[w % nbuf], (unsigned)(w / nbuf) & 1u);
-      __syncthreads();
-      return;
-    }
+    if (counts) outputs(smem + p.out0 + oi * p.out, counts);
+    counts = hd.z;
+    if (u > 0 && ++oi > nbuf) oi = 0;
+    // unit u + 1: its records (not its rows) before the barrier
     if (++bi == nbuf) { bi = 0; phase ^= 1u; }
-    a = e;
-    e = e_next;
-    wu = wu_next;
-    kpf1 = kpf2;
-    kpf2 = kpf3;
-    if (rinv_qc) {
-#pragma unroll
-      for (int j = 0; j < KV; ++j) rcur[j] = rnxt[j];
-    }
+    st = smem + p.stage0 + bi * p.stage;
+    if (u + 1 < nlev) arrive(u + 1);
+    if (FINAL && pend >= 0) contact(pend, Tp0);
+    __syncthreads();
   }
+  if (counts) outputs(smem + p.out0 + oi * p.out, counts);
+  if (FINAL) __syncthreads();
   if (FINAL && !p.det) {
-    for (int j = tid; j < mc; j += blockDim.x) {
+    for (int j = tid; j < mc; j += nthr) {
       p.K[(int64_t)(m0 + j) * p.n_dir + q] = (double)s_k[j];
       p.S_out[(int64_t)(m0 + j) * p.n_dir + q] = (double)s_s[j];
     }
@@ -1189,8 +1370,8 @@ __global__ void det_contact_sum_kernel(const Real* __restrict__ kpart, const Rea
 // ---- table upload ---------------------------------------------------------------
 
 size_t DevSchedule::bytes() const {
-  const DevBuf* all[] = {&rec, &klev_ptr, &klev_off, &knlev, &kwo, &kpf, &pf, &sx, &ksx, &mfp, &tco, &sig, &wo_wall, &wo_geo,
-                         &kcoef, &scoef, &hs, &vals, &cellmap, &Pq, &si, &sr, &wo_off, &spec, &lpt, &rinv};
+  const DevBuf* all[] = {&blk, &desc, &unit_base, &pfe, &xrow, &mfp, &tco, &sig, &kcoef, &scoef, &hs,
+                         &vals, &cellmap, &Pq, &si, &sr, &spec, &lpt, &gain};
   size_t b = 0;
   for (auto* x : all) b += x->bytes;
   return b;
@@ -1203,43 +1384,103 @@ static obte_status upload_real(DevBuf& b, const std::vector<double>& v, cudaStre
   return upload(b, h, st);
 }
 
-
-// Compiled thread shapes (lanes per element G, MFPs per lane KV) for each precision.
-struct Shape { int G, KV; };
-template <typename Real> struct Shapes;
-template <> struct Shapes<float> { static constexpr Shape v[] = {{1, 4}, {1, 8}, {2, 4}, {1, 2}}; };
-template <> struct Shapes<double> { static constexpr Shape v[] = {{1, 2}, {1, 4}, {2, 2}}; };
-constexpr Shape Shapes<float>::v[];
-constexpr Shape Shapes<double>::v[];
-
-// Choose the thread shape.  Measured on the 60k-triangle (100 MFP x 96 directions) and 110k-tetrahedron
-// (30 x 512) benchmark meshes: one thread per element (G = 1) is fastest (2.32 / 10.5 ms per FP32 sweep
-// against 2.40 / 16.7 ms at G = 2 and 2.90 ms at G = 8), because each CTA is a chain of level barriers
-// and more, smaller CTAs per SM keep more chains in flight.
-// OBTE_SWEEP_G / OBTE_SWEEP_KV force a shape (tuning); a shape whose shared memory does not fit is
-// skipped.
+// MFPs per CTA (the MFPs that share a partial sum).  FP32: 8 while a base layout (128-element units, two
+// staged) with 32-byte rows would let at least 4 CTAs share an SM, else 4 (60k triangles: 2.14 ms at 8 against
+// 2.23 at 4; 110k tetrahedra, 2 CTAs per SM at 8: 20.8 against 11.6 ms); 4 for at most 4 MFPs.  The choice fixes
+// the grouping of the FP32 partial sums, so it depends on the mesh and the ordinates alone, not on the
+// launch shape below.  FP64: 2.  OBTE_SWEEP_KV forces a compiled value.
 template <typename Real>
-static Shape choose_shape(const Schedule& s, int rows, int unit_wo, int pf_pad, int unit_sx, int nbuf,
-                          size_t optin) {
-  const char* eg = std::getenv("OBTE_SWEEP_G");
-  const char* ek = std::getenv("OBTE_SWEEP_KV");
-  const int want_g = eg ? std::atoi(eg) : 1;
-  const int want_k = ek ? std::atoi(ek) : V16<Real>::K;
-  auto fits = [&](Shape sh) {
-    return SmemLayout<Real>(s.nf, sh.G * sh.KV, rows, unit_wo, pf_pad, unit_sx, nbuf).total <= optin;
-  };
-  if (eg || ek) {
-    for (Shape sh : Shapes<Real>::v)
-      if (sh.G == want_g && sh.KV == want_k && fits(sh)) return sh;
-  } else {
-    // two vectors per lane halve the per-element overhead per MFP; worth it while at least 4 CTAs still
-    // share an SM (60k triangles: 2.14 against 2.23 ms; 110k tetrahedra, 2 CTAs per SM: 20.8 against 11.6 ms)
-    const Shape wide{1, 2 * V16<Real>::K};
-    const size_t sm = SmemLayout<Real>(s.nf, wide.KV, rows, unit_wo, pf_pad, unit_sx, nbuf).total;
-    if (sizeof(Real) == 4 && sm + 1024 <= (228 * 1024) / 4 && fits(wide)) return wide;
+static int choose_mc(const Schedule& s, const UnitStats& base) {
+  constexpr int kNarrow = 16 / (int)sizeof(Real), kWide = 2 * kNarrow;
+  if (const char* e = std::getenv("OBTE_SWEEP_KV")) {
+    const int v = std::atoi(e);
+    if (v == kNarrow || v == kWide) return v;
   }
-  const Shape base{1, V16<Real>::K};
-  return fits(base) ? base : Shape{0, 0};
+  if (sizeof(Real) == 8 || s.n_mfp <= kNarrow) return kNarrow;
+  const int64_t stage = kBaseUnit * rec_words(sizeof(Real), s.nf) * 4 + (kBaseUnit + 2) * 8 + base.unit_wo * 16 +
+                        ((base.emax + 3) & ~3) * 4 + base.unit_sx * 16;
+  const int64_t rows = s.base_slots + 2 + 2 * base.emax;
+  const int64_t smem = 128 + 2 * stage + kWide * 20 + rows * 32;
+  return smem + 1024 <= 228 * 1024 / 4 ? kWide : kNarrow;
+}
+
+// Lanes per element, threads per CTA, unit size and stages for a plan, by shape alone.
+template <typename Real>
+static obte_status choose_layout(const Schedule& s, size_t optin, Units& un, std::vector<int64_t>& unit_base,
+                                 std::vector<int32_t>& cnt, Layout& lay) {
+  build_units(s, kBaseUnit, un);
+  UnitStats st = count_units(s, un, sizeof(Real), unit_base, cnt);
+  if (st.bad_wo) {
+    set_error("wall re-emission entries are not in sweep order");
+    return OBTE_ERR_BAD_ARG;
+  }
+  const int MC = choose_mc<Real>(s, st);
+  const int n_chunks = (s.n_mfp + MC - 1) / MC;
+  int64_t levels = 0;
+  int widest = 0;
+  for (int q = 0; q < s.n_dir; ++q) {
+    levels += s.nlev[q];
+    const int32_t* lp = s.lev_ptr.data() + s.lev_off[q];
+    for (int L = 0; L < s.nlev[q]; ++L) widest = std::max(widest, (int)(lp[L + 1] - lp[L]));
+  }
+  const double width = levels ? (double)s.n_dir * s.n / (double)levels : 1.0;
+  // CTAs an SM has to run: no more are worth making room for
+  const int64_t want = std::max<int64_t>(1, ((int64_t)s.n_dir * n_chunks + 151) / 152);
+  Layout shape;
+  shape.KV = MC;
+  shape.threads = width <= 64 ? 96 : kMaxThreads;
+  if (const char* e = std::getenv("OBTE_SWEEP_THREADS")) {
+    const int v = std::atoi(e);
+    if (v >= 32 && v <= kMaxThreads && v % 32 == 0) shape.threads = v;
+  }
+  auto layout = [&](const UnitStats& e, int nbuf) { return make_layout<Real>(s, e, shape, nbuf); };
+  auto steps = [&](int cap) {
+    int64_t c = 0;
+    for (int q = 0; q < s.n_dir; ++q) {
+      const int32_t* lp = s.lev_ptr.data() + s.lev_off[q];
+      for (int L = 0; L < s.nlev[q]; ++L) c += (lp[L + 1] - lp[L] + cap - 1) / cap;
+    }
+    return (double)c;
+  };
+  // unit size: a level wider than a unit costs one more step of the chain, a wider unit costs shared memory and
+  // so CTAs per SM: the size with the fewest steps per resident CTA
+  int cap = kBaseUnit;
+  double best = 0;
+  for (int c = kBaseUnit; c <= 256; c += 32) {
+    UnitStats e = st;                       // what wider units would hold, in proportion
+    e.unit_el = std::min(c, widest);
+    if (e.unit_sx > kUnitSx) e.unit_out = e.unit_out * c / kBaseUnit;
+    if (e.emax > kUnitPf) e.emax = e.emax * c / kBaseUnit;
+    const int r = resident<Real>(layout(e, 2));
+    if (r < 1) break;
+    const double cost = steps(c) / (double)std::min<int64_t>(r, want);
+    if (c == kBaseUnit || cost < 0.97 * best) { best = cost; cap = c; }
+    if (c >= widest) break;
+  }
+  if (const char* e = std::getenv("OBTE_SWEEP_UNIT")) cap = std::max(32, std::min(1024, std::atoi(e)));
+  if (cap != kBaseUnit) {
+    build_units(s, cap, un);
+    st = count_units(s, un, sizeof(Real), unit_base, cnt);
+  }
+  // smaller units while two stages do not fit a CTA
+  while (layout(st, 2).smem > optin && cap > 32) {
+    cap /= 2;
+    build_units(s, cap, un);
+    st = count_units(s, un, sizeof(Real), unit_base, cnt);
+  }
+  lay = layout(st, 2);
+  if (lay.smem > optin) {
+    set_error("sweep front needs more shared memory than one CTA can have (" + std::to_string(lay.rows) + " rows)");
+    return OBTE_ERR_UNSUPPORTED;
+  }
+  // more stages where the extra ones cost no resident CTA
+  const char* nb_env = std::getenv("OBTE_SWEEP_NBUF");
+  const int64_t have = std::min<int64_t>(resident<Real>(lay), want);
+  for (int nb = nb_env ? std::max(2, std::min(kMaxBuf, std::atoi(nb_env))) : 4; nb > 2; --nb) {
+    const Layout l = layout(st, nb);
+    if (l.smem <= optin && (nb_env || std::min<int64_t>(resident<Real>(l), want) >= have)) { lay = l; break; }
+  }
+  return OBTE_OK;
 }
 
 template <typename Real>
@@ -1247,44 +1488,44 @@ static obte_status upload_tables(obte_plan plan, DevSchedule& d) {
   PhaseTimer timer(sizeof(Real) == 4 ? "upload_tables fp32" : "upload_tables fp64");
   const Schedule& s = plan->sched;
   cudaStream_t st = plan->stream;
-  // split levels into units of at most kUnit elements (slots were assigned per level, so this stays valid)
   Units un;
-  build_units(s, un);
   Packed pk;
   {
     PhaseTimer tp("pack");
-    OBTE_TRY(pack<Real>(s, un, pk));
+    std::vector<int64_t> unit_base;
+    std::vector<int32_t> cnt;
+    Layout lay;
+    OBTE_TRY(choose_layout<Real>(s, plan->ctx->smem_optin, un, unit_base, cnt, lay));
+    OBTE_TRY(pack<Real>(s, un, unit_base, cnt, lay, pk));
+    OBTE_TRY(upload(d.unit_base, unit_base, st));
+    d.n_units = unit_base[s.n_dir];
   }
-  const int rows = pk.rows;
-  const char* nb_env = std::getenv("OBTE_SWEEP_NBUF");
-  const int nbuf = nb_env ? std::max(2, std::min(kMaxBuf, std::atoi(nb_env))) : kDefaultBuf;
-  const Shape sh = choose_shape<Real>(s, rows, pk.unit_wo, pk.pf_pad, pk.unit_sx, nbuf, plan->ctx->smem_optin);
-  const int G = sh.G;
-  if (!G) {
-    set_error("sweep front needs more shared memory than one CTA can have (" + std::to_string(rows) + " rows)");
-    return OBTE_ERR_UNSUPPORTED;
-  }
-  const int mcp = G * sh.KV;
-  d.G = G;
-  d.KV = sh.KV;
-  d.mc = mcp;
-  d.mcp = mcp;
-  d.n_chunks = (s.n_mfp + mcp - 1) / mcp;
-  d.zero_slot = s.max_slots;
-  d.rows = rows;
-  d.emax = pk.emax;
-  d.unit_wo = pk.unit_wo;
-  d.pf_pad = pk.pf_pad;
-  d.nbuf = nbuf;
-  d.unit_sx = pk.unit_sx;
-  d.smem = SmemLayout<Real>(s.nf, mcp, rows, pk.unit_wo, pk.pf_pad, pk.unit_sx, nbuf).total;
+  const Layout& l = pk.lay;
+  d.mc = l.KV;
+  d.n_chunks = (s.n_mfp + d.mc - 1) / d.mc;
+  d.threads = l.threads;
+  d.prow0 = l.prow0;
+  d.emax = l.emax;
+  d.nbuf = l.nbuf;
+  d.stage0 = kRingOff + l.rows * d.mc * (int)sizeof(Real);
+  d.stage = l.stage();
+  d.out0 = d.stage0 + l.nbuf * l.stage();
+  d.out = l.out;
+  d.val_off = l.blk;
+  d.gain_off = l.blk + l.val;
+  d.smem = l.smem;
+  d.n_pf = pk.n_pf;
+  d.row_stride = pk.n_pf * d.n_chunks * d.mc;
   if (timer.on)
-    std::fprintf(stderr, "[obte trace] sweep shape %s: G %d KV %d, %d chunks x %d directions = %d CTAs, %zu B shared "
-                 "memory (%d rows = %d slots + 2 + 2 x %d bank rows; staging per unit: %d wall entries, %d prefetch ints, %d "
-                 "output entries), <= %zu CTAs per SM by shared memory\n", sizeof(Real) == 4 ? "fp32" : "fp64", G,
-                 sh.KV, d.n_chunks, s.n_dir, d.n_chunks * s.n_dir, d.smem, rows, s.max_slots, pk.emax, pk.unit_wo,
-                 pk.pf_pad, pk.unit_sx, (size_t)(233472 / (d.smem + 1024)));
-  OBTE_TRY(upload(d.rec, pk.rec, st));
+    std::fprintf(stderr, "[obte trace] sweep shape %s: KV %d, %d threads, %d chunks x %d directions = %d CTAs, %zu B "
+                 "shared memory (%d rows = %d slots + 2 + %d x %d bank rows; %d stages of %d B), <= %d CTAs per SM; %lld "
+                 "units, %lld levels\n", sizeof(Real) == 4 ? "fp32" : "fp64", l.KV, l.threads, d.n_chunks, s.n_dir,
+                 d.n_chunks * s.n_dir, l.smem, l.rows, s.max_slots, l.nbuf, l.emax, l.nbuf, l.stage(), resident<Real>(l),
+                 (long long)d.n_units, (long long)std::accumulate(s.nlev.begin(), s.nlev.end(), (int64_t)0));
+  OBTE_TRY(upload(d.blk, pk.blk, st));
+  OBTE_TRY(upload(d.desc, pk.desc, st));
+  OBTE_TRY(upload(d.pfe, pk.pfe, st));
+  OBTE_TRY(d.xrow.alloc(std::max<size_t>((size_t)d.row_stride * sizeof(Real), 32)));
   OBTE_TRY(upload(d.cellmap, pk.cellmap, st));
   OBTE_TRY(upload(d.Pq, pk.P, st));
   OBTE_TRY(upload(d.si, pk.si, st));
@@ -1307,33 +1548,9 @@ static obte_status upload_tables(obte_plan plan, DevSchedule& d) {
       for (int c = 0; c < d.n_chunks; ++c) lpt.push_back(q * d.n_chunks + c);
     OBTE_TRY(upload(d.lpt, lpt, st));
   }
-  OBTE_TRY(upload(d.klev_ptr, un.ptr, st));
-  OBTE_TRY(upload(d.klev_off, un.off, st));
-  OBTE_TRY(upload(d.knlev, un.n, st));
-  OBTE_TRY(upload(d.kwo, pk.kwo, st));
-  OBTE_TRY(upload(d.kpf, pk.kpf, st));
-  OBTE_TRY(upload(d.pf, pk.pf, st));
-  OBTE_TRY(upload(d.sx, pk.sx, st));
-  OBTE_TRY(upload(d.ksx, pk.ksx, st));
-  std::vector<int32_t> wo = s.wo_wall;
-  if (wo.empty()) wo.push_back(0);
-  OBTE_TRY(upload(d.wo_wall, wo, st));
-  OBTE_TRY(upload(d.wo_off, s.wo_off, st));
   OBTE_TRY(upload_real<Real>(d.mfp, s.mfp, st));
   OBTE_TRY(upload_real<Real>(d.tco, s.tco, st));
   OBTE_TRY(upload_real<Real>(d.sig, s.sig, st));
-  {
-    // wall weights regrouped [direction][chunk][entry][mcp] so one unit's entries are one contiguous copy
-    // per wall entry: area vector / volume of the wall's element and 1 / (-sum_mq min(sigma . w, 0))
-    const int64_t n_wo = (int64_t)s.wo_wall.size();
-    std::vector<Real> geo(std::max<size_t>((size_t)n_wo * 4, 4), Real(0));
-    parallel_for(n_wo, [&](int64_t e) {
-      const int32_t w = s.wo_wall[e];
-      for (int k = 0; k < s.dim; ++k) geo[(size_t)e * 4 + k] = (Real)s.w_db[(size_t)w * s.dim + k];
-      geo[(size_t)e * 4 + 3] = s.gbm_sum[w] != 0 ? (Real)(1.0 / (-s.gbm_sum[w])) : Real(0);
-    });
-    OBTE_TRY(upload(d.wo_geo, geo, st));
-  }
   OBTE_TRY(upload_real<Real>(d.kcoef, s.kcoef, st));
   OBTE_TRY(upload_real<Real>(d.scoef, s.scoef, st));
   if (!s.hs.empty()) OBTE_TRY(upload(d.hs, s.hs, st));
@@ -1349,30 +1566,52 @@ static obte_status upload_tables(obte_plan plan, DevSchedule& d) {
   return OBTE_OK;
 }
 
+// Element records of a unit on the device: first record, item of its first element, elements.
+struct UnitRecs {
+  int64_t item0;
+  int64_t word0;
+  int n_el, a;
+};
+template <typename Real>
+__device__ __forceinline__ UnitRecs unit_recs(const int32_t* __restrict__ desc, int64_t u) {
+  const int4 a = reinterpret_cast<const int4*>(desc)[2 * u], b = reinterpret_cast<const int4*>(desc)[2 * u + 1];
+  UnitRecs r;
+  r.item0 = (int64_t)(unsigned)b.y * (16 / (2 * (int)sizeof(Real))) + (a.x >> 16);
+  r.word0 = (int64_t)(unsigned)b.x * 4 + kHeader / 4;
+  r.n_el = a.x & 0xFFFF;
+  r.a = a.y;
+  return r;
+}
+
 // New transmissions: rewrite the coefficient words of the records and the wall inflow coefficients of
 // the special entries (the same walk over the inflow entries as pack), then P and the contact
 // coefficients; indices, units and launch order stay.
 // Coefficient word w of item `it`'s record from inflow slot f: g0 x (t_s, 1 - t_s or 1 by the slot's mode),
-// the same arithmetic as set_transmission on the host, rounded to the record's precision.
+// the same arithmetic as set_transmission on the host, rounded to the record's precision.  A warp per unit.
 template <typename Real, int NF>
-__global__ void refresh_rec_kernel(int64_t items, const double* __restrict__ g0, const int32_t* __restrict__ mode,
-                                   const int8_t* __restrict__ word, const double* __restrict__ t,
-                                   int32_t* __restrict__ rec) {
+__global__ void refresh_rec_kernel(int64_t n_units, const int32_t* __restrict__ desc, const double* __restrict__ g0,
+                                   const int32_t* __restrict__ mode, const int8_t* __restrict__ word,
+                                   const double* __restrict__ t, int32_t* __restrict__ blk) {
   using RR = Rec<Real, NF>;
-  for (int64_t it = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; it < items; it += (int64_t)gridDim.x * blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n_units; u += nw) {
+    const UnitRecs ur = unit_recs<Real>(desc, u);
+    for (int el = lane; el < ur.n_el; el += 32) {
 #pragma unroll
-    for (int f = 0; f < NF; ++f) {
-      const int64_t e = it * NF + f;
-      const int w = word[e];
-      if (w < 0) continue;
-      const int32_t md = mode[e];
-      const double g = md >= 0 ? g0[e] * t[md] : md == -1 ? g0[e] * 1.0 : g0[e] * (1.0 - t[-md - 2]);
-      int32_t* r = rec + it * RR::W + RR::COEF + w * RR::CSTEP;
-      if constexpr (sizeof(Real) == 4) {
-        r[0] = __float_as_int((float)g);
-      } else {
-        r[0] = __double2loint(g);
-        r[1] = __double2hiint(g);
+      for (int f = 0; f < NF; ++f) {
+        const int64_t e = (ur.item0 + el) * NF + f;
+        const int w = word[e];
+        if (w < 0) continue;
+        const int32_t md = mode[e];
+        const double g = md >= 0 ? g0[e] * t[md] : md == -1 ? g0[e] * 1.0 : g0[e] * (1.0 - t[-md - 2]);
+        int32_t* r = blk + ur.word0 + (int64_t)el * RR::W + RR::COEF + w * RR::CSTEP;
+        if constexpr (sizeof(Real) == 4) {
+          r[0] = __float_as_int((float)g);
+        } else {
+          r[0] = __double2loint(g);
+          r[1] = __double2hiint(g);
+        }
       }
     }
   }
@@ -1417,8 +1656,8 @@ static obte_status refresh_impl(obte_plan plan, DevSchedule& d, int64_t* bytes, 
   const int blocks = (int)std::min<int64_t>((items + 255) / 256, (int64_t)plan->ctx->num_sms * 8);
   auto kern = s.nf == 3 ? refresh_rec_kernel<Real, 3> : refresh_rec_kernel<Real, 4>;
   if (s.nf != 3 && s.nf != 4) { d.ready = false; return OBTE_OK; }
-  kern<<<blocks, 256, 0, st>>>(items, plan->tf_g0.as<double>(), plan->tf_mode.as<int32_t>(),
-                               plan->tf_word.as<int8_t>(), plan->tf_t.as<double>(), d.rec.as<int32_t>());
+  kern<<<blocks, 256, 0, st>>>(d.n_units, d.desc.as<int32_t>(), plan->tf_g0.as<double>(), plan->tf_mode.as<int32_t>(),
+                               plan->tf_word.as<int8_t>(), plan->tf_t.as<double>(), d.blk.as<int32_t>());
   count_launch();
   OBTE_CUDA(cudaGetLastError());
   // wall coefficients of the special entries (host, small)
@@ -1473,20 +1712,20 @@ struct Fnv {
 template <typename Real>
 static obte_status tables_digest_impl(const Schedule& s, uint64_t* digest) {
   Units un;
-  {
-    PhaseTimer tu("units");
-    build_units(s, un);
-  }
   Packed pk;
+  std::vector<int64_t> unit_base;
   {
     PhaseTimer tp("pack");
-    OBTE_TRY(pack<Real>(s, un, pk));
+    std::vector<int32_t> cnt;
+    Layout lay;
+    OBTE_TRY(choose_layout<Real>(s, 232448, un, unit_base, cnt, lay));   // 227 KB: the most one CTA can have
+    OBTE_TRY(pack<Real>(s, un, unit_base, cnt, lay, pk));
   }
   Fnv f;
   f.vec(un.ptr); f.vec(un.off); f.vec(un.n);
-  f.vec(pk.rec); f.vec(pk.cellmap); f.vec(pk.si); f.vec(pk.spec); f.vec(pk.P); f.vec(pk.sr);
-  f.vec(pk.pf); f.vec(pk.kpf); f.vec(pk.sx); f.vec(pk.ksx); f.vec(pk.kwo);
-  f.i(pk.unit_sx); f.i(pk.emax); f.i(pk.pf_pad); f.i(pk.unit_wo); f.i(pk.rows);
+  f.vec(pk.blk); f.vec(pk.cellmap); f.vec(pk.si); f.vec(pk.spec); f.vec(pk.P); f.vec(pk.sr);
+  f.vec(pk.desc); f.vec(pk.pfe); f.vec(unit_base);
+  f.i(pk.lay.KV); f.i(pk.lay.threads); f.i(pk.lay.nbuf); f.i(pk.lay.emax); f.i(pk.lay.rows);
   // the schedule's own uploads: contact coefficients, K shifts, wall outputs, periodic sources
   f.vec(s.kcoef); f.vec(s.scoef); f.vec(s.kconst); f.vec(s.kshift); f.vec(s.sshift);
   f.vec(s.wo_wall); f.vec(s.wo_off); f.vec(s.x_cell); f.vec(s.x_base); f.vec(s.ell_B);
@@ -1511,51 +1750,49 @@ obte_status refresh_tables(obte_plan plan, const double* side_transmission, int6
   if (plan->d32.ready) OBTE_TRY(refresh_impl<float>(plan, plan->d32, bytes, plan->d64.ready ? &plan->d64 : nullptr));
   return OBTE_OK;
 }
-
-// 1 / (1 + mfp_m D) for every (direction, chunk, position, MFP of the chunk) of the FP64 tables, D read
-// from the packed records (padded MFPs: 1, as their mfp is 0)
+// mfp_m / (1 + mfp_m D) for every (direction, chunk, position, MFP of the chunk) of the FP64 tables, D read
+// from the packed records (padded MFPs: 0, as their mfp is 0).  A warp per unit, elements on the lanes.
 template <int NF>
-__global__ void rinv_build_kernel(const int32_t* __restrict__ rec, int64_t n, int n_dir, int n_chunks, int mcp,
-                                  int n_mfp, const double* __restrict__ mfp, double* __restrict__ out) {
+__global__ void gain_build_kernel(int64_t n_units, const int32_t* __restrict__ desc, const int32_t* __restrict__ blk,
+                                  int64_t n, int n_chunks, int KV, int n_mfp, const double* __restrict__ mfp,
+                                  double* __restrict__ out) {
   using RR = Rec<double, NF>;
-  const int64_t total = (int64_t)n_dir * n_chunks * n * mcp;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int j = (int)(i % mcp);
-    int64_t t = i / mcp;
-    const int64_t pos = t % n;
-    t /= n;
-    const int chunk = (int)(t % n_chunks);
-    const int64_t q = t / n_chunks;
-    const int m = chunk * mcp + j;
-    const int32_t* r = rec + (q * n + pos) * RR::W;
-    const double D = __hiloint2double(r[RR::D + 1], r[RR::D]);
-    const double L = m < n_mfp ? mfp[m] : 0.0;
-    out[i] = 1.0 / (1.0 + L * D);
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n_units; u += nw) {
+    const UnitRecs ur = unit_recs<double>(desc, u);
+    const int64_t q = ur.item0 / n;
+    const int total = ur.n_el * KV;
+    for (int chunk = 0; chunk < n_chunks; ++chunk)
+      for (int i = lane; i < total; i += 32) {
+        const int el = i / KV, j = i - el * KV, m = chunk * KV + j;
+        const int32_t* r = blk + ur.word0 + (int64_t)el * RR::W;
+        const double D = __hiloint2double(r[RR::D + 1], r[RR::D]);
+        const double L = m < n_mfp ? mfp[m] : 0.0;
+        out[((q * n_chunks + chunk) * n + ur.a) * KV + i] = L / (1.0 + L * D);
+      }
   }
 }
 
-// The FP64 reciprocal table, unless OBTE_SWEEP64_RINV=0 or it would exceed OBTE_SWEEP64_RINV_GB (default 32)
-// or device memory (the sweep then divides)
-static obte_status build_rinv(obte_plan plan, DevSchedule& d) {
+// The FP64 gain table, unless OBTE_SWEEP64_RINV=0 or it would exceed OBTE_SWEEP64_RINV_GB (default 32) or
+// device memory (the sweep then divides)
+static obte_status build_gain(obte_plan plan, DevSchedule& d) {
   const Schedule& s = plan->sched;
   if (const char* e = std::getenv("OBTE_SWEEP64_RINV"))
     if (std::atoi(e) == 0) return OBTE_OK;
   double cap_gb = 32.0;
   if (const char* e = std::getenv("OBTE_SWEEP64_RINV_GB")) cap_gb = std::atof(e);
-  const int64_t total = (int64_t)s.n_dir * d.n_chunks * s.n * d.mcp;
+  const int64_t total = (int64_t)s.n_dir * d.n_chunks * s.n * d.mc;
   if ((double)total * 8.0 > cap_gb * 1e9 || (s.nf != 3 && s.nf != 4)) return OBTE_OK;
-  if (d.rinv.alloc((size_t)total * sizeof(double)) != OBTE_OK) {
+  if (d.gain.alloc((size_t)total * sizeof(double)) != OBTE_OK) {
     cudaGetLastError();
-    d.rinv.release();
+    d.gain.release();
     return OBTE_OK;            // no room: the sweep divides
   }
-  const int blocks = (int)std::min<int64_t>((total + 255) / 256, (int64_t)plan->ctx->num_sms * 16);
-  if (s.nf == 3)
-    rinv_build_kernel<3><<<blocks, 256, 0, plan->stream>>>(d.rec.as<int32_t>(), s.n, s.n_dir, d.n_chunks, d.mcp,
-                                                            s.n_mfp, d.mfp.as<double>(), d.rinv.as<double>());
-  else
-    rinv_build_kernel<4><<<blocks, 256, 0, plan->stream>>>(d.rec.as<int32_t>(), s.n, s.n_dir, d.n_chunks, d.mcp,
-                                                            s.n_mfp, d.mfp.as<double>(), d.rinv.as<double>());
+  const int blocks = (int)std::min<int64_t>((d.n_units + 7) / 8, (int64_t)plan->ctx->num_sms * 16);
+  auto kern = s.nf == 3 ? gain_build_kernel<3> : gain_build_kernel<4>;
+  kern<<<std::max(blocks, 1), 256, 0, plan->stream>>>(d.n_units, d.desc.as<int32_t>(), d.blk.as<int32_t>(), s.n,
+                                                      d.n_chunks, d.mc, s.n_mfp, d.mfp.as<double>(), d.gain.as<double>());
   count_launch();
   OBTE_CUDA(cudaGetLastError());
   return OBTE_OK;
@@ -1571,14 +1808,13 @@ obte_status ensure_tables(obte_plan plan, bool fp32) {
   } else {
     if (!plan->d64.ready) {
       OBTE_TRY(upload_tables<double>(plan, plan->d64));
-      OBTE_TRY(build_rinv(plan, plan->d64));
+      OBTE_TRY(build_gain(plan, plan->d64));
     }
   }
   return OBTE_OK;
 }
 
 // ---- launch -----------------------------------------------------------------------
-
 // Deterministic reductions requested (OBTE_DETERMINISTIC=1, read per call).
 static bool deterministic() {
   const char* e = std::getenv("OBTE_DETERMINISTIC");
@@ -1630,59 +1866,60 @@ static obte_status ensure_det(obte_plan plan, DevSchedule& d) {
   return OBTE_OK;
 }
 
-template <typename Real, int NF, int G, int KV, bool FINAL, bool DF = false>
-static obte_status launch_impl(obte_plan plan, const DevSchedule& d, const double* u_in, double* u_out,
-                               bool with_src, double* Jraw, double* K, double* S) {
+// Scratch of one sweep: the plan's, or the static array's (obte_bte_sweep_static).
+template <typename Real>
+struct SweepScratch {
+  Real* vals;
+  int* err;
+  Real* xrow;
+};
+
+// The per-sweep inputs and the sweep itself (two launches).
+template <typename Real, int NF, int KV, bool FINAL, bool DF = false>
+static obte_status launch_impl(obte_plan plan, const DevSchedule& d, const SweepScratch<Real>& sc, bool plain,
+                               const double* u_in, double* u_out, bool with_src, double* Jraw, double* K, double* S) {
   const Schedule& s = plan->sched;
   cudaStream_t st = plan->stream;
-  // the double-float pass chunks the MFPs by its own thread shape (G KV per CTA), not by the tables'
-  int n_chunks = d.n_chunks;
-  size_t smem = d.smem;
-  if (DF) {
-    n_chunks = (s.n_mfp + G * KV - 1) / (G * KV);
-    smem = SmemLayout<Real>(s.nf, G * KV, d.rows, d.unit_wo, d.pf_pad, d.unit_sx, d.nbuf).total;
-    if (smem > plan->ctx->smem_optin) {
-      set_error("the double-float sweep front needs more shared memory than one CTA can have");
-      return OBTE_ERR_UNSUPPORTED;
-    }
-  }
-  const int64_t total = (int64_t)s.n_dir * s.n;
-  const int vblocks = (int)std::min<int64_t>((total + 255) / 256, (int64_t)plan->ctx->num_sms * 8);
-  sweep_values_kernel<Real><<<vblocks, 256, 0, st>>>(
-      d.cellmap.as<int32_t>(), d.Pq.as<double>(), d.spec.as<int32_t>(), d.si.as<int32_t>(),
-      d.sr.as<Real>(), u_in, s.n, s.hs.empty() ? nullptr : d.hs.as<double>(), with_src ? 1 : 0, total,
-      d.vals.as<Real>());
+  const bool subset = !plain && !FINAL && plan->sweep_cta_map != nullptr;
+  const int batch = subset && plan->sweep_batch > 1 ? plan->sweep_batch : 1;
+  PrepParams<Real> r;
+  r.cellmap = d.cellmap.as<int32_t>(); r.Pq = d.Pq.as<double>(); r.spec = d.spec.as<int32_t>();
+  r.si = d.si.as<int32_t>(); r.sr = d.sr.as<Real>(); r.hs = s.hs.empty() ? nullptr : d.hs.as<double>();
+  r.u_in = u_in; r.n = s.n; r.nd = s.nd; r.total = (int64_t)s.n_dir * s.n; r.with_src = with_src ? 1 : 0;
+  r.vals = sc.vals; r.pfe = d.pfe.as<int32_t>(); r.n_pf = d.n_pf; r.n_mfp = s.n_mfp; r.m_row = d.n_chunks * KV;
+  r.batch = batch; r.batch_stride = batch > 1 ? plan->sweep_batch_stride : 0; r.row_stride = d.row_stride;
+  r.xrow = batch > 1 ? static_cast<Real*>(plan->sweep_batch_rows) : sc.xrow;
+  r.zero0 = u_out; r.nz0 = s.n + s.nd;
+  r.zero1 = FINAL ? Jraw : nullptr; r.nz1 = FINAL ? s.n * s.ds : 0;
+  const int64_t sms = plan->ctx->num_sms;
+  r.row_blocks = (int)std::min<int64_t>((d.n_pf * batch + 7) / 8, sms * 4);
+  const int vblocks = (int)std::max<int64_t>(1, std::min<int64_t>((r.total + 255) / 256, sms * 8));
+  sweep_prep_kernel<Real, KV, DF><<<r.row_blocks + vblocks, 256, 0, st>>>(r);
   count_launch();
   OBTE_CUDA(cudaGetLastError());
-  auto kern = bte_sweep_kernel<Real, NF, G, KV, FINAL, DF>;
+  auto kern = bte_sweep_kernel<Real, NF, KV, FINAL, DF>;
   // the limit is per kernel, shared by every plan and thread: always the device maximum, so concurrent
   // plans with different footprints cannot lower it under each other's launches
   OBTE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan->ctx->smem_optin));
   SweepParams<Real> p;
   p.n = s.n; p.nd = s.nd; p.n_mfp = s.n_mfp; p.n_dir = s.n_dir; p.ds = s.ds; p.m_pad = s.m_pad;
-  p.n_chunks = n_chunks; p.rows = d.rows; p.S = s.max_slots;
-  p.emax = d.emax; p.unit_wo = d.unit_wo; p.pf_pad = d.pf_pad; p.nbuf = d.nbuf;
-  p.rec = d.rec.as<int32_t>(); p.vals = d.vals.as<Real>();
-  p.lev_ptr = d.klev_ptr.as<int32_t>(); p.lev_off = d.klev_off.as<int64_t>(); p.nlev = d.knlev.as<int32_t>();
-  p.kwo = d.kwo.as<int32_t>(); p.kpf = d.kpf.as<int32_t>(); p.pf = d.pf.as<int32_t>();
-  p.ksx = d.ksx.as<int32_t>(); p.sx = d.sx.as<int32_t>(); p.unit_sx = d.unit_sx;
-  p.x_base = plan->x_base_dev.as<int64_t>();
-  p.wo_off = d.wo_off.as<int32_t>();
-  p.wo_wall = d.wo_wall.as<int32_t>();
-  p.mfp = d.mfp.as<Real>(); p.tco = d.tco.as<Real>(); p.sig = d.sig.as<Real>(); p.wo_geo = d.wo_geo.as<Real>();
+  p.n_chunks = d.n_chunks; p.zero_row = s.max_slots; p.prow0 = d.prow0; p.emax = d.emax; p.nbuf = d.nbuf;
+  p.stage0 = d.stage0; p.stage = d.stage; p.out0 = d.out0; p.out = d.out; p.val_off = d.val_off; p.gain_off = d.gain_off;
+  p.blk = d.blk.as<int32_t>(); p.desc = d.desc.as<int32_t>(); p.unit_base = d.unit_base.as<int64_t>();
+  p.vals = sc.vals; p.xrow = r.xrow;
+  p.mfp = d.mfp.as<Real>(); p.tco = d.tco.as<Real>(); p.sig = d.sig.as<Real>();
   p.kcoef = d.kcoef.as<Real>(); p.scoef = d.scoef.as<Real>();
-  p.u_in = u_in; p.u_out = u_out; p.Jraw = Jraw; p.K = K; p.S_out = S;
-  p.err = plan->err.as<int>();
-  p.rinv = (sizeof(Real) == 8 && !DF) ? d.rinv.as<double>() : nullptr;
+  p.u_out = u_out; p.Jraw = Jraw; p.K = K; p.S_out = S;
+  p.err = sc.err;
+  p.gain = (sizeof(Real) == 8 && !DF) ? d.gain.as<double>() : nullptr;
   p.Xs = FINAL ? plan->xstore : nullptr;
   p.xs_add = plan->xstore_add ? 1 : 0;
   p.Xd = FINAL ? plan->xstore64 : nullptr;
-  p.skip_unit = plan->test_skip_unit;
-  p.wait_limit = plan->test_wait_limit > 0 ? plan->test_wait_limit : kWaitPolls;
-  const bool subset = !FINAL && plan->sweep_cta_map != nullptr;
+  p.skip_unit = plain ? -1 : plan->test_skip_unit;
+  p.wait_limit = !plain && plan->test_wait_limit > 0 ? plan->test_wait_limit : kWaitPolls;
   // deterministic reductions: full sweeps of the FP32 and FP64 kernels (not the probes' subset sweeps, not the
   // double-float pass)
-  const bool det = deterministic() && !subset && !DF;
+  const bool det = !plain && deterministic() && !subset && !DF;
   p.det = det ? 1 : 0;
   p.dpart = p.jpart = p.wpart = p.kpart = p.spart = nullptr;
   p.n_wo = (int64_t)s.wo_wall.size();
@@ -1695,20 +1932,19 @@ static obte_status launch_impl(obte_plan plan, const DevSchedule& d, const doubl
     p.spart = d.det_s.as<Real>();
   }
   static const bool index_order = std::getenv("OBTE_SWEEP_NO_LPT") != nullptr;   // plain index order
-  // (the double-float pass runs in index order: the launch order table belongs to the tables' chunking)
   p.cta_map = subset ? plan->sweep_cta_map : (index_order || DF ? nullptr : d.lpt.as<int32_t>());
-  const int batch = subset && plan->sweep_batch > 1 ? plan->sweep_batch : 1;
-  p.n_cta_batch = subset ? plan->sweep_n_cta : 0;
-  p.batch_stride = batch > 1 ? plan->sweep_batch_stride : 0;
-  const int grid = subset ? plan->sweep_n_cta * batch : s.n_dir * n_chunks;
-  kern<<<grid, kUnit * G, smem, st>>>(p);
+  p.n_cta_batch = batch > 1 ? plan->sweep_n_cta : 0;
+  p.batch_stride = r.batch_stride;
+  p.row_stride = batch > 1 ? d.row_stride : 0;
+  const int grid = subset ? plan->sweep_n_cta * batch : s.n_dir * d.n_chunks;
+  kern<<<grid, FINAL ? kMaxThreads : d.threads, d.smem, st>>>(p);
   count_launch();
   OBTE_CUDA(cudaGetLastError());
   if (det) {
     const int nb = plan->ctx->num_sms * 8;
     const int64_t total = (int64_t)s.n_dir * s.n;
     det_pos_sum_kernel<Real><<<(int)std::min<int64_t>((total + 255) / 256, nb), 256, 0, st>>>(
-        d.det_d.as<Real>(), FINAL ? d.det_j.as<Real>() : nullptr, n_chunks, s.n, total, s.ds, d.det_S.as<double>(),
+        d.det_d.as<Real>(), FINAL ? d.det_j.as<Real>() : nullptr, d.n_chunks, s.n, total, s.ds, d.det_S.as<double>(),
         d.det_SJ.as<double>());
     det_elem_sum_kernel<<<(int)std::min<int64_t>((s.n + 255) / 256, nb), 256, 0, st>>>(
         d.det_S.as<double>(), FINAL ? d.det_SJ.as<double>() : nullptr, plan->det_inv.as<int32_t>(), s.n_dir, s.n, s.ds,
@@ -1716,7 +1952,7 @@ static obte_status launch_impl(obte_plan plan, const DevSchedule& d, const doubl
     count_launch(2);
     if (s.nd > 0) {
       det_wall_sum_kernel<Real><<<(int)std::min<int64_t>((s.nd + 255) / 256, nb), 256, 0, st>>>(
-          d.det_w.as<Real>(), n_chunks, p.n_wo, plan->det_wptr.as<int32_t>(), plan->det_went.as<int32_t>(), s.nd,
+          d.det_w.as<Real>(), d.n_chunks, p.n_wo, plan->det_wptr.as<int32_t>(), plan->det_went.as<int32_t>(), s.nd,
           u_out + s.n);
       count_launch();
     }
@@ -1731,52 +1967,58 @@ static obte_status launch_impl(obte_plan plan, const DevSchedule& d, const doubl
   return OBTE_OK;
 }
 
-template <typename Real, int G, int KV>
-static obte_status launch_w(obte_plan plan, const DevSchedule& d, const double* u_in, double* u_out, bool with_src,
-                            bool final_pass, double* Jraw, double* K, double* S) {
+template <typename Real, int KV>
+static obte_status launch_kv(obte_plan plan, const DevSchedule& d, const SweepScratch<Real>& sc, bool plain,
+                             const double* u_in, double* u_out, bool with_src, bool final_pass, double* Jraw, double* K,
+                             double* S) {
   if (plan->sched.nf == 3) {
-    if (final_pass) return launch_impl<Real, 3, G, KV, true>(plan, d, u_in, u_out, with_src, Jraw, K, S);
-    return launch_impl<Real, 3, G, KV, false>(plan, d, u_in, u_out, with_src, Jraw, K, S);
+    if (final_pass) return launch_impl<Real, 3, KV, true>(plan, d, sc, plain, u_in, u_out, with_src, Jraw, K, S);
+    return launch_impl<Real, 3, KV, false>(plan, d, sc, plain, u_in, u_out, with_src, Jraw, K, S);
   }
-  if (final_pass) return launch_impl<Real, 4, G, KV, true>(plan, d, u_in, u_out, with_src, Jraw, K, S);
-  return launch_impl<Real, 4, G, KV, false>(plan, d, u_in, u_out, with_src, Jraw, K, S);
+  if (final_pass) return launch_impl<Real, 4, KV, true>(plan, d, sc, plain, u_in, u_out, with_src, Jraw, K, S);
+  return launch_impl<Real, 4, KV, false>(plan, d, sc, plain, u_in, u_out, with_src, Jraw, K, S);
+}
+
+// plain: no test hook, no deterministic reductions, every CTA (obte_bte_sweep_static)
+template <typename Real>
+static obte_status launch_shape(obte_plan plan, const DevSchedule& d, const SweepScratch<Real>& sc, bool plain,
+                                const double* u_in, double* u_out, bool with_src, bool final_pass, double* Jraw,
+                                double* K, double* S) {
+  constexpr int N = 16 / (int)sizeof(Real);
+  if (d.mc == N) return launch_kv<Real, N>(plan, d, sc, plain, u_in, u_out, with_src, final_pass, Jraw, K, S);
+  return launch_kv<Real, 2 * N>(plan, d, sc, plain, u_in, u_out, with_src, final_pass, Jraw, K, S);
+}
+
+static obte_status check_shape(const Schedule& s) {
+  if (s.ds > 3) { set_error("sigma with more than 3 components"); return OBTE_ERR_UNSUPPORTED; }
+  if (s.nf > 4) { set_error("elements with more than 4 sides are not supported"); return OBTE_ERR_UNSUPPORTED; }
+  return OBTE_OK;
 }
 
 obte_status launch_sweep(obte_plan plan, bool fp32, const double* u_in, double* u_out, bool with_src,
                          bool final_pass, double* Jraw, double* K, double* S) {
   OBTE_TRY(ensure_tables(plan, fp32));
-  const Schedule& s = plan->sched;
-  cudaStream_t st = plan->stream;
-  if (s.ds > 3) { set_error("sigma with more than 3 components"); return OBTE_ERR_UNSUPPORTED; }
-  if (s.nf > 4) { set_error("elements with more than 4 sides are not supported"); return OBTE_ERR_UNSUPPORTED; }
-  OBTE_CUDA(cudaMemsetAsync(u_out, 0, (size_t)(s.n + s.nd) * sizeof(double), st));
-  if (final_pass) OBTE_CUDA(cudaMemsetAsync(Jraw, 0, (size_t)s.n * s.ds * sizeof(double), st));
-  const DevSchedule& d = fp32 ? plan->d32 : plan->d64;
-#define OBTE_W(R, GG, KK) \
-  if (d.G == GG && d.KV == KK) return launch_w<R, GG, KK>(plan, d, u_in, u_out, with_src, final_pass, Jraw, K, S)
-  if (fp32) {
-    OBTE_W(float, 1, 4); OBTE_W(float, 1, 8); OBTE_W(float, 2, 4); OBTE_W(float, 1, 2);
-  } else {
-    OBTE_W(double, 1, 2); OBTE_W(double, 1, 4); OBTE_W(double, 2, 2);
-  }
-#undef OBTE_W
-  set_error("no compiled sweep kernel for this thread shape");
-  return OBTE_ERR_UNSUPPORTED;
+  OBTE_TRY(check_shape(plan->sched));
+  if (fp32)
+    return launch_shape<float>(plan, plan->d32, {plan->d32.vals.as<float>(), plan->err.as<int>(), plan->d32.xrow.as<float>()},
+                               false, u_in, u_out, with_src, final_pass, Jraw, K, S);
+  return launch_shape<double>(plan, plan->d64, {plan->d64.vals.as<double>(), plan->err.as<int>(), plan->d64.xrow.as<double>()},
+                              false, u_in, u_out, with_src, final_pass, Jraw, K, S);
 }
 
 // The output pass in double-float arithmetic on the FP64 tables (J, K and S accumulated like a final pass).
 obte_status launch_sweep_df(obte_plan plan, const double* u_in, double* u_out, bool with_src, double* Jraw, double* K,
                             double* S) {
   OBTE_TRY(ensure_tables(plan, false));
-  const Schedule& s = plan->sched;
-  cudaStream_t st = plan->stream;
-  if (s.ds > 3) { set_error("sigma with more than 3 components"); return OBTE_ERR_UNSUPPORTED; }
-  if (s.nf > 4) { set_error("elements with more than 4 sides are not supported"); return OBTE_ERR_UNSUPPORTED; }
-  OBTE_CUDA(cudaMemsetAsync(u_out, 0, (size_t)(s.n + s.nd) * sizeof(double), st));
-  OBTE_CUDA(cudaMemsetAsync(Jraw, 0, (size_t)s.n * s.ds * sizeof(double), st));
+  OBTE_TRY(check_shape(plan->sched));
   const DevSchedule& d = plan->d64;
-  if (s.nf == 3) return launch_impl<double, 3, 1, 4, true, true>(plan, d, u_in, u_out, with_src, Jraw, K, S);
-  return launch_impl<double, 4, 1, 4, true, true>(plan, d, u_in, u_out, with_src, Jraw, K, S);
+  const SweepScratch<double> sc{d.vals.as<double>(), plan->err.as<int>(), d.xrow.as<double>()};
+  if (d.mc == 2) {
+    if (plan->sched.nf == 3) return launch_impl<double, 3, 2, true, true>(plan, d, sc, false, u_in, u_out, with_src, Jraw, K, S);
+    return launch_impl<double, 4, 2, true, true>(plan, d, sc, false, u_in, u_out, with_src, Jraw, K, S);
+  }
+  if (plan->sched.nf == 3) return launch_impl<double, 3, 4, true, true>(plan, d, sc, false, u_in, u_out, with_src, Jraw, K, S);
+  return launch_impl<double, 4, 4, true, true>(plan, d, sc, false, u_in, u_out, with_src, Jraw, K, S);
 }
 
 // Device error word: nonzero after a bounded wait gave up (cleared on read).
@@ -1792,7 +2034,6 @@ obte_status check_device_error(obte_plan plan) {
   }
   return OBTE_OK;
 }
-
 }  // namespace obte
 
 // ---- sweep on library-owned static scratch ---------------------------------------------
@@ -1838,85 +2079,21 @@ static obte_status static_scratch_address(int device, void** out) {
   return OBTE_OK;
 }
 
-template <typename Real, int NF, int G, int KV>
-static obte_status launch_static_impl(obte_plan plan, const DevSchedule& d, const double* u_in, double* u_out,
-                                      bool with_src, Real* vals, int* err) {
-  const Schedule& s = plan->sched;
-  cudaStream_t st = plan->stream;
-  const int64_t total = (int64_t)s.n_dir * s.n;
-  const int vblocks = (int)std::min<int64_t>((total + 255) / 256, (int64_t)plan->ctx->num_sms * 8);
-  sweep_values_kernel<Real><<<vblocks, 256, 0, st>>>(
-      d.cellmap.as<int32_t>(), d.Pq.as<double>(), d.spec.as<int32_t>(), d.si.as<int32_t>(), d.sr.as<Real>(), u_in,
-      s.n, s.hs.empty() ? nullptr : d.hs.as<double>(), with_src ? 1 : 0, total, vals);
-  count_launch();
-  OBTE_CUDA(cudaGetLastError());
-  auto kern = bte_sweep_kernel<Real, NF, G, KV, false>;
-  OBTE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan->ctx->smem_optin));
-  SweepParams<Real> p;
-  p.n = s.n; p.nd = s.nd; p.n_mfp = s.n_mfp; p.n_dir = s.n_dir; p.ds = s.ds; p.m_pad = s.m_pad;
-  p.n_chunks = d.n_chunks; p.rows = d.rows; p.S = s.max_slots;
-  p.emax = d.emax; p.unit_wo = d.unit_wo; p.pf_pad = d.pf_pad; p.nbuf = d.nbuf;
-  p.rec = d.rec.as<int32_t>(); p.vals = vals;
-  p.lev_ptr = d.klev_ptr.as<int32_t>(); p.lev_off = d.klev_off.as<int64_t>(); p.nlev = d.knlev.as<int32_t>();
-  p.kwo = d.kwo.as<int32_t>(); p.kpf = d.kpf.as<int32_t>(); p.pf = d.pf.as<int32_t>();
-  p.ksx = d.ksx.as<int32_t>(); p.sx = d.sx.as<int32_t>(); p.unit_sx = d.unit_sx;
-  p.x_base = plan->x_base_dev.as<int64_t>();
-  p.wo_off = d.wo_off.as<int32_t>();
-  p.wo_wall = d.wo_wall.as<int32_t>();
-  p.mfp = d.mfp.as<Real>(); p.tco = d.tco.as<Real>(); p.sig = d.sig.as<Real>(); p.wo_geo = d.wo_geo.as<Real>();
-  p.kcoef = d.kcoef.as<Real>(); p.scoef = d.scoef.as<Real>();
-  p.u_in = u_in; p.u_out = u_out; p.Jraw = nullptr; p.K = nullptr; p.S_out = nullptr;
-  p.err = err;
-  p.Xs = nullptr;
-  p.xs_add = 0;
-  p.rinv = nullptr;
-  p.Xd = nullptr;
-  // the launch order of obte_bte_sweep: longest chains first (FP32 tables), unless OBTE_SWEEP_NO_LPT is set
-  static const bool index_order = std::getenv("OBTE_SWEEP_NO_LPT") != nullptr;
-  p.cta_map = index_order ? nullptr : d.lpt.as<int32_t>();
-  p.n_cta_batch = 0;
-  p.batch_stride = 0;
-  p.skip_unit = -1;
-  p.wait_limit = kWaitPolls;
-  p.det = 0;
-  p.dpart = p.jpart = p.wpart = p.kpart = p.spart = nullptr;
-  p.n_wo = 0;
-  kern<<<s.n_dir * d.n_chunks, kUnit * G, d.smem, st>>>(p);
-  count_launch();
-  OBTE_CUDA(cudaGetLastError());
-  return OBTE_OK;
-}
-
-template <typename Real, int G, int KV>
-static obte_status launch_static_w(obte_plan plan, const DevSchedule& d, const double* u_in, double* u_out,
-                                   bool with_src, Real* vals, int* err) {
-  if (plan->sched.nf == 3) return launch_static_impl<Real, 3, G, KV>(plan, d, u_in, u_out, with_src, vals, err);
-  return launch_static_impl<Real, 4, G, KV>(plan, d, u_in, u_out, with_src, vals, err);
-}
-
 // Runs with the plan's device current; the caller restores its own.
 static obte_status sweep_static_on_device(obte_plan plan, bool fp32, const double* u_in, double* u_out,
                                           bool with_src) {
-  const Schedule& s = plan->sched;
-  const DevSchedule& d = fp32 ? plan->d32 : plan->d64;
   cudaStream_t st = plan->stream;
   void* base = nullptr;
   OBTE_TRY(static_scratch_address(plan->ctx->device, &base));
   int* err = static_cast<int*>(base);
   void* vals = static_cast<unsigned char*>(base) + kStaticValsOffset;
   OBTE_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
-  OBTE_CUDA(cudaMemsetAsync(u_out, 0, (size_t)(s.n + s.nd) * sizeof(double), st));
-  obte_status rc = OBTE_ERR_UNSUPPORTED;
-#define OBTE_SW(R, GG, KK) \
-  if (d.G == GG && d.KV == KK) rc = launch_static_w<R, GG, KK>(plan, d, u_in, u_out, with_src, static_cast<R*>(vals), err)
-  if (fp32) {
-    OBTE_SW(float, 1, 4); else OBTE_SW(float, 1, 8); else OBTE_SW(float, 2, 4); else OBTE_SW(float, 1, 2);
-  } else {
-    OBTE_SW(double, 1, 2); else OBTE_SW(double, 1, 4); else OBTE_SW(double, 2, 2);
-  }
-#undef OBTE_SW
-  if (rc == OBTE_ERR_UNSUPPORTED) set_error("no compiled sweep kernel for this thread shape");
-  if (rc != OBTE_OK) return rc;
+  if (fp32)
+    OBTE_TRY(launch_shape<float>(plan, plan->d32, {static_cast<float*>(vals), err, plan->d32.xrow.as<float>()}, true, u_in,
+                                 u_out, with_src, false, nullptr, nullptr, nullptr));
+  else
+    OBTE_TRY(launch_shape<double>(plan, plan->d64, {static_cast<double*>(vals), err, plan->d64.xrow.as<double>()}, true,
+                                  u_in, u_out, with_src, false, nullptr, nullptr, nullptr));
   int h = 0;
   OBTE_CUDA(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, st));
   OBTE_CUDA(cudaStreamSynchronize(st));

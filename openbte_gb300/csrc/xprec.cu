@@ -230,8 +230,11 @@ int64_t xprec_build_bound(obte_plan plan) {
   const int64_t nu = plan->nu;
   // W (capped), per-block tables (at most one block per ordinate, every block's slots at most its
   // direction's), detection norms, CTA map, the batched probe vectors (16 pairs or 2 GB at most)
+  // and the batch's periodic inflow rows (one per cut inflow face)
   const int64_t probes = std::min<int64_t>(16 * 2 * nu * (int64_t)sizeof(double), (int64_t)2e9);
-  return (int64_t)max_bytes() + nord * (4 + 4 + 8 + 8 + 4 + 16 + 4) + nsrc * s.n_mfp * 4 + probes;
+  const int64_t nbat = std::max<int64_t>(1, probes / (16 * std::max<int64_t>(nu, 1)));
+  const int64_t rows = nbat * s.n_cut * ((s.n_mfp + 7) & ~7) * 4;
+  return (int64_t)max_bytes() + nord * (4 + 4 + 8 + 8 + 4 + 16 + 4) + nsrc * s.n_mfp * 4 + probes + rows;
 }
 
 obte_status ensure_xprec(obte_plan plan, SolveWork& wk) {
@@ -376,6 +379,9 @@ obte_status ensure_xprec(obte_plan plan, SolveWork& wk) {
   OBTE_TRY(xb.alloc((size_t)nbat * nu * sizeof(double)));
   OBTE_TRY(yb.alloc((size_t)nbat * nu * sizeof(double)));
   OBTE_CUDA(cudaMemsetAsync(xb.p, 0, (size_t)nbat * nu * sizeof(double), st));
+  DevBuf rows;                    // periodic inflow rows of a batch
+  OBTE_TRY(rows.alloc(std::max<size_t>((size_t)nbat * d.row_stride * sizeof(float), 32)));
+  plan->sweep_batch_rows = rows.p;
   plan->sweep_cta_map = cmap.as<int32_t>();
   plan->sweep_n_cta = (int)ctas.size();
   plan->sweep_batch_stride = nu;
@@ -401,6 +407,7 @@ obte_status ensure_xprec(obte_plan plan, SolveWork& wk) {
   plan->sweep_n_cta = 0;
   plan->sweep_batch = 1;
   plan->sweep_batch_stride = 0;
+  plan->sweep_batch_rows = nullptr;
   OBTE_TRY(ps);
   P.probe_sweeps = launches;
   // 3. (I - T)^-1 - I per block
