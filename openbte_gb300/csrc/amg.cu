@@ -19,8 +19,8 @@
 // G = w D^-1 (2 I - w A D^-1) (symmetric, A's pattern),
 //   b_c = Q^T b    and    x = G b + Q x_c,
 // so the device applies one sparse product per level on the way down and one on the way up, plus one dense
-// product with the coarsest inverse: 2 (levels - 1) + 1 launches per V-cycle instead of 6 per level.  The
-// launches are enqueued on a stream and are therefore capturable in a CUDA graph.
+// product with the coarsest inverse: 2 (levels - 1) + 1 launches per V-cycle instead of 6 per level (amg_apply),
+// or as many phases inside a larger kernel (grid.cuh).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,7 +28,7 @@
 #include <cstdlib>
 #include <vector>
 
-#include "internal.h"
+#include "grid.cuh"
 
 namespace obte {
 
@@ -251,19 +251,18 @@ bool dense_inverse(const HostCsr& A, std::vector<double>& inv) {
 // ---- device V-cycle ----------------------------------------------------------------------------
 
 // y = G gx + Q qx (G optional) with VEC lanes per row (lane-strided products, then an xor tree: a fixed
-// summation order); with `part`, block partials of gx . y as well.  Every thread runs the same number of
-// row passes, so the group shuffles always see full warps.
+// summation order).  Every thread runs the same number of row passes, so the group shuffles always see full
+// warps.
 template <int VEC>
 __global__ void __launch_bounds__(AT) amg_rows_kernel(
     int64_t n, const int32_t* __restrict__ grp, const int32_t* __restrict__ gci, const double* __restrict__ gv,
     const double* __restrict__ gx, const int32_t* __restrict__ qrp, const int32_t* __restrict__ qci,
-    const double* __restrict__ qv, const double* __restrict__ qx, double* __restrict__ y, double* __restrict__ part) {
+    const double* __restrict__ qv, const double* __restrict__ qx, double* __restrict__ y) {
   constexpr int GPB = AT / VEC;
   const int lane = (int)(threadIdx.x % VEC);
   const int64_t stride = (int64_t)gridDim.x * GPB;
   const int64_t first = (int64_t)blockIdx.x * GPB + threadIdx.x / VEC;
   const int64_t trips = (n + stride - 1) / stride;
-  double dot = 0;
   for (int64_t t = 0; t < trips; ++t) {
     const int64_t row = first + t * stride;
     double acc = 0;
@@ -274,21 +273,7 @@ __global__ void __launch_bounds__(AT) amg_rows_kernel(
     }
 #pragma unroll
     for (int o = VEC / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (row < n && lane == 0) {
-      y[row] = acc;
-      if (part) dot += gx[row] * acc;
-    }
-  }
-  if (part) {
-    __shared__ double red[AT / 32];
-    for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = dot;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0;
-      for (int w = 0; w < AT / 32; ++w) t += red[w];
-      part[blockIdx.x] = t;
-    }
+    if (row < n && lane == 0) y[row] = acc;
   }
 }
 
@@ -301,22 +286,6 @@ __global__ void amg_coarse_kernel(int n, const double* __restrict__ inv, const d
     for (int k = lane; k < n; k += 32) s += inv[(size_t)row * n + k] * b[k];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) x[row] = s;
-  }
-}
-
-// block partials of r . z (a one-level hierarchy has no up-sweep product to carry them)
-__global__ void amg_dot_kernel(int64_t n, const double* __restrict__ r, const double* __restrict__ z,
-                               double* __restrict__ part) {
-  __shared__ double red[AT / 32];
-  double dot = 0;
-  for (int64_t i = (int64_t)blockIdx.x * AT + threadIdx.x; i < n; i += (int64_t)gridDim.x * AT) dot += r[i] * z[i];
-  for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = dot;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0;
-    for (int w = 0; w < AT / 32; ++w) t += red[w];
-    part[blockIdx.x] = t;
   }
 }
 
@@ -427,28 +396,40 @@ obte_status amg_build(int64_t n, const std::vector<int32_t>& rp, const std::vect
   return OBTE_OK;
 }
 
-int amg_levels(const AmgHierarchy& H) { return (int)H.lv.size(); }
-int amg_launches(const AmgHierarchy& H, bool with_part) {
+// The hierarchy as a kernel reads it (one level: only the dense inverse).
+void amg_device(const AmgHierarchy& H, AmgDev& d) {
   const int nl = (int)H.lv.size();
-  return 2 * (nl - 1) + 1 + (with_part && nl == 1 ? 1 : 0);
+  d.nl = nl;
+  d.nc = H.nc;
+  d.inv = H.inv.as<double>();
+  auto csr = [](const DevCsr& m) { return CsrDev{m.n, m.rp.as<int32_t>(), m.ci.as<int32_t>(), m.val.as<double>()}; };
+  for (int l = 0; l < nl; ++l) {
+    const AmgLevel& L = *H.lv[l];
+    d.b[l] = l ? L.b.as<double>() : nullptr;
+    d.x[l] = l ? L.x.as<double>() : nullptr;
+    if (l + 1 < nl) {
+      d.G[l] = csr(L.G);
+      d.Q[l] = csr(L.Q);
+      d.Qt[l] = csr(L.Qt);
+    }
+  }
 }
 
+int amg_levels(const AmgHierarchy& H) { return (int)H.lv.size(); }
 namespace {
-// y = G gx + Q qx over n rows, lanes per row from the mean row length; `grid` > 0 fixes the grid (and is
-// then the number of partials written to `part`)
-void rows_launch(const DevCsr* G, const double* gx, const DevCsr& Q, const double* qx, double* y, double* part,
-                 int grid, int num_sms, cudaStream_t st) {
+// y = G gx + Q qx over n rows, lanes per row from the mean row length
+void rows_launch(const DevCsr* G, const double* gx, const DevCsr& Q, const double* qx, double* y, int num_sms,
+                 cudaStream_t st) {
   const int64_t n = Q.n;
   const double mean = (double)(Q.nnz + (G ? G->nnz : 0)) / (double)std::max<int64_t>(n, 1);
   const int vec = mean < 6 ? 1 : mean < 12 ? 2 : mean < 24 ? 4 : mean < 48 ? 8 : mean < 96 ? 16 : 32;
-  const int blocks = grid > 0 ? grid
-                              : (int)std::max<int64_t>(1, std::min<int64_t>((n * vec + AT - 1) / AT, (int64_t)num_sms * 8));
+  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((n * vec + AT - 1) / AT, (int64_t)num_sms * 8));
   const int32_t* grp = G ? G->rp.as<int32_t>() : nullptr;
   const int32_t* gci = G ? G->ci.as<int32_t>() : nullptr;
   const double* gv = G ? G->val.as<double>() : nullptr;
 #define OBTE_AMG_ROWS(V)                                                                                       \
   amg_rows_kernel<V><<<blocks, AT, 0, st>>>(n, grp, gci, gv, gx, Q.rp.as<int32_t>(), Q.ci.as<int32_t>(),      \
-                                            Q.val.as<double>(), qx, y, part)
+                                            Q.val.as<double>(), qx, y)
   switch (vec) {
     case 1: OBTE_AMG_ROWS(1); break;
     case 2: OBTE_AMG_ROWS(2); break;
@@ -461,24 +442,22 @@ void rows_launch(const DevCsr* G, const double* gx, const DevCsr& Q, const doubl
 }
 }  // namespace
 
-// z = M^-1 r (level 0 reads r and writes z directly); with `part`, the nb_part block partials of r . z
-int amg_apply(const AmgHierarchy& H, const double* r, double* z, double* part, int nb_part, cudaStream_t st) {
+// z = M^-1 r (level 0 reads r and writes z directly); the number of launches
+int amg_apply(const AmgHierarchy& H, const double* r, double* z, cudaStream_t st) {
   const int nl = (int)H.lv.size();
   auto bvec = [&](int l) { return l == 0 ? r : H.lv[l]->b.as<double>(); };
   auto xvec = [&](int l) { return l == 0 ? z : H.lv[l]->x.as<double>(); };
   for (int l = 0; l < nl - 1; ++l)                        // b_l+1 = Q_l^T b_l
-    rows_launch(nullptr, nullptr, H.lv[l]->Qt, bvec(l), H.lv[l + 1]->b.as<double>(), nullptr, 0, H.num_sms, st);
+    rows_launch(nullptr, nullptr, H.lv[l]->Qt, bvec(l), H.lv[l + 1]->b.as<double>(), H.num_sms, st);
   {
     const int blocks = std::max(1, std::min(1024, (H.nc * 32 + AT - 1) / AT));
     amg_coarse_kernel<<<blocks, AT, 0, st>>>(H.nc, H.inv.as<double>(), bvec(nl - 1), xvec(nl - 1));
   }
   for (int l = nl - 2; l >= 0; --l) {                     // x_l = G_l b_l + Q_l x_l+1
     const AmgLevel& L = *H.lv[l];
-    rows_launch(&L.G, bvec(l), L.Q, xvec(l + 1), xvec(l), l == 0 ? part : nullptr, l == 0 && part ? nb_part : 0,
-                H.num_sms, st);
+    rows_launch(&L.G, bvec(l), L.Q, xvec(l + 1), xvec(l), H.num_sms, st);
   }
-  if (part && nl == 1) amg_dot_kernel<<<nb_part, AT, 0, st>>>(H.lv[0]->n, r, z, part);
-  return amg_launches(H, part != nullptr);
+  return 2 * (nl - 1) + 1;
 }
 
 }  // namespace obte

@@ -316,11 +316,11 @@ void dsa_add(obte_plan plan, const double* in, double* out) {
   dsa_restrict_kernel<<<gn, DT, 0, st>>>(n, op.vol.as<double>(), op.inv_vol_sum, op.project ? part : nullptr, gn,
                                          in, b);
   count_launch();
-  count_launch(amg_apply(*op.amg, b, d, nullptr, 0, st));
+  count_launch(amg_apply(*op.amg, b, d, st));
   for (int c = 1; c < op.cycles; ++c) {
     dsa_residual_kernel<<<gn, DT, 0, st>>>(n, op.rp.as<int32_t>(), op.ci.as<int32_t>(), op.val.as<double>(), b, d,
                                            op.r.as<double>());
-    count_launch(amg_apply(*op.amg, op.r.as<double>(), op.e.as<double>(), nullptr, 0, st));
+    count_launch(amg_apply(*op.amg, op.r.as<double>(), op.e.as<double>(), st));
     dsa_axpy_kernel<<<gn, DT, 0, st>>>(n, op.e.as<double>(), d);
     count_launch(2);
   }

@@ -12,8 +12,7 @@
 // value is moved to the right-hand side and CG runs on the remaining SPD
 // system.  The least-squares gradient (openbte/objects.py:322-405), the
 // correction gather and the diffusive kappa (openbte/objects.py:139-172) are
-// kernels; CG keeps alpha/beta on the device and the host only reads the
-// residual every few iterations.
+// device code too: the whole solve after assembly is one launch.
 #include <cuda_runtime.h>
 
 #include <cstdlib>
@@ -23,335 +22,267 @@
 #include <map>
 #include <vector>
 
-#include "internal.h"
+#include "grid.cuh"
 
 namespace obte {
 namespace {
 
 constexpr int FT = 256;
 
-__global__ void spmv_kernel(int64_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
-                            const double* __restrict__ v, const double* __restrict__ x, double* __restrict__ y,
-                            double* __restrict__ part) {
-  __shared__ double red[FT / 32];
-  double acc = 0;
-  for (int64_t i = (int64_t)blockIdx.x * FT + threadIdx.x; i < n; i += (int64_t)gridDim.x * FT) {
-    double s = 0;
-    for (int k = rp[i]; k < rp[i + 1]; ++k) s += v[k] * x[ci[k]];
-    y[i] = s;
-    acc += s * x[i];
-  }
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0;
-    for (int w = 0; w < FT / 32; ++w) t += red[w];
-    part[blockIdx.x] = t;
-  }
-}
+// Everything of the solve after assembly, for the one launch that runs it.
+struct FourierParams {
+  int64_t n;
+  CsrDev A;                                  // L
+  int has_amg;
+  AmgDev amg;
+  const double *dinv, *vol, *B, *colpin;
+  int pin, nv, dim;
+  const int32_t* g_nb;                       // gradient stencils
+  const double* g_off;
+  const unsigned char* g_mixed;
+  const double* gw;
+  const int32_t *s_i, *s_j;                  // internal sides
+  const double *s_w, *s_vnon;
+  const int32_t *c_ptr, *c_side;
+  double *T, *C, *r[2], *z, *p[2], *Ap, *grad, *part;
+  int max_iter, cg_max, check;
+  double rtol, cg_rtol;
+  double* out;                               // deferred corrections, CG iterations
+  unsigned* count;
+  int* err;
+};
 
-// scalars: [0] rz  [1] pAp  [2] rz_new  [3] rr
-__global__ void reduce_kernel(const double* __restrict__ part, int nb, double* __restrict__ dst) {
-  __shared__ double red[FT / 32];
-  double acc = 0;
-  for (int b = threadIdx.x; b < nb; b += FT) acc += part[b];
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0;
-    for (int w = 0; w < FT / 32; ++w) t += red[w];
-    *dst = t;
+// The deferred-correction loop (fourier.py:145-178) with its preconditioned CG solves, one launch.  Phases end at
+// a barrier over the blocks; scalars are sums of per-block partials that every block adds up itself, in a
+// fixed order.  A CG iteration takes one barrier for the product with the direction, one for the residual and
+// its restriction (both formed in the gather), and those of the V-cycle; the directions and residuals
+// alternate between two buffers so that neighbours read the values of the phase before.
+//
+// The solve was bound by its launches (60k triangles: 10 corrections, 184 CG iterations, 2,180 launches of 4.6 us
+// with their gaps, 13.3 ms; 600 triangles 6.9 ms).  Its matrices stay in shared memory (60k triangles: 85 KB
+// an SM), so what is left of a phase is the barrier, one gather through L2 and a chain of FP64
+// operations at 64-76 cycles each: 8.8 and 2.9 ms.
+template <typename Bar>
+__global__ void __launch_bounds__(kPhaseThreads, 1) fourier_kernel(const __grid_constant__ FourierParams P) {
+  extern __shared__ __align__(16) char smem[];
+  __shared__ double red[kPhaseThreads];
+  __shared__ Rows sA;
+  __shared__ AmgRows sM;
+  Bar bar(P.count, P.err);
+  const int tid = threadIdx.x, nthr = blockDim.x, nb = gridDim.x;
+  Arena ar{smem, kPhaseSmem};
+  load_rows(P.A, &sA, ar);
+  if (P.has_amg) load_amg(P.amg, &sM, ar);
+  int r0, r1;
+  block_range(P.n, r0, r1);
+  // partials: one row of nb per sum
+  double *p_pap = P.part, *p_rr = P.part + nb, *p_rz = P.part + 2 * nb, *p_bb = P.part + 3 * nb, *p_mx = P.part + 4 * nb,
+         *p_mn = P.part + 5 * nb, *p_cc = P.part + 6 * nb;
+  auto put_slot = [&](double v, int slot, int count, double* row) {
+    const double s = block_sum(v, slot, count, red);
+    if (tid == 0) row[blockIdx.x] = s;
+  };
+  const int own = min(r1 - r0, nthr);
+  auto put = [&](double v, double* row) { put_slot(v, tid < own ? tid : -1, own, row); };      // rows by thread
+  auto put_rows = [&](double v, int vec, double* row) {                                      // of block_rows
+    put_slot(v, tid % vec == 0 ? tid / vec : -1, min(r1 - r0, nthr / vec), row);
+  };
+  for (int i = r0 + tid; i < r1; i += nthr) {
+    P.T[i] = 0.0;
+    P.C[i] = 0.0;
   }
-}
-
-// x += a p; r -= a Ap; z = r * dinv; partials of r.z and r.r
-__global__ void cg_update_kernel(int64_t n, const double* __restrict__ sc, double* __restrict__ x,
-                                 double* __restrict__ r, double* __restrict__ z, const double* __restrict__ p,
-                                 const double* __restrict__ Ap, const double* __restrict__ dinv,
-                                 double* __restrict__ part_rz, double* __restrict__ part_rr) {
-  __shared__ double red[2][FT / 32];
-  const double pap = sc[1];
-  const double a = pap != 0 ? sc[0] / pap : 0.0;
-  double rz = 0, rr = 0;
-  for (int64_t i = (int64_t)blockIdx.x * FT + threadIdx.x; i < n; i += (int64_t)gridDim.x * FT) {
-    x[i] += a * p[i];
-    const double ri = r[i] - a * Ap[i];
-    r[i] = ri;
-    const double zi = ri * dinv[i];
-    z[i] = zi;
-    rz += ri * zi;
-    rr += ri * ri;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    rz += __shfl_xor_sync(0xffffffffu, rz, o);
-    rr += __shfl_xor_sync(0xffffffffu, rr, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    red[0][threadIdx.x >> 5] = rz;
-    red[1][threadIdx.x >> 5] = rr;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t0 = 0, t1 = 0;
-    for (int w = 0; w < FT / 32; ++w) { t0 += red[0][w]; t1 += red[1][w]; }
-    part_rz[blockIdx.x] = t0;
-    part_rr[blockIdx.x] = t1;
-  }
-}
-
-// p = z + (rz_new / rz) p ; rz = rz_new
-__global__ void cg_direction_kernel(int64_t n, double* __restrict__ sc, double* __restrict__ p,
-                                    const double* __restrict__ z) {
-  const double rz = sc[0];
-  const double b = rz != 0 ? sc[2] / rz : 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * FT + threadIdx.x; i < n; i += (int64_t)gridDim.x * FT) p[i] = z[i] + b * p[i];
-}
-
-__global__ void copy_scalar_kernel(double* __restrict__ sc, int dst, int src) { sc[dst] = sc[src]; }
-
-// Sum of per-block partials in a fixed order; every block computes the same value, so a
-// kernel can use a grid-wide reduction of the previous kernel without another launch.
-__device__ __forceinline__ double sum_partials(const double* __restrict__ part, int nb) {
-  __shared__ double red[FT / 32];
-  __shared__ double total;
-  double acc = 0;
-  for (int b = threadIdx.x; b < nb; b += FT) acc += part[b];
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0;
-    for (int w = 0; w < FT / 32; ++w) t += red[w];
-    total = t;
-  }
-  __syncthreads();
-  return total;
-}
-
-// one CG step after the SpMV: alpha = rz / sum(pAp partials); x += a p; r -= a Ap; z = r dinv;
-// partials of r.z (next rz) and r.r.  rz is read from sc[cur].  z == nullptr: another preconditioner
-// writes z and the r.z partials.
-__global__ void cg_step_kernel(int64_t n, const double* __restrict__ part_pap, int nb, const double* __restrict__ sc,
-                               int cur, double* __restrict__ x, double* __restrict__ r, double* __restrict__ z,
-                               const double* __restrict__ p, const double* __restrict__ Ap,
-                               const double* __restrict__ dinv, double* __restrict__ part_rz,
-                               double* __restrict__ part_rr) {
-  __shared__ double red[2][FT / 32];
-  const double pap = sum_partials(part_pap, nb);
-  const double a = pap != 0 ? sc[cur] / pap : 0.0;
-  double rz = 0, rr = 0;
-  for (int64_t i = (int64_t)blockIdx.x * FT + threadIdx.x; i < n; i += (int64_t)gridDim.x * FT) {
-    x[i] += a * p[i];
-    const double ri = r[i] - a * Ap[i];
-    r[i] = ri;
-    const double zi = ri * dinv[i];
-    if (z) z[i] = zi;
-    rz += ri * zi;
-    rr += ri * ri;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    rz += __shfl_xor_sync(0xffffffffu, rz, o);
-    rr += __shfl_xor_sync(0xffffffffu, rr, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    red[0][threadIdx.x >> 5] = rz;
-    red[1][threadIdx.x >> 5] = rr;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t0 = 0, t1 = 0;
-    for (int w = 0; w < FT / 32; ++w) { t0 += red[0][w]; t1 += red[1][w]; }
-    if (z) part_rz[blockIdx.x] = t0;
-    part_rr[blockIdx.x] = t1;
-  }
-}
-
-// p = z + (rz_new / rz) p with rz_new = sum(rz partials); block 0 stores rz_new in sc[cur^1]
-// and r.r in sc[3] (read by the host between batches)
-__global__ void cg_dir_kernel(int64_t n, const double* __restrict__ part_rz, const double* __restrict__ part_rr,
-                              int nb, double* __restrict__ sc, int cur, double* __restrict__ p,
-                              const double* __restrict__ z) {
-  const double rzn = sum_partials(part_rz, nb);
-  const double rz = sc[cur];
-  const double b = rz != 0 ? rzn / rz : 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * FT + threadIdx.x; i < n; i += (int64_t)gridDim.x * FT) p[i] = z[i] + b * p[i];
-  if (blockIdx.x == 0) {
-    const double rr = sum_partials(part_rr, nb);
-    if (threadIdx.x == 0) {
-      sc[cur ^ 1] = rzn;
-      sc[3] = rr;
+  if (!bar.wait()) return;
+  double norm_old = 0, tol = 0, rz = 0;      // thread 0's
+  int it = 0, ncg = 0, rb = 0, pb = 0;       // rb, pb: current buffers of r and p
+  bool more = P.max_iter > 0;
+  while (more) {
+    ++it;
+    // right-hand side V (B + C), the pinned value moved over; the previous T was re-centred: shifted back onto
+    // the pinned value the warm start differs from the new solution only by the change of C
+    const double tn = P.pin >= 0 ? P.B[P.pin] + P.C[P.pin] : 0.0;
+    const double delta = P.pin >= 0 ? tn - P.T[P.pin] : 0.0;
+    {
+      double rr = 0, bb = 0;
+      double* r = P.r[rb];
+      block_rows(sA, [&](int c) { return P.T[c] + delta; }, [&](int i, double Ti) {
+        double v = P.vol[i] * (P.B[i] + P.C[i]);
+        if (P.pin >= 0) v = i == P.pin ? 0.0 : v - P.colpin[i] * tn;
+        const double ri = v - Ti;
+        r[i] = ri;
+        rr += ri * ri;
+        bb += v * v;
+      });
+      put_rows(rr, sA.vec, p_rr);
+      put_rows(bb, sA.vec, p_bb);
     }
-  }
-}
-
-// partials of r.z (the preconditioned residual product); p = z as well when p is given
-__global__ void rz_kernel(int64_t n, const double* __restrict__ r, const double* __restrict__ z, double* __restrict__ p,
-                          double* __restrict__ part) {
-  __shared__ double red[FT / 32];
-  double acc = 0;
-  for (int64_t i = (int64_t)blockIdx.x * FT + threadIdx.x; i < n; i += (int64_t)gridDim.x * FT) {
-    const double zi = z[i];
-    acc += r[i] * zi;
-    if (p) p[i] = zi;
-  }
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0;
-    for (int w = 0; w < FT / 32; ++w) t += red[w];
-    part[blockIdx.x] = t;
-  }
-}
-
-// warm start consistent with the pin: T += (B + C)_N - T_N  (two launches: read, then shift)
-__global__ void pin_delta_kernel(const double* __restrict__ T, const double* __restrict__ B,
-                                 const double* __restrict__ C, int pin, double* __restrict__ out) {
-  *out = B[pin] + C[pin] - T[pin];
-}
-__global__ void shift_by_kernel(int64_t n, double* __restrict__ T, const double* __restrict__ d) {
-  const double v = *d;
-  for (int64_t i = (int64_t)blockIdx.x * FT + threadIdx.x; i < n; i += (int64_t)gridDim.x * FT) T[i] += v;
-}
-
-// r = rhs - Ap; z = r dinv; p = z; partials of r.z, r.r and rhs.rhs
-__global__ void cg_init_kernel(int64_t n, const double* __restrict__ rhs, const double* __restrict__ Ap,
-                               const double* __restrict__ dinv, double* __restrict__ r, double* __restrict__ z,
-                               double* __restrict__ p, double* __restrict__ part_rz, double* __restrict__ part_rr,
-                               double* __restrict__ part_bb) {
-  __shared__ double red[3][FT / 32];
-  double rz = 0, rr = 0, bb = 0;
-  for (int64_t i = (int64_t)blockIdx.x * FT + threadIdx.x; i < n; i += (int64_t)gridDim.x * FT) {
-    const double ri = rhs[i] - Ap[i];
-    const double zi = ri * dinv[i];
-    r[i] = ri;
-    z[i] = zi;
-    p[i] = zi;
-    rz += ri * zi;
-    rr += ri * ri;
-    bb += rhs[i] * rhs[i];
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    rz += __shfl_xor_sync(0xffffffffu, rz, o);
-    rr += __shfl_xor_sync(0xffffffffu, rr, o);
-    bb += __shfl_xor_sync(0xffffffffu, bb, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    red[0][threadIdx.x >> 5] = rz;
-    red[1][threadIdx.x >> 5] = rr;
-    red[2][threadIdx.x >> 5] = bb;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t0 = 0, t1 = 0, t2 = 0;
-    for (int w = 0; w < FT / 32; ++w) { t0 += red[0][w]; t1 += red[1][w]; t2 += red[2][w]; }
-    part_rz[blockIdx.x] = t0;
-    part_rr[blockIdx.x] = t1;
-    part_bb[blockIdx.x] = t2;
-  }
-}
-
-// rhs_i = V_i (B_i + C_i) - L_iN (B_N + C_N) for i != N; rhs_N = 0;  T_N fixed to (B+C)_N
-__global__ void cg_rhs_kernel(int64_t n, const double* __restrict__ vol, const double* __restrict__ B,
-                              const double* __restrict__ C, int pin, const double* __restrict__ colpin,
-                              double* __restrict__ rhs) {
-  const double tn = pin >= 0 ? B[pin] + C[pin] : 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * FT + threadIdx.x; i < n; i += (int64_t)gridDim.x * FT) {
-    double v = vol[i] * (B[i] + C[i]);
-    if (pin >= 0) v = (i == pin) ? 0.0 : v - colpin[i] * tn;
-    rhs[i] = v;
-  }
-}
-
-__global__ void set_pin_kernel(double* __restrict__ T, const double* __restrict__ B, const double* __restrict__ C,
-                               int pin) {
-  T[pin] = B[pin] + C[pin];
-}
-
-// block partial max/min
-__global__ void minmax_kernel(int64_t n, const double* __restrict__ T, double* __restrict__ pmax,
-                              double* __restrict__ pmin) {
-  __shared__ double rmx[FT / 32], rmn[FT / 32];
-  double mx = -INFINITY, mn = INFINITY;
-  for (int64_t i = (int64_t)blockIdx.x * FT + threadIdx.x; i < n; i += (int64_t)gridDim.x * FT) {
-    mx = fmax(mx, T[i]);
-    mn = fmin(mn, T[i]);
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-  }
-  if ((threadIdx.x & 31) == 0) { rmx[threadIdx.x >> 5] = mx; rmn[threadIdx.x >> 5] = mn; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < FT / 32; ++w) { mx = fmax(mx, rmx[w]); mn = fmin(mn, rmn[w]); }
-    mx = rmx[0] > mx ? rmx[0] : mx;
-    mn = rmn[0] < mn ? rmn[0] : mn;
-    pmax[blockIdx.x] = mx;
-    pmin[blockIdx.x] = mn;
-  }
-}
-
-__global__ void shift_kernel(int64_t n, double* __restrict__ T, double s) {
-  for (int64_t i = (int64_t)blockIdx.x * FT + threadIdx.x; i < n; i += (int64_t)gridDim.x * FT) T[i] -= s;
-}
-
-// least-squares gradient: grad[c] = sum_k gw[c][:, k] * diff[c][k]
-//   diff = T[nb] - T[c] + off   (nb >= 0),   off (nb < 0, no mixed),   value - T[c] (mixed)
-__global__ void gradient_kernel(int64_t n, int nv, int dim, const int32_t* __restrict__ nb,
-                                const double* __restrict__ off, const unsigned char* __restrict__ mixed,
-                                const double* __restrict__ gw, const double* __restrict__ T, double* __restrict__ grad) {
-  for (int64_t c = (int64_t)blockIdx.x * FT + threadIdx.x; c < n; c += (int64_t)gridDim.x * FT) {
-    const double tc = T[c];
-    double g[3] = {0, 0, 0};
-    for (int k = 0; k < nv; ++k) {
-      const int j = nb[c * nv + k];
-      double d;
-      if (mixed[c * nv + k]) d = off[c * nv + k] - tc;
-      else d = (j >= 0 ? T[j] - tc : 0.0) + off[c * nv + k];
-      for (int a = 0; a < dim; ++a) g[a] += gw[(c * dim + a) * nv + k] * d;
+    if (!bar.wait()) return;
+    if (P.pin >= 0)
+      for (int i = r0 + tid; i < r1; i += nthr) P.T[i] += delta;
+    grid_sum(p_bb, nb, red, [&](double s) { return tol = P.cg_rtol * fmax(sqrt(fmax(s, 0.0)), 1e-300); });
+    auto open = [&](double s) { return sqrt(fmax(s, 0.0)) <= tol ? 0.0 : 1.0; };
+    bool run = grid_sum(p_rr, nb, red, open) != 0;
+    // z = M^-1 r and the partials of r . z, after the restriction (or nothing) of the phase before
+    auto precondition = [&](const double* r) -> bool {
+      double dot = 0;
+      auto up = [&](int row, double v) {
+        P.z[row] = v;
+        dot += r[row] * v;
+      };
+      int vec = 1;
+      if (!P.has_amg) {
+        for (int i = r0 + tid; i < r1; i += nthr) up(i, r[i] * P.dinv[i]);
+      } else if (P.amg.nl == 1) {
+        block_dense(sM, P.amg.nc, r, up);
+        vec = 32;
+      } else if (!amg_cycle(P.amg, sM, bar, [&](int c) { return r[c]; }, up)) {
+        return false;
+      } else {
+        vec = sM.Q[0].vec;
+      }
+      put_rows(dot, vec, p_rz);
+      return bar.wait();
+    };
+    auto restrict0 = [&](auto value) {         // b_1 = Q_0^T r
+      if (P.has_amg && P.amg.nl > 1) {
+        double* b1 = P.amg.b[1];
+        block_rows(sM.Qt[0], value, [&](int row, double v) { b1[row] = v; });
+      }
+    };
+    if (run) {
+      const double* r = P.r[rb];
+      restrict0([&](int c) { return r[c]; });
+      if (!bar.wait()) return;
+      if (!precondition(r)) return;
+      grid_sum(p_rz, nb, red, [&](double s) { return rz = s; });
     }
-    for (int a = 0; a < dim; ++a) grad[c * dim + a] = g[a];
-  }
-}
-
-// per internal side: tmp = (w grad_i + (1-w) grad_j) . vnon
-__global__ void side_flux_kernel(int64_t ns, int dim, const int32_t* __restrict__ si, const int32_t* __restrict__ sj,
-                                 const double* __restrict__ w, const double* __restrict__ vnon,
-                                 const double* __restrict__ grad, double* __restrict__ tmp) {
-  for (int64_t s = (int64_t)blockIdx.x * FT + threadIdx.x; s < ns; s += (int64_t)gridDim.x * FT) {
-    const int i = si[s], j = sj[s];
-    double t = 0;
-    for (int a = 0; a < dim; ++a) t += (w[s] * grad[i * dim + a] + (1.0 - w[s]) * grad[j * dim + a]) * vnon[s * dim + a];
-    tmp[s] = t;
-  }
-}
-
-// C[c] = sum over its internal sides of +-tmp / V_c  (gather, fixed order); partial ‖C‖^2
-__global__ void correction_kernel(int64_t n, const int32_t* __restrict__ cp, const int32_t* __restrict__ cs,
-                                  const double* __restrict__ tmp, const double* __restrict__ vol,
-                                  double* __restrict__ C, double* __restrict__ part) {
-  __shared__ double red[FT / 32];
-  double acc = 0;
-  for (int64_t c = (int64_t)blockIdx.x * FT + threadIdx.x; c < n; c += (int64_t)gridDim.x * FT) {
-    double v = 0;
-    for (int k = cp[c]; k < cp[c + 1]; ++k) {
-      const int e = cs[k];
-      v += e >= 0 ? tmp[e] : -tmp[-e - 1];
+    double beta = 0;
+    bool fresh = true;                         // first direction: p = z
+    for (int k = 0; run; ++k) {
+      // p = z + beta p, Ap, partials of p . Ap
+      {
+        const double* po = P.p[pb];
+        double* pn = P.p[pb ^ 1];
+        double pap = 0;
+        auto dir = [&](int c) { return fresh ? P.z[c] : P.z[c] + beta * po[c]; };
+        block_rows(sA, dir, [&](int i, double s) {
+          const double pi = dir(i);
+          pn[i] = pi;
+          P.Ap[i] = s;
+          pap += s * pi;
+        });
+        pb ^= 1;
+        fresh = false;
+        put_rows(pap, sA.vec, p_pap);
+      }
+      if (!bar.wait()) return;
+      const double a = grid_sum(p_pap, nb, red, [&](double pap) { return pap != 0 ? rz / pap : 0.0; });
+      {
+        const double *ro = P.r[rb], *p = P.p[pb];
+        double* rn = P.r[rb ^ 1];
+        double s = 0;
+        for (int i = r0 + tid; i < r1; i += nthr) {
+          P.T[i] += a * p[i];
+          const double ri = ro[i] - a * P.Ap[i];
+          rn[i] = ri;
+          s += ri * ri;
+        }
+        restrict0([&](int c) { return ro[c] - a * P.Ap[c]; });
+        rb ^= 1;
+        if ((k + 1) % P.check == 0) put(s, p_rr);        // the residual is tested every `check` iterations
+      }
+      if (!bar.wait()) return;
+      if (!precondition(P.r[rb])) return;
+      beta = grid_sum(p_rz, nb, red, [&](double s) {
+        const double b = rz != 0 ? s / rz : 0.0;
+        rz = s;
+        return b;
+      });
+      if ((k + 1) % P.check == 0) {
+        ncg += P.check;
+        run = grid_sum(p_rr, nb, red, open) != 0 && k + 1 < P.cg_max;
+      }
     }
-    v /= vol[c];
-    C[c] = v;
-    acc += v * v;
+    // T_pin, then T -= (max + min) / 2 (fourier.py:155-156)
+    double shift = 0;
+    if (P.pin >= 0) {
+      double mx = -INFINITY, mn = INFINITY;
+      for (int i = r0 + tid; i < r1; i += nthr) {
+        if (i == P.pin) P.T[i] = tn;
+        mx = fmax(mx, P.T[i]);
+        mn = fmin(mn, P.T[i]);
+      }
+      mx = block_max(mx, red);
+      mn = -block_max(-mn, red);
+      if (tid == 0) {
+        p_mx[blockIdx.x] = mx;
+        p_mn[blockIdx.x] = mn;
+      }
+      if (!bar.wait()) return;
+      mx = -INFINITY;
+      mn = INFINITY;
+      if (tid < nb) {                        // more threads than blocks
+        mx = p_mx[tid];
+        mn = p_mn[tid];
+      }
+      mx = block_max(mx, red);
+      mn = -block_max(-mn, red);
+      __syncthreads();
+      if (tid == 0) red[0] = (mx + mn) * 0.5;
+      __syncthreads();
+      shift = red[0];
+    } else if (!bar.wait()) {
+      return;
+    }
+    // least-squares gradient of the shifted T: grad[c] = sum_k gw[c][:, k] diff[c][k],
+    //   diff = T[nb] - T[c] + off (nb >= 0), off (nb < 0, no mixed), value - T[c] (mixed)
+    const int nv = P.nv, dim = P.dim;
+    for (int64_t c = r0 + tid; c < r1; c += nthr) {
+      const double tc = P.T[c] - shift;
+      double g[3] = {0, 0, 0};
+      for (int k = 0; k < nv; ++k) {
+        const int j = P.g_nb[c * nv + k];
+        double d;
+        if (P.g_mixed[c * nv + k]) d = P.g_off[c * nv + k] - tc;
+        else d = (j >= 0 ? (P.T[j] - shift) - tc : 0.0) + P.g_off[c * nv + k];
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+          if (a < dim) g[a] += P.gw[(c * dim + a) * nv + k] * d;
+      }
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+        if (a < dim) P.grad[c * dim + a] = g[a];
+    }
+    if (!bar.wait()) return;
+    // C[c] = sum over its internal sides of +-(w grad_i + (1 - w) grad_j) . v_nonorth / V_c; partial |C|^2
+    double cc = 0;
+    for (int64_t c = r0 + tid; c < r1; c += nthr) {
+      if (P.pin >= 0) P.T[c] -= shift;
+      double v = 0;
+      for (int k = P.c_ptr[c]; k < P.c_ptr[c + 1]; ++k) {
+        const int e = P.c_side[k], sd = e >= 0 ? e : -e - 1;
+        const int64_t i = P.s_i[sd], j = P.s_j[sd];
+        const double w = P.s_w[sd];
+        double f = 0;
+        for (int a = 0; a < dim; ++a)
+          f += (w * P.grad[i * dim + a] + (1.0 - w) * P.grad[j * dim + a]) * P.s_vnon[(int64_t)sd * dim + a];
+        v += e >= 0 ? f : -f;
+      }
+      v /= P.vol[c];
+      P.C[c] = v;
+      cc += v * v;
+    }
+    put(cc, p_cc);
+    if (!bar.wait()) return;
+    more = grid_sum(p_cc, nb, red, [&](double s) {
+             const double norm = sqrt(fmax(s, 0.0));
+             const double err = norm == 0 ? 0 : fabs(norm - norm_old) / norm;   // fourier.py:168-171
+             norm_old = norm;
+             return err > P.rtol && it < P.max_iter ? 1.0 : 0.0;
+           }) != 0;
   }
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0;
-    for (int w = 0; w < FT / 32; ++w) t += red[w];
-    part[blockIdx.x] = t;
+  if (blockIdx.x == 0 && tid == 0) {
+    P.out[0] = (double)it;
+    P.out[1] = (double)ncg;
   }
 }
 
@@ -389,17 +320,10 @@ struct obte_fourier_plan_s {
   obte::DevBuf rp, ci, val, dinv, vol, B, colpin, g_nb, g_off, g_mixed, gw, s_i, s_j, s_w, s_vnon, c_ptr, c_side,
       k_e1, k_e2, k_coef, kap;
   // work
-  obte::DevBuf C, rhs, r, z, p, Ap, part, part2, part3, sc, grad, tmp, kout, pmx, pmn;
-  // CG iterations between two convergence checks as one CUDA graph (captured per solution pointer)
-  cudaStream_t capture_stream = nullptr;
-  cudaGraphExec_t cg_exec = nullptr;
-  const double* cg_exec_T = nullptr;
+  obte::DevBuf C, r, z, p, Ap, part, sc, grad, kout;
+  obte::HostBuf hout;               // the two counts of a solve and the error word, read back
   // smoothed-aggregation AMG V-cycle as the CG preconditioner (null: Jacobi)
   obte::AmgPtr amg;
-  ~obte_fourier_plan_s() {
-    if (cg_exec) cudaGraphExecDestroy(cg_exec);
-    if (capture_stream) cudaStreamDestroy(capture_stream);
-  }
 };
 
 using namespace obte;
@@ -584,12 +508,11 @@ extern "C" obte_status obte_fourier_plan_create(obte_context ctx, const obte_fou
   up(upload(P->k_e1, ke1, st)); up(upload(P->k_e2, ke2, st)); up(upload(P->k_coef, kco, st));
   up(upload(P->kap, P->kappa, st));
   const size_t vb = (size_t)n * sizeof(double);
-  up(P->C.alloc(vb)); up(P->rhs.alloc(vb)); up(P->r.alloc(vb)); up(P->z.alloc(vb)); up(P->p.alloc(vb));
-  up(P->Ap.alloc(vb)); up(P->part.alloc((size_t)P->nb * sizeof(double))); up(P->part2.alloc((size_t)P->nb * sizeof(double)));
-  up(P->part3.alloc((size_t)P->nb * sizeof(double)));
-  up(P->sc.alloc(8 * sizeof(double))); up(P->grad.alloc(vb * dim)); up(P->tmp.alloc((size_t)std::max<int64_t>(ni, 1) * 8));
+  // r and p alternate between two buffers; partials: seven sums of one value per block
+  up(P->C.alloc(vb)); up(P->r.alloc(2 * vb)); up(P->z.alloc(vb)); up(P->p.alloc(2 * vb));
+  up(P->Ap.alloc(vb)); up(P->part.alloc(7 * sizeof(double) * (size_t)phase_shape(n, ctx->num_sms).blocks));
+  up(P->sc.alloc(4 * sizeof(double))); up(P->grad.alloc(vb * dim));
   up(P->kout.alloc((size_t)std::max<int64_t>(P->nc, 1) * 8));
-  up(P->pmx.alloc((size_t)P->nb * 8)); up(P->pmn.alloc((size_t)P->nb * 8));
   // OBTE_FOURIER_JACOBI=1 keeps the diagonal preconditioner (same solution, ~40x more CG iterations)
   const char* jac = std::getenv("OBTE_FOURIER_JACOBI");
   if (s0 == OBTE_OK && !(jac && std::atoi(jac) != 0))
@@ -609,84 +532,6 @@ extern "C" obte_status obte_fourier_plan_destroy(obte_fourier_plan plan) {
   return OBTE_OK;
 }
 
-// Preconditioned CG (AMG V-cycle, or Jacobi) on the masked system, warm-started from T (device). Returns iterations.
-static obte_status cg_solve(obte_fourier_plan P, double* T, double rtol, int max_iter, int& iters) {
-  cudaStream_t st = P->ctx->stream;
-  const int64_t n = P->n;
-  const int nb = P->nb;
-  double* sc = P->sc.as<double>();
-  double *r = P->r.as<double>(), *z = P->z.as<double>(), *p = P->p.as<double>(), *Ap = P->Ap.as<double>();
-  const int32_t *rp = P->rp.as<int32_t>(), *ci = P->ci.as<int32_t>();
-  const double* val = P->val.as<double>();
-  // r = rhs - L T, z = r dinv, p = z; rz -> sc[0], rr -> sc[3], ‖rhs‖^2 -> sc[5]
-  const AmgHierarchy* amg = P->amg.get();
-  spmv_kernel<<<nb, FT, 0, st>>>(n, rp, ci, val, T, Ap, P->part.as<double>());
-  cg_init_kernel<<<nb, FT, 0, st>>>(n, P->rhs.as<double>(), Ap, P->dinv.as<double>(), r, z, p, P->part.as<double>(),
-                                    P->part2.as<double>(), P->part3.as<double>());
-  if (amg) {                         // z = M^-1 r, p = z, r.z
-    count_launch(amg_apply(*amg, r, z, nullptr, 0, st));
-    rz_kernel<<<nb, FT, 0, st>>>(n, r, z, p, P->part.as<double>());
-    count_launch();
-  }
-  reduce_kernel<<<1, FT, 0, st>>>(P->part.as<double>(), nb, sc + 0);
-  reduce_kernel<<<1, FT, 0, st>>>(P->part2.as<double>(), nb, sc + 3);
-  reduce_kernel<<<1, FT, 0, st>>>(P->part3.as<double>(), nb, sc + 5);
-  count_launch(5);
-  OBTE_CUDA(cudaGetLastError());
-  double hs[6];
-  OBTE_CUDA(cudaMemcpyAsync(hs, sc, 6 * sizeof(double), cudaMemcpyDeviceToHost, st));
-  OBTE_CUDA(cudaStreamSynchronize(st));
-  {
-    const double tol = rtol * std::max(std::sqrt(std::max(hs[5], 0.0)), 1e-300);
-    iters = 0;
-    if (std::sqrt(std::max(hs[3], 0.0)) <= tol) return OBTE_OK;
-    // three launches per iteration; rz alternates between sc[0] and sc[1].  At a few microseconds of work
-    // per launch the loop is launch-bound, so the `check` iterations between two convergence tests are
-    // captured once as a CUDA graph (on a private stream: capture is not allowed on the legacy default
-    // stream) and replayed on the plan's stream.  `check` is even, so every block starts with cur = 0.
-    // With the AMG preconditioner a solve takes a few tens of iterations, so the check comes every 4.
-    // The V-cycle writes z and the partials of r.z (cg_step_kernel then skips its Jacobi z).
-    const int check = amg ? 4 : 8;
-    double* pp = P->part.as<double>();
-    double* prz = P->part2.as<double>();
-    double* prr = P->part3.as<double>();
-    const int per_iter = amg ? 3 + amg_launches(*amg, true) : 3;
-    auto enqueue = [&](cudaStream_t s2) {
-      for (int k = 0; k < check; ++k) {
-        const int cur = k & 1;
-        spmv_kernel<<<nb, FT, 0, s2>>>(n, rp, ci, val, p, Ap, pp);
-        cg_step_kernel<<<nb, FT, 0, s2>>>(n, pp, nb, sc, cur, T, r, amg ? nullptr : z, p, Ap, P->dinv.as<double>(),
-                                          prz, prr);
-        if (amg) amg_apply(*amg, r, z, prz, nb, s2);
-        cg_dir_kernel<<<nb, FT, 0, s2>>>(n, prz, prr, nb, sc, cur, p, z);
-      }
-    };
-    if (P->cg_exec_T != T && !std::getenv("OBTE_NO_GRAPHS")) {
-      if (P->cg_exec) { cudaGraphExecDestroy(P->cg_exec); P->cg_exec = nullptr; }
-      if (!P->capture_stream) OBTE_CUDA(cudaStreamCreateWithFlags(&P->capture_stream, cudaStreamNonBlocking));
-      cudaGraph_t g = nullptr;
-      OBTE_CUDA(cudaStreamBeginCapture(P->capture_stream, cudaStreamCaptureModeThreadLocal));
-      enqueue(P->capture_stream);
-      OBTE_CUDA(cudaStreamEndCapture(P->capture_stream, &g));
-      const cudaError_t e = cudaGraphInstantiate(&P->cg_exec, g, 0);
-      cudaGraphDestroy(g);
-      if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate", __FILE__, __LINE__);
-      P->cg_exec_T = T;
-    }
-    while (iters < max_iter) {
-      if (P->cg_exec && P->cg_exec_T == T) OBTE_CUDA(cudaGraphLaunch(P->cg_exec, st));
-      else enqueue(st);
-      count_launch(per_iter * check);
-      iters += check;
-      OBTE_CUDA(cudaGetLastError());
-      OBTE_CUDA(cudaMemcpyAsync(hs, sc, 4 * sizeof(double), cudaMemcpyDeviceToHost, st));
-      OBTE_CUDA(cudaStreamSynchronize(st));
-      if (std::sqrt(std::max(hs[3], 0.0)) <= tol) break;
-    }
-  }
-  return OBTE_OK;
-}
-
 extern "C" obte_status obte_fourier_solve(obte_fourier_plan P, const obte_fourier_opts* opts, double* T, double* J,
                                           obte_fourier_info* info) {
   if (!P || !opts || !T) { set_error("null argument"); return OBTE_ERR_BAD_ARG; }
@@ -697,78 +542,56 @@ extern "C" obte_status obte_fourier_solve(obte_fourier_plan P, const obte_fourie
   const double rtol = opts->rtol > 0 ? opts->rtol : 1e-8;
   const double cg_rtol = opts->cg_rtol > 0 ? opts->cg_rtol : 1e-13;
   const int cg_max = opts->cg_max_iter > 0 ? opts->cg_max_iter : 20000;
-  double* C = P->C.as<double>();
-  OBTE_CUDA(cudaMemsetAsync(C, 0, n * sizeof(double), st));
-  OBTE_CUDA(cudaMemsetAsync(T, 0, n * sizeof(double), st));
-  double norm_old = 0, err = 1, kappa = 0;
-  int it = 0, ncg = 0;
-  while (err > rtol && it < max_iter) {                                          // fourier.py:149
-    ++it;
-    cg_rhs_kernel<<<nb, FT, 0, st>>>(n, P->vol.as<double>(), P->B.as<double>(), C, P->pin, P->colpin.as<double>(),
-                                     P->rhs.as<double>());
+  if (!P->hout.p) OBTE_TRY(P->hout.alloc(4 * sizeof(double)));
+  FourierParams f = {};
+  f.n = n;
+  f.A = CsrDev{n, P->rp.as<int32_t>(), P->ci.as<int32_t>(), P->val.as<double>()};
+  f.has_amg = P->amg ? 1 : 0;
+  if (P->amg) amg_device(*P->amg, f.amg);
+  f.dinv = P->dinv.as<double>(); f.vol = P->vol.as<double>(); f.B = P->B.as<double>(); f.colpin = P->colpin.as<double>();
+  f.pin = P->pin; f.nv = P->nv; f.dim = P->dim;
+  f.g_nb = P->g_nb.as<int32_t>(); f.g_off = P->g_off.as<double>(); f.g_mixed = P->g_mixed.as<unsigned char>();
+  f.gw = P->gw.as<double>();
+  f.s_i = P->s_i.as<int32_t>(); f.s_j = P->s_j.as<int32_t>(); f.s_w = P->s_w.as<double>(); f.s_vnon = P->s_vnon.as<double>();
+  f.c_ptr = P->c_ptr.as<int32_t>(); f.c_side = P->c_side.as<int32_t>();
+  f.T = T; f.C = P->C.as<double>();
+  f.r[0] = P->r.as<double>(); f.r[1] = f.r[0] + n;
+  f.p[0] = P->p.as<double>(); f.p[1] = f.p[0] + n;
+  f.z = P->z.as<double>(); f.Ap = P->Ap.as<double>(); f.grad = P->grad.as<double>(); f.part = P->part.as<double>();
+  f.max_iter = max_iter; f.cg_max = cg_max;
+  f.check = P->amg ? 4 : 8;          // iterations between two convergence tests
+  f.rtol = rtol; f.cg_rtol = cg_rtol;
+  f.out = P->sc.as<double>();
+  f.count = reinterpret_cast<unsigned*>(f.out + 2);
+  f.err = reinterpret_cast<int*>(f.out + 3);
+  OBTE_CUDA(cudaMemsetAsync(P->sc.p, 0, 4 * sizeof(double), st));
+  OBTE_CUDA(phase_launch(phase_shape(n, P->ctx->num_sms), fourier_kernel<ClusterBarrier>, fourier_kernel<GridBarrier>, f, st));
+  count_launch();
+  double kappa = 0;
+  std::vector<double> kh(std::max<int64_t>(P->nc, 1));
+  if (P->nc > 0) {
+    contact_kernel<<<nb, FT, 0, st>>>(P->nc, P->k_e1.as<int32_t>(), P->k_e2.as<int32_t>(), P->k_coef.as<double>(),
+                                      P->contact_t2, T, P->kout.as<double>());
     count_launch();
-    int k = 0;
-    if (P->pin >= 0) {
-      // the previous T was re-centred; shift it back onto the pinned value so the warm start
-      // differs from the new solution only by the change of C (a uniform shift is in L's null space)
-      pin_delta_kernel<<<1, 1, 0, st>>>(T, P->B.as<double>(), C, P->pin, P->sc.as<double>() + 6);
-      shift_by_kernel<<<nb, FT, 0, st>>>(n, T, P->sc.as<double>() + 6);
-      count_launch(2);
-    }
-    OBTE_TRY(cg_solve(P, T, cg_rtol, cg_max, k));                                // fourier.py:152
-    ncg += k;
-    if (P->pin >= 0) {
-      set_pin_kernel<<<1, 1, 0, st>>>(T, P->B.as<double>(), C, P->pin);
-      count_launch();
-      // T -= (max + min)/2                                                      // fourier.py:155-156
-      minmax_kernel<<<nb, FT, 0, st>>>(n, T, P->pmx.as<double>(), P->pmn.as<double>());
-      count_launch();
-      std::vector<double> mx(nb), mn(nb);
-      OBTE_CUDA(cudaMemcpyAsync(mx.data(), P->pmx.p, nb * 8, cudaMemcpyDeviceToHost, st));
-      OBTE_CUDA(cudaMemcpyAsync(mn.data(), P->pmn.p, nb * 8, cudaMemcpyDeviceToHost, st));
-      OBTE_CUDA(cudaStreamSynchronize(st));
-      double a = mx[0], b = mn[0];
-      for (int i = 1; i < nb; ++i) { a = std::max(a, mx[i]); b = std::min(b, mn[i]); }
-      shift_kernel<<<nb, FT, 0, st>>>(n, T, (a + b) * 0.5);
-      count_launch();
-    }
-    gradient_kernel<<<nb, FT, 0, st>>>(n, P->nv, P->dim, P->g_nb.as<int32_t>(), P->g_off.as<double>(),
-                                       P->g_mixed.as<unsigned char>(), P->gw.as<double>(), T, P->grad.as<double>());
-    side_flux_kernel<<<nb, FT, 0, st>>>(P->ns_int, P->dim, P->s_i.as<int32_t>(), P->s_j.as<int32_t>(),
-                                        P->s_w.as<double>(), P->s_vnon.as<double>(), P->grad.as<double>(),
-                                        P->tmp.as<double>());
-    correction_kernel<<<nb, FT, 0, st>>>(n, P->c_ptr.as<int32_t>(), P->c_side.as<int32_t>(), P->tmp.as<double>(),
-                                         P->vol.as<double>(), C, P->part.as<double>());
-    reduce_kernel<<<1, FT, 0, st>>>(P->part.as<double>(), nb, P->sc.as<double>() + 4);
-    count_launch(4);
-    OBTE_CUDA(cudaGetLastError());
-    double cc;
-    OBTE_CUDA(cudaMemcpyAsync(&cc, P->sc.as<double>() + 4, sizeof(double), cudaMemcpyDeviceToHost, st));
-    OBTE_CUDA(cudaStreamSynchronize(st));
-    const double norm_C = std::sqrt(std::max(cc, 0.0));
-    err = norm_C == 0 ? 0 : std::fabs(norm_C - norm_old) / norm_C;                  // fourier.py:168-171
-    norm_old = norm_C;
-    if (P->nc > 0) {
-      contact_kernel<<<nb, FT, 0, st>>>(P->nc, P->k_e1.as<int32_t>(), P->k_e2.as<int32_t>(), P->k_coef.as<double>(),
-                                        P->contact_t2, T, P->kout.as<double>());
-      count_launch();
-      std::vector<double> kh(P->nc);
-      OBTE_CUDA(cudaMemcpyAsync(kh.data(), P->kout.p, P->nc * 8, cudaMemcpyDeviceToHost, st));
-      OBTE_CUDA(cudaStreamSynchronize(st));
-      kappa = 0;
-      for (double v : kh) kappa += v;
-    }
+    OBTE_CUDA(cudaMemcpyAsync(kh.data(), P->kout.p, P->nc * 8, cudaMemcpyDeviceToHost, st));
   }
   if (J) {
     flux_kernel<<<nb, FT, 0, st>>>(n, P->dim, P->kap.as<double>(), P->grad.as<double>(), J);
     count_launch();
   }
   OBTE_CUDA(cudaGetLastError());
+  double* h = P->hout.as<double>();
+  OBTE_CUDA(cudaMemcpyAsync(h, P->sc.p, 4 * sizeof(double), cudaMemcpyDeviceToHost, st));
   OBTE_CUDA(cudaStreamSynchronize(st));
+  if (reinterpret_cast<int*>(h + 3)[0] != 0) {
+    set_error("a device-side wait timed out in the Fourier kernel");
+    return OBTE_ERR_DEVICE_TIMEOUT;
+  }
+  for (int64_t k = 0; k < P->nc; ++k) kappa += kh[k];
   if (info) {
     info->kappa = kappa;
-    info->n_iter = it;
-    info->n_cg = ncg;
+    info->n_iter = (int32_t)h[0];
+    info->n_cg = (int32_t)h[1];
   }
   return OBTE_OK;
 }

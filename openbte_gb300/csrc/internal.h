@@ -165,11 +165,9 @@ using AmgPtr = std::unique_ptr<AmgHierarchy, AmgDeleter>;
 obte_status amg_build(int64_t n, const std::vector<int32_t>& rp, const std::vector<int32_t>& ci,
                       const std::vector<double>& val, int pin, int num_sms, cudaStream_t st, AmgPtr& out,
                       int coarse_max = 400);
-// Enqueue z = M^-1 r (one symmetric V-cycle) on `st`; with `part`, also the nb_part block partials of
-// r . z (launched on exactly nb_part blocks).  Returns the number of kernel launches.
-int amg_apply(const AmgHierarchy& H, const double* r, double* z, double* part, int nb_part, cudaStream_t st);
+// Enqueue z = M^-1 r (one symmetric V-cycle) on `st`.  Returns the number of kernel launches.
+int amg_apply(const AmgHierarchy& H, const double* r, double* z, cudaStream_t st);
 int amg_levels(const AmgHierarchy& H);
-int amg_launches(const AmgHierarchy& H, bool with_part);   // kernel launches of one amg_apply
 
 }  // namespace obte
 
