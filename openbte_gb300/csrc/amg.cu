@@ -19,8 +19,8 @@
 // G = w D^-1 (2 I - w A D^-1) (symmetric, A's pattern),
 //   b_c = Q^T b    and    x = G b + Q x_c,
 // so the device applies one sparse product per level on the way down and one on the way up, plus one dense
-// product with the coarsest inverse: 2 (levels - 1) + 1 launches per V-cycle instead of 6 per level (amg_apply),
-// or as many phases inside a larger kernel (grid.cuh).
+// product with the coarsest inverse: 2 (levels - 1) + 1 phases of a larger kernel (amg_cycle in grid.cuh) instead of
+// 6 per level.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -34,7 +34,6 @@ namespace obte {
 
 namespace {
 
-constexpr int AT = 256;
 
 struct HostCsr {
   int64_t n = 0, m = 0;
@@ -248,47 +247,6 @@ bool dense_inverse(const HostCsr& A, std::vector<double>& inv) {
   return true;
 }
 
-// ---- device V-cycle ----------------------------------------------------------------------------
-
-// y = G gx + Q qx (G optional) with VEC lanes per row (lane-strided products, then an xor tree: a fixed
-// summation order).  Every thread runs the same number of row passes, so the group shuffles always see full
-// warps.
-template <int VEC>
-__global__ void __launch_bounds__(AT) amg_rows_kernel(
-    int64_t n, const int32_t* __restrict__ grp, const int32_t* __restrict__ gci, const double* __restrict__ gv,
-    const double* __restrict__ gx, const int32_t* __restrict__ qrp, const int32_t* __restrict__ qci,
-    const double* __restrict__ qv, const double* __restrict__ qx, double* __restrict__ y) {
-  constexpr int GPB = AT / VEC;
-  const int lane = (int)(threadIdx.x % VEC);
-  const int64_t stride = (int64_t)gridDim.x * GPB;
-  const int64_t first = (int64_t)blockIdx.x * GPB + threadIdx.x / VEC;
-  const int64_t trips = (n + stride - 1) / stride;
-  for (int64_t t = 0; t < trips; ++t) {
-    const int64_t row = first + t * stride;
-    double acc = 0;
-    if (row < n) {
-      if (gv)
-        for (int k = grp[row] + lane; k < grp[row + 1]; k += VEC) acc += gv[k] * gx[gci[k]];
-      for (int k = qrp[row] + lane; k < qrp[row + 1]; k += VEC) acc += qv[k] * qx[qci[k]];
-    }
-#pragma unroll
-    for (int o = VEC / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (row < n && lane == 0) y[row] = acc;
-  }
-}
-
-// x = Ainv b (dense, one warp per row, fixed summation order)
-__global__ void amg_coarse_kernel(int n, const double* __restrict__ inv, const double* __restrict__ b,
-                                  double* __restrict__ x) {
-  const int lane = threadIdx.x & 31;
-  for (int row = (blockIdx.x * AT + threadIdx.x) >> 5; row < n; row += (gridDim.x * AT) >> 5) {
-    double s = 0;
-    for (int k = lane; k < n; k += 32) s += inv[(size_t)row * n + k] * b[k];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) x[row] = s;
-  }
-}
-
 struct DevCsr {
   int64_t n = 0, nnz = 0;
   DevBuf rp, ci, val;
@@ -308,7 +266,6 @@ struct AmgHierarchy {
   std::vector<std::unique_ptr<AmgLevel>> lv;
   DevBuf inv;                        // dense inverse of the coarsest operator
   int nc = 0;
-  int num_sms = 1;
 };
 
 void AmgDeleter::operator()(AmgHierarchy* h) const { delete h; }
@@ -324,7 +281,7 @@ static obte_status upload_csr(const HostCsr& A, DevCsr& d, cudaStream_t st) {
 }
 
 obte_status amg_build(int64_t n, const std::vector<int32_t>& rp, const std::vector<int32_t>& ci,
-                      const std::vector<double>& val, int pin, int num_sms, cudaStream_t st, AmgPtr& out,
+                      const std::vector<double>& val, int pin, cudaStream_t st, AmgPtr& out,
                       int coarse_max) {
   PhaseTimer timer("amg_build");
   if (n >= (int64_t)1 << 31 || rp.back() < 0) { set_error("AMG: matrix too large"); return OBTE_ERR_BAD_ARG; }
@@ -352,7 +309,6 @@ obte_status amg_build(int64_t n, const std::vector<int32_t>& rp, const std::vect
     A = std::move(B);
   }
   std::unique_ptr<AmgHierarchy> H(new AmgHierarchy());
-  H->num_sms = std::max(1, num_sms);
   const double theta = 0.08;
   while (true) {
     H->lv.emplace_back(new AmgLevel());
@@ -396,68 +352,29 @@ obte_status amg_build(int64_t n, const std::vector<int32_t>& rp, const std::vect
   return OBTE_OK;
 }
 
-// The hierarchy as a kernel reads it (one level: only the dense inverse).
-void amg_device(const AmgHierarchy& H, AmgDev& d) {
+// The hierarchy as a kernel reads it (one level: only the dense inverse).  fixed_order: the lanes of a row, and with
+// them the order of its sum, follow from the level's mean row length alone.
+void amg_device(const AmgHierarchy& H, AmgDev& d, bool fixed_order) {
   const int nl = (int)H.lv.size();
   d.nl = nl;
   d.nc = H.nc;
   d.inv = H.inv.as<double>();
-  auto csr = [](const DevCsr& m) { return CsrDev{m.n, m.rp.as<int32_t>(), m.ci.as<int32_t>(), m.val.as<double>()}; };
+  auto csr = [&](const DevCsr& m, int64_t extra) {
+    const double mean = (double)(m.nnz + extra) / (double)std::max<int64_t>(m.n, 1);
+    const int vec = mean < 6 ? 1 : mean < 12 ? 2 : mean < 24 ? 4 : mean < 48 ? 8 : mean < 96 ? 16 : 32;
+    return CsrDev{m.n, m.rp.as<int32_t>(), m.ci.as<int32_t>(), m.val.as<double>(), fixed_order ? vec : 0};
+  };
   for (int l = 0; l < nl; ++l) {
     const AmgLevel& L = *H.lv[l];
     d.b[l] = l ? L.b.as<double>() : nullptr;
     d.x[l] = l ? L.x.as<double>() : nullptr;
     if (l + 1 < nl) {
-      d.G[l] = csr(L.G);
-      d.Q[l] = csr(L.Q);
-      d.Qt[l] = csr(L.Qt);
+      d.G[l] = csr(L.G, 0);
+      d.Q[l] = csr(L.Q, L.G.nnz);
+      d.Qt[l] = csr(L.Qt, 0);
     }
   }
 }
 
 int amg_levels(const AmgHierarchy& H) { return (int)H.lv.size(); }
-namespace {
-// y = G gx + Q qx over n rows, lanes per row from the mean row length
-void rows_launch(const DevCsr* G, const double* gx, const DevCsr& Q, const double* qx, double* y, int num_sms,
-                 cudaStream_t st) {
-  const int64_t n = Q.n;
-  const double mean = (double)(Q.nnz + (G ? G->nnz : 0)) / (double)std::max<int64_t>(n, 1);
-  const int vec = mean < 6 ? 1 : mean < 12 ? 2 : mean < 24 ? 4 : mean < 48 ? 8 : mean < 96 ? 16 : 32;
-  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((n * vec + AT - 1) / AT, (int64_t)num_sms * 8));
-  const int32_t* grp = G ? G->rp.as<int32_t>() : nullptr;
-  const int32_t* gci = G ? G->ci.as<int32_t>() : nullptr;
-  const double* gv = G ? G->val.as<double>() : nullptr;
-#define OBTE_AMG_ROWS(V)                                                                                       \
-  amg_rows_kernel<V><<<blocks, AT, 0, st>>>(n, grp, gci, gv, gx, Q.rp.as<int32_t>(), Q.ci.as<int32_t>(),      \
-                                            Q.val.as<double>(), qx, y)
-  switch (vec) {
-    case 1: OBTE_AMG_ROWS(1); break;
-    case 2: OBTE_AMG_ROWS(2); break;
-    case 4: OBTE_AMG_ROWS(4); break;
-    case 8: OBTE_AMG_ROWS(8); break;
-    case 16: OBTE_AMG_ROWS(16); break;
-    default: OBTE_AMG_ROWS(32); break;
-  }
-#undef OBTE_AMG_ROWS
-}
-}  // namespace
-
-// z = M^-1 r (level 0 reads r and writes z directly); the number of launches
-int amg_apply(const AmgHierarchy& H, const double* r, double* z, cudaStream_t st) {
-  const int nl = (int)H.lv.size();
-  auto bvec = [&](int l) { return l == 0 ? r : H.lv[l]->b.as<double>(); };
-  auto xvec = [&](int l) { return l == 0 ? z : H.lv[l]->x.as<double>(); };
-  for (int l = 0; l < nl - 1; ++l)                        // b_l+1 = Q_l^T b_l
-    rows_launch(nullptr, nullptr, H.lv[l]->Qt, bvec(l), H.lv[l + 1]->b.as<double>(), H.num_sms, st);
-  {
-    const int blocks = std::max(1, std::min(1024, (H.nc * 32 + AT - 1) / AT));
-    amg_coarse_kernel<<<blocks, AT, 0, st>>>(H.nc, H.inv.as<double>(), bvec(nl - 1), xvec(nl - 1));
-  }
-  for (int l = nl - 2; l >= 0; --l) {                     // x_l = G_l b_l + Q_l x_l+1
-    const AmgLevel& L = *H.lv[l];
-    rows_launch(&L.G, bvec(l), L.Q, xvec(l + 1), xvec(l), H.num_sms, st);
-  }
-  return 2 * (nl - 1) + 1;
-}
-
 }  // namespace obte

@@ -41,89 +41,130 @@
 #include <cstdlib>
 #include <vector>
 
-#include "internal.h"
+#include "grid.cuh"
 
 namespace obte {
 
 namespace {
 
-constexpr int DT = 256;
+struct DsaParams {
+  int64_t n, nd, nu;
+  int n_mfp, project, cycles;
+  double inv_vol_sum;
+  CsrDev A;                                  // L
+  AmgDev amg;
+  const double* vol;
+  const int32_t *wcell, *xcell;
+  const double *in, *base;
+  double *out, *b, *d, *r, *e, *part;
+  unsigned *count, *count_next;
+  int* err;
+};
 
-__device__ __forceinline__ double block_sum(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+// out = base + E L^-1 R in, one launch.  Phases end at a barrier (grid.cuh): the weighted sum of `in`; the
+// right-hand side b = V (in - mean) formed in the gather of its restriction; the V-cycle; the weighted sum of
+// d; the extension out[i] = base[i] + d[cell(i)] - mean over the state: temperatures, wall temperatures (element
+// of the wall), periodic inflow (element of the source slot, every MFP).
+//
+// As 12 launches of 3.9 us each with its gap an application took 47 us (64^2 and 128^2 pixels); with the Arnoldi
+// step in one launch as well, 64^2 pixels x 20 x 32 went from 33.1 to 26.5 ms a gradient evaluation.
+template <typename Bar>
+__global__ void __launch_bounds__(kPhaseThreads, 1) dsa_kernel(const __grid_constant__ DsaParams P) {
+  __shared__ double red[kPhaseThreads];
+  __shared__ Rows sA;
+  __shared__ AmgRows sM;
+  Bar bar(P.count, P.err);
+  const int tid = threadIdx.x, nthr = blockDim.x, nb = gridDim.x;
+  if (blockIdx.x == 0 && tid == 0) *P.count_next = 0;
+  Arena ar{nullptr, 0};                      // read once: not worth copying
+  load_amg(P.amg, &sM, ar, 32);
+  if (P.cycles > 1) load_rows(P.A, &sA, ar, 32);
+  int r0, r1;
+  block_range(P.n, r0, r1, 32);
+  // V x over each 32 consecutive elements of the block (x complete in the block)
+  const int segments = (int)((P.n + 31) / 32);
+  auto weigh = [&](const double* x, double* seg) {
+    for (int i0 = r0 + (tid & ~31); i0 < r1; i0 += nthr) {       // whole warps
+      const int i = i0 + (tid & 31);
+      double v = i < r1 ? P.vol[i] * x[i] : 0.0;
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if ((tid & 31) == 0) seg[i0 >> 5] = v;
+    }
+  };
+  // The mean from the segments' sums (after a barrier), in one order for every number of blocks: the correction
+  // of a nearly singular operator is sensitive to the rounding of the means, and an FP32 basis turns that
+  // into another, equally good, iterate.
+  auto mean = [&](const double* seg) {
+    double v = 0;
+    if (tid < 256)
+      for (int i = tid * 8; i < segments; i += 8 * 256) {
+        double a[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[j] = i + j < segments ? seg[i + j] : 0.0;
+        v += ((a[0] + a[4]) + (a[2] + a[6])) + ((a[1] + a[5]) + (a[3] + a[7]));
+      }
+    if (tid < 256)
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if (tid < 256 && (tid & 31) == 0) red[1 + (tid >> 5)] = v;
+    __syncthreads();
+    if (tid == 0) {
+      const double* a = red + 1;
+      red[0] = (((a[0] + a[4]) + (a[2] + a[6])) + ((a[1] + a[5]) + (a[3] + a[7]))) * P.inv_vol_sum;
+    }
+    __syncthreads();
+    return red[0];
+  };
   __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  v = (threadIdx.x < (blockDim.x >> 5)) ? red[threadIdx.x] : 0.0;
-  if (w == 0)
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if (threadIdx.x == 0) red[0] = v;
-  __syncthreads();
-  return red[0];
-}
-
-// part[block] = sum over the block's grid-stride range of V x (fixed order)
-__global__ void dsa_partial_kernel(int64_t n, const double* __restrict__ vol, const double* __restrict__ x,
-                                   double* __restrict__ part) {
-  __shared__ double red[32];
-  double s = 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    s += vol[i] * x[i];
-  s = block_sum(s, red);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
-}
-
-// sum of the np partials, the same value (same order) in every block
-__device__ __forceinline__ double sum_partials(const double* __restrict__ part, int np, double* red) {
-  double s = 0;
-  for (int i = threadIdx.x; i < np; i += blockDim.x) s += part[i];
-  return block_sum(s, red);
-}
-
-// b = V in[0:n], minus V times the volume-weighted mean of in when `part` (the partials of V in) is given
-__global__ void dsa_restrict_kernel(int64_t n, const double* __restrict__ vol, double inv_vol_sum,
-                                    const double* __restrict__ part, int np, const double* __restrict__ in,
-                                    double* __restrict__ b) {
-  __shared__ double red[32];
-  const double mu = part ? sum_partials(part, np, red) * inv_vol_sum : 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    b[i] = vol[i] * (in[i] - mu);
-}
-
-// r = b - L d (CSR, one thread per row)
-__global__ void dsa_residual_kernel(int64_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
-                                    const double* __restrict__ val, const double* __restrict__ b,
-                                    const double* __restrict__ d, double* __restrict__ r) {
-  for (int64_t i = (int64_t)blockIdx.x * DT + threadIdx.x; i < n; i += (int64_t)gridDim.x * DT) {
-    double acc = b[i];
-    for (int32_t k = rp[i]; k < rp[i + 1]; ++k) acc -= val[k] * d[ci[k]];
-    r[i] = acc;
+  double mu = 0;
+  if (P.project) {
+    weigh(P.in, P.part);
+    if (!bar.wait()) return;
+    mu = mean(P.part);
   }
-}
-
-__global__ void dsa_axpy_kernel(int64_t n, const double* __restrict__ e, double* __restrict__ d) {
-  for (int64_t i = (int64_t)blockIdx.x * DT + threadIdx.x; i < n; i += (int64_t)gridDim.x * DT) d[i] += e[i];
-}
-
-// out[i] += d[cell(i)] - mean over the state: temperatures, wall temperatures (element of the wall),
-// periodic inflow (element of the source slot, every MFP); the mean is the volume-weighted one of d from its
-// partials (or 0 without them)
-__global__ void dsa_extend_kernel(int64_t n, int64_t nd, int64_t nu, int n_mfp, const int32_t* __restrict__ wcell,
-                                  const int32_t* __restrict__ xcell, const double* __restrict__ d,
-                                  const double* __restrict__ part, int np, double inv_vol_sum,
-                                  double* __restrict__ out) {
-  __shared__ double red[32];
-  const double mu = part ? sum_partials(part, np, red) * inv_vol_sum : 0.0;
-  const int64_t xoff = n + nd;
-  for (int64_t i = (int64_t)blockIdx.x * DT + threadIdx.x; i < nu; i += (int64_t)gridDim.x * DT) {
-    const int64_t c = i < n ? i : i < xoff ? (int64_t)wcell[i - n] : (int64_t)xcell[(i - xoff) / n_mfp];
-    out[i] += d[c] - mu;
+  const int nl = P.amg.nl;
+  for (int i = r0 + tid; i < r1; i += nthr) P.b[i] = P.vol[i] * (P.in[i] - mu);
+  auto restrict0 = [&](auto value) {         // b_1 = Q_0^T b
+    double* b1 = P.amg.b[1];
+    block_rows(sM.Qt[0], value, [&](int row, double v) { b1[row] = v; });
+  };
+  if (nl > 1) restrict0([&](int c) { return P.vol[c] * (P.in[c] - mu); });
+  if (!bar.wait()) return;
+  // x = B rhs with one V-cycle, after the restriction
+  auto cycle = [&](const double* rhs, double* x) -> bool {
+    auto up = [&](int row, double v) { x[row] = v; };
+    if (nl == 1) {
+      block_dense(sM, P.amg.nc, rhs, up);
+      return true;
+    }
+    return amg_cycle(P.amg, sM, bar, [&](int c) { return rhs[c]; }, up);
+  };
+  if (!cycle(P.b, P.d)) return;
+  for (int c = 1; c < P.cycles; ++c) {       // d += B (b - L d)
+    if (!bar.wait()) return;
+    block_rows(sA, [&](int j) { return P.d[j]; }, [&](int i, double s) { P.r[i] = P.b[i] - s; });
+    if (!bar.wait()) return;
+    if (nl > 1) {
+      restrict0([&](int j) { return P.r[j]; });
+      if (!bar.wait()) return;
+    }
+    if (!cycle(P.r, P.e)) return;
+    if (!bar.wait()) return;
+    for (int i = r0 + tid; i < r1; i += nthr) P.d[i] += P.e[i];
   }
-}
-
-int grid_for(int64_t n, int num_sms) {
-  return (int)std::max<int64_t>(1, std::min<int64_t>((n + DT - 1) / DT, (int64_t)num_sms * 8));
+  __syncthreads();                           // the block's rows of d, by other threads than those that add them up
+  mu = 0;
+  if (P.project) weigh(P.d, P.part + segments);
+  if (!bar.wait()) return;
+  if (P.project) mu = mean(P.part + segments);
+  const int64_t n = P.n, xoff = P.n + P.nd, t = (int64_t)blockIdx.x * nthr + tid, stride = (int64_t)nb * nthr;
+  for (int64_t i = t; i < P.nu; i += stride) {
+    const int64_t x = i - xoff;
+    int64_t c = i;
+    if (x >= 0) c = P.xcell[P.nu < ((int64_t)1 << 31) ? (int64_t)((unsigned)x / (unsigned)P.n_mfp) : x / P.n_mfp];
+    else if (i >= n) c = P.wcell[i - n];
+    P.out[i] = P.base[i] + (P.d[c] - mu);
+  }
 }
 
 }  // namespace
@@ -253,13 +294,16 @@ obte_status ensure_dsa(obte_plan plan) {
   // rebuilt for every density field of a design loop: coarsen down to 64 rows, whose dense inverse costs
   // little (on 128^2 pixels the hierarchy's set-up took 16.5 ms with the default 400-row coarsest
   // operator, 6.8 ms with 64 rows, for one more sweep per solve)
-  OBTE_TRY(amg_build(n, rp, ci, val, -1, plan->ctx->num_sms, st, op->amg, 64));
+  OBTE_TRY(amg_build(n, rp, ci, val, -1, st, op->amg, 64));
   OBTE_TRY(upload(op->rp, rp, st));
   OBTE_TRY(upload(op->ci, ci, st));
   OBTE_TRY(upload(op->val, val, st));
   OBTE_TRY(upload(op->vol, D.vol, st));
   for (DevBuf* b : {&op->b, &op->d, &op->r, &op->e}) OBTE_TRY(b->alloc((size_t)n * sizeof(double)));
-  OBTE_TRY(op->mean.alloc((size_t)grid_for(n, plan->ctx->num_sms) * sizeof(double)));   // partial sums
+  // partial sums of the two weighted means, and the two barrier counters that launches use in turn
+  const int64_t segments = (n + 31) / 32;
+  OBTE_TRY(op->mean.alloc((size_t)(2 * segments + 1) * sizeof(double)));
+  OBTE_CUDA(cudaMemsetAsync(op->mean.as<double>() + 2 * segments, 0, sizeof(double), st));
   double vs = 0;
   for (double v : D.vol) vs += v;
   op->inv_vol_sum = vs > 0 ? 1.0 / vs : 0.0;
@@ -299,39 +343,31 @@ obte_status dsa_join(obte_plan plan) {
   return st;
 }
 
-void dsa_add(obte_plan plan, const double* in, double* out) {
+obte_status dsa_add(obte_plan plan, const double* in, const double* base, double* out) {
   DsaOp& op = *plan->dsa;
   const Schedule& s = plan->sched;
-  const int64_t n = s.n;
-  cudaStream_t st = plan->stream;
-  const int num_sms = plan->ctx->num_sms;
-  const int gn = grid_for(n, num_sms);
-  double* b = op.b.as<double>();
-  double* d = op.d.as<double>();
-  double* part = op.mean.as<double>();          // partial sums, one per block of the n-element grid
-  if (op.project) {
-    dsa_partial_kernel<<<gn, DT, 0, st>>>(n, op.vol.as<double>(), in, part);
-    count_launch();
-  }
-  dsa_restrict_kernel<<<gn, DT, 0, st>>>(n, op.vol.as<double>(), op.inv_vol_sum, op.project ? part : nullptr, gn,
-                                         in, b);
+  const PhaseShape ps = phase_shape(s.n, plan->ctx->num_sms);
+  DsaParams f = {};
+  f.n = s.n; f.nd = s.nd; f.nu = plan->nu; f.n_mfp = s.n_mfp;
+  f.project = op.project ? 1 : 0;
+  f.cycles = op.cycles;
+  f.inv_vol_sum = op.inv_vol_sum;
+  f.A = CsrDev{s.n, op.rp.as<int32_t>(), op.ci.as<int32_t>(), op.val.as<double>()};
+  amg_device(*op.amg, f.amg, true);
+  f.vol = op.vol.as<double>();
+  f.wcell = plan->diffuse_cell.as<int32_t>();
+  f.xcell = plan->x_cell.as<int32_t>();
+  f.in = in; f.base = base; f.out = out;
+  f.b = op.b.as<double>(); f.d = op.d.as<double>(); f.r = op.r.as<double>(); f.e = op.e.as<double>();
+  f.part = op.mean.as<double>();
+  unsigned* count = reinterpret_cast<unsigned*>(f.part + 2 * ((s.n + 31) / 32));
+  f.count = count + op.turn;
+  f.count_next = count + (op.turn ^ 1);
+  op.turn ^= 1;
+  f.err = plan->err.as<int>();
+  OBTE_CUDA(phase_launch(ps, dsa_kernel<ClusterBarrier>, dsa_kernel<GridBarrier>, f, 0, plan->stream));
   count_launch();
-  count_launch(amg_apply(*op.amg, b, d, st));
-  for (int c = 1; c < op.cycles; ++c) {
-    dsa_residual_kernel<<<gn, DT, 0, st>>>(n, op.rp.as<int32_t>(), op.ci.as<int32_t>(), op.val.as<double>(), b, d,
-                                           op.r.as<double>());
-    count_launch(amg_apply(*op.amg, op.r.as<double>(), op.e.as<double>(), st));
-    dsa_axpy_kernel<<<gn, DT, 0, st>>>(n, op.e.as<double>(), d);
-    count_launch(2);
-  }
-  if (op.project) {
-    dsa_partial_kernel<<<gn, DT, 0, st>>>(n, op.vol.as<double>(), d, part);
-    count_launch();
-  }
-  dsa_extend_kernel<<<grid_for(plan->nu, num_sms), DT, 0, st>>>(
-      n, s.nd, plan->nu, s.n_mfp, plan->diffuse_cell.as<int32_t>(), plan->x_cell.as<int32_t>(), d,
-      op.project ? part : nullptr, gn, op.inv_vol_sum, out);
-  count_launch();
+  return OBTE_OK;
 }
 
 }  // namespace obte

@@ -516,7 +516,7 @@ extern "C" obte_status obte_fourier_plan_create(obte_context ctx, const obte_fou
   // OBTE_FOURIER_JACOBI=1 keeps the diagonal preconditioner (same solution, ~40x more CG iterations)
   const char* jac = std::getenv("OBTE_FOURIER_JACOBI");
   if (s0 == OBTE_OK && !(jac && std::atoi(jac) != 0))
-    up(amg_build(n, rp, ci, val, pin, ctx->num_sms, st, P->amg));
+    up(amg_build(n, rp, ci, val, pin, st, P->amg));
   if (s0 == OBTE_OK) {
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) s0 = cuda_fail(e, "cudaStreamSynchronize", __FILE__, __LINE__);
@@ -547,7 +547,7 @@ extern "C" obte_status obte_fourier_solve(obte_fourier_plan P, const obte_fourie
   f.n = n;
   f.A = CsrDev{n, P->rp.as<int32_t>(), P->ci.as<int32_t>(), P->val.as<double>()};
   f.has_amg = P->amg ? 1 : 0;
-  if (P->amg) amg_device(*P->amg, f.amg);
+  if (P->amg) amg_device(*P->amg, f.amg, false);
   f.dinv = P->dinv.as<double>(); f.vol = P->vol.as<double>(); f.B = P->B.as<double>(); f.colpin = P->colpin.as<double>();
   f.pin = P->pin; f.nv = P->nv; f.dim = P->dim;
   f.g_nb = P->g_nb.as<int32_t>(); f.g_off = P->g_off.as<double>(); f.g_mixed = P->g_mixed.as<unsigned char>();
@@ -565,7 +565,8 @@ extern "C" obte_status obte_fourier_solve(obte_fourier_plan P, const obte_fourie
   f.count = reinterpret_cast<unsigned*>(f.out + 2);
   f.err = reinterpret_cast<int*>(f.out + 3);
   OBTE_CUDA(cudaMemsetAsync(P->sc.p, 0, 4 * sizeof(double), st));
-  OBTE_CUDA(phase_launch(phase_shape(n, P->ctx->num_sms), fourier_kernel<ClusterBarrier>, fourier_kernel<GridBarrier>, f, st));
+  OBTE_CUDA(phase_launch(phase_shape(n, P->ctx->num_sms), fourier_kernel<ClusterBarrier>, fourier_kernel<GridBarrier>, f,
+                         kPhaseSmem, st));
   count_launch();
   double kappa = 0;
   std::vector<double> kh(std::max<int64_t>(P->nc, 1));

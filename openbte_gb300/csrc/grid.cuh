@@ -14,6 +14,14 @@
 
 namespace obte {
 
+// float -> double, exactly, on the integer pipe for normal numbers (GB300's FP64 pipe converts two lanes a
+// clock per SM; zeros, denormals, infinities and NaN take the conversion instruction)
+__device__ __forceinline__ double widen(float f) {
+  const unsigned b = __float_as_uint(f), e = b & 0x7f800000u;
+  if (e == 0u || e == 0x7f800000u) return (double)f;
+  return __hiloint2double((int)(((b & 0x7fffffffu) >> 3) + (896u << 20) | (b & 0x80000000u)), (int)(b << 29));
+}
+
 // Barrier over the blocks of a cluster.
 struct ClusterBarrier {
   __device__ ClusterBarrier(unsigned*, int*) {}
@@ -125,6 +133,7 @@ struct CsrDev {
   const int32_t* rp;
   const int32_t* ci;
   const double* val;
+  int vec = 0;              // lanes per row, 0: by the block's rows (load_rows)
 };
 constexpr int kAmgMaxLevels = 12;
 struct AmgDev {
@@ -135,7 +144,7 @@ struct AmgDev {
   double* b[kAmgMaxLevels];
   double* x[kAmgMaxLevels];
 };
-void amg_device(const AmgHierarchy& H, AmgDev& d);
+void amg_device(const AmgHierarchy& H, AmgDev& d, bool fixed_order);
 
 // A block's rows [r0, r1) of a matrix; rp, ci and val are its own part, in shared memory where they fit.
 struct Rows {
@@ -164,17 +173,18 @@ struct Arena {
     return r;
   }
 };
-__device__ __forceinline__ void block_range(int64_t n, int& r0, int& r1) {
-  const int per = (int)((n + gridDim.x - 1) / gridDim.x);
+__device__ __forceinline__ void block_range(int64_t n, int& r0, int& r1, int align = 1) {
+  int per = (int)((n + gridDim.x - 1) / gridDim.x);
+  per = (per + align - 1) / align * align;
   r0 = (int)min((int64_t)per * blockIdx.x, n);
   r1 = (int)min((int64_t)per * (blockIdx.x + 1), n);
 }
 // This block's part of a matrix (called by all threads; thread 0 fills `d` in shared memory; a __syncthreads
-// must follow).  The launch reads its matrices some hundred times over: from shared memory the gather of
-// the vector is the only trip to L2 between two barriers.
-__device__ __forceinline__ void load_rows(const CsrDev& m, Rows* d, Arena& ar) {
+// must follow).  A solve reads its matrices some hundred times over: from shared memory the gather of
+// the vector is the only trip to L2 between two barriers.  (An empty arena leaves them where they are.)
+__device__ __forceinline__ void load_rows(const CsrDev& m, Rows* d, Arena& ar, int align = 1) {
   int r0, r1;
-  block_range(m.n, r0, r1);
+  block_range(m.n, r0, r1, align);
   const int nr = r1 - r0, k0 = nr ? m.rp[r0] : 0, k1 = nr ? m.rp[r1] : 0;
   const int32_t *rp = m.rp + r0, *ci = m.ci + k0;
   const double* val = m.val + k0;
@@ -195,18 +205,19 @@ __device__ __forceinline__ void load_rows(const CsrDev& m, Rows* d, Arena& ar) {
     // as many lanes as keep the block's threads on one pass over its rows, at most half a row's entries
     int vec = 1;
     while (vec < 32 && 2 * vec * nr <= (int)blockDim.x && 4 * vec * nr <= k1 - k0) vec *= 2;
-    vec = vec <= 1 ? 1 : vec <= 4 ? 4 : vec <= 8 ? 8 : 32;
+    if (m.vec) vec = m.vec;
     *d = Rows{r0, r1, k0, vec, rp, ci, val};
   }
 }
-__device__ __forceinline__ void load_amg(const AmgDev& A, AmgRows* d, Arena& ar) {
+// align: the blocks' rows of level 0 start at multiples of it
+__device__ __forceinline__ void load_amg(const AmgDev& A, AmgRows* d, Arena& ar, int align = 1) {
   for (int l = 0; l < A.nl - 1; ++l) {
     load_rows(A.Qt[l], &d->Qt[l], ar);
-    load_rows(A.G[l], &d->G[l], ar);
-    load_rows(A.Q[l], &d->Q[l], ar);
+    load_rows(A.G[l], &d->G[l], ar, l == 0 ? align : 1);
+    load_rows(A.Q[l], &d->Q[l], ar, l == 0 ? align : 1);
   }
   int c0, c1;
-  block_range(A.nc, c0, c1);
+  block_range(A.nc, c0, c1, A.nl == 1 ? align : 1);
   const double* inv = A.inv + (size_t)c0 * A.nc;
   const int nv = (c1 - c0) * A.nc;
   if (nv > 0 && nv < (1 << 24))
@@ -247,10 +258,14 @@ __device__ __forceinline__ void block_rows_vec(const Rows* G, FG gx, const Rows&
 template <typename FG, typename FQ, typename FO>
 __device__ __forceinline__ void block_rows(const Rows* G, FG gx, const Rows& Qs, FQ qx, FO out) {
   const Rows Q = Qs;
-  if (Q.vec == 1) block_rows_vec<1>(G, gx, Q, qx, out);
-  else if (Q.vec == 4) block_rows_vec<4>(G, gx, Q, qx, out);
-  else if (Q.vec == 8) block_rows_vec<8>(G, gx, Q, qx, out);
-  else block_rows_vec<32>(G, gx, Q, qx, out);
+  switch (Q.vec) {
+    case 1: block_rows_vec<1>(G, gx, Q, qx, out); break;
+    case 2: block_rows_vec<2>(G, gx, Q, qx, out); break;
+    case 4: block_rows_vec<4>(G, gx, Q, qx, out); break;
+    case 8: block_rows_vec<8>(G, gx, Q, qx, out); break;
+    case 16: block_rows_vec<16>(G, gx, Q, qx, out); break;
+    default: block_rows_vec<32>(G, gx, Q, qx, out);
+  }
 }
 template <typename FQ, typename FO>
 __device__ __forceinline__ void block_rows(const Rows& Q, FQ qx, FO out) {
@@ -309,16 +324,18 @@ inline PhaseShape phase_shape(int64_t n, int num_sms) {
   if (n <= kClusterElems) return {8, kPhaseThreads, true};
   return {num_sms, kPhaseThreads, false};
 }
-constexpr int kPhaseSmem = 200 * 1024;     // of the 227 KB a block can have
+constexpr int kPhaseSmem = 200 * 1024;     // of the 227 KB a block can have, for a solve's matrices
 // Launch kern<ClusterBarrier> or kern<GridBarrier> by the shape.
 template <typename Params>
 cudaError_t phase_launch(const PhaseShape& ps, void (*clustered)(Params), void (*coop)(Params), const Params& p,
-                         cudaStream_t st) {
+                         int smem, cudaStream_t st) {
   void (*kern)(Params) = ps.cluster ? clustered : coop;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPhaseSmem);
-  if (e != cudaSuccess) return e;
+  if (smem > 0) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+  }
   cudaLaunchConfig_t cfg = {};
-  cfg.dynamicSmemBytes = kPhaseSmem;
+  cfg.dynamicSmemBytes = smem;
   cfg.gridDim = dim3(ps.blocks);
   cfg.blockDim = dim3(ps.threads);
   cfg.stream = st;

@@ -163,10 +163,8 @@ using AmgPtr = std::unique_ptr<AmgHierarchy, AmgDeleter>;
 // Hierarchy of the SPD CSR matrix (rp, ci, val); row `pin` (>= 0) is replaced by the identity.  Coarsening
 // stops at `coarse_max` rows or fewer, whose operator is inverted densely (host Gauss-Jordan, O(rows^3)).
 obte_status amg_build(int64_t n, const std::vector<int32_t>& rp, const std::vector<int32_t>& ci,
-                      const std::vector<double>& val, int pin, int num_sms, cudaStream_t st, AmgPtr& out,
+                      const std::vector<double>& val, int pin, cudaStream_t st, AmgPtr& out,
                       int coarse_max = 400);
-// Enqueue z = M^-1 r (one symmetric V-cycle) on `st`.  Returns the number of kernel launches.
-int amg_apply(const AmgHierarchy& H, const double* r, double* z, cudaStream_t st);
 int amg_levels(const AmgHierarchy& H);
 
 }  // namespace obte
@@ -350,8 +348,8 @@ struct SolveWork {
   DevBuf pz;         // preconditioned vector (allocated when the plan has a preconditioner)
   DevBuf rc, Jraw2, Kraw2, Sraw2;   // refinement: correction right-hand side, outputs of the correction
   DevBuf V32, w32;   // FP32 basis and working vector (stages with FP32 sweeps), allocated on first use
-  DevBuf gs;         // device Arnoldi step: second-pass coefficients, Hessenberg column, flags
-  HostBuf hcol;      // pinned copy of the Hessenberg column
+  DevBuf gs;         // barrier counters of the Arnoldi steps
+  HostBuf hcol;      // the Hessenberg column, written by the device
 };
 
 // Diffusion-synthetic acceleration (dsa.cu): right preconditioner term E L^-1 R, with R the volume-
@@ -364,7 +362,8 @@ struct DsaOp {
   DevBuf rp, ci, val;            // L (CSR, symmetric, volume-weighted)
   DevBuf vol;                    // [n]
   DevBuf b, d, r, e, mean;       // right-hand side, correction, residual, cycle update; partial sums of the
-                                 // weighted means (one per block)
+                                 // weighted means and barrier counters
+  int turn = 0;                  // barrier counter of the next application
   double inv_vol_sum = 0;
   bool project = true;           // L has the constant null vector (no isothermal walls)
   int cycles = 1;
@@ -460,7 +459,7 @@ void xprec_add(obte_plan plan, const double* in, double* out, bool fp32);
 int64_t xprec_resident_bytes(const XPrec* P);
 // Diffusion-synthetic acceleration (dsa.cu).
 obte_status ensure_dsa(obte_plan plan);
-void dsa_add(obte_plan plan, const double* in, double* out);    // out += E L^-1 R in
+obte_status dsa_add(obte_plan plan, const double* in, const double* base, double* out);   // out = base + E L^-1 R in
 bool dsa_default(const Schedule& s);                            // on by default for this problem?
 void dsa_start_async(obte_plan plan);                           // build `dsa` on a host thread
 obte_status dsa_join(obte_plan plan);                           // wait for it (OBTE_OK if none ran)

@@ -31,14 +31,13 @@
 #include <cstdlib>
 #include <vector>
 
-#include "internal.h"
+#include "grid.cuh"
 
 namespace obte {
 
 namespace {
 
 constexpr int VT = 256;       // threads per vector block
-constexpr int DOT_TILE = 8;   // vectors per multidot pass
 
 int vec_blocks(const obte_plan plan, int64_t n) {
   const int64_t want = (n + VT - 1) / VT;
@@ -46,244 +45,302 @@ int vec_blocks(const obte_plan plan, int64_t n) {
   return (int)std::max<int64_t>(1, std::min(want, cap));
 }
 
-// partial[b * kk + j] = sum over block b's range of V[j*ld + i] * w[i] for j < k, and w.w for
-// j == k when self != 0 (kk = k + self)
-__global__ void __launch_bounds__(VT) multidot_kernel(const double* __restrict__ V, int64_t ld, int k, int self,
-                                                      const double* __restrict__ w, int64_t n,
-                                                      double* __restrict__ partial, const int* __restrict__ skip) {
-  if (skip && *skip) return;
-  __shared__ double red[VT / 32][DOT_TILE];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int kk = k + self;
-  for (int jt = 0; jt < kk; jt += DOT_TILE) {
-    double acc[DOT_TILE];
-#pragma unroll
-    for (int t = 0; t < DOT_TILE; ++t) acc[t] = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * VT + threadIdx.x; i < n; i += (int64_t)gridDim.x * VT) {
-      const double wi = w[i];
-#pragma unroll
-      for (int t = 0; t < DOT_TILE; ++t) {
-        const int j = jt + t;
-        if (j < k) acc[t] += V[(int64_t)j * ld + i] * wi;
-        else if (j < kk) acc[t] += wi * wi;
-      }
-    }
-#pragma unroll
-    for (int t = 0; t < DOT_TILE; ++t) {
-      double v = acc[t];
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) red[warp][t] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < DOT_TILE && jt + (int)threadIdx.x < kk) {
-      double v = 0;
-      for (int w2 = 0; w2 < VT / 32; ++w2) v += red[w2][threadIdx.x];
-      partial[(int64_t)blockIdx.x * kk + jt + threadIdx.x] = v;
-    }
-    __syncthreads();
-  }
+// partial[b] = sum over block b's range of v[i] w[i]
+__global__ void __launch_bounds__(VT) dot_kernel(const double* __restrict__ v, const double* __restrict__ w, int64_t n,
+                                                 double* __restrict__ partial) {
+  __shared__ double red[VT];
+  double acc = 0.0;
+  for (int64_t i = (int64_t)blockIdx.x * VT + threadIdx.x; i < n; i += (int64_t)gridDim.x * VT) acc += v[i] * w[i];
+  acc = block_sum(acc, threadIdx.x, VT, red);
+  if (threadIdx.x == 0) partial[blockIdx.x] = acc;
 }
 
-// out[j] = sum_b partial[b * k + j]: one block per output, fixed summation tree (deterministic)
-__global__ void __launch_bounds__(VT) reduce_partials_kernel(const double* __restrict__ partial, int nb, int k,
+// out[0] = sum of the nb partials, fixed order
+__global__ void __launch_bounds__(VT) reduce_partials_kernel(const double* __restrict__ partial, int nb,
                                                              double* __restrict__ out) {
-  __shared__ double red[VT / 32];
-  const int j = blockIdx.x;
-  double v = 0;
-  for (int b = threadIdx.x; b < nb; b += VT) v += partial[(int64_t)b * k + j];
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0;
-    for (int w = 0; w < VT / 32; ++w) t += red[w];
-    out[j] = t;
-  }
+  __shared__ double red[VT];
+  const double s = grid_sum(partial, nb, red, [](double v) { return v; });
+  if (threadIdx.x == 0) out[0] = s;
 }
 
-// w -= sum_j h[j] V[j]; partial[b] = sum over block b of the new w^2.  The coefficients sit in
-// shared memory and the basis is read eight vectors at a time, so each thread keeps eight
-// independent loads in flight instead of one load per dependent FMA.
+// x -= sum_j h[j] V[j].  The coefficients sit in shared memory and the basis is read eight vectors at a
+// time, so each thread keeps eight independent loads in flight instead of one load per dependent FMA.
 constexpr int MAX_BASIS = 256;
-__global__ void __launch_bounds__(VT) update_kernel(double* __restrict__ w, const double* __restrict__ V, int64_t ld,
-                                                    int k, const double* __restrict__ h, int64_t n,
-                                                    double* __restrict__ partial, const int* __restrict__ skip) {
-  if (skip && *skip) return;
-  __shared__ double red[VT / 32];
+__device__ __forceinline__ double subtract8(double acc, const double* V, int64_t ld, int k, const double* hs, int64_t i) {
+  int j = 0;
+  for (; j + 8 <= k; j += 8) {
+    double v[8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) v[t] = V[(int64_t)(j + t) * ld + i];
+    double s = 0;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) s += hs[j + t] * v[t];
+    acc -= s;
+  }
+  for (; j < k; ++j) acc -= hs[j] * V[(int64_t)j * ld + i];
+  return acc;
+}
+__global__ void __launch_bounds__(VT) update_kernel(double* __restrict__ x, const double* __restrict__ V, int64_t ld,
+                                                    int k, const double* __restrict__ h, int64_t n) {
   __shared__ double hs[MAX_BASIS];
   for (int j = threadIdx.x; j < k; j += VT) hs[j] = h[j];
   __syncthreads();
-  double ss = 0;
-  for (int64_t i = (int64_t)blockIdx.x * VT + threadIdx.x; i < n; i += (int64_t)gridDim.x * VT) {
-    double acc = w[i];
-    int j = 0;
-    for (; j + 8 <= k; j += 8) {
-      double v[8];
+  for (int64_t i = (int64_t)blockIdx.x * VT + threadIdx.x; i < n; i += (int64_t)gridDim.x * VT)
+    x[i] = subtract8(x[i], V, ld, k, hs, i);
+}
+
+// ---- the Arnoldi step ---------------------------------------------------------------------------
+// One launch orthogonalises w = z - K z against the basis V[0..k) and normalises it: classical Gram-Schmidt with
+// a second pass only when the first one cancelled most of w (Daniel-Gragg-Kaufman-Stewart criterion, |w| after
+// < 0.7 |w| before).  Phases end at a barrier over the blocks (grid.cuh): the products V^T w and w.w, the
+// difference formed on the way; w -= V h and its norm; the same again after the test; the scaled vector and
+// its FP64 copy for the next sweep.  Every block adds up the blocks' sums itself, in a fixed order.  The host
+// reads the Hessenberg column, written to its memory, once per step.
+//
+// As 13 launches of 3.9 us each with its gap a step took 50 us beside its sweep (8,000 triangles x 60 x 48: 46 steps,
+// 14.7 ms a solve; now 12.8).
+//
+// On GB300 the FP64 pipe cannot keep up with HBM for one FMA per 8 loaded bytes, so the stages with FP32 sweeps keep
+// V and w in FP32: FP32 products, per-thread sums and warp sums, FP64 across warps and blocks.  The sweep still
+// takes FP64 input and the solution x stays FP64.  FP32 rows are read 16 bytes at a time (rows padded to a
+// multiple of 4 floats; the n % 4 tail goes through share 0).  The vector is cut into nvb shares of
+// about four float4 per thread, which fixes the order of the FP32 sums whatever the number of blocks; where
+// there are fewer shares than SMs, sp blocks split the basis vectors of a share, in tiles of 16, between them.
+constexpr int DOT_TILE = 16;
+template <typename Real>
+struct ArnoldiParams {
+  int64_t n, ld;
+  int k, nvb, groups, sp;
+  const double *z, *kz;
+  const Real* V;
+  Real *w, *vnext;
+  double* v64;                               // FP64 copy of vnext (FP32 basis)
+  double *part, *s_part;                     // block sums: of the products [k + 1][groups], of w.w [2][groups]
+  double* col;                               // h (+ h2) [k], |w|, second pass ran, 0 when complete
+  unsigned *count, *count_next;
+  int* err;
+};
+
+template <typename Real>
+__device__ __forceinline__ void arnoldi_dots(const ArnoldiParams<Real>& P, bool first, int kk, Real* buf) {
+  const int tid = threadIdx.x, g = blockIdx.x / P.sp, q = blockIdx.x % P.sp, k = P.k;
+  if (g >= P.groups) return;
+  if constexpr (sizeof(Real) == 4) {
+    const int lane = tid & 31, warp = tid >> 5;
+    const int64_t n4 = P.n >> 2, stride = (int64_t)P.nvb * VT;
+    const double2 *z2 = reinterpret_cast<const double2*>(P.z), *kz2 = reinterpret_cast<const double2*>(P.kz);
+    float4* w4 = reinterpret_cast<float4*>(P.w);
+    int ping = 0;
+    for (int jt = q * DOT_TILE; jt < kk; jt += DOT_TILE * P.sp) {
+      // a block forms the differences with its first tile; with several blocks to a share w is written by one
+      // of them, so the others go on forming them
+      const bool form = first && (P.sp > 1 || jt == 0);
+      const float* Vt = P.V + (int64_t)jt * P.ld;
+      const int nt = k - jt;                 // basis vectors of this tile (then w itself, then padding)
+      double tot = 0;
+      for (int vb = g; vb < P.nvb; vb += P.groups) {
+        float acc[DOT_TILE];
 #pragma unroll
-      for (int t = 0; t < 8; ++t) v[t] = V[(int64_t)(j + t) * ld + i];
-      double s = 0;
+        for (int t = 0; t < DOT_TILE; ++t) acc[t] = 0.f;
+        for (int64_t i = (int64_t)vb * VT + tid; i < n4; i += stride) {
+          float4 b;
+          if (form) {
+            const double2 a0 = z2[2 * i], a1 = z2[2 * i + 1], c0 = kz2[2 * i], c1 = kz2[2 * i + 1];
+            b = make_float4((float)(a0.x - c0.x), (float)(a0.y - c0.y), (float)(a1.x - c1.x), (float)(a1.y - c1.y));
+            if (jt == 0) w4[i] = b;
+          } else {
+            b = w4[i];
+          }
 #pragma unroll
-      for (int t = 0; t < 8; ++t) s += hs[j + t] * v[t];
-      acc -= s;
+          for (int t = 0; t < DOT_TILE; ++t) {
+            const float4 a = t < nt ? reinterpret_cast<const float4*>(Vt + (int64_t)t * P.ld)[i] : b;
+            acc[t] = fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, acc[t]))));
+          }
+        }
+        if (vb == 0)
+          for (int64_t i = 4 * n4 + tid; i < P.n; i += VT) {
+            const float b = form ? (float)(P.z[i] - P.kz[i]) : P.w[i];
+            if (form && jt == 0) P.w[i] = b;
+#pragma unroll
+            for (int t = 0; t < DOT_TILE; ++t) acc[t] = fmaf(t < nt ? Vt[(int64_t)t * P.ld + i] : b, b, acc[t]);
+          }
+        float mine = 0.f;
+#pragma unroll
+        for (int t = 0; t < DOT_TILE; ++t) {
+          float v = acc[t];
+          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+          if (lane == t) mine = v;
+        }
+        float* row = buf + ping * (VT / 32) * DOT_TILE;
+        if (lane < DOT_TILE) row[warp * DOT_TILE + lane] = mine;
+        __syncthreads();
+        if (warp == 0) {                     // lane: product lane % 16, warps 4 (lane / 16) to + 3
+          const float* r = row + (lane >> 4) * 4 * DOT_TILE + (lane & 15);
+          double v = (widen(r[0]) + widen(r[DOT_TILE])) + (widen(r[2 * DOT_TILE]) + widen(r[3 * DOT_TILE]));
+          v += __shfl_xor_sync(0xffffffffu, v, 16);
+          tot += v;
+        }
+        ping ^= 1;
+      }
+      if (warp == 0 && lane < DOT_TILE && jt + lane < kk) P.part[(int64_t)(jt + lane) * P.groups + g] = tot;
     }
-    for (; j < k; ++j) acc -= hs[j] * V[(int64_t)j * ld + i];
-    w[i] = acc;
-    ss += acc * acc;
-  }
-  if (partial) {
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0;
-      for (int w2 = 0; w2 < VT / 32; ++w2) t += red[w2];
-      partial[blockIdx.x] = t;
+  } else {
+    for (int jt = q * DOT_TILE; jt < kk; jt += DOT_TILE * P.sp) {
+      const bool form = first && (P.sp > 1 || jt == 0);
+      const double* Vt = P.V + (int64_t)jt * P.ld;
+      const int nt = k - jt, used = min(DOT_TILE, kk - jt);
+      double acc[DOT_TILE];
+#pragma unroll
+      for (int t = 0; t < DOT_TILE; ++t) acc[t] = 0.0;
+      for (int64_t i = (int64_t)g * VT + tid; i < P.n; i += (int64_t)P.groups * VT) {
+        double b;
+        if (form) {
+          b = P.z[i] - P.kz[i];
+          if (jt == 0) P.w[i] = b;
+        } else {
+          b = P.w[i];
+        }
+#pragma unroll
+        for (int t = 0; t < DOT_TILE; ++t)
+          if (t < used) acc[t] += (t < nt ? Vt[(int64_t)t * P.ld + i] : b) * b;
+      }
+      // transposed through shared memory: 16 threads to a product (a shuffle tree per product and warp
+      // would hold the FP64 pipe for longer than the products)
+#pragma unroll
+      for (int t = 0; t < DOT_TILE; ++t)
+        if (t < used) buf[t * VT + tid] = acc[t];
+      __syncthreads();
+      const int t = tid >> 4, part = tid & 15;
+      if ((t & ~1) < used) {                 // whole warps
+        double v[4] = {0, 0, 0, 0};
+        if (t < used)
+#pragma unroll
+          for (int r = 0; r < VT / 16; r += 4)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) v[c] += buf[t * VT + part + 16 * (r + c)];
+        double s = (v[0] + v[1]) + (v[2] + v[3]);
+        for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (part == 0 && t < used) P.part[(int64_t)(jt + t) * P.groups + g] = s;
+      }
+      __syncthreads();
     }
   }
 }
 
-// ---- FP32 Krylov basis (stages whose sweeps are FP32) ------------------------------------------
-// On GB300 the FP64 pipe cannot keep up with HBM for one FMA per 8 loaded bytes, so the Gram-Schmidt
-// passes of the FP32 stages keep the basis V and the new vector w in FP32: FP32 products and
-// per-thread sums, FP64 across threads and blocks.  The sweep still takes FP64 input (one widening
-// pass per Krylov vector) and the solution x stays FP64.
-
-// The two Gram-Schmidt products read 16 bytes per load: V's rows (stride ld) and w must be 16-byte
-// aligned (the FP32 basis rows are padded to a multiple of 4 floats); the n % 4 tail goes through
-// block 0.  They run on fewer blocks than the elementwise kernels so that each thread streams several
-// float4 per tile: with small states (0.9M entries) one scalar per thread and 8-vector tile left the
-// per-tile reductions and barriers dominant.  Warp sums are FP32 (32 partial sums of a few elements
-// each), FP64 from the warp level up: FP64 shuffles kept these kernels on the FP64 pipe.
-
-// partial[b * kk + j] = block b's part of V[j] . w (j < k) and of w . w (j == k when self)
-constexpr int DOT_TILE4 = 16;
-__global__ void __launch_bounds__(VT) multidot32v_kernel(const float* __restrict__ V, int64_t ld, int k, int self,
-                                                         const float* __restrict__ w, int64_t n,
-                                                         double* __restrict__ partial, const int* __restrict__ skip) {
-  if (skip && *skip) return;
-  __shared__ double red[VT / 32][DOT_TILE4];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int kk = k + self;
-  const int64_t n4 = n >> 2;
-  const float4* w4 = reinterpret_cast<const float4*>(w);
-  for (int jt = 0; jt < kk; jt += DOT_TILE4) {
-    const float* vp[DOT_TILE4];
-#pragma unroll
-    for (int t = 0; t < DOT_TILE4; ++t) vp[t] = jt + t < k ? V + (int64_t)(jt + t) * ld : w;   // self / padding read w
-    float acc[DOT_TILE4];
-#pragma unroll
-    for (int t = 0; t < DOT_TILE4; ++t) acc[t] = 0.f;
-    for (int64_t i = (int64_t)blockIdx.x * VT + threadIdx.x; i < n4; i += (int64_t)gridDim.x * VT) {
-      const float4 b = w4[i];
-#pragma unroll
-      for (int t = 0; t < DOT_TILE4; ++t) {
-        const float4 a = reinterpret_cast<const float4*>(vp[t])[i];
-        acc[t] = fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, acc[t]))));
-      }
+// h[j] = sum of product j's block sums, in every block: 8 threads to a product
+template <typename Real>
+__device__ __forceinline__ void arnoldi_sums(const ArnoldiParams<Real>& P, int kk, double* h) {
+  const int part = threadIdx.x & 7;
+  for (int j0 = 0; j0 < kk; j0 += VT / 8) {
+    const int j = j0 + (threadIdx.x >> 3);
+    if (j0 + (int)(threadIdx.x >> 5) * 4 >= kk) break;      // whole warps
+    double v = 0;
+    if (j < kk) {
+      const double* row = P.part + (int64_t)j * P.groups;
+#pragma unroll 8
+      for (int b = part; b < P.groups; b += 8) v += row[b];
     }
-    if (blockIdx.x == 0)
-      for (int64_t i = 4 * n4 + threadIdx.x; i < n; i += VT) {
-        const float b = w[i];
-#pragma unroll
-        for (int t = 0; t < DOT_TILE4; ++t) acc[t] = fmaf(vp[t][i], b, acc[t]);
-      }
-#pragma unroll
-    for (int t = 0; t < DOT_TILE4; ++t) {
-      float v = acc[t];
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) red[warp][t] = (double)v;
-    }
-    __syncthreads();
-    if (threadIdx.x < DOT_TILE4 && jt + (int)threadIdx.x < kk) {
-      double v = 0;
-      for (int w2 = 0; w2 < VT / 32; ++w2) v += red[w2][threadIdx.x];
-      partial[(int64_t)blockIdx.x * kk + jt + threadIdx.x] = v;
-    }
-    __syncthreads();
+    if (P.groups > 1)
+      for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (part == 0 && j < kk) h[j] = v;
   }
-}
-
-// w -= sum_j h[j] V[j] (FP32); partial[b] = block b's part of the new w . w
-__global__ void __launch_bounds__(VT) update32v_kernel(float* __restrict__ w, const float* __restrict__ V, int64_t ld,
-                                                       int k, const double* __restrict__ h, int64_t n,
-                                                       double* __restrict__ partial, const int* __restrict__ skip) {
-  if (skip && *skip) return;
-  __shared__ double red[VT / 32];
-  __shared__ float hs[MAX_BASIS];
-  for (int j = threadIdx.x; j < k; j += VT) hs[j] = (float)h[j];
   __syncthreads();
-  const int64_t n4 = n >> 2;
-  float4* w4 = reinterpret_cast<float4*>(w);
-  float ss = 0.f;
-  for (int64_t i = (int64_t)blockIdx.x * VT + threadIdx.x; i < n4; i += (int64_t)gridDim.x * VT) {
-    float4 acc = w4[i];
-#pragma unroll 4
-    for (int j = 0; j < k; ++j) {
-      const float4 v = reinterpret_cast<const float4*>(V + (int64_t)j * ld)[i];
-      const float c = -hs[j];
-      acc.x = fmaf(c, v.x, acc.x);
-      acc.y = fmaf(c, v.y, acc.y);
-      acc.z = fmaf(c, v.z, acc.z);
-      acc.w = fmaf(c, v.w, acc.w);
+}
+
+// w -= V h on the share's first block; its part of w.w
+template <typename Real>
+__device__ __forceinline__ void arnoldi_update(const ArnoldiParams<Real>& P, const double* h, double* s_part,
+                                               Real* hs, double* red) {
+  const int tid = threadIdx.x, g = blockIdx.x / P.sp, k = P.k;
+  if (g >= P.groups || blockIdx.x % P.sp != 0) return;
+  for (int j = tid; j < k; j += VT) hs[j] = (Real)h[j];
+  __syncthreads();
+  double sum = 0;
+  if constexpr (sizeof(Real) == 4) {
+    const int64_t n4 = P.n >> 2, stride = (int64_t)P.nvb * VT;
+    float4* w4 = reinterpret_cast<float4*>(P.w);
+    for (int vb = g; vb < P.nvb; vb += P.groups) {
+      float ss = 0.f;
+      for (int64_t i = (int64_t)vb * VT + tid; i < n4; i += stride) {
+        float4 acc = w4[i];
+#pragma unroll 8
+        for (int j = 0; j < k; ++j) {
+          const float4 v = reinterpret_cast<const float4*>(P.V + (int64_t)j * P.ld)[i];
+          const float c = -hs[j];
+          acc.x = fmaf(c, v.x, acc.x);
+          acc.y = fmaf(c, v.y, acc.y);
+          acc.z = fmaf(c, v.z, acc.z);
+          acc.w = fmaf(c, v.w, acc.w);
+        }
+        w4[i] = acc;
+        ss = fmaf(acc.x, acc.x, fmaf(acc.y, acc.y, fmaf(acc.z, acc.z, fmaf(acc.w, acc.w, ss))));
+      }
+      if (vb == 0)
+        for (int64_t i = 4 * n4 + tid; i < P.n; i += VT) {
+          float acc = P.w[i];
+          for (int j = 0; j < k; ++j) acc = fmaf(-hs[j], P.V[(int64_t)j * P.ld + i], acc);
+          P.w[i] = acc;
+          ss = fmaf(acc, acc, ss);
+        }
+      sum += widen(ss);
     }
-    w4[i] = acc;
-    ss = fmaf(acc.x, acc.x, fmaf(acc.y, acc.y, fmaf(acc.z, acc.z, fmaf(acc.w, acc.w, ss))));
+  } else {
+    for (int64_t i = (int64_t)g * VT + tid; i < P.n; i += (int64_t)P.groups * VT) {
+      const double acc = subtract8(P.w[i], P.V, P.ld, k, hs, i);
+      P.w[i] = acc;
+      sum += acc * acc;
+    }
+  }
+  sum = block_sum(sum, tid, VT, red);
+  if (tid == 0) s_part[g] = sum;
+}
+
+template <typename Bar, typename Real>
+__global__ void __launch_bounds__(VT, 2) arnoldi_kernel(const __grid_constant__ ArnoldiParams<Real> P) {
+  __shared__ double red[VT];
+  __shared__ double h[MAX_BASIS + 1], h2[MAX_BASIS];
+  __shared__ Real hs[MAX_BASIS];
+  __shared__ Real buf[sizeof(Real) == 4 ? 2 * (VT / 32) * DOT_TILE : DOT_TILE * VT];
+  __shared__ double sc;
+  Bar bar(P.count, P.err);
+  const int tid = threadIdx.x, k = P.k;
+  if (blockIdx.x == 0 && tid == 0) *P.count_next = 0;
+  arnoldi_dots(P, true, k + 1, buf);
+  if (!bar.wait()) return;
+  arnoldi_sums(P, k + 1, h);
+  arnoldi_update(P, h, P.s_part, hs, red);
+  if (!bar.wait()) return;
+  double s = 0;                              // w.w after the passes so far; thread 0's
+  const bool two = grid_sum(P.s_part, P.groups, red, [&](double v) {
+                     s = v;
+                     return sqrt(fmax(v, 0.0)) < 0.7 * sqrt(fmax(h[k], 0.0)) ? 1.0 : 0.0;
+                   }) != 0;
+  if (two) {
+    arnoldi_dots(P, false, k, buf);
+    if (!bar.wait()) return;
+    arnoldi_sums(P, k, h2);
+    arnoldi_update(P, h2, P.s_part + P.groups, hs, red);
+    if (!bar.wait()) return;
+    grid_sum(P.s_part + P.groups, P.groups, red, [&](double v) { return s = v; });
+  }
+  if (tid == 0) {
+    const double hn = sqrt(fmax(s, 0.0));
+    sc = hn > 0 ? 1.0 / hn : 0.0;
+    if (blockIdx.x == 0) {
+      P.col[k] = hn;
+      P.col[k + 1] = two ? 1.0 : 0.0;
+      P.col[k + 2] = 0.0;
+    }
   }
   if (blockIdx.x == 0)
-    for (int64_t i = 4 * n4 + threadIdx.x; i < n; i += VT) {
-      float acc = w[i];
-      for (int j = 0; j < k; ++j) acc = fmaf(-hs[j], V[(int64_t)j * ld + i], acc);
-      w[i] = acc;
-      ss = fmaf(acc, acc, ss);
-    }
-  double sd = (double)ss;
-  for (int o = 16; o > 0; o >>= 1) sd += __shfl_xor_sync(0xffffffffu, sd, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sd;
+    for (int i = tid; i < k; i += VT) P.col[i] = two ? h[i] + h2[i] : h[i];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0;
-    for (int w2 = 0; w2 < VT / 32; ++w2) t += red[w2];
-    partial[blockIdx.x] = t;
+  const Real inv = (Real)sc;
+  for (int64_t i = (int64_t)blockIdx.x * VT + tid; i < P.n; i += (int64_t)gridDim.x * VT) {
+    const Real v = inv * P.w[i];
+    P.vnext[i] = v;
+    if constexpr (sizeof(Real) == 4) P.v64[i] = widen(v);
   }
-}
-
-// Device side of the Arnoldi step (no host round trip between the Gram-Schmidt passes).
-// DGKS test after the first pass: skip[0] = 1 (no second pass) unless the projection left less than
-// 0.7 of the norm w had before it (h[k] = w . w before, s[0] = w . w after).
-__global__ void gs_check_kernel(const double* __restrict__ h, int k, const double* __restrict__ s,
-                                int* __restrict__ skip) {
-  if (threadIdx.x == 0) skip[0] = sqrt(fmax(s[0], 0.0)) < 0.7 * sqrt(fmax(h[k], 0.0)) ? 0 : 1;
-}
-
-// Hessenberg column of the step: col[i] = h[i] (+ h2[i] after a second pass) for i < k, col[k] = ‖w‖,
-// col[k + 1] = 1 when the second pass ran; inv[0] = 1 / ‖w‖ in FP32 and inv64[0] in FP64 (0 for a zero
-// vector).
-__global__ void gs_finish_kernel(const double* __restrict__ h, const double* __restrict__ h2, int k,
-                                 const double* __restrict__ s, const int* __restrict__ skip,
-                                 double* __restrict__ col, float* __restrict__ inv, double* __restrict__ inv64) {
-  const bool two = skip[0] == 0;
-  for (int i = threadIdx.x; i < k; i += blockDim.x) col[i] = two ? h[i] + h2[i] : h[i];
-  if (threadIdx.x == 0) {
-    const double hn = sqrt(fmax(two ? s[1] : s[0], 0.0));
-    col[k] = hn;
-    col[k + 1] = two ? 1.0 : 0.0;
-    inv[0] = hn > 0 ? (float)(1.0 / hn) : 0.f;
-    inv64[0] = hn > 0 ? 1.0 / hn : 0.0;
-  }
-}
-
-// y = a[0] x (scale read from the device)
-__global__ void scaled_kernel(const double* __restrict__ a, const double* __restrict__ x, double* __restrict__ y,
-                              int64_t n) {
-  const double s = *a;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    y[i] = s * x[i];
-}
-__global__ void scale32d_kernel(const float* __restrict__ a, const float* __restrict__ x, float* __restrict__ y,
-                                int64_t n) {
-  const float s = *a;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    y[i] = s * x[i];
 }
 
 // x += sum_j y[j] V[j] (FP32 combination, FP64 accumulate into x)
@@ -299,23 +356,15 @@ __global__ void __launch_bounds__(VT) xupdate32_kernel(double* __restrict__ x, c
   }
 }
 
-// y = (float)(a * x)
-__global__ void scale_to_f32_kernel(double a, const double* __restrict__ x, float* __restrict__ y, int64_t n) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    y[i] = (float)(a * x[i]);
+// y = (float)(a * x), y64 = (double)y
+__global__ void scale_to_f32_kernel(double a, const double* __restrict__ x, float* __restrict__ y,
+                                    double* __restrict__ y64, int64_t n) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const float v = (float)(a * x[i]);
+    y[i] = v;
+    y64[i] = widen(v);
+  }
 }
-// y = (double)x
-__global__ void widen_kernel(const float* __restrict__ x, double* __restrict__ y, int64_t n) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    y[i] = (double)x[i];
-}
-// w = (float)(a - b)
-__global__ void diff_to_f32_kernel(const double* __restrict__ a, const double* __restrict__ b, float* __restrict__ w,
-                                   int64_t n) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    w[i] = (float)(a[i] - b[i]);
-}
-
 // y = a*x + b*y
 // y += x
 __global__ void add_kernel(double* __restrict__ y, const double* __restrict__ x, int64_t n) {
@@ -407,18 +456,20 @@ struct Solver {
   // a final pass that recomputes the true residual follows every gmres call: end a cycle whose Arnoldi
   // estimate met the tolerance without the confirming sweep
   bool estimate_exit = false;
-  // out += (M^-1 - I) in: W in on the slow inflow blocks, E L^-1 R in of the diffusion correction
-  void prec_add(const double* in, double* out, bool fp32) {
-    if (xblocks) xprec_add(plan, in, out, fp32);
-    if (dsa) dsa_add(plan, in, out);
-  }
-  // out = M^-1 in
-  obte_status prec(const double* in, double* out, bool fp32) {
-    OBTE_CUDA(cudaMemcpyAsync(out, in, (size_t)wk.nu * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    prec_add(in, out, fp32);
+  // out = base + (M^-1 - I) in: W in on the slow inflow blocks, E L^-1 R in of the diffusion correction
+  obte_status prec_add(const double* in, const double* base, double* out, bool fp32) {
+    if (xblocks) {
+      if (base != out)
+        OBTE_CUDA(cudaMemcpyAsync(out, base, (size_t)wk.nu * sizeof(double), cudaMemcpyDeviceToDevice, st));
+      xprec_add(plan, in, out, fp32);
+      base = out;
+    }
+    if (dsa) OBTE_TRY(dsa_add(plan, in, base, out));
     OBTE_CUDA(cudaGetLastError());
     return OBTE_OK;
   }
+  // out = M^-1 in
+  obte_status prec(const double* in, double* out, bool fp32) { return prec_add(in, in, out, fp32); }
 
   obte_status sweep(bool fp32, const double* in, double* out, bool src, bool fin = false) {
     ++sweeps;
@@ -432,23 +483,19 @@ struct Solver {
     ++sweeps_df;
     return launch_sweep_df(plan, in, out, true, wk.Jraw.as<double>(), wk.Kraw.as<double>(), wk.Sraw.as<double>());
   }
-  // h[0..k) = V[0..k)^T w (and h[k] = w.w when self), copied to host
-  obte_status multidot(const double* V, int k, const double* w, std::vector<double>& h, bool self = false) {
-    const int64_t n = wk.nu;
-    const int kk = k + (self ? 1 : 0);
-    multidot_kernel<<<wk.nb, VT, 0, st>>>(V, n, k, self ? 1 : 0, w, n, wk.partial.as<double>(), nullptr);
-    reduce_partials_kernel<<<kk, VT, 0, st>>>(wk.partial.as<double>(), wk.nb, kk, wk.hdev.as<double>());
+  // out = v . w, on the host
+  obte_status dot(const double* v, const double* w, double& out) {
+    dot_kernel<<<wk.nb, VT, 0, st>>>(v, w, wk.nu, wk.partial.as<double>());
+    reduce_partials_kernel<<<1, VT, 0, st>>>(wk.partial.as<double>(), wk.nb, wk.hdev.as<double>());
     count_launch(2);
     OBTE_CUDA(cudaGetLastError());
-    h.resize(kk);
-    OBTE_CUDA(cudaMemcpyAsync(h.data(), wk.hdev.p, kk * sizeof(double), cudaMemcpyDeviceToHost, st));
+    OBTE_CUDA(cudaMemcpyAsync(&out, wk.hdev.p, sizeof(double), cudaMemcpyDeviceToHost, st));
     OBTE_CUDA(wait_stream(st));
     return OBTE_OK;
   }
   obte_status norm(const double* x, double& out) {
-    std::vector<double> h;
-    OBTE_TRY(multidot(x, 1, x, h));
-    out = std::sqrt(std::max(h[0], 0.0));
+    OBTE_TRY(dot(x, x, out));
+    out = std::sqrt(std::max(out, 0.0));
     return OBTE_OK;
   }
   obte_status lincomb(double a, const double* x, double b, const double* y, double* z) {
@@ -477,27 +524,55 @@ struct Solver {
     return OBTE_OK;
   }
 
-  // Device Arnoldi scratch: second-pass coefficients [m+1], Hessenberg column [m+3], norms [2], DGKS flag,
-  // 1/‖w‖ in FP32 and FP64; and the pinned host copy of the column.
-  struct GsScratch {
-    double *h2, *col, *s, *inv64;
-    int* skip;
-    float* inv;
-  };
-  obte_status gs_scratch(GsScratch& g) {
-    const int m = wk.restart;
-    if (!wk.gs.p) OBTE_TRY(wk.gs.alloc((size_t)(2 * m + 9) * sizeof(double)));
-    if (!wk.hcol.p) OBTE_TRY(wk.hcol.alloc((size_t)(m + 3) * sizeof(double)));
-    g.h2 = wk.gs.as<double>();
-    g.col = g.h2 + (m + 1);
-    g.s = g.col + (m + 3);
-    g.skip = reinterpret_cast<int*>(g.s + 2);
-    g.inv = reinterpret_cast<float*>(g.s + 3);
-    g.inv64 = g.s + 4;
+  // Barrier counters of the Arnoldi steps, two that steps use in turn, and the host's Hessenberg column.
+  int turn = 0;
+  obte_status arnoldi_begin() {
+    if (!wk.gs.p) OBTE_TRY(wk.gs.alloc(2 * sizeof(unsigned)));
+    if (!wk.hcol.p) OBTE_TRY(wk.hcol.alloc((size_t)(wk.restart + 4) * sizeof(double)));
+    OBTE_CUDA(cudaMemsetAsync(wk.gs.p, 0, 2 * sizeof(unsigned), st));
+    turn = 0;
+    return OBTE_OK;
+  }
+  // V[k] and the Hessenberg column of w = z - kz against V[0..k), column in wk.hcol
+  template <typename Real>
+  obte_status arnoldi(const double* z, const double* kz, Real* V, int64_t ld, int k, Real* w, double* v64) {
+    const int64_t n = wk.nu;
+    const int num_sms = plan->ctx->num_sms;
+    ArnoldiParams<Real> f = {};
+    f.n = n; f.ld = ld; f.k = k;
+    f.z = z; f.kz = kz; f.V = V; f.w = w; f.vnext = V + (int64_t)k * ld; f.v64 = v64;
+    const int tiles = (k + DOT_TILE) / DOT_TILE;
+    // shares: about 4 float4 per thread and tile, at most the elementwise grid (FP32); a row per thread (FP64)
+    f.nvb = sizeof(Real) == 4 ? (int)std::max<int64_t>(1, std::min<int64_t>(wk.nb, (n / 4 + 4 * VT - 1) / (4 * VT)))
+                              : (int)std::min<int64_t>((n + VT - 1) / VT, 2 * num_sms);
+    f.groups = std::min(f.nvb, 2 * num_sms);             // two blocks to an SM
+    f.sp = std::max(1, std::min(tiles, num_sms / f.groups));
+    PhaseShape ps{f.groups * f.sp, VT, false};
+    if (ps.blocks <= 8) {
+      ps.cluster = true;
+      while (ps.blocks & (ps.blocks - 1)) ++ps.blocks;   // blocks above groups * sp only wait
+    }
+    f.part = wk.partial.as<double>();
+    f.s_part = f.part + (int64_t)(k + 1) * f.groups;
+    unsigned* count = wk.gs.as<unsigned>();
+    f.count = count + turn;
+    f.count_next = count + (turn ^ 1);
+    turn ^= 1;
+    f.col = wk.hcol.as<double>();
+    f.col[k + 2] = 1.0;                                  // until the kernel is through
+    f.err = plan->err.as<int>();
+    OBTE_CUDA(phase_launch(ps, arnoldi_kernel<ClusterBarrier, Real>, arnoldi_kernel<GridBarrier, Real>, f, 0, st));
+    count_launch();
+    OBTE_CUDA(wait_stream(st));
+    if (f.col[k + 2] != 0.0) {
+      OBTE_TRY(check_device_error(plan));
+      set_error("the Arnoldi kernel did not complete");
+      return OBTE_ERR_DEVICE_TIMEOUT;
+    }
     return OBTE_OK;
   }
 
-  // Restarted GMRES with the FP32 basis (see multidot32v_kernel); same contract as gmres().
+  // Restarted GMRES with the FP32 basis (see arnoldi_kernel); same contract as gmres().
   obte_status gmres32(const double* rhs, double* x, double tol_rel, double tol_abs, double& res_out, bool& ok) {
     const int64_t n = wk.nu;
     const int m = wk.restart;
@@ -511,18 +586,8 @@ struct Solver {
     double* vj64 = wk.w.as<double>();
     double* r = wk.r.as<double>();
     const int nb = wk.nb;
-    // Gram-Schmidt kernels: about 4 float4 per thread and tile, at most the elementwise grid
-    const int nbg = (int)std::max<int64_t>(1, std::min<int64_t>(nb, (n / 4 + 4 * VT - 1) / (4 * VT)));
-    GsScratch gsd;
-    OBTE_TRY(gs_scratch(gsd));
-    double* h2d = gsd.h2;
-    double* cold = gsd.col;
-    double* sd = gsd.s;
-    int* skipd = gsd.skip;
-    float* invd = gsd.inv;
+    OBTE_TRY(arnoldi_begin());
     const double* hc = wk.hcol.as<double>();
-    double* hdev = wk.hdev.as<double>();
-    double* part = wk.partial.as<double>();
     std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1);
     ok = false;
     if (x_zero && rhs) OBTE_TRY(lincomb(1.0, rhs, 0.0, rhs, r));
@@ -537,7 +602,7 @@ struct Solver {
       const double tol = std::max(tol_abs, tol_rel * std::max(xn, beta));
       if (beta <= tol) { ok = true; return OBTE_OK; }
       if (sweeps >= max_sweeps) return OBTE_OK;
-      scale_to_f32_kernel<<<nb, VT, 0, st>>>(1.0 / beta, r, V, n);
+      scale_to_f32_kernel<<<nb, VT, 0, st>>>(1.0 / beta, r, V, vj64, n);
       count_launch();
       std::fill(g.begin(), g.end(), 0.0);
       g[0] = beta;
@@ -546,37 +611,15 @@ struct Solver {
       for (; j < m && sweeps < max_sweeps; ++j) {
         const auto w0 = std::chrono::steady_clock::now();
         if (trace) cudaEventRecord(ev[0], st);
-        widen_kernel<<<nb, VT, 0, st>>>(V + (int64_t)j * ld, vj64, n);
-        count_launch();
-        const double* zj = vj64;              // z_j = M^-1 v_j
+        const double* zj = vj64;              // z_j = M^-1 v_j (vj64: V[j] in FP64)
         if (xp) {
           OBTE_TRY(prec(vj64, wk.pz.as<double>(), true));
           zj = wk.pz.as<double>();
         }
         OBTE_TRY(sweep(true, zj, wk.tmp.as<double>(), false));
         if (trace) cudaEventRecord(ev[1], st);
-        diff_to_f32_kernel<<<nb, VT, 0, st>>>(zj, wk.tmp.as<double>(), w, n);
-        count_launch();
-        OBTE_CUDA(cudaGetLastError());
-        // classical Gram-Schmidt with one conditional re-orthogonalisation (as in gmres()), all on the
-        // device: the second pass's kernels return at once when the DGKS test declines it, and the
-        // host reads the finished Hessenberg column once per step
         const int k = j + 1;
-        multidot32v_kernel<<<nbg, VT, 0, st>>>(V, ld, k, 1, w, n, part, nullptr);
-        reduce_partials_kernel<<<k + 1, VT, 0, st>>>(part, nbg, k + 1, hdev);
-        update32v_kernel<<<nbg, VT, 0, st>>>(w, V, ld, k, hdev, n, part, nullptr);
-        reduce_partials_kernel<<<1, VT, 0, st>>>(part, nbg, 1, sd);
-        gs_check_kernel<<<1, 32, 0, st>>>(hdev, k, sd, skipd);
-        multidot32v_kernel<<<nbg, VT, 0, st>>>(V, ld, k, 0, w, n, part, skipd);
-        reduce_partials_kernel<<<k, VT, 0, st>>>(part, nbg, k, h2d);
-        update32v_kernel<<<nbg, VT, 0, st>>>(w, V, ld, k, h2d, n, part, skipd);
-        reduce_partials_kernel<<<1, VT, 0, st>>>(part, nbg, 1, sd + 1);
-        gs_finish_kernel<<<1, 128, 0, st>>>(hdev, h2d, k, sd, skipd, cold, invd, gsd.inv64);
-        scale32d_kernel<<<nb, VT, 0, st>>>(invd, w, V + (int64_t)k * ld, n);
-        count_launch(11);
-        OBTE_CUDA(cudaGetLastError());
-        OBTE_CUDA(cudaMemcpyAsync(wk.hcol.p, cold, (size_t)(k + 2) * sizeof(double), cudaMemcpyDeviceToHost, st));
-        OBTE_CUDA(wait_stream(st));
+        OBTE_TRY(arnoldi<float>(zj, wk.tmp.as<double>(), V, ld, k, w, vj64));
         const double hn = hc[k];
         for (int i = 0; i <= j; ++i) H[(size_t)i * m + j] = hc[i];
         H[(size_t)(j + 1) * m + j] = hn;
@@ -621,7 +664,7 @@ struct Solver {
           xupdate32_kernel<<<nb, VT, 0, st>>>(z, V, ld, j, wk.hdev.as<double>(), n);
           count_launch();
           OBTE_TRY(axpby(1.0, z, 1.0, x));
-          prec_add(z, x, true);
+          OBTE_TRY(prec_add(z, x, x, true));
         } else {
           xupdate32_kernel<<<nb, VT, 0, st>>>(x, V, ld, j, wk.hdev.as<double>(), n);
           count_launch();
@@ -656,12 +699,8 @@ struct Solver {
     double* V = wk.V.as<double>();
     double* w = wk.w.as<double>();
     double* r = wk.r.as<double>();
-    GsScratch gsd;
-    OBTE_TRY(gs_scratch(gsd));
+    OBTE_TRY(arnoldi_begin());
     const double* hc = wk.hcol.as<double>();
-    double* hdev = wk.hdev.as<double>();
-    double* part = wk.partial.as<double>();
-    const int nb = wk.nb;
     std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1);
     ok = false;
     if (x_zero && rhs) OBTE_TRY(lincomb(1.0, rhs, 0.0, rhs, r));
@@ -692,27 +731,8 @@ struct Solver {
         }
         OBTE_TRY(sweep(fp32, zj, wk.tmp.as<double>(), false));
         if (trace) cudaEventRecord(ev[1], st);
-        OBTE_TRY(lincomb(1.0, zj, -1.0, wk.tmp.as<double>(), w));
-        // classical Gram-Schmidt; a second pass only when the first one cancelled most of w
-        // (Daniel-Gragg-Kaufman-Stewart criterion, ‖w‖ after < 0.7 ‖w‖ before).  The whole step runs on
-        // the device (the second pass's kernels return at once when the test declines it) and the host
-        // reads the Hessenberg column once.
         const int k = j + 1;
-        multidot_kernel<<<nb, VT, 0, st>>>(V, n, k, 1, w, n, part, nullptr);   // h[0..j] and w.w in one pass
-        reduce_partials_kernel<<<k + 1, VT, 0, st>>>(part, nb, k + 1, hdev);
-        update_kernel<<<nb, VT, 0, st>>>(w, V, n, k, hdev, n, part, nullptr);
-        reduce_partials_kernel<<<1, VT, 0, st>>>(part, nb, 1, gsd.s);
-        gs_check_kernel<<<1, 32, 0, st>>>(hdev, k, gsd.s, gsd.skip);
-        multidot_kernel<<<nb, VT, 0, st>>>(V, n, k, 0, w, n, part, gsd.skip);
-        reduce_partials_kernel<<<k, VT, 0, st>>>(part, nb, k, gsd.h2);
-        update_kernel<<<nb, VT, 0, st>>>(w, V, n, k, gsd.h2, n, part, gsd.skip);
-        reduce_partials_kernel<<<1, VT, 0, st>>>(part, nb, 1, gsd.s + 1);
-        gs_finish_kernel<<<1, 128, 0, st>>>(hdev, gsd.h2, k, gsd.s, gsd.skip, gsd.col, gsd.inv, gsd.inv64);
-        scaled_kernel<<<nb, VT, 0, st>>>(gsd.inv64, w, V + (int64_t)k * n, n);
-        count_launch(11);
-        OBTE_CUDA(cudaGetLastError());
-        OBTE_CUDA(cudaMemcpyAsync(wk.hcol.p, gsd.col, (size_t)(k + 2) * sizeof(double), cudaMemcpyDeviceToHost, st));
-        OBTE_CUDA(wait_stream(st));
+        OBTE_TRY(arnoldi<double>(zj, wk.tmp.as<double>(), V, n, k, w, nullptr));
         const double hn = hc[k];
         // Hessenberg column j
         for (int i = 0; i <= j; ++i) H[(size_t)i * m + j] = hc[i];
@@ -757,12 +777,12 @@ struct Solver {
         if (xp) {                             // x += M^-1 (V y)
           double* z = wk.pz.as<double>();
           OBTE_CUDA(cudaMemsetAsync(z, 0, (size_t)n * sizeof(double), st));
-          update_kernel<<<wk.nb, VT, 0, st>>>(z, V, n, j, wk.hdev.as<double>(), n, nullptr, nullptr);
+          update_kernel<<<wk.nb, VT, 0, st>>>(z, V, n, j, wk.hdev.as<double>(), n);
           count_launch();
           OBTE_TRY(axpby(1.0, z, 1.0, x));
-          prec_add(z, x, false);
+          OBTE_TRY(prec_add(z, x, x, false));
         } else {
-          update_kernel<<<wk.nb, VT, 0, st>>>(x, V, n, j, wk.hdev.as<double>(), n, nullptr, nullptr);
+          update_kernel<<<wk.nb, VT, 0, st>>>(x, V, n, j, wk.hdev.as<double>(), n);
           count_launch();
         }
         OBTE_CUDA(cudaGetLastError());
@@ -783,6 +803,10 @@ struct Solver {
 
 }  // namespace
 
+// block sums of a product (dot) and of an Arnoldi step ([restart + 1] products and two norms, at most two blocks to an SM)
+static size_t partial_doubles(obte_plan plan, int nb, int restart) {
+  return std::max<size_t>(nb, (size_t)(restart + 3) * std::min(nb, 2 * plan->ctx->num_sms));
+}
 static obte_status alloc_work(obte_plan plan, Work& wk, int restart) {
   PhaseTimer timer("alloc_work");
   const Schedule& s = plan->sched;
@@ -796,7 +820,7 @@ static obte_status alloc_work(obte_plan plan, Work& wk, int restart) {
   OBTE_TRY(wk.w.alloc(vb));
   OBTE_TRY(wk.tmp.alloc(vb));
   OBTE_TRY(wk.delta.alloc(vb));
-  OBTE_TRY(wk.partial.alloc((size_t)wk.nb * (restart + 1) * sizeof(double)));
+  OBTE_TRY(wk.partial.alloc(partial_doubles(plan, wk.nb, restart) * sizeof(double)));
   OBTE_TRY(wk.hdev.alloc((size_t)(restart + 2) * sizeof(double)));
   OBTE_TRY(wk.sdev.alloc(8 * sizeof(double)));
   OBTE_TRY(wk.Jraw.alloc((size_t)s.n * s.ds * sizeof(double)));
@@ -810,7 +834,7 @@ int64_t solve_scratch_bytes(obte_plan plan, int restart) {
   const int64_t vb = plan->nu * (int64_t)sizeof(double);
   // u Fu r w tmp delta pz rc, the FP64 and FP32 bases, two sets of J/K/S accumulators, partials, Arnoldi scratch
   return vb * (8 + restart + 1) + ((plan->nu + 3) & ~3LL) * 4LL * (restart + 2) + 2 * ((int64_t)s.n * s.ds * 8 + 2LL * s.n_mfp * s.n_dir * 8) +
-         (int64_t)plan->ctx->num_sms * 4 * (restart + 1) * 8 + (2LL * restart + 9) * 8;
+         (int64_t)plan->ctx->num_sms * 2 * (restart + 3) * 8 + 8;
 }
 
 }  // namespace obte
@@ -939,9 +963,8 @@ extern "C" obte_status obte_bte_solve(obte_plan plan, const obte_solve_opts* opt
   count_launch();
   OBTE_CUDA(cudaGetLastError());
   // conserved ell.u of the initial state (DeltaT and T_B parts)
-  std::vector<double> h;
-  OBTE_TRY(sv.multidot(u0, 1, plan->ell.as<double>(), h));
-  const double ell0 = h[0];
+  double ell0;
+  OBTE_TRY(sv.dot(u0, plan->ell.as<double>(), ell0));
 
   double unorm;
   OBTE_TRY(sv.norm(u, unorm));
@@ -1040,8 +1063,9 @@ extern "C" obte_status obte_bte_solve(obte_plan plan, const obte_solve_opts* opt
   // offset: ell.(Fu + c) = ell0 (none with isothermal walls, whose fixed point is unique)
   double c = 0;
   if (!s.isothermal) {
-    OBTE_TRY(sv.multidot(Fu, 1, plan->ell.as<double>(), h));
-    c = (ell0 - h[0]) / plan->ell_sum;
+    double ell1;
+    OBTE_TRY(sv.dot(Fu, plan->ell.as<double>(), ell1));
+    c = (ell0 - ell1) / plan->ell_sum;
   }
   const double s0 = s.ds > 0 ? s.sig_sum[0] : 0, s1 = s.ds > 1 ? s.sig_sum[1] : 0, s2 = s.ds > 2 ? s.sig_sum[2] : 0;
   finalize_kernel<<<wk.nb, VT, 0, st>>>(Fu, u, s.n, c, wk.Jraw.as<double>(), s.ds, s0, s1, s2,

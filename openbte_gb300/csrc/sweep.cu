@@ -34,7 +34,7 @@
 #include <mutex>
 #include <numeric>
 
-#include "internal.h"
+#include "grid.cuh"
 
 namespace obte {
 
@@ -593,13 +593,6 @@ __device__ __forceinline__ float dpack_lo(double x) { return __int_as_float(__do
 __device__ __forceinline__ double dpack_value(double x) { return (double)dpack_hi(x) + (double)dpack_lo(x); }
 __device__ __forceinline__ df2 dunpack2(double a, double b) {   // two packed pairs -> lanes x, y
   return {make_float2(dpack_hi(a), dpack_hi(b)), make_float2(dpack_lo(a), dpack_lo(b))};
-}
-// float -> double, exactly, on the integer pipe for normal numbers (GB300's FP64 pipe converts two lanes a
-// clock per SM; zeros, denormals, infinities and NaN take the conversion instruction)
-__device__ __forceinline__ double widen(float f) {
-  const unsigned b = __float_as_uint(f), e = b & 0x7f800000u;
-  if (e == 0u || e == 0x7f800000u) return (double)f;
-  return __hiloint2double((int)(((b & 0x7fffffffu) >> 3) + (896u << 20) | (b & 0x80000000u)), (int)(b << 29));
 }
 __device__ __forceinline__ double widen(double f) { return f; }
 
