@@ -228,6 +228,7 @@ struct Schedule {
   std::vector<int32_t> nlev;       // [n_dir]
   std::vector<int32_t> nslots;     // [n_dir]
   int max_slots = 0;
+  int n_up = 2;       // most cell and periodic inflow faces of an element, at least 2: the rows a sweep reads for it
   int base_slots = 0;              // rows alive at once when outputs are read back within their own level
   int64_t n_cut = 0;               // cut periodic inflow faces of all directions
   int max_src = 0;                 // largest number of periodic source elements of one direction

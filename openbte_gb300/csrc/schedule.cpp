@@ -407,6 +407,7 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
 
   struct DirOut {
     int64_t n_cut = 0;
+    int n_up = 2;
     std::vector<int32_t> lev, x_cell, wo_wall;
     std::vector<double> kcoef, scoef;
     int nslots = 0, base_slots = 0;
@@ -551,24 +552,67 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
       live += alive[L];
       o.base_slots = std::max(o.base_slots, live);
     }
+    // As many slots as are ever alive at once, each taken by the class (slot mod 8) that collides least.  The sweep
+    // accesses 16 bytes per lane, eight lanes (an octet of a level's elements) per pass, and rows of the
+    // same class share their banks (ring_field): a row's class should differ from those that its octet
+    // stores and that each octet which reads it reads with the same instruction.  groups[octet][0] counts the
+    // classes stored, [octet][1 + k] those read as inflow k, eight one-byte counters to a word.
     {
+      std::fill(alive.begin(), alive.end(), 0);
+      for (int64_t e = 0; e < n; ++e)
+        if (last_use[e] >= 0) { ++alive[level[e]]; if (last_use[e] + 1 <= nl) --alive[last_use[e] + 1]; }
+      int32_t live = 0;
+      o.nslots = 0;
+      for (int32_t L = 0; L < nl; ++L) {
+        live += alive[L];
+        o.nslots = std::max(o.nslots, live);
+      }
       std::vector<std::vector<int32_t>> release(nl + 2);
-      std::vector<int32_t> free_slots;
-      int32_t next = 0;
-      int64_t p = 0;
+      std::vector<int32_t> free_slots[8];
+      for (int32_t sl = o.nslots - 1; sl >= 0; --sl) free_slots[sl & 7].push_back(sl);
+      std::vector<int32_t> octet(n);
+      int32_t n_oct = 0;
       for (int L = 0; L < nl; ++L) {
-        for (int32_t sl : release[L]) free_slots.push_back(sl);
-        for (; p < n && level[order[p]] == L; ++p) {
+        for (int32_t p = o.lev[L]; p < o.lev[L + 1]; ++p) octet[order[p]] = n_oct + ((p - o.lev[L]) >> 3);
+        n_oct += (o.lev[L + 1] - o.lev[L] + 7) >> 3;
+      }
+      const int ng = nf + 1;
+      std::vector<uint64_t> groups((size_t)n_oct * ng, 0);
+      std::vector<uint64_t*> touched;
+      for (int L = 0; L < nl; ++L) {
+        for (int32_t sl : release[L]) free_slots[sl & 7].push_back(sl);
+        for (int32_t p = o.lev[L]; p < o.lev[L + 1]; ++p) {
           const int32_t e = order[p];
           if (last_use[e] < 0) continue;
-          int32_t sl;
-          if (!free_slots.empty()) { sl = free_slots.back(); free_slots.pop_back(); }
-          else sl = next++;
+          touched.clear();
+          touched.push_back(&groups[(size_t)octet[e] * ng]);
+          for (int64_t k = out_ptr[e]; k < out_ptr[e + 1]; ++k) {
+            const int32_t d = out_adj[k];
+            for (int64_t t = in_ptr[d]; t < in_ptr[d + 1] && t - in_ptr[d] < nf; ++t)
+              if (f_nb[in_face[t]] == e && !f_cut[in_face[t]])
+                touched.push_back(&groups[(size_t)octet[d] * ng + 1 + (t - in_ptr[d])]);
+          }
+          // a counter holds at most 8; the few words of an element add up without carries below 32 of them
+          uint64_t sum = 0;
+          for (size_t k = 0; k < std::min<size_t>(touched.size(), 24); ++k) sum += *touched[k];
+          int best = -1, best_score = 0;
+          for (int c = 0; c < 8; ++c) {
+            if (free_slots[c].empty()) continue;
+            const int score = (int)((sum >> (8 * c)) & 0xFF);
+            if (best < 0 || score < best_score ||
+                (score == best_score && free_slots[c].size() > free_slots[best].size())) {
+              best = c;
+              best_score = score;
+            }
+          }
+          const int32_t sl = free_slots[best].back();
+          free_slots[best].pop_back();
+          for (uint64_t* w : touched)
+            if (((*w >> (8 * best)) & 0xFF) < 8) *w += (uint64_t)1 << (8 * best);
           slot_of[e] = sl;
           release[last_use[e] + 1].push_back(sl);
         }
       }
-      o.nslots = next;
     }
 
     // items in level order (wout and contact indices local to the direction; rebased on merge)
@@ -589,6 +633,7 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
       for (int64_t t = in_ptr[e]; t < in_ptr[e + 1]; ++t) {
         const int32_t f = in_face[t];
         if (k >= nf) { o.st = OBTE_ERR_BAD_ARG; o.err = "more inflow faces than element sides"; return; }
+        o.n_up = std::max(o.n_up, k + 1);
         if (f_cut[f]) { s.in_idx[it * nf + k] = pack_item(ITEM_PERIODIC, src_of[f_nb[f]]); ++o.n_cut; }
         else s.in_idx[it * nf + k] = pack_item(ITEM_CELL, slot_of[f_nb[f]]);
         s.in_coef[it * nf + k] = g[f] * f_t[f];
@@ -688,6 +733,7 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
   s.kcoef.clear();
   s.scoef.clear();
   s.max_slots = s.max_src = s.max_wo = 0;
+  s.n_up = 2;
   s.n_cut = 0;
   s.base_slots = 0;
   std::vector<int32_t> wo_base(n_dir), ce_base(n_dir);
@@ -699,6 +745,7 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
     s.nlev[q] = (int32_t)o.lev.size() - 1;
     s.nslots[q] = o.nslots;
     s.max_slots = std::max(s.max_slots, o.nslots);
+    s.n_up = std::max(s.n_up, o.n_up);
     s.base_slots = std::max(s.base_slots, o.base_slots);
     s.n_cut += o.n_cut;
     s.x_base[q + 1] = s.x_base[q] + (int64_t)o.x_cell.size();

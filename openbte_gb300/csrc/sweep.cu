@@ -44,9 +44,12 @@ static constexpr int kBaseUnit = 128;     // elements per unit of the base layou
 // ---- packed element records -------------------------------------------------------
 // 32-bit words, ring rows as 16-bit halves in units of 16 bytes (ring_field):
 //   w0 cell | w1 so, s0 | w2 s1, s2 | w3 s3, kc | the reals c0 .. c(NF-1), D | padding to 16 B
-// so = output row, s* = inflow rows (s3 only for NF = 4), kc = 1 + index of a contact element's entry in its
-// unit's list of wall / contact entries (0: no contact side), bit 15 set for a periodic source.  Triangles: 32 B (FP32) / 48 B (FP64); tetrahedra:
-// 48 B / 64 B.
+// so = output row, s* = inflow rows, kc = 1 + index of a contact element's entry in its unit's list of wall /
+// contact entries (0: no contact side), bit 15 set for a periodic source.  NF = the most cell and periodic inflow
+// faces of an element (Schedule::n_up): a convex cell has at least one outflow face, so triangles and squares
+// need two rows, tetrahedra three, not one per side.  32 B (FP32) / 48 B (FP64), tetrahedra 32 B / 64 B.  Leaving
+// out the rows that every element read as zero, with the rows' bank classes (schedule.cpp), took the 60k-triangle
+// sweep (100 x 96, FP32) from 1,430 to 1,167 us and 5 of 7 spilled words from its element loop.
 // A unit's static data: its record block (header, records), followed by its output block:
 //   header 0: elements | (values start one pair into their window) << 16, first position, periodic outputs |
 //             wall and contact outputs << 16, then of unit u + nbuf: bank rows | size of its output block << 16
@@ -69,7 +72,8 @@ static constexpr int kHeader = 32;   // bytes
 // row as two 16-byte halves; eight lanes (128 bytes) are served per pass, and with the halves in plain
 // order all first halves would share 4 of the 8 16-byte bank groups.  Rows whose index has bit 2 set keep
 // their halves swapped, so eight consecutive rows' first halves cover all the banks (60k-triangle cell,
-// random row order: 9.0 -> 7.0 passes per 32-lane load; 3.6 would be conflict-free).
+// random row order: 9.0 -> 7.0 passes per 32-lane load); with rows chosen by their class mod 8 (schedule.cpp) 4.7;
+// 3.6 would be conflict-free.
 __host__ __device__ constexpr int ring_field(int row, int row_bytes) {
   return row_bytes == 32 ? 2 * row + ((row >> 2) & 1) : row;
 }
@@ -253,7 +257,7 @@ static Layout make_layout(const Schedule& s, const UnitStats& st, const Layout& 
   l.emax = (st.emax + al) & ~al;
   l.prow0 = (s.max_slots + 2 + al) & ~al;
   l.rows = l.prow0 + nbuf * l.emax;
-  l.blk = kHeader + over * rec_words(sizeof(Real), s.nf) * 4;
+  l.blk = kHeader + over * rec_words(sizeof(Real), s.n_up) * 4;
   l.val = ((over + 2) * 2 * (int)sizeof(Real) + 15) & ~15;
   l.gain = sizeof(Real) == 8 ? over * row_bytes : 0;
   l.out = st.unit_out;
@@ -287,7 +291,7 @@ struct Packed {
 template <typename Real>
 static obte_status pack(const Schedule& s, const Units& un, const std::vector<int64_t>& unit_base,
                         const std::vector<int32_t>& cnt, const Layout& lay, Packed& pk) {
-  const int W = rec_words(sizeof(Real), s.nf);
+  const int W = rec_words(sizeof(Real), s.n_up);
   constexpr int CSTEP = sizeof(Real) / 4, COEF = 4, VB = 2 * sizeof(Real);
   const int row_bytes = lay.KV * (int)sizeof(Real);
   const int n_chunks = (s.n_mfp + lay.KV - 1) / lay.KV;
@@ -469,13 +473,13 @@ static obte_status pack(const Schedule& s, const Units& un, const std::vector<in
         } else {
           pk.spec[it] = -1;
         }
-        for (int f = 0; f < s.nf; ++f) {
+        for (int f = 0; f < s.n_up; ++f) {
           const Real v = (Real)coef[f];
           std::memcpy(&r[COEF + f * CSTEP], &v, sizeof(Real));
         }
         const Real dv = (Real)s.D[it];
-        std::memcpy(&r[COEF + s.nf * CSTEP], &dv, sizeof(Real));
-        for (int wd = COEF + (s.nf + 1) * CSTEP; wd < W; ++wd) r[wd] = 0;   // padding to 16 bytes
+        std::memcpy(&r[COEF + s.n_up * CSTEP], &dv, sizeof(Real));
+        for (int wd = COEF + (s.n_up + 1) * CSTEP; wd < W; ++wd) r[wd] = 0;   // padding to 16 bytes
       }
       wo_run += nwo;
     }
@@ -1076,11 +1080,11 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
     Real Tp0[FINAL ? KV : 1];
     int el = tid;
     // read together: while the row loads are in flight the issuer refills the stage of unit u - 1
-    Real v0[KV], v1[KV], v2[KV], v3[NF > 3 ? KV : 1];
+    Real v0[KV], v1[KV], v2[NF > 2 ? KV : 1], v3[NF > 3 ? KV : 1];
     auto rows = [&]() {
       row_load<MC, KV>(ring, ((unsigned)r[1] >> 12) & 0xFFFF0u, 0, v0);
       row_load<MC, KV>(ring, ((unsigned)r[2] << 4) & 0xFFFF0u, 0, v1);
-      row_load<MC, KV>(ring, ((unsigned)r[2] >> 12) & 0xFFFF0u, 0, v2);
+      if constexpr (NF > 2) row_load<MC, KV>(ring, ((unsigned)r[2] >> 12) & 0xFFFF0u, 0, v2);
       if constexpr (NF > 3) row_load<MC, KV>(ring, ((unsigned)r[3] << 4) & 0xFFFF0u, 0, v3);
     };
     if (el < n_el) rows();
@@ -1106,7 +1110,7 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
       const Real b = bv;
       const Real c0 = word_real<Real>(r, RR::COEF);
       const Real c1 = word_real<Real>(r, RR::COEF + RR::CSTEP);
-      const Real c2 = word_real<Real>(r, RR::COEF + 2 * RR::CSTEP);
+      const Real c2 = NF > 2 ? word_real<Real>(r, RR::COEF + 2 * RR::CSTEP) : Real(0);
       const Real c3 = NF > 3 ? word_real<Real>(r, RR::COEF + 3 * RR::CSTEP) : Real(0);
       const Real D = word_real<Real>(r, RR::D);
       Real T[KV];
@@ -1125,7 +1129,7 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
         for (int j = 0; j < KV; j += 2) {
           df2 sm = dmul2(C0, dunpack2(v0[j], v0[j + 1]));
           sm = dadd2(sm, dmul2(C1, dunpack2(v1[j], v1[j + 1])));
-          sm = dadd2(sm, dmul2(C2, dunpack2(v2[j], v2[j + 1])));
+          if constexpr (NF > 2) sm = dadd2(sm, dmul2(C2, dunpack2(v2[j], v2[j + 1])));
           if constexpr (NF > 3) sm = dadd2(sm, dmul2(C3, dunpack2(v3[j], v3[j + 1])));
           const df2 LM = lam2[j / 2];
           const df2 num = dadd2(BB, dmul2(LM, dadd2(PW, dneg2(sm))));   // b + L (pw - sm)
@@ -1157,7 +1161,7 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
         for (int j = 0; j < KV; j += 2) {
           float2 sm = __fmul2_rn(C0, make_float2(v0[j], v0[j + 1]));
           sm = __ffma2_rn(C1, make_float2(v1[j], v1[j + 1]), sm);
-          sm = __ffma2_rn(C2, make_float2(v2[j], v2[j + 1]), sm);
+          if constexpr (NF > 2) sm = __ffma2_rn(C2, make_float2(v2[j], v2[j + 1]), sm);
           if constexpr (NF > 3) sm = __ffma2_rn(C3, make_float2(v3[j], v3[j + 1]), sm);
           const float2 lm = make_float2(lam[j], lam[j + 1]);
           const float2 num = __ffma2_rn(lm, __ffma2_rn(NEG, sm, PW), BB);    // b + L (pw - sm)
@@ -1189,14 +1193,15 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
           for (int j = 0; j < KV; ++j) {
             Real z = fma(-c0, v0[j], y);
             z = fma(-c1, v1[j], z);
-            z = fma(-c2, v2[j], z);
+            if constexpr (NF > 2) z = fma(-c2, v2[j], z);
             if constexpr (NF > 3) z = fma(-c3, v3[j], z);
             T[j] = fma((Real)gn[kGain ? j : 0], z, b);
           }
         } else {
 #pragma unroll
           for (int j = 0; j < KV; ++j) {
-            Real sm = c0 * v0[j] + c1 * v1[j] + c2 * v2[j];
+            Real sm = c0 * v0[j] + c1 * v1[j];
+            if constexpr (NF > 2) sm += c2 * v2[j];
             if constexpr (NF > 3) sm += c3 * v3[j];
             T[j] = quot(b + lam[j] * (pw - sm), Real(1) + lam[j] * D);
           }
@@ -1582,7 +1587,7 @@ __device__ __forceinline__ UnitRecs unit_recs(const int32_t* __restrict__ desc, 
 // Coefficient word w of item `it`'s record from inflow slot f: g0 x (t_s, 1 - t_s or 1 by the slot's mode),
 // the same arithmetic as set_transmission on the host, rounded to the record's precision.  A warp per unit.
 template <typename Real, int NF>
-__global__ void refresh_rec_kernel(int64_t n_units, const int32_t* __restrict__ desc, const double* __restrict__ g0,
+__global__ void refresh_rec_kernel(int64_t n_units, int nf, const int32_t* __restrict__ desc, const double* __restrict__ g0,
                                    const int32_t* __restrict__ mode, const int8_t* __restrict__ word,
                                    const double* __restrict__ t, int32_t* __restrict__ blk) {
   using RR = Rec<Real, NF>;
@@ -1591,9 +1596,8 @@ __global__ void refresh_rec_kernel(int64_t n_units, const int32_t* __restrict__ 
   for (int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n_units; u += nw) {
     const UnitRecs ur = unit_recs<Real>(desc, u);
     for (int el = lane; el < ur.n_el; el += 32) {
-#pragma unroll
-      for (int f = 0; f < NF; ++f) {
-        const int64_t e = (ur.item0 + el) * NF + f;
+      for (int f = 0; f < nf; ++f) {
+        const int64_t e = (ur.item0 + el) * nf + f;
         const int w = word[e];
         if (w < 0) continue;
         const int32_t md = mode[e];
@@ -1647,9 +1651,9 @@ static obte_status refresh_impl(obte_plan plan, DevSchedule& d, int64_t* bytes, 
   const int64_t items = (int64_t)s.n_dir * s.n;
   // the records' coefficient words, on the device from the transmission-free factors and t
   const int blocks = (int)std::min<int64_t>((items + 255) / 256, (int64_t)plan->ctx->num_sms * 8);
-  auto kern = s.nf == 3 ? refresh_rec_kernel<Real, 3> : refresh_rec_kernel<Real, 4>;
+  auto kern = s.n_up == 2 ? refresh_rec_kernel<Real, 2> : s.n_up == 3 ? refresh_rec_kernel<Real, 3> : refresh_rec_kernel<Real, 4>;
   if (s.nf != 3 && s.nf != 4) { d.ready = false; return OBTE_OK; }
-  kern<<<blocks, 256, 0, st>>>(d.n_units, d.desc.as<int32_t>(), plan->tf_g0.as<double>(), plan->tf_mode.as<int32_t>(),
+  kern<<<blocks, 256, 0, st>>>(d.n_units, s.nf, d.desc.as<int32_t>(), plan->tf_g0.as<double>(), plan->tf_mode.as<int32_t>(),
                                plan->tf_word.as<int8_t>(), plan->tf_t.as<double>(), d.blk.as<int32_t>());
   count_launch();
   OBTE_CUDA(cudaGetLastError());
@@ -1783,7 +1787,7 @@ static obte_status build_gain(obte_plan plan, DevSchedule& d) {
     return OBTE_OK;            // no room: the sweep divides
   }
   const int blocks = (int)std::min<int64_t>((d.n_units + 7) / 8, (int64_t)plan->ctx->num_sms * 16);
-  auto kern = s.nf == 3 ? gain_build_kernel<3> : gain_build_kernel<4>;
+  auto kern = s.n_up == 2 ? gain_build_kernel<2> : s.n_up == 3 ? gain_build_kernel<3> : gain_build_kernel<4>;
   kern<<<std::max(blocks, 1), 256, 0, plan->stream>>>(d.n_units, d.desc.as<int32_t>(), d.blk.as<int32_t>(), s.n,
                                                       d.n_chunks, d.mc, s.n_mfp, d.mfp.as<double>(), d.gain.as<double>());
   count_launch();
@@ -1964,7 +1968,11 @@ template <typename Real, int KV>
 static obte_status launch_kv(obte_plan plan, const DevSchedule& d, const SweepScratch<Real>& sc, bool plain,
                              const double* u_in, double* u_out, bool with_src, bool final_pass, double* Jraw, double* K,
                              double* S) {
-  if (plan->sched.nf == 3) {
+  if (plan->sched.n_up == 2) {
+    if (final_pass) return launch_impl<Real, 2, KV, true>(plan, d, sc, plain, u_in, u_out, with_src, Jraw, K, S);
+    return launch_impl<Real, 2, KV, false>(plan, d, sc, plain, u_in, u_out, with_src, Jraw, K, S);
+  }
+  if (plan->sched.n_up == 3) {
     if (final_pass) return launch_impl<Real, 3, KV, true>(plan, d, sc, plain, u_in, u_out, with_src, Jraw, K, S);
     return launch_impl<Real, 3, KV, false>(plan, d, sc, plain, u_in, u_out, with_src, Jraw, K, S);
   }
@@ -2007,10 +2015,12 @@ obte_status launch_sweep_df(obte_plan plan, const double* u_in, double* u_out, b
   const DevSchedule& d = plan->d64;
   const SweepScratch<double> sc{d.vals.as<double>(), plan->err.as<int>(), d.xrow.as<double>()};
   if (d.mc == 2) {
-    if (plan->sched.nf == 3) return launch_impl<double, 3, 2, true, true>(plan, d, sc, false, u_in, u_out, with_src, Jraw, K, S);
+    if (plan->sched.n_up == 2) return launch_impl<double, 2, 2, true, true>(plan, d, sc, false, u_in, u_out, with_src, Jraw, K, S);
+    if (plan->sched.n_up == 3) return launch_impl<double, 3, 2, true, true>(plan, d, sc, false, u_in, u_out, with_src, Jraw, K, S);
     return launch_impl<double, 4, 2, true, true>(plan, d, sc, false, u_in, u_out, with_src, Jraw, K, S);
   }
-  if (plan->sched.nf == 3) return launch_impl<double, 3, 4, true, true>(plan, d, sc, false, u_in, u_out, with_src, Jraw, K, S);
+  if (plan->sched.n_up == 2) return launch_impl<double, 2, 4, true, true>(plan, d, sc, false, u_in, u_out, with_src, Jraw, K, S);
+  if (plan->sched.n_up == 3) return launch_impl<double, 3, 4, true, true>(plan, d, sc, false, u_in, u_out, with_src, Jraw, K, S);
   return launch_impl<double, 4, 4, true, true>(plan, d, sc, false, u_in, u_out, with_src, Jraw, K, S);
 }
 
