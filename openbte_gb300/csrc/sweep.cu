@@ -630,30 +630,46 @@ struct PrepParams {
 };
 
 template <typename Real, int MC, bool DF>
-__global__ void __launch_bounds__(256) sweep_prep_kernel(const __grid_constant__ PrepParams<Real> p) {
+__global__ void __launch_bounds__(256, 8) sweep_prep_kernel(const __grid_constant__ PrepParams<Real> p) {
   if ((int)blockIdx.x < p.row_blocks) {
     constexpr bool kWide = MC * sizeof(Real) == 32;
-    constexpr int U = 4;                 // loads in flight per lane
+    constexpr int U = 4;                 // loads in flight per lane, over the pieces of 32 MFPs of consecutive rows
     const double* __restrict__ X = p.u_in + p.n + p.nd;
     const int lane = threadIdx.x & 31;
-    const int64_t nw = (int64_t)p.row_blocks * (blockDim.x >> 5);
-    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < p.n_pf * p.batch; w += nw) {
-      const int64_t t = p.batch > 1 ? w / p.n_pf : 0;
-      const int4 e = reinterpret_cast<const int4*>(p.pfe)[w - t * p.n_pf];
-      const double* src = X + t * p.batch_stride + (int64_t)(e.x & 0x3fffffff) * p.n_mfp;
-      Real* dst = p.xrow + t * p.row_stride + (int64_t)e.y * MC;
-      const int flip = kWide && (e.x >> 30) ? MC / 2 : 0;
-      for (int m0 = lane; m0 < p.m_row; m0 += 32 * U) {
-        double v[U];
+    const int np = (p.m_row + 31) >> 5;  // pieces of a row
+    const int64_t nw = (int64_t)p.row_blocks * (blockDim.x >> 5), total = p.n_pf * p.batch * np;
+    const int4* __restrict__ pfe = reinterpret_cast<const int4*>(p.pfe);
+    // the entries of a row are read again for its stores (an L1 hit): kept, they would cost a third of the warps
+    for (int64_t f = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * U; f < total; f += nw * U) {
+      const int64_t w0 = f / np;
+      const int piece0 = (int)(f - w0 * np), left = (int)min((int64_t)U, total - f);
+      double v[U];
+      int64_t w = w0;
+      int piece = piece0;
 #pragma unroll
-        for (int k = 0; k < U; ++k) v[k] = m0 + 32 * k < p.n_mfp ? src[m0 + 32 * k] : 0.0;
+      for (int k = 0; k < U; ++k) {
+        v[k] = 0.0;
+        const int m = lane + 32 * piece;
+        if (k < left && m < p.n_mfp) {
+          const int64_t t = p.batch > 1 ? w / p.n_pf : 0;
+          v[k] = X[t * p.batch_stride + (int64_t)(pfe[w - t * p.n_pf].x & 0x3fffffff) * p.n_mfp + m];
+        }
+        if (++piece == np) { piece = 0; ++w; }
+      }
+      w = w0;
+      piece = piece0;
 #pragma unroll
-        for (int k = 0; k < U; ++k) {
-          const int m = m0 + 32 * k;
+      for (int k = 0; k < U; ++k) {
+        const int m = lane + 32 * piece;
+        if (k < left && m < p.m_row) {
+          const int64_t t = p.batch > 1 ? w / p.n_pf : 0;
+          const int4 e = pfe[w - t * p.n_pf];
+          const int flip = kWide && (e.x >> 30) ? MC / 2 : 0;
           Real r = (Real)v[k];
           if constexpr (DF) r = dpack_split((double)r);
-          if (m < p.m_row) dst[(int64_t)(m / MC) * e.z * MC + ((m % MC) ^ flip)] = r;
+          p.xrow[t * p.row_stride + ((int64_t)e.y + (int64_t)(m / MC) * e.z) * MC + ((m % MC) ^ flip)] = r;
         }
+        if (++piece == np) { piece = 0; ++w; }
       }
     }
     return;
