@@ -200,7 +200,7 @@ void dsa_matrix(const Schedule& s, std::vector<int32_t>& rp, std::vector<int32_t
       }
     }
     coef[k] = D.area[k] * c;
-  });
+  }, std::max<int64_t>(64, 20000 / std::max(n_mfp, 1)));
   std::vector<double> diag(n, 0.0);
   std::vector<int32_t> deg(n + 1, 0);
   for (int64_t k = 0; k < nfc; ++k) {

@@ -52,10 +52,11 @@ inline int host_threads() {
   return std::max(1, std::min(t, 32));
 }
 
-// f(i) for i in [0, n) over host threads in contiguous blocks (results must not depend on the split).
+// f(i) for i in [0, n) over host threads in contiguous blocks of at least `grain` (results must not depend on the
+// split).  Starting a thread costs about 60 us: a grain should hold a few times that.
 template <typename F>
-void parallel_for(int64_t n, F&& f) {
-  const int nt = (int)std::min<int64_t>(host_threads(), std::max<int64_t>(1, n / 64));
+void parallel_for(int64_t n, F&& f, int64_t grain = 64) {
+  const int nt = (int)std::min<int64_t>(host_threads(), std::max<int64_t>(1, n / grain));
   if (nt <= 1) {
     for (int64_t i = 0; i < n; ++i) f(i);
     return;
@@ -69,10 +70,11 @@ void parallel_for(int64_t n, F&& f) {
 }
 
 // f(i) for i in [0, n) where each i is a large task (a direction): one task at a time per host thread,
-// handed out in index order from a shared counter (results must not depend on the assignment).
+// handed out in index order from a shared counter (results must not depend on the assignment), on at most
+// max_threads.
 template <typename F>
-void parallel_tasks(int64_t n, F&& f) {
-  const int nt = (int)std::min<int64_t>(host_threads(), n);
+void parallel_tasks(int64_t n, F&& f, int64_t max_threads = 32) {
+  const int nt = (int)std::min<int64_t>({(int64_t)host_threads(), n, max_threads});
   if (nt <= 1) {
     for (int64_t i = 0; i < n; ++i) f(i);
     return;
@@ -329,11 +331,9 @@ struct DevSchedule {
   DevBuf gain;
   // deterministic reductions (OBTE_DETERMINISTIC=1): per-(direction, chunk) partials and per-position sums
   DevBuf det_d, det_j, det_w, det_k, det_s, det_S, det_SJ;
-  // transmission plans: the special-entry index of each item (host), so that new transmissions rewrite
-  // the wall coefficients; the records' coefficient words are rewritten on the device (refresh_tables)
-  RawVec<int32_t> h_spec;
+  // transmission plans: new transmissions rewrite the records' coefficient words and the wall coefficients on the
+  // device (refresh_tables)
   bool refreshable = false;
-  int64_t n_spec = 0;
   size_t bytes() const;
 };
 

@@ -792,13 +792,14 @@ obte_status set_transmission(Schedule& s, const double* t) {
     if (!(t[k] > 0 && t[k] <= 1)) { set_error("side transmission outside (0, 1]"); return OBTE_ERR_BAD_ARG; }
   const int64_t n = s.n;
   const int nf = s.nf, n_dir = s.n_dir, n_mfp = s.n_mfp, m_pad = s.m_pad, ds = s.ds, dim = s.dim;
+  constexpr int64_t kGrain = 1 << 15;        // items of a few hundred us
   parallel_for((int64_t)n_dir * n, [&](int64_t it) {
     for (int k = 0; k < nf; ++k) {
       const size_t e = (size_t)it * nf + k;
       const int32_t md = tf.mode[e];
       s.in_coef[e] = md >= 0 ? tf.g0[e] * t[md] : md == -1 ? tf.g0[e] * 1.0 : tf.g0[e] * (1.0 - t[-md - 2]);
     }
-  });
+  }, kGrain);
   const int64_t np = (int64_t)tf.per_i.size();
   const int64_t nc = (int64_t)tf.c_side.size();
   const double nrm = s.normalization;
@@ -841,7 +842,7 @@ obte_status set_transmission(Schedule& s, const double* t) {
         for (int64_t k = 0; k < nc; ++k) acc += std::min(sigma_n(m, q, k), 0.0) * t[tf.c_side[k]];
         s.kconst[(size_t)m * n_dir + q] = s.contact_alpha * acc * nrm;
       }
-  });
+  }, std::max<int64_t>(1, (int64_t)n_dir * (n + nc * n_mfp * 4) / kGrain));
   for (int64_t w = 0; w < s.nd; ++w)
     s.ell_B[w] = tf.ell0[w] * (tf.w_side[w] < 0 ? 1.0 : 1.0 - t[tf.w_side[w]]);
   for (size_t k = 0; k < s.dsa.t.size(); ++k) s.dsa.t[k] = t[s.dsa.side[k]];

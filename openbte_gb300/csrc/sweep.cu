@@ -1573,8 +1573,6 @@ static obte_status upload_tables(obte_plan plan, DevSchedule& d) {
   OBTE_CUDA(cudaMemsetAsync(d.vals.p, 0, d.vals.bytes, st));
   if (s.tf.ok) {   // transmission plans: keep what refresh_tables rewrites
     d.refreshable = true;
-    d.h_spec = std::move(pk.spec);
-    d.n_spec = (int64_t)(pk.sr.size() / SR);
   }
   d.ready = true;
   return OBTE_OK;
@@ -1601,23 +1599,32 @@ __device__ __forceinline__ UnitRecs unit_recs(const int32_t* __restrict__ desc, 
 // the special entries (the same walk over the inflow entries as pack), then P and the contact
 // coefficients; indices, units and launch order stay.
 // Coefficient word w of item `it`'s record from inflow slot f: g0 x (t_s, 1 - t_s or 1 by the slot's mode),
-// the same arithmetic as set_transmission on the host, rounded to the record's precision.  A warp per unit.
+// the same arithmetic as set_transmission on the host, rounded to the record's precision; the wall inflow (w = -2)
+// goes to the item's special entry, in order.  A warp per unit.  (Formed on the host and uploaded, the wall
+// coefficients took 7.5 of the 10 ms between two evaluations on 128^2 pixels x 50 x 64, where every item has some.)
 template <typename Real, int NF>
 __global__ void refresh_rec_kernel(int64_t n_units, int nf, const int32_t* __restrict__ desc, const double* __restrict__ g0,
                                    const int32_t* __restrict__ mode, const int8_t* __restrict__ word,
-                                   const double* __restrict__ t, int32_t* __restrict__ blk) {
+                                   const double* __restrict__ t, int32_t* __restrict__ blk,
+                                   const int32_t* __restrict__ spec, Real* __restrict__ sr) {
   using RR = Rec<Real, NF>;
   const int lane = threadIdx.x & 31;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n_units; u += nw) {
     const UnitRecs ur = unit_recs<Real>(desc, u);
     for (int el = lane; el < ur.n_el; el += 32) {
+      const int32_t sp = spec[ur.item0 + el];
+      int j = 0;
       for (int f = 0; f < nf; ++f) {
         const int64_t e = (ur.item0 + el) * nf + f;
         const int w = word[e];
-        if (w < 0) continue;
+        if (w == -1) continue;
         const int32_t md = mode[e];
         const double g = md >= 0 ? g0[e] * t[md] : md == -1 ? g0[e] * 1.0 : g0[e] * (1.0 - t[-md - 2]);
+        if (w < 0) {
+          sr[(int64_t)sp * SR + j++] = (Real)g;
+          continue;
+        }
         int32_t* r = blk + ur.word0 + (int64_t)el * RR::W + RR::COEF + w * RR::CSTEP;
         if constexpr (sizeof(Real) == 4) {
           r[0] = __float_as_int((float)g);
@@ -1642,6 +1649,7 @@ static obte_status upload_transmission(obte_plan plan, const double* t) {
       for (int f = 0; f < s.nf; ++f) {
         const int kind = (int)((uint32_t)s.in_idx[it * s.nf + f] >> ITEM_SHIFT);
         if (kind == ITEM_CELL || kind == ITEM_PERIODIC) word[(size_t)it * s.nf + f] = (int8_t)k++;
+        else if (kind == ITEM_WALL) word[(size_t)it * s.nf + f] = -2;
       }
     });
     OBTE_TRY(upload(plan->tf_g0, s.tf.g0, st));
@@ -1670,21 +1678,11 @@ static obte_status refresh_impl(obte_plan plan, DevSchedule& d, int64_t* bytes, 
   auto kern = s.n_up == 2 ? refresh_rec_kernel<Real, 2> : s.n_up == 3 ? refresh_rec_kernel<Real, 3> : refresh_rec_kernel<Real, 4>;
   if (s.nf != 3 && s.nf != 4) { d.ready = false; return OBTE_OK; }
   kern<<<blocks, 256, 0, st>>>(d.n_units, s.nf, d.desc.as<int32_t>(), plan->tf_g0.as<double>(), plan->tf_mode.as<int32_t>(),
-                               plan->tf_word.as<int8_t>(), plan->tf_t.as<double>(), d.blk.as<int32_t>());
+                               plan->tf_word.as<int8_t>(), plan->tf_t.as<double>(), d.blk.as<int32_t>(),
+                               d.spec.as<int32_t>(), d.sr.as<Real>());
   count_launch();
   OBTE_CUDA(cudaGetLastError());
-  // wall coefficients of the special entries (host, small)
-  PhaseTimer th(sizeof(Real) == 4 ? "refresh fp32: walls and uploads" : "refresh fp64: walls and uploads");
-  std::vector<double> sr((size_t)d.n_spec * SR, 0.0);
-  parallel_for(items, [&](int64_t it) {
-    const int32_t sp = d.h_spec[it];
-    if (sp < 0) return;
-    int j = 0;
-    for (int f = 0; f < s.nf; ++f) {
-      const int32_t code = s.in_idx[it * s.nf + f];
-      if ((int)((uint32_t)code >> ITEM_SHIFT) == ITEM_WALL) sr[(size_t)sp * SR + j++] = s.in_coef[it * s.nf + f];
-    }
-  });
+  PhaseTimer th(sizeof(Real) == 4 ? "refresh fp32: uploads" : "refresh fp64: uploads");
   const size_t kc_n = std::max<size_t>(s.kcoef.size(), 1);
   const bool reuse = sizeof(Real) == 4 && done && done->Pq.p && d.Pq.bytes == done->Pq.bytes && done->kcoef.p &&
                      d.kcoef.p && d.kcoef.bytes >= kc_n * sizeof(Real) && done->kcoef.bytes >= kc_n * sizeof(double);
@@ -1698,9 +1696,8 @@ static obte_status refresh_impl(obte_plan plan, DevSchedule& d, int64_t* bytes, 
     OBTE_CUDA(cudaMemcpyAsync(d.Pq.p, s.P.data(), s.P.size() * sizeof(double), cudaMemcpyHostToDevice, st));
   }
   OBTE_CUDA(wait_stream(st));
-  OBTE_TRY(upload_real<Real>(d.sr, sr, st));
   if (!reuse) OBTE_TRY(upload_real<Real>(d.kcoef, s.kcoef, st));
-  if (bytes) *bytes += (int64_t)(sr.size() * sizeof(Real) + (reuse ? 0 : s.kcoef.size() * sizeof(Real) + s.P.size() * 8));
+  if (bytes) *bytes += (int64_t)(reuse ? 0 : s.kcoef.size() * sizeof(Real) + s.P.size() * 8);
   return OBTE_OK;
 }
 
