@@ -261,19 +261,33 @@ __device__ __forceinline__ void arnoldi_update(const ArnoldiParams<Real>& P, con
     float4* w4 = reinterpret_cast<float4*>(P.w);
     for (int vb = g; vb < P.nvb; vb += P.groups) {
       float ss = 0.f;
-      for (int64_t i = (int64_t)vb * VT + tid; i < n4; i += stride) {
-        float4 acc = w4[i];
-#pragma unroll 8
+      // a share is about four float4 per thread: all of them against four basis vectors at a time, 16 loads in
+      // flight (one float4 against eight vectors left the loop waiting for L2)
+      for (int64_t i0 = (int64_t)vb * VT + tid; i0 < n4; i0 += 4 * stride) {
+        float4 acc[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (i0 + e * stride < n4) acc[e] = w4[i0 + e * stride];
+#pragma unroll 4
         for (int j = 0; j < k; ++j) {
-          const float4 v = reinterpret_cast<const float4*>(P.V + (int64_t)j * P.ld)[i];
+          const float4* row = reinterpret_cast<const float4*>(P.V + (int64_t)j * P.ld);
           const float c = -hs[j];
-          acc.x = fmaf(c, v.x, acc.x);
-          acc.y = fmaf(c, v.y, acc.y);
-          acc.z = fmaf(c, v.z, acc.z);
-          acc.w = fmaf(c, v.w, acc.w);
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (i0 + e * stride < n4) {
+              const float4 v = row[i0 + e * stride];
+              acc[e].x = fmaf(c, v.x, acc[e].x);
+              acc[e].y = fmaf(c, v.y, acc[e].y);
+              acc[e].z = fmaf(c, v.z, acc[e].z);
+              acc[e].w = fmaf(c, v.w, acc[e].w);
+            }
         }
-        w4[i] = acc;
-        ss = fmaf(acc.x, acc.x, fmaf(acc.y, acc.y, fmaf(acc.z, acc.z, fmaf(acc.w, acc.w, ss))));
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (i0 + e * stride < n4) {
+            w4[i0 + e * stride] = acc[e];
+            ss = fmaf(acc[e].x, acc[e].x, fmaf(acc[e].y, acc[e].y, fmaf(acc[e].z, acc[e].z, fmaf(acc[e].w, acc[e].w, ss))));
+          }
       }
       if (vb == 0)
         for (int64_t i = 4 * n4 + tid; i < P.n; i += VT) {
