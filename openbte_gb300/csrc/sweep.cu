@@ -1402,7 +1402,7 @@ static obte_status upload_real(DevBuf& b, const std::vector<double>& v, cudaStre
 // staged) with 32-byte rows would let at least 4 CTAs share an SM, else 4 (60k triangles: 2.14 ms at 8 against
 // 2.23 at 4; 110k tetrahedra, 2 CTAs per SM at 8: 20.8 against 11.6 ms); 4 for at most 4 MFPs.  The choice fixes
 // the grouping of the FP32 partial sums, so it depends on the mesh and the ordinates alone, not on the
-// launch shape below.  FP64: 2.  OBTE_SWEEP_KV forces a compiled value.
+// launch shape below.  FP64: 2 or 4, see there.  OBTE_SWEEP_KV forces a compiled value.
 template <typename Real>
 static int choose_mc(const Schedule& s, const UnitStats& base) {
   constexpr int kNarrow = 16 / (int)sizeof(Real), kWide = 2 * kNarrow;
@@ -1410,7 +1410,13 @@ static int choose_mc(const Schedule& s, const UnitStats& base) {
     const int v = std::atoi(e);
     if (v == kNarrow || v == kWide) return v;
   }
-  if (sizeof(Real) == 8 || s.n_mfp <= kNarrow) return kNarrow;
+  // FP64: four MFPs to a CTA halve the passes over the records, but also the CTAs, and only with two inflow rows do they
+  // fit the registers.  Measured, two MFPs against four: 60,000 triangles x 100 x 96 6,550 and 6,018 us, 20,000 2,749
+  // and 2,596, 8,000 x 60 x 48 (720 CTAs of four) 503 and 456; 2,000 x 30 x 48 (384) 146 and 194, 1,000 x 12 x 24 104
+  // and 137; 8,000 tetrahedra x 30 x 128 704 and 718.
+  if (sizeof(Real) == 8)
+    return s.n_up == 2 && (int64_t)s.n_dir * ((s.n_mfp + kWide - 1) / kWide) >= 4 * 152 ? kWide : kNarrow;
+  if (s.n_mfp <= kNarrow) return kNarrow;
   const int64_t stage = kBaseUnit * rec_words(sizeof(Real), s.nf) * 4 + (kBaseUnit + 2) * 8 + base.unit_wo * 16 +
                         ((base.emax + 3) & ~3) * 4 + base.unit_sx * 16;
   const int64_t rows = s.base_slots + 2 + 2 * base.emax;
