@@ -742,7 +742,7 @@ def run_resident(args, dev, world, rank, local):
             ev[1].synchronize()
             ms[prec] = ev[0].elapsed_time(ev[1]) / max(1, args.profile_sweeps - args.profile_sweeps // 2)
         print(json.dumps({"profile_sweeps": args.profile_sweeps, "workload": args.workload,
-                          "ms_per_sweep": ms, "group_env": os.environ.get("OBTE_SWEEP_G")}))
+                          "ms_per_sweep": ms}))
         return
     dT0 = torch.zeros(geo.n_elems, dtype=torch.float64, device=dev)
     flush = torch.empty(2 * L2_BYTES // 4, dtype=torch.float32, device=dev)
