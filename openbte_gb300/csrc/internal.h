@@ -221,6 +221,7 @@ struct Schedule {
   int64_t nd = 0;                  // diffuse wall sides (T_B entries)
   // per direction, per position (n_dir * n); written by build_schedule's direction workers
   RawVec<int32_t> cell, slot, xk, wout, contact;
+  RawVec<uint8_t> info;   // cut inflow faces | 8: periodic source | 16: wall or contact entry | wall entries << 5
   RawVec<int32_t> in_idx;          // n_dir * n * nf
   RawVec<double> in_coef;          // n_dir * n * nf
   RawVec<double> D, P;             // n_dir * n
@@ -349,7 +350,7 @@ struct SolveWork {
   DevBuf pz;         // preconditioned vector (allocated when the plan has a preconditioner)
   DevBuf rc, Jraw2, Kraw2, Sraw2;   // refinement: correction right-hand side, outputs of the correction
   DevBuf V32, w32;   // FP32 basis and working vector (stages with FP32 sweeps), allocated on first use
-  DevBuf gs;         // barrier counters of the Arnoldi steps
+  DevBuf gs;         // what an Arnoldi step passes between its launches
   HostBuf hcol;      // the Hessenberg column, written by the device
 };
 

@@ -90,15 +90,17 @@ __global__ void __launch_bounds__(VT) update_kernel(double* __restrict__ x, cons
 }
 
 // ---- the Arnoldi step ---------------------------------------------------------------------------
-// One launch orthogonalises w = z - K z against the basis V[0..k) and normalises it: classical Gram-Schmidt with
+// A step orthogonalises w = z - K z against the basis V[0..k) and normalises it: classical Gram-Schmidt with
 // a second pass only when the first one cancelled most of w (Daniel-Gragg-Kaufman-Stewart criterion, |w| after
-// < 0.7 |w| before).  Phases end at a barrier over the blocks (grid.cuh): the products V^T w and w.w, the
-// difference formed on the way; w -= V h and its norm; the same again after the test; the scaled vector and
-// its FP64 copy for the next sweep.  Every block adds up the blocks' sums itself, in a fixed order.  The host
-// reads the Hessenberg column, written to its memory, once per step.
+// < 0.7 |w| before).  Its phases: the products V^T w and w.w, the difference formed on the way; w -= V h and its
+// norm; the same again after the test; the scaled vector and its FP64 copy for the next sweep.  Every block adds up the
+// blocks' sums itself, in a fixed order.  The host reads the Hessenberg column, written to its memory, once per step.
 //
-// As 13 launches of 3.9 us each with its gap a step took 50 us beside its sweep (8,000 triangles x 60 x 48: 46 steps,
-// 14.7 ms a solve; now 12.8).
+// Small states (up to 8 blocks) run as one launch, a cluster whose barrier ends the phases; larger ones as one
+// launch per phase.  As a cooperative launch those ran a step 6 us faster alone, but such a launch waits until all
+// its blocks fit at once: twelve concurrent solves then waited for each other (512 requests at 50 a second: median
+// latency 465 ms against 266 ms with ordinary launches).  As 13 launches of 3.9 us each with its gap a step took 50 us
+// beside its sweep (8,000 triangles x 60 x 48: 46 steps, 14.7 ms a solve).
 //
 // On GB300 the FP64 pipe cannot keep up with HBM for one FMA per 8 loaded bytes, so the stages with FP32 sweeps keep
 // V and w in FP32: FP32 products, per-thread sums and warp sums, FP64 across warps and blocks.  The sweep still
@@ -116,9 +118,9 @@ struct ArnoldiParams {
   Real *w, *vnext;
   double* v64;                               // FP64 copy of vnext (FP32 basis)
   double *part, *s_part;                     // block sums: of the products [k + 1][groups], of w.w [2][groups]
-  double* col;                               // h (+ h2) [k], |w|, second pass ran, 0 when complete
-  unsigned *count, *count_next;
-  int* err;
+  double *h, *h2;                            // coefficients of the passes between launches [k + 1], [k]
+  int* two;                                  // the second pass runs
+  double* col;                               // h (+ h2) [k], |w|, second pass ran
 };
 
 template <typename Real>
@@ -309,51 +311,100 @@ __device__ __forceinline__ void arnoldi_update(const ArnoldiParams<Real>& P, con
   if (tid == 0) s_part[g] = sum;
 }
 
-template <typename Bar, typename Real>
-__global__ void __launch_bounds__(VT, 2) arnoldi_kernel(const __grid_constant__ ArnoldiParams<Real> P) {
-  __shared__ double red[VT];
-  __shared__ double h[MAX_BASIS + 1], h2[MAX_BASIS];
-  __shared__ Real hs[MAX_BASIS];
-  __shared__ Real buf[sizeof(Real) == 4 ? 2 * (VT / 32) * DOT_TILE : DOT_TILE * VT];
-  __shared__ double sc;
-  Bar bar(P.count, P.err);
+// DGKS test, from the block sums of w.w after the first pass; s: w.w (thread 0)
+template <typename Real>
+__device__ __forceinline__ bool arnoldi_test(const ArnoldiParams<Real>& P, double before, double& s, double* red) {
+  return grid_sum(P.s_part, P.groups, red, [&](double v) {
+           s = v;
+           return sqrt(fmax(v, 0.0)) < 0.7 * sqrt(fmax(before, 0.0)) ? 1.0 : 0.0;
+         }) != 0;
+}
+// Hessenberg column (block 0) and the scaled vector; s: w.w (thread 0)
+template <typename Real>
+__device__ __forceinline__ void arnoldi_finish(const ArnoldiParams<Real>& P, const double* h, const double* h2, bool two,
+                                               double s, double* sc) {
   const int tid = threadIdx.x, k = P.k;
-  if (blockIdx.x == 0 && tid == 0) *P.count_next = 0;
-  arnoldi_dots(P, true, k + 1, buf);
-  if (!bar.wait()) return;
-  arnoldi_sums(P, k + 1, h);
-  arnoldi_update(P, h, P.s_part, hs, red);
-  if (!bar.wait()) return;
-  double s = 0;                              // w.w after the passes so far; thread 0's
-  const bool two = grid_sum(P.s_part, P.groups, red, [&](double v) {
-                     s = v;
-                     return sqrt(fmax(v, 0.0)) < 0.7 * sqrt(fmax(h[k], 0.0)) ? 1.0 : 0.0;
-                   }) != 0;
-  if (two) {
-    arnoldi_dots(P, false, k, buf);
-    if (!bar.wait()) return;
-    arnoldi_sums(P, k, h2);
-    arnoldi_update(P, h2, P.s_part + P.groups, hs, red);
-    if (!bar.wait()) return;
-    grid_sum(P.s_part + P.groups, P.groups, red, [&](double v) { return s = v; });
-  }
   if (tid == 0) {
     const double hn = sqrt(fmax(s, 0.0));
-    sc = hn > 0 ? 1.0 / hn : 0.0;
+    *sc = hn > 0 ? 1.0 / hn : 0.0;
     if (blockIdx.x == 0) {
       P.col[k] = hn;
       P.col[k + 1] = two ? 1.0 : 0.0;
-      P.col[k + 2] = 0.0;
     }
   }
   if (blockIdx.x == 0)
     for (int i = tid; i < k; i += VT) P.col[i] = two ? h[i] + h2[i] : h[i];
   __syncthreads();
-  const Real inv = (Real)sc;
+  const Real inv = (Real)*sc;
   for (int64_t i = (int64_t)blockIdx.x * VT + tid; i < P.n; i += (int64_t)gridDim.x * VT) {
     const Real v = inv * P.w[i];
     P.vnext[i] = v;
     if constexpr (sizeof(Real) == 4) P.v64[i] = widen(v);
+  }
+}
+
+template <typename Real>
+constexpr int kDotBuf = sizeof(Real) == 4 ? 2 * (VT / 32) * DOT_TILE : DOT_TILE * VT;
+
+// A whole step in one cluster.
+template <typename Real>
+__global__ void __launch_bounds__(VT, 2) arnoldi_kernel(const __grid_constant__ ArnoldiParams<Real> P) {
+  __shared__ double red[VT];
+  __shared__ double h[MAX_BASIS + 1], h2[MAX_BASIS];
+  __shared__ Real hs[MAX_BASIS];
+  __shared__ Real buf[kDotBuf<Real>];
+  __shared__ double sc;
+  ClusterBarrier bar(nullptr, nullptr);
+  const int k = P.k;
+  arnoldi_dots(P, true, k + 1, buf);
+  bar.wait();
+  arnoldi_sums(P, k + 1, h);
+  arnoldi_update(P, h, P.s_part, hs, red);
+  bar.wait();
+  double s = 0;                              // w.w after the passes so far; thread 0's
+  const bool two = arnoldi_test(P, h[k], s, red);
+  if (two) {
+    arnoldi_dots(P, false, k, buf);
+    bar.wait();
+    arnoldi_sums(P, k, h2);
+    arnoldi_update(P, h2, P.s_part + P.groups, hs, red);
+    bar.wait();
+    grid_sum(P.s_part + P.groups, P.groups, red, [&](double v) { return s = v; });
+  }
+  arnoldi_finish(P, h, h2, two, s, &sc);
+}
+
+// One phase of a step: 0 products, 1 update, 2 test and products of the second pass, 3 its update, 4 column and vector.
+template <typename Real, int PHASE>
+__global__ void __launch_bounds__(VT, 2) arnoldi_phase_kernel(const __grid_constant__ ArnoldiParams<Real> P) {
+  const int tid = threadIdx.x, k = P.k;
+  if constexpr (PHASE == 0 || PHASE == 2) {
+    __shared__ Real buf[kDotBuf<Real>];
+    if constexpr (PHASE == 2) {
+      __shared__ double red[VT];
+      double s;
+      const bool two = arnoldi_test(P, P.h[k], s, red);
+      if (blockIdx.x == 0 && tid == 0) *P.two = two ? 1 : 0;
+      if (!two) return;
+    }
+    arnoldi_dots(P, PHASE == 0, PHASE == 0 ? k + 1 : k, buf);
+  } else if constexpr (PHASE == 1 || PHASE == 3) {
+    __shared__ double red[VT];
+    __shared__ double h[MAX_BASIS + 1];
+    __shared__ Real hs[MAX_BASIS];
+    if (PHASE == 3 && *P.two == 0) return;
+    const int kk = PHASE == 1 ? k + 1 : k;
+    arnoldi_sums(P, kk, h);
+    if (blockIdx.x == 0)
+      for (int i = tid; i < kk; i += VT) (PHASE == 1 ? P.h : P.h2)[i] = h[i];
+    arnoldi_update(P, h, P.s_part + (PHASE == 1 ? 0 : P.groups), hs, red);
+  } else {
+    __shared__ double red[VT];
+    __shared__ double sc;
+    const bool two = *P.two != 0;
+    double s = 0;
+    grid_sum(P.s_part + (two ? P.groups : 0), P.groups, red, [&](double v) { return s = v; });
+    arnoldi_finish(P, P.h, P.h2, two, s, &sc);
   }
 }
 
@@ -538,13 +589,10 @@ struct Solver {
     return OBTE_OK;
   }
 
-  // Barrier counters of the Arnoldi steps, two that steps use in turn, and the host's Hessenberg column.
-  int turn = 0;
+  // What an Arnoldi step passes between its launches, and the host's Hessenberg column.
   obte_status arnoldi_begin() {
-    if (!wk.gs.p) OBTE_TRY(wk.gs.alloc(2 * sizeof(unsigned)));
-    if (!wk.hcol.p) OBTE_TRY(wk.hcol.alloc((size_t)(wk.restart + 4) * sizeof(double)));
-    OBTE_CUDA(cudaMemsetAsync(wk.gs.p, 0, 2 * sizeof(unsigned), st));
-    turn = 0;
+    if (!wk.gs.p) OBTE_TRY(wk.gs.alloc((size_t)(2 * wk.restart + 4) * sizeof(double)));
+    if (!wk.hcol.p) OBTE_TRY(wk.hcol.alloc((size_t)(wk.restart + 3) * sizeof(double)));
     return OBTE_OK;
   }
   // V[k] and the Hessenberg column of w = z - kz against V[0..k), column in wk.hcol
@@ -561,28 +609,27 @@ struct Solver {
                               : (int)std::min<int64_t>((n + VT - 1) / VT, 2 * num_sms);
     f.groups = std::min(f.nvb, 2 * num_sms);             // two blocks to an SM
     f.sp = std::max(1, std::min(tiles, num_sms / f.groups));
-    PhaseShape ps{f.groups * f.sp, VT, false};
-    if (ps.blocks <= 8) {
-      ps.cluster = true;
-      while (ps.blocks & (ps.blocks - 1)) ++ps.blocks;   // blocks above groups * sp only wait
-    }
     f.part = wk.partial.as<double>();
     f.s_part = f.part + (int64_t)(k + 1) * f.groups;
-    unsigned* count = wk.gs.as<unsigned>();
-    f.count = count + turn;
-    f.count_next = count + (turn ^ 1);
-    turn ^= 1;
+    f.h = wk.gs.as<double>();
+    f.h2 = f.h + (wk.restart + 1);
+    f.two = reinterpret_cast<int*>(f.h2 + (wk.restart + 1));
     f.col = wk.hcol.as<double>();
-    f.col[k + 2] = 1.0;                                  // until the kernel is through
-    f.err = plan->err.as<int>();
-    OBTE_CUDA(phase_launch(ps, arnoldi_kernel<ClusterBarrier, Real>, arnoldi_kernel<GridBarrier, Real>, f, 0, st));
-    count_launch();
-    OBTE_CUDA(wait_stream(st));
-    if (f.col[k + 2] != 0.0) {
-      OBTE_TRY(check_device_error(plan));
-      set_error("the Arnoldi kernel did not complete");
-      return OBTE_ERR_DEVICE_TIMEOUT;
+    int blocks = f.groups * f.sp;
+    if (blocks <= 8) {
+      while (blocks & (blocks - 1)) ++blocks;            // blocks above groups * sp only wait
+      OBTE_CUDA(phase_launch({blocks, VT, true}, arnoldi_kernel<Real>, arnoldi_kernel<Real>, f, 0, st));
+      count_launch();
+    } else {
+      arnoldi_phase_kernel<Real, 0><<<blocks, VT, 0, st>>>(f);
+      arnoldi_phase_kernel<Real, 1><<<blocks, VT, 0, st>>>(f);
+      arnoldi_phase_kernel<Real, 2><<<blocks, VT, 0, st>>>(f);
+      arnoldi_phase_kernel<Real, 3><<<blocks, VT, 0, st>>>(f);
+      arnoldi_phase_kernel<Real, 4><<<wk.nb, VT, 0, st>>>(f);
+      count_launch(5);
     }
+    OBTE_CUDA(cudaGetLastError());
+    OBTE_CUDA(wait_stream(st));
     return OBTE_OK;
   }
 
@@ -848,7 +895,7 @@ int64_t solve_scratch_bytes(obte_plan plan, int restart) {
   const int64_t vb = plan->nu * (int64_t)sizeof(double);
   // u Fu r w tmp delta pz rc, the FP64 and FP32 bases, two sets of J/K/S accumulators, partials, Arnoldi scratch
   return vb * (8 + restart + 1) + ((plan->nu + 3) & ~3LL) * 4LL * (restart + 2) + 2 * ((int64_t)s.n * s.ds * 8 + 2LL * s.n_mfp * s.n_dir * 8) +
-         (int64_t)plan->ctx->num_sms * 2 * (restart + 3) * 8 + 8;
+         (int64_t)plan->ctx->num_sms * 2 * (restart + 3) * 8 + (2LL * restart + 4) * 8;
 }
 
 }  // namespace obte

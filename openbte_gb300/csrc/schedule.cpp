@@ -16,6 +16,7 @@
 // depend on the thread count.
 #include <algorithm>
 #include <array>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <numeric>
@@ -383,6 +384,7 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
   s.xk.resize((size_t)n_dir * n);
   s.wout.resize((size_t)n_dir * n);
   s.contact.resize((size_t)n_dir * n);
+  s.info.resize((size_t)n_dir * n);
   s.in_idx.resize((size_t)n_dir * n * nf);
   s.in_coef.resize((size_t)n_dir * n * nf);
   s.D.resize((size_t)n_dir * n);
@@ -421,7 +423,7 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
                        std::vector<int32_t>& last_use, std::vector<int32_t>& slot_of, std::vector<int64_t>& out_ptr,
                        std::vector<int64_t>& in_ptr, std::vector<int32_t>& out_adj, std::vector<int32_t>& in_face,
                        std::vector<std::vector<int32_t>>& wall_in, std::vector<std::vector<int32_t>>& wall_out,
-                       std::vector<int32_t>& src_of) {
+                       std::vector<int32_t>& src_of, std::vector<uint8_t>& out_slot) {
     const double* sq = mt->vmfp + (int64_t)q * dd;
     std::fill(D.begin(), D.end(), 0.0);
     std::fill(P.begin(), P.end(), 0.0);
@@ -478,13 +480,18 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
       }
     for (int64_t e = 0; e < n; ++e) { out_ptr[e + 1] += out_ptr[e]; in_ptr[e + 1] += in_ptr[e]; }
     out_adj.assign(out_ptr[n], 0);
+    out_slot.assign(out_ptr[n], 0);          // which inflow of its reader each outflow is
     in_face.assign(in_ptr[n], 0);
     {
       std::vector<int64_t> oc(out_ptr.begin(), out_ptr.end() - 1), ic(in_ptr.begin(), in_ptr.end() - 1);
       for (int64_t f = 0; f < nfd; ++f)
         if (g[f] < 0) {
-          in_face[ic[f_row[f]]++] = (int32_t)f;
-          if (!f_cut[f]) out_adj[oc[f_nb[f]]++] = f_row[f];
+          const int64_t k = ic[f_row[f]]++;
+          in_face[k] = (int32_t)f;
+          if (!f_cut[f]) {
+            out_slot[oc[f_nb[f]]] = (uint8_t)std::min<int64_t>(k - in_ptr[f_row[f]], 255);
+            out_adj[oc[f_nb[f]]++] = f_row[f];
+          }
         }
     }
     // Kahn topological order + longest-path levels
@@ -567,9 +574,11 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
         live += alive[L];
         o.nslots = std::max(o.nslots, live);
       }
-      std::vector<std::vector<int32_t>> release(nl + 2);
-      std::vector<int32_t> free_slots[8];
-      for (int32_t sl = o.nslots - 1; sl >= 0; --sl) free_slots[sl & 7].push_back(sl);
+      // free rows of each class (a stack each), the rows that a level frees (a list through next_freed)
+      std::vector<int32_t> stack((size_t)8 * (o.nslots / 8 + 1)), freed(nl + 3, -1), next_freed(o.nslots, -1);
+      const int32_t cap = o.nslots / 8 + 1;
+      int32_t top[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      for (int32_t sl = o.nslots - 1; sl >= 0; --sl) stack[(sl & 7) * cap + top[sl & 7]++] = sl;
       std::vector<int32_t> octet(n);
       int32_t n_oct = 0;
       for (int L = 0; L < nl; ++L) {
@@ -578,39 +587,32 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
       }
       const int ng = nf + 1;
       std::vector<uint64_t> groups((size_t)n_oct * ng, 0);
-      std::vector<uint64_t*> touched;
+      constexpr int kTouched = 24;           // more readers than that (none in a mesh) are left out of the choice
+      uint64_t* touched[kTouched];
       for (int L = 0; L < nl; ++L) {
-        for (int32_t sl : release[L]) free_slots[sl & 7].push_back(sl);
+        for (int32_t sl = freed[L]; sl >= 0; sl = next_freed[sl]) stack[(sl & 7) * cap + top[sl & 7]++] = sl;
         for (int32_t p = o.lev[L]; p < o.lev[L + 1]; ++p) {
           const int32_t e = order[p];
-          if (last_use[e] < 0) continue;
-          touched.clear();
-          touched.push_back(&groups[(size_t)octet[e] * ng]);
-          for (int64_t k = out_ptr[e]; k < out_ptr[e + 1]; ++k) {
-            const int32_t d = out_adj[k];
-            for (int64_t t = in_ptr[d]; t < in_ptr[d + 1] && t - in_ptr[d] < nf; ++t)
-              if (f_nb[in_face[t]] == e && !f_cut[in_face[t]])
-                touched.push_back(&groups[(size_t)octet[d] * ng + 1 + (t - in_ptr[d])]);
-          }
-          // a counter holds at most 8; the few words of an element add up without carries below 32 of them
+          const int32_t lu = last_use[e];
+          if (lu < 0) continue;
+          int nt = 0;
+          touched[nt++] = &groups[(size_t)octet[e] * ng];
+          for (int64_t k = out_ptr[e]; k < out_ptr[e + 1] && nt < kTouched; ++k)
+            if (out_slot[k] < nf) touched[nt++] = &groups[(size_t)octet[out_adj[k]] * ng + 1 + out_slot[k]];
+          // a counter holds at most 8: the sum of 24 words has no carries
           uint64_t sum = 0;
-          for (size_t k = 0; k < std::min<size_t>(touched.size(), 24); ++k) sum += *touched[k];
-          int best = -1, best_score = 0;
-          for (int c = 0; c < 8; ++c) {
-            if (free_slots[c].empty()) continue;
-            const int score = (int)((sum >> (8 * c)) & 0xFF);
-            if (best < 0 || score < best_score ||
-                (score == best_score && free_slots[c].size() > free_slots[best].size())) {
-              best = c;
-              best_score = score;
-            }
+          for (int k = 0; k < nt; ++k) sum += *touched[k];
+          int best = 0, best_key = INT_MAX;
+          for (int c = 0; c < 8; ++c) {      // fewest collisions, then the fullest stack
+            const int key = top[c] == 0 ? INT_MAX : ((int)((sum >> (8 * c)) & 0xFF) << 20) - top[c];
+            if (key < best_key) { best = c; best_key = key; }
           }
-          const int32_t sl = free_slots[best].back();
-          free_slots[best].pop_back();
-          for (uint64_t* w : touched)
-            if (((*w >> (8 * best)) & 0xFF) < 8) *w += (uint64_t)1 << (8 * best);
+          const int32_t sl = stack[best * cap + --top[best]];
+          for (int k = 0; k < nt; ++k)
+            if (((*touched[k] >> (8 * best)) & 0xFF) < 8) *touched[k] += (uint64_t)1 << (8 * best);
           slot_of[e] = sl;
-          release[last_use[e] + 1].push_back(sl);
+          next_freed[sl] = freed[lu + 1];
+          freed[lu + 1] = sl;
         }
       }
     }
@@ -629,12 +631,12 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
       s.slot[it] = slot_of[e];
       s.D[it] = D[e];
       s.P[it] = P[e];
-      int k = 0;
+      int k = 0, cut = 0;
       for (int64_t t = in_ptr[e]; t < in_ptr[e + 1]; ++t) {
         const int32_t f = in_face[t];
         if (k >= nf) { o.st = OBTE_ERR_BAD_ARG; o.err = "more inflow faces than element sides"; return; }
         o.n_up = std::max(o.n_up, k + 1);
-        if (f_cut[f]) { s.in_idx[it * nf + k] = pack_item(ITEM_PERIODIC, src_of[f_nb[f]]); ++o.n_cut; }
+        if (f_cut[f]) { s.in_idx[it * nf + k] = pack_item(ITEM_PERIODIC, src_of[f_nb[f]]); ++o.n_cut; ++cut; }
         else s.in_idx[it * nf + k] = pack_item(ITEM_CELL, slot_of[f_nb[f]]);
         s.in_coef[it * nf + k] = g[f] * f_t[f];
         if (keep_tf) {
@@ -655,6 +657,9 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
         }
         ++k;
       }
+      const bool contact = ck == OBTE_CONTACT_NANOWIRE || co_ptr[e] != co_ptr[e + 1];
+      s.info[it] = (uint8_t)(std::min(cut, 7) | (src_of[e] >= 0 ? 8 : 0) | (contact || !wall_out[e].empty() ? 16 : 0) |
+                             ((int)wall_out[e].size() << 5));
       if (src_of[e] >= 0) s.xk[it] = src_of[e];
       if (!wall_out[e].empty()) {
         const int32_t begin = (int32_t)o.wo_wall.size();
@@ -708,10 +713,11 @@ obte_status build_schedule(const obte_problem* pb, const obte_material* mt, Sche
     std::vector<int32_t> indeg(n), level(n), order(n), last_use(n), slot_of(n), out_adj, in_face;
     std::vector<int64_t> out_ptr(n + 1), in_ptr(n + 1);
     std::vector<std::vector<int32_t>> wall_in(n), wall_out(n);
+    std::vector<uint8_t> out_slot;
     std::vector<int32_t> src_of(n, -1);   // periodic source index of an element in the current direction
     for (int q = tid; q < n_dir; q += nthreads) {
       build_dir(q, outs[q], D, P, g, indeg, level, order, last_use, slot_of, out_ptr, in_ptr, out_adj, in_face,
-                wall_in, wall_out, src_of);
+                wall_in, wall_out, src_of, out_slot);
       for (int32_t e : outs[q].x_cell) src_of[e] = -1;
     }
   };

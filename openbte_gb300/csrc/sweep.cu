@@ -117,11 +117,7 @@ static void build_units_capped(const Schedule& s, int cap, int cap_pf, int cap_s
         cnt = npf = nsx = 0;
       };
       for (int32_t pos = lp[Lv]; pos < lp[Lv + 1]; ++pos) {
-        const size_t it = (size_t)q * s.n + pos;
-        int pf = 0;
-        for (int f = 0; f < s.nf; ++f)
-          if ((int)((uint32_t)s.in_idx[it * s.nf + f] >> ITEM_SHIFT) == ITEM_PERIODIC) ++pf;
-        const int sx = (s.xk[it] >= 0 || s.wout[it] != 0 || s.contact[it] >= 0) ? 1 : 0;
+        const int info = s.info[(size_t)q * s.n + pos], pf = info & 7, sx = info & 24 ? 1 : 0;
         if (cnt > 0 && (cnt == cap || npf + pf > cap_pf || nsx + sx > cap_sx)) close(pos);
         ++cnt;
         npf += pf;
@@ -168,11 +164,6 @@ struct UnitStats {
 static inline bool has_outputs(const Schedule& s, size_t it) {
   return s.xk[it] >= 0 || s.wout[it] != 0 || s.contact[it] >= 0;
 }
-static inline int cut_faces(const Schedule& s, size_t it) {
-  int c = 0;
-  for (int f = 0; f < s.nf; ++f) c += (int)((uint32_t)s.in_idx[it * s.nf + f] >> ITEM_SHIFT) == ITEM_PERIODIC;
-  return c;
-}
 
 // Output block of a unit: nx periodic sources, nw wall / contact entries, nwo wall entries.
 static inline int out_bytes(int nx, int nw, int nwo, int real_bytes) {
@@ -195,12 +186,13 @@ static UnitStats count_units(const Schedule& s, const Units& un, int real_bytes,
     for (int u = 0; u < un.n[q]; ++u) {
       int npf = 0, nwo = 0, nsx = 0, nx = 0, nw = 0;
       for (int32_t pos = up[u]; pos < up[u + 1]; ++pos) {
-        const size_t it = (size_t)q * s.n + pos;
-        npf += cut_faces(s, it);
-        nwo += s.wout[it] & 7;
-        nsx += has_outputs(s, it) ? 1 : 0;
-        nx += s.xk[it] >= 0 ? 1 : 0;
-        nw += s.wout[it] != 0 || s.contact[it] >= 0 ? 1 : 0;
+        const int info = s.info[(size_t)q * s.n + pos];
+        if (info == 0) continue;
+        npf += info & 7;
+        nwo += info >> 5;
+        nsx += info & 24 ? 1 : 0;
+        nx += (info >> 3) & 1;
+        nw += (info >> 4) & 1;
       }
       int32_t* c = cnt.data() + 4 * (size_t)(unit_base[q] + u);
       c[0] = npf; c[1] = nwo; c[2] = nx; c[3] = nw;
@@ -265,11 +257,12 @@ static Layout make_layout(const Schedule& s, const UnitStats& st, const Layout& 
   return l;
 }
 
-// CTAs that share an SM: by shared memory and by registers (launch bounds of the kernel).
+// CTAs that share an SM: by shared memory (handed out in 128-byte pieces: 45,600 B a CTA leave room for four, not five,
+// and took the 60k-triangle benchmark cell's sweep from 1.43 to 1.73 ms) and by registers (launch bounds of the kernel).
 template <typename Real>
 static int resident(const Layout& l) {
   const int by_regs = (sizeof(Real) == 4 && l.KV == 8 ? 5 : 4) * kMaxThreads / l.threads;
-  return (int)std::min<size_t>((size_t)std::min(by_regs, 32), kSmemPerSM / (l.smem + kSmemPerCta));
+  return (int)std::min<size_t>((size_t)std::min(by_regs, 32), kSmemPerSM / (((l.smem + 127) & ~(size_t)127) + kSmemPerCta));
 }
 
 struct Packed {
