@@ -17,16 +17,18 @@
 // the ring while the next unit runs.
 //
 // Data movement: everything a unit reads arrives in its stage of shared memory by TMA bulk copies
-// (cp.async.bulk + mbarrier), `nbuf` units ahead: the unit's records, its list of outputs, its (b, p) values, its periodic inflow rows (gathered per sweep by
+// (cp.async.bulk + mbarrier), `nbuf` units ahead: the unit's records, its list of outputs, its (b, p) values, its
+// periodic inflow rows (gathered per sweep by
 // sweep_prep_kernel, already in the table's precision and row layout) and, in FP64, its rows of the gain
 // table.  The header carries the source addresses of the unit nbuf further, so the loop reads no global
 // metadata.  T never goes to HBM.  Reductions of openbte/bte.py:222-243 are register accumulations over the
-// MFPs followed by one FP64 atomic per element (DeltaT', T_B', J) or per MFP (K, S).
+// MFPs followed by one FP64 atomic per element (DeltaT', T_B', J); K and S are sums of one thread per MFP.
 // Every mbarrier wait is bounded; on timeout the thread raises the device error word and skips the unit,
 // and the CTA waits (bounded) for its copies in flight and leaves after the next block-wide barrier.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <climits>
 #include <cmath>
 #include <cstdlib>
@@ -43,21 +45,21 @@ static constexpr int kBaseUnit = 128;     // elements per unit of the base layou
 
 // ---- packed element records -------------------------------------------------------
 // 32-bit words, ring rows as 16-bit halves in units of 16 bytes (ring_field):
-//   w0 cell | w1 so, s0 | w2 s1, s2 | w3 s3, kc | the reals c0 .. c(NF-1), D | padding to 16 B
-// so = output row, s* = inflow rows, kc = 1 + index of a contact element's entry in its unit's list of wall /
-// contact entries (0: no contact side), bit 15 set for a periodic source.  NF = the most cell and periodic inflow
+//   w0 cell | w1 so, s0 | w2 s1, s2 | w3 s3 | the reals c0 .. c(NF-1), D | padding to 16 B
+// so = output row, s* = inflow rows.  NF = the most cell and periodic inflow
 // faces of an element (Schedule::n_up): a convex cell has at least one outflow face, so triangles and squares
 // need two rows, tetrahedra three, not one per side.  32 B (FP32) / 48 B (FP64), tetrahedra 32 B / 64 B.  Leaving
 // out the rows that every element read as zero, with the rows' bank classes (schedule.cpp), took the 60k-triangle
 // sweep (100 x 96, FP32) from 1,430 to 1,167 us and 5 of 7 spilled words from its element loop.
 // A unit's static data: its record block (header, records), followed by its output block:
-//   header 0: elements | (values start one pair into their window) << 16, first position, periodic outputs |
-//             wall and contact outputs << 16, then of unit u + nbuf: bank rows | size of its output block << 16
+//   header 0: elements | (values start one pair into their window) << 16 | contact outputs << 17, first position,
+//             periodic outputs | wall and contact outputs << 16, then of unit u + nbuf: bank rows | size of its
+//             output block << 16
 //   header 1: of unit u + nbuf: record block and value sources (16-byte units), their sizes (16-byte units,
 //             block | values << 16), its first bank row among all units' rows
 //   outputs:  periodic sources (int2: source slot, row; padded to 16 B), wall / contact entries (int4: row,
 //             count | first of the unit's wall entries << 3 | wall entries of the unit << 16, contact entry, first
-//             wall entry overall), wall entries (4 reals: area vector / volume, 1 / (-sum_mq min(sigma . w, 0))),
+//             wall entry overall; those with a contact entry first, in the order of their sums), wall entries (4 reals: area vector / volume, 1 / (-sum_mq min(sigma . w, 0))),
 //             their wall indices
 __host__ __device__ constexpr int rec_words(int real_bytes, int nf) {
   return ((4 + (nf + 1) * (real_bytes / 4)) + 3) & ~3;
@@ -219,12 +221,12 @@ static UnitStats count_units(const Schedule& s, const Units& un, int real_bytes,
 }
 
 // ---- shared memory of a CTA (bytes) --------------------------------------------------
-//   [0, 64) mbarriers | [64, 68) first unit that timed out | [96, ...) sigma [3][KV], K, S accumulators [KV]
+//   [0, 64) mbarriers | [64, 68) first unit that timed out | [96, ...) sigma [3][KV]
 //   | [kRingOff, ...) ring | nbuf stages of (record block | values | gain rows) | nbuf + 1 output blocks
 // (a unit's outputs are written while the next unit runs, so its output block outlives its stage)
 static constexpr int kMaxBuf = 8;
 static constexpr int kFailOff = 64, kSigOff = 96, kRingOff = 384;
-static_assert(kSigOff + 5 * 32 <= kRingOff, "sigma and accumulators of 32-byte rows");
+static_assert(kSigOff + 3 * 32 <= kRingOff, "sigma of 32-byte rows");
 static constexpr size_t kSmemPerSM = 233472, kSmemPerCta = 1024;   // capacity, reserved per CTA
 
 struct Layout {
@@ -281,8 +283,40 @@ struct Packed {
   int64_t n_pf = 0;
 };
 
+// The place of each contact entry of direction q in the sums K and S of an output pass, by entry (relative to the
+// direction's first).  The sums are in the sweep's precision, so their order is part of the result: unit by unit
+// of the base layout, in a unit the 32-element groups with fewer contact elements first (of equal ones the later
+// group), elements of a group in order.  That is the order in which one FP32 shared-memory atomic per element and MFP
+// arrives most often from a CTA with one element of a base unit to a thread: on 8,000 triangles x 60 x 48 at least
+// 2,876 of 2,880 sums have these bits (2,858 in position order; two runs of the atomics agree on as many), while
+// sums in FP64 would be 1e-7 off.  Beside it the atomics cost time: the resident solve of 60,000 triangles x 100 x 96
+// went from 46.1 to 45.0 ms without them, 8,000 x 60 x 48 from 11.95 to 11.83 ms.
+static void contact_order(const Schedule& s, const Units& base, int q, std::vector<int32_t>& place) {
+  struct Entry { int32_t unit, count, group, pos; };
+  std::vector<Entry> e;
+  const int32_t* up = base.ptr.data() + base.off[q];
+  for (int32_t u = 0, pos = 0; u < base.n[q]; ++u)
+    for (; pos < up[u + 1]; ++pos)
+      if (s.contact[(size_t)q * s.n + pos] >= 0) e.push_back({u, 0, (pos - up[u]) >> 5, pos});
+  for (size_t a = 0, b = 0; a < e.size(); a = b) {
+    while (b < e.size() && e[b].unit == e[a].unit && e[b].group == e[a].group) ++b;
+    for (size_t k = a; k < b; ++k) e[k].count = (int32_t)(b - a);
+  }
+  std::vector<int32_t> ord(e.size());
+  std::iota(ord.begin(), ord.end(), 0);
+  std::sort(ord.begin(), ord.end(), [&](int32_t i, int32_t j) {
+    const Entry &x = e[i], &y = e[j];
+    if (x.unit != y.unit) return x.unit < y.unit;
+    if (x.count != y.count) return x.count < y.count;
+    return x.group != y.group ? x.group > y.group : x.pos < y.pos;
+  });
+  place.resize(e.size());
+  for (size_t k = 0; k < ord.size(); ++k) place[ord[k]] = (int32_t)k;
+}
+
+// base: the units of the base layout
 template <typename Real>
-static obte_status pack(const Schedule& s, const Units& un, const std::vector<int64_t>& unit_base,
+static obte_status pack(const Schedule& s, const Units& un, const Units& base, const std::vector<int64_t>& unit_base,
                         const std::vector<int32_t>& cnt, const Layout& lay, Packed& pk) {
   const int W = rec_words(sizeof(Real), s.n_up);
   constexpr int CSTEP = sizeof(Real) / 4, COEF = 4, VB = 2 * sizeof(Real);
@@ -365,29 +399,35 @@ static obte_status pack(const Schedule& s, const Units& un, const std::vector<in
     int64_t nsp = spec_base[q];
     const int32_t* up = un.ptr.data() + un.off[q];
     int32_t wo_run = s.wo_off[q];          // first wall entry of the unit
+    std::vector<int32_t> place;            // of the direction's contact entries in their sums
+    contact_order(s, base, q, place);
+    size_t ce = 0;                         // contact entries before the element
+    std::vector<std::pair<int32_t, std::array<int32_t, 4>>> entries;   // the unit's wall / contact entries
     for (int u = 0; u < un.n[q]; ++u) {
       const int64_t gu = unit_base[q] + u;
       const int n_el = up[u + 1] - up[u], npf = cnt[4 * gu], nwo = cnt[4 * gu + 1], nx = cnt[4 * gu + 2],
                 nw = cnt[4 * gu + 3];
-      int32_t* base = pk.blk.data() + (size_t)boff[gu] * 4;
-      int32_t* recs = base + kHeader / 4;
+      int32_t* head = pk.blk.data() + (size_t)boff[gu] * 4;
+      int32_t* recs = head + kHeader / 4;
       int32_t* xo = recs + (size_t)n_el * W;
       int32_t* wo = xo + (((size_t)nx * 2 + 3) & ~(size_t)3);
       int32_t* wg = wo + (size_t)nw * 4;
+      entries.clear();
+      int n_contact = 0;
       if (nx & 1) xo[2 * nx] = xo[2 * nx + 1] = 0;
       // header: this unit, and the source addresses of the unit nbuf further
       const int32_t* own = pk.desc.data() + 8 * (size_t)gu;
-      base[0] = own[0];
-      base[1] = own[1];
-      base[2] = nx | (nw << 16);
-      std::fill(base + 3, base + 8, 0);
+      head[0] = own[0];
+      head[1] = own[1];
+      head[2] = nx | (nw << 16);
+      std::fill(head + 3, head + 8, 0);
       if (u + lay.nbuf < un.n[q]) {
         const int32_t* f = pk.desc.data() + 8 * (size_t)(gu + lay.nbuf);
-        base[3] = f[3];
-        base[4] = f[4];
-        base[5] = f[5];
-        base[6] = f[6];
-        base[7] = f[2];
+        head[3] = f[3];
+        head[4] = f[4];
+        head[5] = f[5];
+        head[6] = f[6];
+        head[7] = f[2];
       }
       for (int e = 0; e < nwo; ++e) {      // wall geometry
         const int32_t w = s.wo_wall[wo_run + e];
@@ -398,7 +438,7 @@ static obte_status pack(const Schedule& s, const Units& un, const std::vector<in
         wg[(size_t)nwo * 4 * CSTEP + e] = w;
       }
       for (int e = nwo; e & 3; ++e) wg[(size_t)nwo * 4 * CSTEP + e] = 0;
-      int ent = 0, nwl = 0;
+      int ent = 0;
       const int bank = lay.prow0 + (u % lay.nbuf) * lay.emax;
       for (int32_t pos = up[u]; pos < up[u + 1]; ++pos) {
         const size_t it = (size_t)q * s.n + pos;
@@ -446,15 +486,17 @@ static obte_status pack(const Schedule& s, const Units& un, const std::vector<in
           xo[1] = field(so) << 4;
           xo += 2;
         }
-        r[3] = field(row_in[3]) | (s.xk[it] >= 0 ? (int)0x80000000 : 0);
+        r[3] = field(row_in[3]);
         if (s.wout[it] != 0 || s.contact[it] >= 0) {
-          if (s.contact[it] >= 0) r[3] |= (nwl + 1) << 16;
-          ++nwl;
-          wo[0] = field(so) << 4;
-          wo[1] = (s.wout[it] ? (((s.wout[it] >> 3) - wo_run) << 3) | (s.wout[it] & 7) : 0) | (nwo << 16);
-          wo[2] = s.contact[it];
-          wo[3] = s.wout[it] >> 3;
-          wo += 4;
+          const bool contact = s.contact[it] >= 0;
+          entries.push_back({contact ? place[ce] : INT_MAX,
+                             {field(so) << 4,
+                              (s.wout[it] ? (((s.wout[it] >> 3) - wo_run) << 3) | (s.wout[it] & 7) : 0) | (nwo << 16),
+                              s.contact[it], s.wout[it] >> 3}});
+          if (contact) {
+            ++ce;
+            ++n_contact;
+          }
         }
         r[1] = field(so) | (field(row_in[0]) << 16);
         r[2] = field(row_in[1]) | (field(row_in[2]) << 16);
@@ -474,6 +516,10 @@ static obte_status pack(const Schedule& s, const Units& un, const std::vector<in
         std::memcpy(&r[COEF + s.n_up * CSTEP], &dv, sizeof(Real));
         for (int wd = COEF + (s.n_up + 1) * CSTEP; wd < W; ++wd) r[wd] = 0;   // padding to 16 bytes
       }
+      // contact entries in the order of their sums, then the others
+      std::stable_sort(entries.begin(), entries.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
+      for (const auto& e : entries) wo = std::copy(e.second.begin(), e.second.end(), wo);
+      head[0] |= n_contact << 17;
       wo_run += nwo;
     }
   });
@@ -847,6 +893,10 @@ __device__ __forceinline__ void row_store(unsigned char* ring, unsigned off, int
   }
 }
 
+// a b, rounded (never contracted into an addition)
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
 // 1 / x for a normal x (the sweep's denominators are 1 + L D >= 1)
 __device__ __forceinline__ float rcp(float x) {
   float r;
@@ -907,8 +957,6 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
   int* s_fail = reinterpret_cast<int*>(smem + kFailOff);
   Real* s_sig = reinterpret_cast<Real*>(smem + kSigOff);    // [3][MC]
-  Real* s_k = s_sig + 3 * MC;
-  Real* s_s = s_k + MC;
   unsigned char* ring = smem + kRingOff;
 
   int bid = (int)blockIdx.x;
@@ -955,10 +1003,7 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
       tt2[j / 2] = {make_float2(t0.x, t1.x), make_float2(t0.y, t1.y)};
     }
   }
-  for (int j = tid; j < MC; j += nthr) {
-    reinterpret_cast<Real*>(ring + (size_t)p.zero_row * ROWB)[j] = Real(0);
-    if (FINAL) { s_k[j] = 0; s_s[j] = 0; }
-  }
+  for (int j = tid; j < MC; j += nthr) reinterpret_cast<Real*>(ring + (size_t)p.zero_row * ROWB)[j] = Real(0);
   if (tid == 0) {
     for (int i = 0; i < nbuf; ++i) mbar_init(&bars[i], 1);
     *s_fail = INT_MAX;
@@ -1025,19 +1070,54 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
   unsigned phase = 0;    // parity of its mbarrier phase ((u / nbuf) & 1)
   const unsigned char* st = smem + p.stage0;
   int4 hd = make_int4(0, 0, 0, 0);
+  // final pass: kappa and suppression sums of the direction, MFP `cj` in this thread (a warp before the issuer's)
+  const int cj = nthr >= 64 ? tid - (nthr - 64) : tid;
+  Real ksum = 0, ssum = 0;
+  // MFP j of the row at byte offset `off`
+  auto row_value = [&](unsigned off, int j) -> Real {
+    constexpr int H = 16 / (int)sizeof(Real);
+    const Real v = reinterpret_cast<const Real*>(ring + (off ^ (j >= H ? 16u : 0u)))[j % H];
+    if constexpr (DF) return dpack_value(v);
+    else return v;
+  };
+  // The unit's part of the contact sums in its entries' order (contact_order): products rounded, then added one by
+  // one, loads four entries ahead.  One thread per MFP instead of one shared-memory atomic per element and MFP:
+  // the sums are the same in every pass and whatever the threads and stages.
+  auto contacts = [&](const int4* ent, int count) {
+    for (int i0 = 0; i0 < count; i0 += 4) {
+      Real kv[4], sv[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        kv[k] = sv[k] = Real(0);
+        if (i0 + k < count) {
+          const int4 e = ent[i0 + k];
+          const Real T = row_value((unsigned)e.x, cj);
+          kv[k] = mul_rn(p.kcoef[(int64_t)e.z * p.m_pad + m0 + cj], T);
+          sv[k] = mul_rn(p.scoef[e.z], T);
+          if (p.det) {
+            p.kpart[(int64_t)e.z * p.m_pad + m0 + cj] = kv[k];
+            p.spart[(int64_t)e.z * p.m_pad + m0 + cj] = sv[k];
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        ksum += kv[k];
+        ssum += sv[k];
+      }
+    }
+  };
   // Per-MFP outputs of a finished unit, from its rows in the ring: one lane per (periodic source, MFP) from the
   // last thread down, one lane per wall element from the warp before (the high threads have no
-  // element in most units).  Done while the next unit runs, off the chain from level to level; inside the
-  // element loop they would take ~150 instructions of every warp with one such element.
-  auto outputs = [&](const unsigned char* ob, int counts) {
+  // element in most units), one lane per MFP for the contact sums.  Done while the next unit runs, off the chain
+  // from level to level; inside the element loop they would take ~150 instructions of every warp with one such
+  // element.
+  auto outputs = [&](const unsigned char* ob, int counts, int n_contact) {
     const int nx = counts & 0xFFFF, nw = (int)((unsigned)counts >> 16);
     for (int i = nthr - 1 - tid; i < nx * MC; i += nthr) {
       const int k = i / MC, j = MC - 1 - (i - k * MC);      // consecutive lanes, consecutive MFPs
       const int2 e = reinterpret_cast<const int2*>(ob)[k];
-      constexpr int H = 16 / (int)sizeof(Real);
-      const unsigned off = (unsigned)e.y ^ (j >= H ? 16u : 0u);
-      Real v = reinterpret_cast<const Real*>(ring + off)[j % H];
-      if constexpr (DF) v = dpack_value(v);
+      const Real v = row_value((unsigned)e.y, j);
       if (j < mc) dT_out[p.n + p.nd + (int64_t)e.x * p.n_mfp + m0 + j] = widen(v);
     }
     if (nw) {
@@ -1047,21 +1127,8 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
       for (; i < nw; i += nthr) {
         wall_outputs<Real, MC, DF>(p, wb, nw, i, ring, s_sig, dT_out, chunk);
       }
-    }
-  };
-  // kappa and suppression sums of contact entry ce (final pass)
-  auto contact = [&](int ce, const Real* Tc) {
-#pragma unroll
-    for (int j = 0; j < KV; ++j) {
-      if (j < mc) {
-        const Real kv = p.kcoef[(int64_t)ce * p.m_pad + m0 + j] * Tc[j], sv = p.scoef[ce] * Tc[j];
-        if (p.det) {
-          p.kpart[(int64_t)ce * p.m_pad + m0 + j] = kv;
-          p.spart[(int64_t)ce * p.m_pad + m0 + j] = sv;
-        } else {
-          atomicAdd(&s_k[j], kv);
-          atomicAdd(&s_s[j], sv);
-        }
+      if constexpr (FINAL) {
+        if (cj >= 0 && cj < mc) contacts(reinterpret_cast<const int4*>(wb), n_contact);
       }
     }
   };
@@ -1070,7 +1137,7 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
   auto arrive = [&](int u) {
     if (mbar_wait_bounded(&bars[bi], phase, p.wait_limit)) {
       hd = *reinterpret_cast<const int4*>(st);
-      fetch(st, hd.x >> 16, tid);
+      fetch(st, (hd.x >> 16) & 1, tid);
     } else {
       hd = make_int4(0, 0, 0, 0);
       atomicOr(p.err, 1);
@@ -1079,14 +1146,11 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
   };
   arrive(0);
   __syncthreads();
-  int counts = 0;        // outputs of unit u - 1
+  int counts = 0, n_contact = 0;         // outputs of unit u - 1
   for (int u = 0; u < nlev; ++u) {
     // the first failed unit, written before the barrier above; later ones carry a larger number
     const int fail = *(volatile int*)s_fail;
     const int n_el = hd.x & 0xFFFF;
-    const int co = u == 0 ? 0 : oi == nbuf ? 0 : oi + 1;   // output block of this unit
-    int pend = -1;                                         // final pass: contact entry summed at the unit's end
-    Real Tp0[FINAL ? KV : 1];
     int el = tid;
     // read together: while the row loads are in flight the issuer refills the stage of unit u - 1
     Real v0[KV], v1[KV], v2[NF > 2 ? KV : 1], v3[NF > 3 ? KV : 1];
@@ -1156,8 +1220,8 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
         j1 = ((double)jb.h.x + (double)jb.h.y) + ((double)jb.l.x + (double)jb.l.y);
         j2 = ((double)jc.h.x + (double)jc.h.y) + ((double)jc.l.x + (double)jc.l.y);
         row_store<MC, KV>(ring, so, 0, Tp);
-        // real values for the stored fields and contact sums below
-        const bool need = p.Xs != nullptr || p.Xd != nullptr || (((unsigned)r[3] >> 16) & 0x7FFFu) != 0u;
+        // real values for the stored fields below
+        const bool need = p.Xs != nullptr || p.Xd != nullptr;
 #pragma unroll
         for (int j = 0; j < KV; ++j) T[j] = need ? dpack_value(Tp[j]) : Real(0);
       } else if constexpr (sizeof(Real) == 4) {
@@ -1253,48 +1317,26 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
           if (p.ds > 2) atomicAdd(&p.Jraw[(int64_t)c * p.ds + 2], widen(j2));
         }
       }
-      if (FINAL) {
-        // contact elements; those of a warp with a periodic source after the others of the unit (the sums are in
-        // the sweep's precision: this keeps their order, inflow side first)
-        const int kc = (int)((unsigned)r[3] >> 16);
-        const bool late = __any_sync(__activemask(), (kc & 0x8000) != 0);
-        if (pend >= 0) contact(pend, Tp0);
-        pend = -1;
-        if (kc & 0x7FFF) {
-          const int nx = hd.z & 0xFFFF;
-          const int ce = reinterpret_cast<const int4*>(smem + p.out0 + co * p.out + ((nx * 8 + 15) & ~15))[(kc & 0x7FFF) - 1].z;
-          if (late) {
-            pend = ce;
-#pragma unroll
-            for (int j = 0; j < KV; ++j) Tp0[FINAL ? j : 0] = T[j];
-          } else {
-            contact(ce, T);
-          }
-        }
-      }
       el += nthr;
       if (el < n_el) {           // units wider than the CTA
-        fetch(st, hd.x >> 16, el);
+        fetch(st, (hd.x >> 16) & 1, el);
         rows();
       }
     }
-    if (counts) outputs(smem + p.out0 + oi * p.out, counts);
+    if (counts) outputs(smem + p.out0 + oi * p.out, counts, n_contact);
     counts = hd.z;
+    if constexpr (FINAL) n_contact = hd.x >> 17;
     if (u > 0 && ++oi > nbuf) oi = 0;
     // unit u + 1: its records (not its rows) before the barrier
     if (++bi == nbuf) { bi = 0; phase ^= 1u; }
     st = smem + p.stage0 + bi * p.stage;
     if (u + 1 < nlev) arrive(u + 1);
-    if (FINAL && pend >= 0) contact(pend, Tp0);
     __syncthreads();
   }
-  if (counts) outputs(smem + p.out0 + oi * p.out, counts);
-  if (FINAL) __syncthreads();
-  if (FINAL && !p.det) {
-    for (int j = tid; j < mc; j += nthr) {
-      p.K[(int64_t)(m0 + j) * p.n_dir + q] = (double)s_k[j];
-      p.S_out[(int64_t)(m0 + j) * p.n_dir + q] = (double)s_s[j];
-    }
+  if (counts) outputs(smem + p.out0 + oi * p.out, counts, n_contact);
+  if (FINAL && !p.det && cj >= 0 && cj < mc) {
+    p.K[(int64_t)(m0 + cj) * p.n_dir + q] = (double)ksum;
+    p.S_out[(int64_t)(m0 + cj) * p.n_dir + q] = (double)ssum;
   }
 }
 
@@ -1423,9 +1465,10 @@ static int choose_mc(const Schedule& s, const UnitStats& base) {
 // (60,000) 1,159 and 1,422; units of 96, 128 and 192 elements on the 60k benchmark cell 1,549, 1,430 and 1,649 us (5, 5
 // and 4 CTAs an SM).
 template <typename Real>
-static obte_status choose_layout(const Schedule& s, size_t optin, Units& un, std::vector<int64_t>& unit_base,
-                                 std::vector<int32_t>& cnt, Layout& lay) {
-  build_units(s, kBaseUnit, un);
+static obte_status choose_layout(const Schedule& s, size_t optin, Units& un, Units& base,
+                                 std::vector<int64_t>& unit_base, std::vector<int32_t>& cnt, Layout& lay) {
+  build_units(s, kBaseUnit, base);
+  un = base;
   UnitStats st = count_units(s, un, sizeof(Real), unit_base, cnt);
   if (st.bad_wo) {
     set_error("wall re-emission entries are not in sweep order");
@@ -1512,8 +1555,9 @@ static obte_status upload_tables(obte_plan plan, DevSchedule& d) {
     std::vector<int64_t> unit_base;
     std::vector<int32_t> cnt;
     Layout lay;
-    OBTE_TRY(choose_layout<Real>(s, plan->ctx->smem_optin, un, unit_base, cnt, lay));
-    OBTE_TRY(pack<Real>(s, un, unit_base, cnt, lay, pk));
+    Units base;
+    OBTE_TRY(choose_layout<Real>(s, plan->ctx->smem_optin, un, base, unit_base, cnt, lay));
+    OBTE_TRY(pack<Real>(s, un, base, unit_base, cnt, lay, pk));
     OBTE_TRY(upload(d.unit_base, unit_base, st));
     d.n_units = unit_base[s.n_dir];
   }
@@ -1731,8 +1775,9 @@ static obte_status tables_digest_impl(const Schedule& s, uint64_t* digest) {
     PhaseTimer tp("pack");
     std::vector<int32_t> cnt;
     Layout lay;
-    OBTE_TRY(choose_layout<Real>(s, 232448, un, unit_base, cnt, lay));   // 227 KB: the most one CTA can have
-    OBTE_TRY(pack<Real>(s, un, unit_base, cnt, lay, pk));
+    Units base;
+    OBTE_TRY(choose_layout<Real>(s, 232448, un, base, unit_base, cnt, lay));   // 227 KB: the most one CTA can have
+    OBTE_TRY(pack<Real>(s, un, base, unit_base, cnt, lay, pk));
   }
   Fnv f;
   f.vec(un.ptr); f.vec(un.off); f.vec(un.n);
