@@ -376,5 +376,16 @@ void amg_device(const AmgHierarchy& H, AmgDev& d, bool fixed_order) {
   }
 }
 
+int64_t amg_bytes(const AmgHierarchy& H) {
+  int64_t b = (int64_t)H.nc * H.nc * 8;
+  auto csr = [&](const DevCsr& m) { b += m.nnz * 12 + m.n * 4; };
+  for (size_t l = 0; l + 1 < H.lv.size(); ++l) {
+    csr(H.lv[l]->G);
+    csr(H.lv[l]->Q);
+    csr(H.lv[l]->Qt);
+  }
+  return b;
+}
+
 int amg_levels(const AmgHierarchy& H) { return (int)H.lv.size(); }
 }  // namespace obte

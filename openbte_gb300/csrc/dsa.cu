@@ -69,8 +69,8 @@ struct DsaParams {
 // As 12 launches of 3.9 us each with its gap an application took 47 us (64^2 and 128^2 pixels); with the Arnoldi
 // step in one launch as well, 64^2 pixels x 20 x 32 went from 33.1 to 26.5 ms a gradient evaluation.
 template <typename Bar>
-__global__ void __launch_bounds__(kPhaseThreads, 1) dsa_kernel(const __grid_constant__ DsaParams P) {
-  __shared__ double red[kPhaseThreads];
+__global__ void __launch_bounds__(Bar::kThreads, Bar::kBlocks == 1 ? 1 : 4) dsa_kernel(const __grid_constant__ DsaParams P) {
+  __shared__ double red[Bar::kThreads];
   __shared__ Rows sA;
   __shared__ AmgRows sM;
   Bar bar(P.count, P.err);

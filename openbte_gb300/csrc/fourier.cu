@@ -29,6 +29,15 @@ namespace {
 
 constexpr int FT = 256;
 
+// Blocks of a solve: as many as its rows fill, 104 to a block: the barrier is cheaper with fewer blocks, and the other SMs
+// are left to other streams (8,000 triangles: 77 blocks 3.55 ms, 152 3.7, 39 3.95); at least a quarter of the SMs
+// (2,000 triangles: 20 blocks 3.9 ms, 38 3.45).
+PhaseShape fourier_shape(int64_t n, int num_sms) {
+  PhaseShape s = phase_shape(n, num_sms);
+  if (!s.cluster) s.blocks = (int)std::min<int64_t>(num_sms, std::max<int64_t>(num_sms / 4, (n + 103) / 104));
+  return s;
+}
+
 // Everything of the solve after assembly, for the one launch that runs it.
 struct FourierParams {
   int64_t n;
@@ -46,6 +55,7 @@ struct FourierParams {
   const int32_t *c_ptr, *c_side;
   double *T, *C, *r[2], *z, *p[2], *Ap, *grad, *part;
   int max_iter, cg_max, check;
+  int smem;                                  // bytes of shared memory for the matrices
   double rtol, cg_rtol;
   double* out;                               // deferred corrections, CG iterations
   unsigned* count;
@@ -59,18 +69,18 @@ struct FourierParams {
 // alternate between two buffers so that neighbours read the values of the phase before.
 //
 // The solve was bound by its launches (60k triangles: 10 corrections, 184 CG iterations, 2,180 launches of 4.6 us
-// with their gaps, 13.3 ms; 600 triangles 6.9 ms).  Its matrices stay in shared memory (60k triangles: 85 KB
-// an SM), so what is left of a phase is the barrier, one gather through L2 and a chain of FP64
-// operations at 64-76 cycles each: 8.8 and 2.9 ms.
+// with their gaps, 11.7 ms; 600 triangles 6.9 ms).  Its matrices stay in shared memory as far as a third of an SM
+// has room (60k triangles: 69 of 85 KB an SM), so what is left of a phase is the barrier, one gather through L2 and
+// a chain of FP64 operations at 64-76 cycles each: 7.3 and 2.7 ms.
 template <typename Bar>
-__global__ void __launch_bounds__(kPhaseThreads, 1) fourier_kernel(const __grid_constant__ FourierParams P) {
+__global__ void __launch_bounds__(Bar::kThreads, Bar::kBlocks) fourier_kernel(const __grid_constant__ FourierParams P) {
   extern __shared__ __align__(16) char smem[];
-  __shared__ double red[kPhaseThreads];
+  __shared__ double red[Bar::kThreads];
   __shared__ Rows sA;
   __shared__ AmgRows sM;
   Bar bar(P.count, P.err);
   const int tid = threadIdx.x, nthr = blockDim.x, nb = gridDim.x;
-  Arena ar{smem, kPhaseSmem};
+  Arena ar{smem, P.smem};
   load_rows(P.A, &sA, ar);
   if (P.has_amg) load_amg(P.amg, &sM, ar);
   int r0, r1;
@@ -510,7 +520,7 @@ extern "C" obte_status obte_fourier_plan_create(obte_context ctx, const obte_fou
   const size_t vb = (size_t)n * sizeof(double);
   // r and p alternate between two buffers; partials: seven sums of one value per block
   up(P->C.alloc(vb)); up(P->r.alloc(2 * vb)); up(P->z.alloc(vb)); up(P->p.alloc(2 * vb));
-  up(P->Ap.alloc(vb)); up(P->part.alloc(7 * sizeof(double) * (size_t)phase_shape(n, ctx->num_sms).blocks));
+  up(P->Ap.alloc(vb)); up(P->part.alloc(7 * sizeof(double) * (size_t)fourier_shape(n, ctx->num_sms).blocks));
   up(P->sc.alloc(4 * sizeof(double))); up(P->grad.alloc(vb * dim));
   up(P->kout.alloc((size_t)std::max<int64_t>(P->nc, 1) * 8));
   // OBTE_FOURIER_JACOBI=1 keeps the diagonal preconditioner (same solution, ~40x more CG iterations)
@@ -565,8 +575,12 @@ extern "C" obte_status obte_fourier_solve(obte_fourier_plan P, const obte_fourie
   f.count = reinterpret_cast<unsigned*>(f.out + 2);
   f.err = reinterpret_cast<int*>(f.out + 3);
   OBTE_CUDA(cudaMemsetAsync(P->sc.p, 0, 4 * sizeof(double), st));
-  OBTE_CUDA(phase_launch(phase_shape(n, P->ctx->num_sms), fourier_kernel<ClusterBarrier>, fourier_kernel<GridBarrier>, f,
-                         kPhaseSmem, st));
+  const PhaseShape shape = fourier_shape(n, P->ctx->num_sms);
+  // shared memory for a block's part of the matrices (an eighth more, as rows differ), as far as it may have
+  const int64_t bytes = (int64_t)(P->val.bytes + P->ci.bytes + P->rp.bytes) + (P->amg ? amg_bytes(*P->amg) : 0);
+  f.smem = (int)std::min<int64_t>(shape.cluster ? ClusterBarrier::kSmem : GridBarrier::kSmem,
+                                  (bytes / shape.blocks * 9 / 8 + 2048 + 127) & ~(int64_t)127);
+  OBTE_CUDA(phase_launch(shape, fourier_kernel<ClusterBarrier>, fourier_kernel<GridBarrier>, f, f.smem, st));
   count_launch();
   double kappa = 0;
   std::vector<double> kh(std::max<int64_t>(P->nc, 1));

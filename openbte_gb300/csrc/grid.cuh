@@ -4,7 +4,7 @@
 // The phases of a multigrid-preconditioned iteration on a few thousand to a hundred thousand elements take
 // 1-2 us each, less than the launch between two of them (3.9-4.6 us with its gap); here a phase ends at a
 // barrier instead.  Small problems run as one cluster of 8 CTAs (hardware barrier, 0.4-0.8 us), larger ones on
-// every SM as a cooperative launch (all blocks resident) with an arrive counter in global memory (1.3 us).
+// a part of every SM as a cooperative launch (all blocks resident) with an arrive counter in global memory (1.3 us).
 // Vectors that change between phases are read with plain loads (never through the read-only path).
 #pragma once
 
@@ -24,6 +24,8 @@ __device__ __forceinline__ double widen(float f) {
 
 // Barrier over the blocks of a cluster.
 struct ClusterBarrier {
+  static constexpr int kThreads = 512, kBlocks = 1;      // threads per block, blocks an SM has registers for
+  static constexpr int kSmem = 200 * 1024;               // shared memory for a solve's matrices at most
   __device__ ClusterBarrier(unsigned*, int*) {}
   __device__ bool wait() {
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
@@ -36,6 +38,7 @@ struct ClusterBarrier {
 // barrier.  The wait is bounded; when it gives up (on any block) the error word is set and wait() is false in
 // every thread of that block, whose caller returns; the other blocks run into their own bounds.
 struct GridBarrier {
+  static constexpr int kThreads = 256, kBlocks = 3, kSmem = 69 * 1024;
   static constexpr int kPolls = 1 << 21;
   unsigned* count;
   int* err;
@@ -145,6 +148,7 @@ struct AmgDev {
   double* x[kAmgMaxLevels];
 };
 void amg_device(const AmgHierarchy& H, AmgDev& d, bool fixed_order);
+int64_t amg_bytes(const AmgHierarchy& H);      // of the matrices that a V-cycle reads
 
 // A block's rows [r0, r1) of a matrix; rp, ci and val are its own part, in shared memory where they fit.
 struct Rows {
@@ -315,23 +319,32 @@ struct PhaseShape {
   int blocks, threads;
   bool cluster;
 };
-constexpr int kPhaseThreads = 512;
 // A cluster's barrier is the cheaper one, but its 8 SMs have a twentieth of the FP64 rate.  Fourier solves of 2D
-// cells, cluster against grid: 600 elements 2.93 and 3.76 ms, 1,100 3.45 and 3.96, 2,000 4.24 and 3.69, 8,000
-// 5.96 and 4.23; of a 3D one with 2,000, 17.6 and 15.6.
+// cells, cluster against grid: 600 elements 2.75 and 3.76 ms, 1,100 3.45 and 3.96, 2,000 4.24 and 3.42, 8,000
+// 5.96 and 3.55; of a 3D one with 2,000, 17.6 and 15.6.
+//
+// A cooperative launch waits until all its blocks fit and then holds their room for the whole solve, while other
+// streams' kernels wait for theirs.  So a block takes no more than a third of an SM: 256 threads of 80 registers
+// and 69 KB.  With 512 threads of 128 registers and 200 KB a solve held every SM: four streams of solves of 8,000 triangles
+// x 60 x 48 beside one that repeats Fourier solves of 60,000 went from 189 to 6 a second (129 now; with
+// Fourier solves of 4-5 us launches 138, beside a fifth of the Fourier solves), four streams of Fourier solves of 8,000
+// from 492 a second to 274 (1,075 now), of 60,000 from 234 to 162 (357 now).  Alone, Fourier solves of
+// 60,000 triangles take 7.3 ms for the 6.3 of a whole-SM block (half an SM 7.1, a quarter 8.2), of 8,000 3.55 for 3.7.
 constexpr int64_t kClusterElems = 1536;
 inline PhaseShape phase_shape(int64_t n, int num_sms) {
-  if (n <= kClusterElems) return {8, kPhaseThreads, true};
-  return {num_sms, kPhaseThreads, false};
+  if (n <= kClusterElems) return {8, ClusterBarrier::kThreads, true};
+  return {num_sms, GridBarrier::kThreads, false};
 }
-constexpr int kPhaseSmem = 200 * 1024;     // of the 227 KB a block can have, for a solve's matrices
 // Launch kern<ClusterBarrier> or kern<GridBarrier> by the shape.
 template <typename Params>
 cudaError_t phase_launch(const PhaseShape& ps, void (*clustered)(Params), void (*coop)(Params), const Params& p,
                          int smem, cudaStream_t st) {
   void (*kern)(Params) = ps.cluster ? clustered : coop;
   if (smem > 0) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // the limit is the kernel's, shared by every plan and thread: always the largest, so that no launch lowers it
+    // under another's
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               ps.cluster ? ClusterBarrier::kSmem : GridBarrier::kSmem);
     if (e != cudaSuccess) return e;
   }
   cudaLaunchConfig_t cfg = {};
