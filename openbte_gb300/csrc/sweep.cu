@@ -42,6 +42,7 @@ namespace obte {
 
 static constexpr int kMaxThreads = 128;   // threads per CTA at most
 static constexpr int kBaseUnit = 128;     // elements per unit of the base layout
+static constexpr int kMaxUnit = 1023;     // of any layout (counts of a header have ten bits)
 
 // ---- packed element records -------------------------------------------------------
 // 32-bit words, ring rows as 16-bit halves in units of 16 bytes (ring_field):
@@ -52,8 +53,8 @@ static constexpr int kBaseUnit = 128;     // elements per unit of the base layou
 // out the rows that every element read as zero, with the rows' bank classes (schedule.cpp), took the 60k-triangle
 // sweep (100 x 96, FP32) from 1,430 to 1,167 us and 5 of 7 spilled words from its element loop.
 // A unit's static data: its record block (header, records), followed by its output block:
-//   header 0: elements | (values start one pair into their window) << 16 | contact outputs << 17, first position,
-//             periodic outputs | wall and contact outputs << 16, then of unit u + nbuf: bank rows | size of its
+//   header 0: elements | (values start one pair into their window) << 16, first position, periodic outputs |
+//             wall and contact outputs << 10 | contact outputs << 20, then of unit u + nbuf: bank rows | size of its
 //             output block << 16
 //   header 1: of unit u + nbuf: record block and value sources (16-byte units), their sizes (16-byte units,
 //             block | values << 16), its first bank row among all units' rows
@@ -419,7 +420,7 @@ static obte_status pack(const Schedule& s, const Units& un, const Units& base, c
       const int32_t* own = pk.desc.data() + 8 * (size_t)gu;
       head[0] = own[0];
       head[1] = own[1];
-      head[2] = nx | (nw << 16);
+      head[2] = nx | (nw << 10);             // at most kMaxUnit each
       std::fill(head + 3, head + 8, 0);
       if (u + lay.nbuf < un.n[q]) {
         const int32_t* f = pk.desc.data() + 8 * (size_t)(gu + lay.nbuf);
@@ -519,7 +520,7 @@ static obte_status pack(const Schedule& s, const Units& un, const Units& base, c
       // contact entries in the order of their sums, then the others
       std::stable_sort(entries.begin(), entries.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
       for (const auto& e : entries) wo = std::copy(e.second.begin(), e.second.end(), wo);
-      head[0] |= n_contact << 17;
+      head[2] |= n_contact << 20;
       wo_run += nwo;
     }
   });
@@ -1112,8 +1113,8 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
   // element in most units), one lane per MFP for the contact sums.  Done while the next unit runs, off the chain
   // from level to level; inside the element loop they would take ~150 instructions of every warp with one such
   // element.
-  auto outputs = [&](const unsigned char* ob, int counts, int n_contact) {
-    const int nx = counts & 0xFFFF, nw = (int)((unsigned)counts >> 16);
+  auto outputs = [&](const unsigned char* ob, int counts) {
+    const int nx = counts & 0x3FF, nw = (counts >> 10) & 0x3FF;
     for (int i = nthr - 1 - tid; i < nx * MC; i += nthr) {
       const int k = i / MC, j = MC - 1 - (i - k * MC);      // consecutive lanes, consecutive MFPs
       const int2 e = reinterpret_cast<const int2*>(ob)[k];
@@ -1128,7 +1129,7 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
         wall_outputs<Real, MC, DF>(p, wb, nw, i, ring, s_sig, dT_out, chunk);
       }
       if constexpr (FINAL) {
-        if (cj >= 0 && cj < mc) contacts(reinterpret_cast<const int4*>(wb), n_contact);
+        if (cj >= 0 && cj < mc) contacts(reinterpret_cast<const int4*>(wb), counts >> 20);
       }
     }
   };
@@ -1137,7 +1138,7 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
   auto arrive = [&](int u) {
     if (mbar_wait_bounded(&bars[bi], phase, p.wait_limit)) {
       hd = *reinterpret_cast<const int4*>(st);
-      fetch(st, (hd.x >> 16) & 1, tid);
+      fetch(st, hd.x >> 16, tid);
     } else {
       hd = make_int4(0, 0, 0, 0);
       atomicOr(p.err, 1);
@@ -1146,7 +1147,7 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
   };
   arrive(0);
   __syncthreads();
-  int counts = 0, n_contact = 0;         // outputs of unit u - 1
+  int counts = 0;        // outputs of unit u - 1
   for (int u = 0; u < nlev; ++u) {
     // the first failed unit, written before the barrier above; later ones carry a larger number
     const int fail = *(volatile int*)s_fail;
@@ -1319,13 +1320,12 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
       }
       el += nthr;
       if (el < n_el) {           // units wider than the CTA
-        fetch(st, (hd.x >> 16) & 1, el);
+        fetch(st, hd.x >> 16, el);
         rows();
       }
     }
-    if (counts) outputs(smem + p.out0 + oi * p.out, counts, n_contact);
+    if (counts) outputs(smem + p.out0 + oi * p.out, counts);
     counts = hd.z;
-    if constexpr (FINAL) n_contact = hd.x >> 17;
     if (u > 0 && ++oi > nbuf) oi = 0;
     // unit u + 1: its records (not its rows) before the barrier
     if (++bi == nbuf) { bi = 0; phase ^= 1u; }
@@ -1333,7 +1333,7 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
     if (u + 1 < nlev) arrive(u + 1);
     __syncthreads();
   }
-  if (counts) outputs(smem + p.out0 + oi * p.out, counts, n_contact);
+  if (counts) outputs(smem + p.out0 + oi * p.out, counts);
   if (FINAL && !p.det && cj >= 0 && cj < mc) {
     p.K[(int64_t)(m0 + cj) * p.n_dir + q] = (double)ksum;
     p.S_out[(int64_t)(m0 + cj) * p.n_dir + q] = (double)ssum;
@@ -1517,7 +1517,7 @@ static obte_status choose_layout(const Schedule& s, size_t optin, Units& un, Uni
     if (c == kBaseUnit || cost < 0.97 * best) { best = cost; cap = c; }
     if (c >= widest) break;
   }
-  if (const char* e = std::getenv("OBTE_SWEEP_UNIT")) cap = std::max(32, std::min(1024, std::atoi(e)));
+  if (const char* e = std::getenv("OBTE_SWEEP_UNIT")) cap = std::max(32, std::min(kMaxUnit, std::atoi(e)));
   if (cap != kBaseUnit) {
     build_units(s, cap, un);
     st = count_units(s, un, sizeof(Real), unit_base, cnt);
