@@ -318,7 +318,7 @@ obte_status set_transmission(Schedule& s, const double* side_transmission);
 struct DevSchedule {
   bool ready = false;
   int mc = 0, n_chunks = 0;                // MFPs per CTA, chunks of them
-  int threads = 128;                       // per CTA
+  int threads = 128, final_threads = 128;  // per CTA of a plain sweep, of an output pass
   int prow0 = 0, emax = 0;                 // first periodic bank row of the ring, rows per bank
   int nbuf = 2;                            // units staged at once
   int stage0 = 0, stage = 0, val_off = 0, gain_off = 0;   // shared-memory stages (bytes)

@@ -232,7 +232,8 @@ static constexpr size_t kSmemPerSM = 233472, kSmemPerCta = 1024;   // capacity, 
 
 struct Layout {
   int KV = 0;         // MFPs per thread and per CTA
-  int threads = 0;
+  int threads = 0;    // of a plain sweep
+  int final_threads = kMaxThreads;   // of an output pass
   int nbuf = 2;
   int emax = 0;       // rows of one periodic bank
   int prow0 = 0;      // first bank row
@@ -247,7 +248,7 @@ template <typename Real>
 static Layout make_layout(const Schedule& s, const UnitStats& st, const Layout& shape, int nbuf) {
   Layout l = shape;
   const int row_bytes = l.KV * (int)sizeof(Real), al = row_bytes == 32 ? 7 : 0;   // swapped halves: runs of 8 rows
-  const int over = std::max(st.unit_el, kMaxThreads);   // every thread reads a record, its own or a stale one
+  const int over = std::max(st.unit_el, l.final_threads);   // every thread reads a record, its own or a stale one
   l.nbuf = nbuf;
   l.emax = (st.emax + al) & ~al;
   l.prow0 = (s.max_slots + 2 + al) & ~al;
@@ -1433,66 +1434,70 @@ static obte_status upload_real(DevBuf& b, const std::vector<double>& v, cudaStre
   return upload(b, h, st);
 }
 
-// MFPs per CTA (the MFPs that share a partial sum).  FP32: 8 while a base layout (128-element units, two
-// staged) with 32-byte rows would let at least 4 CTAs share an SM, else 4 (60k triangles: 2.14 ms at 8 against
-// 2.23 at 4; 110k tetrahedra, 2 CTAs per SM at 8: 20.8 against 11.6 ms); 4 for at most 4 MFPs.  The choice fixes
-// the grouping of the FP32 partial sums, so it depends on the mesh and the ordinates alone, not on the
-// launch shape below.  FP64: 2 or 4, see there.  OBTE_SWEEP_KV forces a compiled value.
-template <typename Real>
-static int choose_mc(const Schedule& s, const UnitStats& base) {
-  constexpr int kNarrow = 16 / (int)sizeof(Real), kWide = 2 * kNarrow;
-  if (const char* e = std::getenv("OBTE_SWEEP_KV")) {
-    const int v = std::atoi(e);
-    if (v == kNarrow || v == kWide) return v;
-  }
-  // FP64: four MFPs to a CTA halve the passes over the records, but also the CTAs, and only with two inflow rows do they
-  // fit the registers.  Measured, two MFPs against four: 60,000 triangles x 100 x 96 6,550 and 6,018 us, 20,000 2,749
-  // and 2,596, 8,000 x 60 x 48 (720 CTAs of four) 503 and 456; 2,000 x 30 x 48 (384) 146 and 194, 1,000 x 12 x 24 104
-  // and 137; 8,000 tetrahedra x 30 x 128 704 and 718.
-  if (sizeof(Real) == 8)
-    return s.n_up == 2 && (int64_t)s.n_dir * ((s.n_mfp + kWide - 1) / kWide) >= 4 * 152 ? kWide : kNarrow;
-  if (s.n_mfp <= kNarrow) return kNarrow;
-  const int64_t stage = kBaseUnit * rec_words(sizeof(Real), s.nf) * 4 + (kBaseUnit + 2) * 8 + base.unit_wo * 16 +
+// Shared memory a CTA can have and SMs of the device that a layout is for (a GB300's where no device is at hand).
+struct DeviceShape {
+  size_t smem = 232448;
+  int sms = 152;
+};
+
+// FP32: the MFPs that share a partial sum.  The grouping is part of the results' rounding, so it stays what it was
+// when the rule was made: 8 while a layout of that time (records with a word per side, two staged units of 128
+// elements, output entries and prefetch lists, rows read back in their own level) would let at least 4 CTAs
+// share an SM, else 4; 4 for at most 4 MFPs.  On the present kernel the other choice costs (4 and 8 MFPs): 2,000
+// triangles x 30 x 48 117 and 120 us, 8,000 x 60 x 48 217 and 217, 11,000 x 77 x 48 355 and 281, 60,000 x 100 x 96 1,861
+// and 1,178, 120,000 x 60 x 48 1,278 and 977; 8,000 tetrahedra x 30 x 128 304 and 222, 24,000 x 30 x 512 1,652 and 1,539.
+static int frozen_mc32(const Schedule& s, const UnitStats& base) {
+  if (s.n_mfp <= 4) return 4;
+  const int64_t stage = kBaseUnit * rec_words(4, s.nf) * 4 + (kBaseUnit + 2) * 8 + base.unit_wo * 16 +
                         ((base.emax + 3) & ~3) * 4 + base.unit_sx * 16;
   const int64_t rows = s.base_slots + 2 + 2 * base.emax;
-  const int64_t smem = 128 + 2 * stage + kWide * 20 + rows * 32;
-  return smem + 1024 <= 228 * 1024 / 4 ? kWide : kNarrow;
+  const int64_t smem = 128 + 2 * stage + 8 * 20 + rows * 32;
+  return smem + 1024 <= 228 * 1024 / 4 ? 8 : 4;
 }
 
-// Threads per CTA, unit size and stages for a plan, by shape alone.  Measured (FP32 sweep calls): 96 and 128 threads on
-// levels of 53 elements (11,000 triangles) 274 and 278 us, of 102 (60,000) 1,309 and 1,159; two and four stages on 11,000
-// triangles (one or two CTAs an SM either way) 279 and 274 us, two and three where the third costs a resident CTA
-// (60,000) 1,159 and 1,422; units of 96, 128 and 192 elements on the 60k benchmark cell 1,549, 1,430 and 1,649 us (5, 5
-// and 4 CTAs an SM).
+// FP64: four MFPs to a CTA halve the passes over the records, but also the CTAs, and their rows take twice the room.
+// They pay while four CTAs still share an SM and the last wave of CTAs is not much emptier than the others.  Two
+// against four MFPs, with CTAs of four and how many share an SM: 8,000 triangles x 60 x 48 (720, 5) 506 and 458
+// us, 20,000 x 100 x 96 (2,400, 4) 2,754 and 2,594, 60,000 x 100 x 96 (2,400, 4) 6,554 and 6,008, x 100 x 48 (1,200, 4) 3,421
+// and 3,119; with 1.03 and 1.18 waves 60,000 x 52 x 48 (624, 4) 2,003 and 2,295, 20,000 x 60 x 48 (720, 4) 958 and
+// 1,181; with three to an SM 40,000 x 100 x 96 5,075 and 5,151, with two 180,000 x 60 x 48 5,830 and 6,843; in half a
+// wave 2,000 x 30 x 48 (384, 5) 146 and 194.  Only with two inflow rows do they fit the registers (8,000
+// tetrahedra x 30 x 128 704 and 718).
+static bool wide64(int64_t ctas, int resident, int sms) {
+  const double waves = (double)ctas / ((double)std::max(resident, 1) * sms);
+  return resident >= 4 && std::ceil(waves) <= 1.3 * waves;
+}
+
+// A plan's launch shape and the units it is for.
+struct Shaped {
+  Units un;
+  std::vector<int64_t> unit_base;
+  std::vector<int32_t> cnt;
+  Layout lay;
+  bool fits = false;
+};
+
+// Unit size and stages for KV MFPs per CTA and `threads`, by shape alone.  Measured (FP32 sweep calls): 96 and 128
+// threads on levels of 53 elements (11,000 triangles) 274 and 278 us, of 102 (60,000) 1,309 and 1,159; two and four
+// stages on 11,000 triangles (one or two CTAs an SM either way) 279 and 274 us, two and three where the third costs a
+// resident CTA (60,000) 1,159 and 1,422; units of 96, 128 and 192 elements on the 60k benchmark cell 1,549, 1,430 and
+// 1,649 us (5, 5 and 4 CTAs an SM).
 template <typename Real>
-static obte_status choose_layout(const Schedule& s, size_t optin, Units& un, Units& base,
-                                 std::vector<int64_t>& unit_base, std::vector<int32_t>& cnt, Layout& lay) {
-  build_units(s, kBaseUnit, base);
-  un = base;
-  UnitStats st = count_units(s, un, sizeof(Real), unit_base, cnt);
-  if (st.bad_wo) {
-    set_error("wall re-emission entries are not in sweep order");
-    return OBTE_ERR_BAD_ARG;
-  }
-  const int MC = choose_mc<Real>(s, st);
-  const int n_chunks = (s.n_mfp + MC - 1) / MC;
-  int64_t levels = 0;
+static void shape_units(const Schedule& s, const DeviceShape& dev, const Units& base, const UnitStats& base_stats, int KV,
+                        int threads, int final_threads, Shaped& r) {
   int widest = 0;
   for (int q = 0; q < s.n_dir; ++q) {
-    levels += s.nlev[q];
     const int32_t* lp = s.lev_ptr.data() + s.lev_off[q];
     for (int L = 0; L < s.nlev[q]; ++L) widest = std::max(widest, (int)(lp[L + 1] - lp[L]));
   }
-  const double width = levels ? (double)s.n_dir * s.n / (double)levels : 1.0;
+  const int n_chunks = (s.n_mfp + KV - 1) / KV;
   // CTAs an SM has to run: no more are worth making room for
-  const int64_t want = std::max<int64_t>(1, ((int64_t)s.n_dir * n_chunks + 151) / 152);
+  const int64_t want = std::max<int64_t>(1, ((int64_t)s.n_dir * n_chunks + dev.sms - 1) / dev.sms);
   Layout shape;
-  shape.KV = MC;
-  shape.threads = width <= 64 ? 96 : kMaxThreads;
-  if (const char* e = std::getenv("OBTE_SWEEP_THREADS")) {
-    const int v = std::atoi(e);
-    if (v >= 32 && v <= kMaxThreads && v % 32 == 0) shape.threads = v;
-  }
+  shape.KV = KV;
+  shape.threads = threads;
+  shape.final_threads = final_threads;
+  UnitStats st = base_stats;
   auto layout = [&](const UnitStats& e, int nbuf) { return make_layout<Real>(s, e, shape, nbuf); };
   auto steps = [&](int cap) {
     int64_t c = 0;
@@ -1511,36 +1516,75 @@ static obte_status choose_layout(const Schedule& s, size_t optin, Units& un, Uni
     e.unit_el = std::min(c, widest);
     if (e.unit_sx > kUnitSx) e.unit_out = e.unit_out * c / kBaseUnit;
     if (e.emax > kUnitPf) e.emax = e.emax * c / kBaseUnit;
-    const int r = resident<Real>(layout(e, 2));
-    if (r < 1) break;
-    const double cost = steps(c) / (double)std::min<int64_t>(r, want);
+    const int res = resident<Real>(layout(e, 2));
+    if (res < 1) break;
+    const double cost = steps(c) / (double)std::min<int64_t>(res, want);
     if (c == kBaseUnit || cost < 0.97 * best) { best = cost; cap = c; }
     if (c >= widest) break;
   }
   if (const char* e = std::getenv("OBTE_SWEEP_UNIT")) cap = std::max(32, std::min(kMaxUnit, std::atoi(e)));
-  if (cap != kBaseUnit) {
-    build_units(s, cap, un);
-    st = count_units(s, un, sizeof(Real), unit_base, cnt);
-  }
+  auto build = [&]() {
+    if (cap == kBaseUnit) r.un = base;
+    else build_units(s, cap, r.un);
+    st = count_units(s, r.un, sizeof(Real), r.unit_base, r.cnt);
+  };
+  build();
   // smaller units while two stages do not fit a CTA
-  while (layout(st, 2).smem > optin && cap > 32) {
+  while (layout(st, 2).smem > dev.smem && cap > 32) {
     cap /= 2;
-    build_units(s, cap, un);
-    st = count_units(s, un, sizeof(Real), unit_base, cnt);
+    build();
   }
-  lay = layout(st, 2);
-  if (lay.smem > optin) {
-    set_error("sweep front needs more shared memory than one CTA can have (" + std::to_string(lay.rows) + " rows)");
-    return OBTE_ERR_UNSUPPORTED;
-  }
+  r.lay = layout(st, 2);
+  r.fits = r.lay.smem <= dev.smem;
+  if (!r.fits) return;
   // more stages where the extra ones cost no resident CTA
   const char* nb_env = std::getenv("OBTE_SWEEP_NBUF");
-  const int64_t have = std::min<int64_t>(resident<Real>(lay), want);
+  const int64_t have = std::min<int64_t>(resident<Real>(r.lay), want);
   for (int nb = nb_env ? std::max(2, std::min(kMaxBuf, std::atoi(nb_env))) : 4; nb > 2; --nb) {
     const Layout l = layout(st, nb);
-    if (l.smem <= optin && (nb_env || std::min<int64_t>(resident<Real>(l), want) >= have)) { lay = l; break; }
+    if (l.smem <= dev.smem && (nb_env || std::min<int64_t>(resident<Real>(l), want) >= have)) { r.lay = l; break; }
   }
-  return OBTE_OK;
+}
+
+// The launch shape of a plan: MFPs per CTA by the rules above (OBTE_SWEEP_KV forces a compiled value), threads by the
+// width of the levels.  A front too wide for that is tried with narrow rows, then with units of 32 elements and as
+// many threads, whose stages are a quarter.
+template <typename Real>
+static obte_status choose_layout(const Schedule& s, const DeviceShape& dev, Units& base, Shaped& out) {
+  constexpr int kNarrow = 16 / (int)sizeof(Real), kWide = 2 * kNarrow;
+  build_units(s, kBaseUnit, base);
+  const UnitStats st = count_units(s, base, sizeof(Real), out.unit_base, out.cnt);
+  if (st.bad_wo) {
+    set_error("wall re-emission entries are not in sweep order");
+    return OBTE_ERR_BAD_ARG;
+  }
+  int64_t levels = 0;
+  for (int q = 0; q < s.n_dir; ++q) levels += s.nlev[q];
+  const double width = levels ? (double)s.n_dir * s.n / (double)levels : 1.0;
+  int threads = width <= 64 ? 96 : kMaxThreads;
+  if (const char* e = std::getenv("OBTE_SWEEP_THREADS")) {
+    const int v = std::atoi(e);
+    if (v >= 32 && v <= kMaxThreads && v % 32 == 0) threads = v;
+  }
+  auto attempt = [&](int KV, int thr, int final_thr) {
+    out.fits = false;
+    shape_units<Real>(s, dev, base, st, KV, thr, final_thr, out);
+    return out.fits;
+  };
+  const char* kv_env = std::getenv("OBTE_SWEEP_KV");
+  const int forced = kv_env ? std::atoi(kv_env) : 0;
+  if (forced == kNarrow || forced == kWide) {
+    if (attempt(forced, threads, kMaxThreads)) return OBTE_OK;
+  } else if constexpr (sizeof(Real) == 4) {
+    if (frozen_mc32(s, st) == kWide && attempt(kWide, threads, kMaxThreads)) return OBTE_OK;
+  } else if (s.n_up == 2) {
+    const int64_t ctas = (int64_t)s.n_dir * ((s.n_mfp + kWide - 1) / kWide);
+    if (ctas >= 3 * dev.sms && attempt(kWide, threads, kMaxThreads) && wide64(ctas, resident<Real>(out.lay), dev.sms))
+      return OBTE_OK;
+  }
+  if (attempt(kNarrow, threads, kMaxThreads) || attempt(kNarrow, 32, 32)) return OBTE_OK;
+  set_error("sweep front needs more shared memory than one CTA can have (" + std::to_string(out.lay.rows) + " rows)");
+  return OBTE_ERR_UNSUPPORTED;
 }
 
 template <typename Real>
@@ -1548,23 +1592,22 @@ static obte_status upload_tables(obte_plan plan, DevSchedule& d) {
   PhaseTimer timer(sizeof(Real) == 4 ? "upload_tables fp32" : "upload_tables fp64");
   const Schedule& s = plan->sched;
   cudaStream_t st = plan->stream;
-  Units un;
+  Shaped sh;
   Packed pk;
   {
     PhaseTimer tp("pack");
-    std::vector<int64_t> unit_base;
-    std::vector<int32_t> cnt;
-    Layout lay;
     Units base;
-    OBTE_TRY(choose_layout<Real>(s, plan->ctx->smem_optin, un, base, unit_base, cnt, lay));
-    OBTE_TRY(pack<Real>(s, un, base, unit_base, cnt, lay, pk));
-    OBTE_TRY(upload(d.unit_base, unit_base, st));
-    d.n_units = unit_base[s.n_dir];
+    OBTE_TRY(choose_layout<Real>(s, {(size_t)plan->ctx->smem_optin, plan->ctx->num_sms}, base, sh));
+    OBTE_TRY(pack<Real>(s, sh.un, base, sh.unit_base, sh.cnt, sh.lay, pk));
+    OBTE_TRY(upload(d.unit_base, sh.unit_base, st));
+    d.n_units = sh.unit_base[s.n_dir];
   }
+  const Units& un = sh.un;
   const Layout& l = pk.lay;
   d.mc = l.KV;
   d.n_chunks = (s.n_mfp + d.mc - 1) / d.mc;
   d.threads = l.threads;
+  d.final_threads = l.final_threads;
   d.prow0 = l.prow0;
   d.emax = l.emax;
   d.nbuf = l.nbuf;
@@ -1768,17 +1811,16 @@ struct Fnv {
 
 template <typename Real>
 static obte_status tables_digest_impl(const Schedule& s, uint64_t* digest) {
-  Units un;
+  Shaped sh;
   Packed pk;
-  std::vector<int64_t> unit_base;
   {
     PhaseTimer tp("pack");
-    std::vector<int32_t> cnt;
-    Layout lay;
     Units base;
-    OBTE_TRY(choose_layout<Real>(s, 232448, un, base, unit_base, cnt, lay));   // 227 KB: the most one CTA can have
-    OBTE_TRY(pack<Real>(s, un, base, unit_base, cnt, lay, pk));
+    OBTE_TRY(choose_layout<Real>(s, DeviceShape(), base, sh));
+    OBTE_TRY(pack<Real>(s, sh.un, base, sh.unit_base, sh.cnt, sh.lay, pk));
   }
+  const Units& un = sh.un;
+  const std::vector<int64_t>& unit_base = sh.unit_base;
   Fnv f;
   f.vec(un.ptr); f.vec(un.off); f.vec(un.n);
   f.vec(pk.blk); f.vec(pk.cellmap); f.vec(pk.si); f.vec(pk.spec); f.vec(pk.P); f.vec(pk.sr);
@@ -1995,7 +2037,7 @@ static obte_status launch_impl(obte_plan plan, const DevSchedule& d, const Sweep
   p.batch_stride = r.batch_stride;
   p.row_stride = batch > 1 ? d.row_stride : 0;
   const int grid = subset ? plan->sweep_n_cta * batch : s.n_dir * d.n_chunks;
-  kern<<<grid, FINAL ? kMaxThreads : d.threads, d.smem, st>>>(p);
+  kern<<<grid, FINAL ? d.final_threads : d.threads, d.smem, st>>>(p);
   count_launch();
   OBTE_CUDA(cudaGetLastError());
   if (det) {
