@@ -397,9 +397,9 @@ extern "C" obte_status obte_bte_plan_footprint(obte_plan plan, int32_t precision
           s.lev_ptr.size() + s.wo_wall.size()) * 4;
     b += (s.in_coef.size() + s.D.size() + s.P.size() + s.mfp.size() + s.tco.size() + s.sig.size() +
           s.wo_wall.size() * 4 + s.kcoef.size() + s.scoef.size() + s.hs.size()) * rb;
-    // unit descriptors and headers (a unit per level, or per 32 elements of a level), periodic bank rows: their
+    // unit descriptors, headers and padding (a unit per level, or per 32 elements of a level), periodic bank rows: their
     // list and their per-sweep values
-    b += (s.lev_ptr.size() + s.cell.size() / 32) * 64;
+    b += (s.lev_ptr.size() + s.cell.size() / 32) * (64 + 48);
     b += s.n_cut * (16 + (int64_t)((s.n_mfp + 7) & ~7) * (int64_t)rb);
     b += (s.lev_ptr.size() + s.in_idx.size()) * 8; // (bound)
     return (int64_t)b;

@@ -56,7 +56,7 @@ static constexpr int kMaxUnit = 1023;     // of any layout (counts of a header h
 //   header 0: elements | (values start one pair into their window) << 16, first position, periodic outputs |
 //             wall and contact outputs << 10 | contact outputs << 20, then of unit u + nbuf: bank rows | size of its
 //             output block << 16
-//   header 1: of unit u + nbuf: record block and value sources (16-byte units), their sizes (16-byte units,
+//   header 1: of unit u + nbuf: record block (kBlkUnit bytes) and value (16 bytes) sources, their sizes (16-byte units,
 //             block | values << 16), its first bank row among all units' rows
 //   outputs:  periodic sources (int2: source slot, row; padded to 16 B), wall / contact entries (int4: row,
 //             count | first of the unit's wall entries << 3 | wall entries of the unit << 16, contact entry, first
@@ -269,6 +269,10 @@ static int resident(const Layout& l) {
   return (int)std::min<size_t>((size_t)std::min(by_regs, 32), kSmemPerSM / (((l.smem + 127) & ~(size_t)127) + kSmemPerCta));
 }
 
+// Alignment and unit of a static block's offset: 32 bits reach 256 GB of blocks.  (Of the values, 16 bytes an item in
+// FP64, 32 bits of 16-byte units reach more items than their blocks leave room for.)
+constexpr int kBlkUnit = 64;
+
 struct Packed {
   Layout lay;
   RawVec<int32_t> blk;                  // static blocks of all units, direction by direction
@@ -277,11 +281,11 @@ struct Packed {
   std::vector<int32_t> si;
   std::vector<double> sr;
   // 8 ints per unit: elements | odd << 16, first position, first bank row, bank rows | output block's size << 16;
-  // record block and value offsets (16-byte units), their sizes (block | values << 16), periodic outputs | wall
-  // and contact outputs << 16
+  // record block (kBlkUnit bytes) and value offsets (16-byte units), their sizes (16-byte units, block | values << 16),
+  // periodic outputs | wall and contact outputs << 16
   std::vector<int32_t> desc;
-  std::vector<int32_t> pfe;             // 4 ints per bank row: source slot | swapped halves << 30, its row among
-                                        // chunk 0's rows of all units, rows of its unit, 0
+  std::vector<int32_t> pfe;             // 4 ints per bank row: source slot, its unit's first row among all units'
+                                        // rows, rows of its unit, its row in the unit | swapped halves << 31
   int64_t n_pf = 0;
 };
 
@@ -323,11 +327,10 @@ static obte_status pack(const Schedule& s, const Units& un, const Units& base, c
   const int W = rec_words(sizeof(Real), s.n_up);
   constexpr int CSTEP = sizeof(Real) / 4, COEF = 4, VB = 2 * sizeof(Real);
   const int row_bytes = lay.KV * (int)sizeof(Real);
-  const int n_chunks = (s.n_mfp + lay.KV - 1) / lay.KV;
   auto field = [&](int row) { return ring_field(row, row_bytes); };
   const int zero_row = s.max_slots, trash_row = s.max_slots + 1;
   pk.lay = lay;
-  if (field(lay.rows) >= 65535 || s.x_base[s.n_dir] >= ((int64_t)1 << 30)) {
+  if (field(lay.rows) >= 65535 || s.x_base[s.n_dir] >= ((int64_t)1 << 32)) {
     set_error("sweep ring rows do not fit 16-bit indices");
     return OBTE_ERR_UNSUPPORTED;
   }
@@ -340,19 +343,20 @@ static obte_status pack(const Schedule& s, const Units& un, const Units& base, c
       const int32_t* up = un.ptr.data() + un.off[q];
       for (int k = 0; k < un.n[q]; ++k, ++u) {
         const int32_t* c = cnt.data() + 4 * (size_t)u;
-        boff[u + 1] = boff[u] + (kHeader + (int64_t)(up[k + 1] - up[k]) * W * 4 + out_bytes(c[2], c[3], c[1], sizeof(Real))) / 16;
+        const int64_t bytes = kHeader + (int64_t)(up[k + 1] - up[k]) * W * 4 + out_bytes(c[2], c[3], c[1], sizeof(Real));
+        boff[u + 1] = boff[u] + (bytes + kBlkUnit - 1) / kBlkUnit;
         poff[u + 1] = poff[u] + c[0];
       }
     }
   }
   pk.n_pf = poff[n_units];
   const int64_t total = (int64_t)s.n_dir * s.n;
-  if (boff[n_units] >= ((int64_t)1 << 32) || pk.n_pf * n_chunks >= ((int64_t)1 << 31) ||
+  if (boff[n_units] >= ((int64_t)1 << 32) || pk.n_pf >= ((int64_t)1 << 31) ||
       total / (16 / VB) >= ((int64_t)1 << 32)) {
     set_error("sweep tables too large");
     return OBTE_ERR_UNSUPPORTED;
   }
-  pk.blk.resize((size_t)boff[n_units] * 4);   // uninitialised: every word is written below
+  pk.blk.resize((size_t)boff[n_units] * (kBlkUnit / 4));   // uninitialised: every word is written below
   pk.desc.assign((size_t)std::max<int64_t>(n_units, 1) * 8, 0);
   pk.pfe.assign((size_t)std::max<int64_t>(pk.n_pf, 1) * 4, 0);
   pk.cellmap.resize(total);
@@ -371,10 +375,11 @@ static obte_status pack(const Schedule& s, const Units& un, const Units& base, c
       d[2] = (int32_t)poff[u];
       const int32_t* c = cnt.data() + 4 * (size_t)u;
       const int out16 = out_bytes(c[2], c[3], c[1], sizeof(Real)) / 16;
+      const int rec16 = (kHeader + (up[k + 1] - up[k]) * W * 4) / 16;
       d[3] = (int32_t)(poff[u + 1] - poff[u]) | (out16 << 16);
       d[4] = (int32_t)(uint32_t)boff[u];
       d[5] = (int32_t)(uint32_t)(v0 >> 4);
-      d[6] = (int32_t)((uint32_t)(boff[u + 1] - boff[u] - out16) | ((uint32_t)(((v1 + 15) >> 4) - (v0 >> 4)) << 16));
+      d[6] = (int32_t)((uint32_t)rec16 | ((uint32_t)(((v1 + 15) >> 4) - (v0 >> 4)) << 16));
       d[7] = c[2] | (c[3] << 16);
     }
   });
@@ -409,7 +414,7 @@ static obte_status pack(const Schedule& s, const Units& un, const Units& base, c
       const int64_t gu = unit_base[q] + u;
       const int n_el = up[u + 1] - up[u], npf = cnt[4 * gu], nwo = cnt[4 * gu + 1], nx = cnt[4 * gu + 2],
                 nw = cnt[4 * gu + 3];
-      int32_t* head = pk.blk.data() + (size_t)boff[gu] * 4;
+      int32_t* head = pk.blk.data() + (size_t)boff[gu] * (kBlkUnit / 4);
       int32_t* recs = head + kHeader / 4;
       int32_t* xo = recs + (size_t)n_el * W;
       int32_t* wo = xo + (((size_t)nx * 2 + 3) & ~(size_t)3);
@@ -440,6 +445,7 @@ static obte_status pack(const Schedule& s, const Units& un, const Units& base, c
         wg[(size_t)nwo * 4 * CSTEP + e] = w;
       }
       for (int e = nwo; e & 3; ++e) wg[(size_t)nwo * 4 * CSTEP + e] = 0;
+      std::fill(wg + (size_t)nwo * 4 * CSTEP + ((nwo + 3) & ~3), pk.blk.data() + (size_t)boff[gu + 1] * (kBlkUnit / 4), 0);
       int ent = 0;
       const int bank = lay.prow0 + (u % lay.nbuf) * lay.emax;
       for (int32_t pos = up[u]; pos < up[u + 1]; ++pos) {
@@ -468,9 +474,10 @@ static obte_status pack(const Schedule& s, const Units& un, const Units& base, c
             } else {
               row_in[k] = bank + ent;
               int32_t* pe = pk.pfe.data() + 4 * (size_t)(poff[gu] + ent);
-              pe[0] = (int32_t)(s.x_base[q] + idx) | ((row_bytes == 32 ? ((bank + ent) >> 2) & 1 : 0) << 30);
-              pe[1] = (int32_t)(poff[gu] * n_chunks + ent);
+              pe[0] = (int32_t)(uint32_t)(s.x_base[q] + idx);
+              pe[1] = (int32_t)poff[gu];
               pe[2] = npf;
+              pe[3] = (int32_t)((uint32_t)ent | (uint32_t)(row_bytes == 32 ? ((bank + ent) >> 2) & 1 : 0) << 31);
               ++ent;
             }
             coef[k] = g;
@@ -484,7 +491,7 @@ static obte_status pack(const Schedule& s, const Units& un, const Units& base, c
           }
         }
         if (s.xk[it] >= 0) {
-          xo[0] = (int32_t)(s.x_base[q] + s.xk[it]);
+          xo[0] = (int32_t)(uint32_t)(s.x_base[q] + s.xk[it]);
           xo[1] = field(so) << 4;
           xo += 2;
         }
@@ -693,7 +700,7 @@ __global__ void __launch_bounds__(256, 8) sweep_prep_kernel(const __grid_constan
         const int m = lane + 32 * piece;
         if (k < left && m < p.n_mfp) {
           const int64_t t = p.batch > 1 ? w / p.n_pf : 0;
-          v[k] = X[t * p.batch_stride + (int64_t)(pfe[w - t * p.n_pf].x & 0x3fffffff) * p.n_mfp + m];
+          v[k] = X[t * p.batch_stride + (int64_t)(unsigned)pfe[w - t * p.n_pf].x * p.n_mfp + m];
         }
         if (++piece == np) { piece = 0; ++w; }
       }
@@ -705,10 +712,11 @@ __global__ void __launch_bounds__(256, 8) sweep_prep_kernel(const __grid_constan
         if (k < left && m < p.m_row) {
           const int64_t t = p.batch > 1 ? w / p.n_pf : 0;
           const int4 e = pfe[w - t * p.n_pf];
-          const int flip = kWide && (e.x >> 30) ? MC / 2 : 0;
+          const int flip = kWide && e.w < 0 ? MC / 2 : 0;
           Real r = (Real)v[k];
           if constexpr (DF) r = dpack_split((double)r);
-          p.xrow[t * p.row_stride + ((int64_t)e.y + (int64_t)(m / MC) * e.z) * MC + ((m % MC) ^ flip)] = r;
+          const int64_t row = (int64_t)e.y * (p.m_row / MC) + (e.w & 0x7fffffff) + (int64_t)(m / MC) * e.z;
+          p.xrow[t * p.row_stride + row * MC + ((m % MC) ^ flip)] = r;
         }
         if (++piece == np) { piece = 0; ++w; }
       }
@@ -1014,13 +1022,13 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
   __syncthreads();
 
   // Bulk copies of a unit into stage bi and output block oi: records, values, outputs, periodic inflow rows, gain
-  // rows.  blk16, val16 = record and value sources, size = their sizes in 16-byte units, prow = first bank row,
+  // rows.  blk64, val16 = record and value sources, size = their sizes in 16-byte units, prow = first bank row,
   // np = bank rows | size of the output block << 16
-  auto issue = [&](int u, int bi, int oi, unsigned blk16, unsigned val16, unsigned size, int prow, unsigned np) {
+  auto issue = [&](int u, int bi, int oi, unsigned blk64, unsigned val16, unsigned size, int prow, unsigned np) {
     if (u == p.skip_unit) return;   // test of the bounded wait: this unit's copies never arrive
     const unsigned bb = (size & 0xFFFFu) << 4, vb = (size >> 16) << 4, ob = (np >> 16) << 4, npf = np & 0xFFFFu;
     unsigned char* st = smem + p.stage0 + bi * p.stage;
-    const unsigned char* src = reinterpret_cast<const unsigned char*>(p.blk) + ((uint64_t)blk16 << 4);
+    const unsigned char* src = reinterpret_cast<const unsigned char*>(p.blk) + (uint64_t)blk64 * kBlkUnit;
     uint64_t* bar = &bars[bi];
     unsigned gb = 0;
     if constexpr (kGain) gb = gain_qc ? (vb / VB) * ROWB : 0u;     // FP64 values are 16 bytes: vb / 16 elements
@@ -1120,7 +1128,7 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
       const int k = i / MC, j = MC - 1 - (i - k * MC);      // consecutive lanes, consecutive MFPs
       const int2 e = reinterpret_cast<const int2*>(ob)[k];
       const Real v = row_value((unsigned)e.y, j);
-      if (j < mc) dT_out[p.n + p.nd + (int64_t)e.x * p.n_mfp + m0 + j] = widen(v);
+      if (j < mc) dT_out[p.n + p.nd + (int64_t)(unsigned)e.x * p.n_mfp + m0 + j] = widen(v);
     }
     if (nw) {
       const unsigned char* wb = ob + ((nx * 8 + 15) & ~15);
@@ -1679,7 +1687,7 @@ __device__ __forceinline__ UnitRecs unit_recs(const int32_t* __restrict__ desc, 
   const int4 a = reinterpret_cast<const int4*>(desc)[2 * u], b = reinterpret_cast<const int4*>(desc)[2 * u + 1];
   UnitRecs r;
   r.item0 = (int64_t)(unsigned)b.y * (16 / (2 * (int)sizeof(Real))) + (a.x >> 16);
-  r.word0 = (int64_t)(unsigned)b.x * 4 + kHeader / 4;
+  r.word0 = (int64_t)(unsigned)b.x * (kBlkUnit / 4) + kHeader / 4;
   r.n_el = a.x & 0xFFFF;
   r.a = a.y;
   return r;
