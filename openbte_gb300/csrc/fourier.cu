@@ -29,6 +29,9 @@ namespace {
 
 constexpr int FT = 256;
 
+// the root of a sum of squares; NaN stays NaN (fmax would turn it into a converged residual of zero)
+__device__ __forceinline__ double root(double s) { return sqrt(s < 0 ? 0.0 : s); }
+
 // Blocks of a solve: as many as its rows fill, 104 to a block: the barrier is cheaper with fewer blocks, and the other SMs
 // are left to other streams (8,000 triangles: 77 blocks 3.55 ms, 152 3.7, 39 3.95); at least a quarter of the SMs
 // (2,000 triangles: 20 blocks 3.9 ms, 38 3.45).
@@ -128,8 +131,8 @@ __global__ void __launch_bounds__(Bar::kThreads, Bar::kBlocks) fourier_kernel(co
     if (!bar.wait()) return;
     if (P.pin >= 0)
       for (int i = r0 + tid; i < r1; i += nthr) P.T[i] += delta;
-    grid_sum(p_bb, nb, red, [&](double s) { return tol = P.cg_rtol * fmax(sqrt(fmax(s, 0.0)), 1e-300); });
-    auto open = [&](double s) { return sqrt(fmax(s, 0.0)) <= tol ? 0.0 : 1.0; };
+    grid_sum(p_bb, nb, red, [&](double s) { return tol = P.cg_rtol * fmax(root(s), 1e-300); });
+    auto open = [&](double s) { return root(s) <= tol ? 0.0 : 1.0; };
     bool run = grid_sum(p_rr, nb, red, open) != 0;
     // z = M^-1 r and the partials of r . z, after the restriction (or nothing) of the phase before
     auto precondition = [&](const double* r) -> bool {
@@ -209,7 +212,8 @@ __global__ void __launch_bounds__(Bar::kThreads, Bar::kBlocks) fourier_kernel(co
       });
       if ((k + 1) % P.check == 0) {
         ncg += P.check;
-        run = grid_sum(p_rr, nb, red, open) != 0 && k + 1 < P.cg_max;
+        // (a residual that is not a number has reached T and stays one)
+        run = grid_sum(p_rr, nb, red, [&](double s) { return s == s ? open(s) : 0.0; }) != 0 && k + 1 < P.cg_max;
       }
     }
     // T_pin, then T -= (max + min) / 2 (fourier.py:155-156)
@@ -284,7 +288,7 @@ __global__ void __launch_bounds__(Bar::kThreads, Bar::kBlocks) fourier_kernel(co
     put(cc, p_cc);
     if (!bar.wait()) return;
     more = grid_sum(p_cc, nb, red, [&](double s) {
-             const double norm = sqrt(fmax(s, 0.0));
+             const double norm = root(s);
              const double err = norm == 0 ? 0 : fabs(norm - norm_old) / norm;   // fourier.py:168-171
              norm_old = norm;
              return err > P.rtol && it < P.max_iter ? 1.0 : 0.0;
