@@ -269,6 +269,13 @@ obte_status obte_bte_sweep_fields(obte_plan plan, int32_t precision, const doubl
  * normally again after (-1, 0).
  */
 obte_status obte_bte_plan_test_wait_timeout(obte_plan plan, int32_t skip_unit, int32_t wait_limit);
+/*
+ * The same for the barriers inside the one-launch diffusion correction of a plan's solves (more than 1,536
+ * elements): at barrier skip_barrier of an application block 0 does not arrive (-1: every block arrives), and a
+ * wait gives up after wait_limit polls (0: the default).  The solve then ends with OBTE_ERR_DEVICE_TIMEOUT after
+ * the step in which it happened; the plan solves normally again after (-1, 0).
+ */
+obte_status obte_bte_plan_test_barrier_timeout(obte_plan plan, int32_t skip_barrier, int32_t wait_limit);
 
 /*
  * Inverse design: dkappa_eff/dt_s for every side of a plan created with side_transmission
@@ -398,6 +405,9 @@ typedef struct {
 obte_status obte_fourier_plan_create(obte_context ctx, const obte_fourier_problem* prob,
                                      obte_fourier_plan* out);
 obte_status obte_fourier_plan_destroy(obte_fourier_plan plan);
+/* Test hook of the solve's barriers, as obte_bte_plan_test_barrier_timeout. */
+obte_status obte_fourier_plan_test_barrier_timeout(obte_fourier_plan plan, int32_t skip_barrier,
+                                                   int32_t wait_limit);
 /*   T device [n_elems] Temperature_Fourier;  J device [n_elems, dim] Flux_Fourier / 1e9 */
 obte_status obte_fourier_solve(obte_fourier_plan plan, const obte_fourier_opts* opts, double* T,
                                double* J, obte_fourier_info* info);

@@ -109,6 +109,7 @@ SIGNATURES = [
     ("obte_bte_sweep_static", C.c_int, [C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_int32]),
     ("obte_bte_sweep_fields", C.c_int, [C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p]),
     ("obte_bte_plan_test_wait_timeout", C.c_int, [C.c_void_p, C.c_int32, C.c_int32]),
+    ("obte_bte_plan_test_barrier_timeout", C.c_int, [C.c_void_p, C.c_int32, C.c_int32]),
     ("obte_bte_kappa_gradient", C.c_int, [C.c_void_p, C.POINTER(SolveOpts), C.c_void_p, C.c_void_p,
                                           C.POINTER(SolveInfo)]),
     ("obte_bte_kappa_gradient_adjoint", C.c_int, [C.c_void_p, C.c_void_p, C.POINTER(SolveOpts), C.c_void_p,
@@ -124,6 +125,7 @@ SIGNATURES = [
     ("obte_bte_tables_digest", C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_uint64)]),
     ("obte_fourier_plan_create", C.c_int, [C.c_void_p, C.POINTER(FourierProblem), C.POINTER(C.c_void_p)]),
     ("obte_fourier_plan_destroy", C.c_int, [C.c_void_p]),
+    ("obte_fourier_plan_test_barrier_timeout", C.c_int, [C.c_void_p, C.c_int32, C.c_int32]),
     ("obte_fourier_solve", C.c_int, [C.c_void_p, C.POINTER(FourierOpts), C.c_void_p, C.c_void_p,
                                      C.POINTER(FourierInfo)]),
 ]

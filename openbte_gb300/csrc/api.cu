@@ -528,6 +528,14 @@ extern "C" obte_status obte_bte_sweep_fields(obte_plan plan, int32_t precision, 
   return check_device_error(plan);
 }
 
+extern "C" obte_status obte_bte_plan_test_barrier_timeout(obte_plan plan, int32_t skip_barrier, int32_t wait_limit) {
+  if (!plan) { set_error("null plan"); return OBTE_ERR_BAD_ARG; }
+  if (skip_barrier < -1 || wait_limit < 0) { set_error("skip_barrier must be >= -1 and wait_limit >= 0"); return OBTE_ERR_BAD_ARG; }
+  plan->test_barrier_skip = skip_barrier;
+  plan->test_barrier_polls = wait_limit;
+  return OBTE_OK;
+}
+
 extern "C" obte_status obte_bte_plan_test_wait_timeout(obte_plan plan, int32_t skip_unit, int32_t wait_limit) {
   if (!plan) { set_error("null plan"); return OBTE_ERR_BAD_ARG; }
   if (skip_unit < -1 || wait_limit < 0) { set_error("skip_unit must be >= -1 and wait_limit >= 0"); return OBTE_ERR_BAD_ARG; }

@@ -57,8 +57,8 @@ struct DsaParams {
   const int32_t *wcell, *xcell;
   const double *in, *base;
   double *out, *b, *d, *r, *e, *part;
-  unsigned *count, *count_next;
-  int* err;
+  BarrierParams bar;
+  unsigned* count_next;                      // the next application's barrier counter, cleared here
 };
 
 // out = base + E L^-1 R in, one launch.  Phases end at a barrier (grid.cuh): the weighted sum of `in`; the
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(Bar::kThreads, Bar::kBlocks == 1 ? 1 : 4) dsa_
   __shared__ double red[Bar::kThreads];
   __shared__ Rows sA;
   __shared__ AmgRows sM;
-  Bar bar(P.count, P.err);
+  Bar bar(P.bar);
   const int tid = threadIdx.x, nthr = blockDim.x, nb = gridDim.x;
   if (blockIdx.x == 0 && tid == 0) *P.count_next = 0;
   Arena ar{nullptr, 0};                      // read once: not worth copying
@@ -361,11 +361,11 @@ obte_status dsa_add(obte_plan plan, const double* in, const double* base, double
   f.b = op.b.as<double>(); f.d = op.d.as<double>(); f.r = op.r.as<double>(); f.e = op.e.as<double>();
   f.part = op.mean.as<double>();
   unsigned* count = reinterpret_cast<unsigned*>(f.part + 2 * ((s.n + 31) / 32));
-  f.count = count + op.turn;
+  f.bar = {count + op.turn, plan->err.as<int>(),
+           plan->test_barrier_polls > 0 ? plan->test_barrier_polls : kBarrierPolls, plan->test_barrier_skip};
   f.count_next = count + (op.turn ^ 1);
-  op.turn ^= 1;
-  f.err = plan->err.as<int>();
   OBTE_CUDA(phase_launch(ps, dsa_kernel<ClusterBarrier>, dsa_kernel<GridBarrier>, f, 0, plan->stream));
+  op.turn ^= 1;                   // a launch that failed has cleared nothing: its counter is still the next one
   count_launch();
   return OBTE_OK;
 }

@@ -61,8 +61,7 @@ struct FourierParams {
   int smem;                                  // bytes of shared memory for the matrices
   double rtol, cg_rtol;
   double* out;                               // deferred corrections, CG iterations
-  unsigned* count;
-  int* err;
+  BarrierParams bar;
 };
 
 // The deferred-correction loop (fourier.py:145-178) with its preconditioned CG solves, one launch.  Phases end at
@@ -81,7 +80,7 @@ __global__ void __launch_bounds__(Bar::kThreads, Bar::kBlocks) fourier_kernel(co
   __shared__ double red[Bar::kThreads];
   __shared__ Rows sA;
   __shared__ AmgRows sM;
-  Bar bar(P.count, P.err);
+  Bar bar(P.bar);
   const int tid = threadIdx.x, nthr = blockDim.x, nb = gridDim.x;
   Arena ar{smem, P.smem};
   load_rows(P.A, &sA, ar);
@@ -336,6 +335,7 @@ struct obte_fourier_plan_s {
   // work
   obte::DevBuf C, r, z, p, Ap, part, sc, grad, kout;
   obte::HostBuf hout;               // the two counts of a solve and the error word, read back
+  int test_skip = -1, test_polls = 0;   // obte_fourier_plan_test_barrier_timeout
   // smoothed-aggregation AMG V-cycle as the CG preconditioner (null: Jacobi)
   obte::AmgPtr amg;
 };
@@ -546,6 +546,15 @@ extern "C" obte_status obte_fourier_plan_destroy(obte_fourier_plan plan) {
   return OBTE_OK;
 }
 
+extern "C" obte_status obte_fourier_plan_test_barrier_timeout(obte_fourier_plan plan, int32_t skip_barrier,
+                                                              int32_t wait_limit) {
+  if (!plan) { set_error("null plan"); return OBTE_ERR_BAD_ARG; }
+  if (skip_barrier < -1 || wait_limit < 0) { set_error("skip_barrier must be >= -1 and wait_limit >= 0"); return OBTE_ERR_BAD_ARG; }
+  plan->test_skip = skip_barrier;
+  plan->test_polls = wait_limit;
+  return OBTE_OK;
+}
+
 extern "C" obte_status obte_fourier_solve(obte_fourier_plan P, const obte_fourier_opts* opts, double* T, double* J,
                                           obte_fourier_info* info) {
   if (!P || !opts || !T) { set_error("null argument"); return OBTE_ERR_BAD_ARG; }
@@ -576,8 +585,8 @@ extern "C" obte_status obte_fourier_solve(obte_fourier_plan P, const obte_fourie
   f.check = P->amg ? 4 : 8;          // iterations between two convergence tests
   f.rtol = rtol; f.cg_rtol = cg_rtol;
   f.out = P->sc.as<double>();
-  f.count = reinterpret_cast<unsigned*>(f.out + 2);
-  f.err = reinterpret_cast<int*>(f.out + 3);
+  f.bar = {reinterpret_cast<unsigned*>(f.out + 2), reinterpret_cast<int*>(f.out + 3),
+           P->test_polls > 0 ? P->test_polls : kBarrierPolls, P->test_skip};
   OBTE_CUDA(cudaMemsetAsync(P->sc.p, 0, 4 * sizeof(double), st));
   const PhaseShape shape = fourier_shape(n, P->ctx->num_sms);
   // shared memory for a block's part of the matrices (an eighth more, as rows differ), as far as it may have

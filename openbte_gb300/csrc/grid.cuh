@@ -22,11 +22,21 @@ __device__ __forceinline__ double widen(float f) {
   return __hiloint2double((int)(((b & 0x7fffffffu) >> 3) + (896u << 20) | (b & 0x80000000u)), (int)(b << 29));
 }
 
+// What the barrier of a cooperative launch needs: its counter (zero at launch) and error word, the polls after which
+// a wait gives up (a wait of 1-2 s by default), and for the test of that the barrier at which block 0 does not arrive
+// (-1: none).
+struct BarrierParams {
+  unsigned* count;
+  int* err;
+  int polls, skip;
+};
+constexpr int kBarrierPolls = 1 << 21;
+
 // Barrier over the blocks of a cluster.
 struct ClusterBarrier {
   static constexpr int kThreads = 512, kBlocks = 1;      // threads per block, blocks an SM has registers for
   static constexpr int kSmem = 200 * 1024;               // shared memory for a solve's matrices at most
-  __device__ ClusterBarrier(unsigned*, int*) {}
+  __device__ ClusterBarrier(const BarrierParams&) {}
   __device__ bool wait() {
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
@@ -34,29 +44,28 @@ struct ClusterBarrier {
   }
 };
 
-// Barrier over the blocks of a cooperative launch: count (zero at launch) grows by the number of blocks per
+// Barrier over the blocks of a cooperative launch: the counter grows by the number of blocks per
 // barrier.  The wait is bounded; when it gives up (on any block) the error word is set and wait() is false in
 // every thread of that block, whose caller returns; the other blocks run into their own bounds.
 struct GridBarrier {
   static constexpr int kThreads = 256, kBlocks = 3, kSmem = 69 * 1024;
-  static constexpr int kPolls = 1 << 21;
-  unsigned* count;
-  int* err;
+  const BarrierParams& p;
   unsigned target = 0;
-  __device__ GridBarrier(unsigned* c, int* e) : count(c), err(e) {}
+  __device__ GridBarrier(const BarrierParams& params) : p(params) {}
   __device__ bool wait() {
     __shared__ int ok;
     __syncthreads();
     target += gridDim.x;
     if (threadIdx.x == 0) {
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+      if (blockIdx.x != 0 || target != (unsigned)(p.skip + 1) * gridDim.x)
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.count) : "memory");
       int done = 0;
-      for (int i = 0; i < kPolls && !done; ++i) {
+      for (int i = 0; i < p.polls && !done; ++i) {
         unsigned v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.count) : "memory");
         done = (int)(v - target) >= 0;
       }
-      if (!done) atomicOr(err, 1);
+      if (!done) atomicOr(p.err, 1);
       ok = done;
     }
     __syncthreads();

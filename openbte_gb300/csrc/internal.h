@@ -419,6 +419,8 @@ struct obte_plan_s {
   bool xstore_add = false;          // the final pass adds its temperatures to xstore (pass at a correction)
   double* xstore64 = nullptr;       // set during obte_bte_sweep_fields in FP64: the same in FP64
   obte::DevBuf fields_J, fields_K, fields_S;   // final-pass outputs of obte_bte_sweep_fields (discarded)
+  // bounded-wait test of the grid barrier (obte_bte_plan_test_barrier_timeout)
+  int test_barrier_skip = -1, test_barrier_polls = 0;
   // bounded-wait test (obte_bte_plan_test_wait_timeout): level unit whose bulk copy the sweeps skip
   // (-1: none) and the poll cap of their copy waits (0: the default)
   int test_skip_unit = -1;

@@ -120,7 +120,8 @@ struct ArnoldiParams {
   double *part, *s_part;                     // block sums: of the products [k + 1][groups], of w.w [2][groups]
   double *h, *h2;                            // coefficients of the passes between launches [k + 1], [k]
   int* two;                                  // the second pass runs
-  double* col;                               // h (+ h2) [k], |w|, second pass ran
+  double* col;                               // h (+ h2) [k], |w|, second pass ran, the plan's error word
+  const int* err;
 };
 
 template <typename Real>
@@ -330,6 +331,7 @@ __device__ __forceinline__ void arnoldi_finish(const ArnoldiParams<Real>& P, con
     if (blockIdx.x == 0) {
       P.col[k] = hn;
       P.col[k + 1] = two ? 1.0 : 0.0;
+      P.col[k + 2] = (double)*P.err;
     }
   }
   if (blockIdx.x == 0)
@@ -354,7 +356,7 @@ __global__ void __launch_bounds__(VT, 2) arnoldi_kernel(const __grid_constant__ 
   __shared__ Real hs[MAX_BASIS];
   __shared__ Real buf[kDotBuf<Real>];
   __shared__ double sc;
-  ClusterBarrier bar(nullptr, nullptr);
+  ClusterBarrier bar(BarrierParams{});
   const int k = P.k;
   arnoldi_dots(P, true, k + 1, buf);
   bar.wait();
@@ -615,6 +617,7 @@ struct Solver {
     f.h2 = f.h + (wk.restart + 1);
     f.two = reinterpret_cast<int*>(f.h2 + (wk.restart + 1));
     f.col = wk.hcol.as<double>();
+    f.err = plan->err.as<int>();
     int blocks = f.groups * f.sp;
     if (blocks <= 8) {
       while (blocks & (blocks - 1)) ++blocks;            // blocks above groups * sp only wait
@@ -630,7 +633,8 @@ struct Solver {
     }
     OBTE_CUDA(cudaGetLastError());
     OBTE_CUDA(wait_stream(st));
-    return OBTE_OK;
+    // a wait of the step's sweep or correction that gave up: its vector is not complete
+    return f.col[k + 2] != 0 ? check_device_error(plan) : OBTE_OK;
   }
 
   // Restarted GMRES with the FP32 basis (see arnoldi_kernel); same contract as gmres().

@@ -2143,7 +2143,7 @@ obte_status check_device_error(obte_plan plan) {
   OBTE_CUDA(wait_stream(plan->stream));
   if (h) {
     OBTE_CUDA(cudaMemsetAsync(plan->err.p, 0, sizeof(int), plan->stream));
-    set_error("a device-side wait timed out in the sweep kernel");
+    set_error("a device-side wait timed out in a sweep or a diffusion correction");
     return OBTE_ERR_DEVICE_TIMEOUT;
   }
   return OBTE_OK;
