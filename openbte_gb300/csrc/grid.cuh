@@ -49,23 +49,25 @@ struct ClusterBarrier {
 // every thread of that block, whose caller returns; the other blocks run into their own bounds.
 struct GridBarrier {
   static constexpr int kThreads = 256, kBlocks = 3, kSmem = 69 * 1024;
-  const BarrierParams& p;
-  unsigned target = 0;
-  __device__ GridBarrier(const BarrierParams& params) : p(params) {}
+  unsigned* count;
+  int* err;
+  int polls;
+  unsigned target = 0, skip;                 // skip: the target at which this block does not arrive, 0: none
+  __device__ GridBarrier(const BarrierParams& p)
+      : count(p.count), err(p.err), polls(p.polls), skip(blockIdx.x == 0 ? (unsigned)(p.skip + 1) * gridDim.x : 0) {}
   __device__ bool wait() {
     __shared__ int ok;
     __syncthreads();
     target += gridDim.x;
     if (threadIdx.x == 0) {
-      if (blockIdx.x != 0 || target != (unsigned)(p.skip + 1) * gridDim.x)
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.count) : "memory");
+      if (target != skip) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
       int done = 0;
-      for (int i = 0; i < p.polls && !done; ++i) {
+      for (int i = 0; i < polls && !done; ++i) {
         unsigned v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.count) : "memory");
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
         done = (int)(v - target) >= 0;
       }
-      if (!done) atomicOr(p.err, 1);
+      if (!done) atomicOr(err, 1);
       ok = done;
     }
     __syncthreads();
