@@ -234,7 +234,8 @@ obte_status obte_bte_sweep(obte_plan plan, int32_t precision, const double* u_in
  * This call allocates nothing: its scratch (the per-sweep values, n_dir x
  * n_elems x 8 bytes in FP32 modes or x 16 in FP64, plus 288 bytes) lives in an
  * 8 MiB array inside the library, which every GPU that loads the library holds
- * until the process exits.  A larger problem is rejected with
+ * until the process exits, and its periodic inflow rows in a buffer that comes
+ * with the plan's device tables.  A larger problem is rejected with
  * OBTE_ERR_UNSUPPORTED (use obte_bte_sweep).  The plan's device tables for the
  * precision must already exist: building them allocates, so run obte_bte_sweep
  * or obte_bte_solve once in that precision at set-up, or this returns

@@ -432,13 +432,13 @@ __global__ void scale_to_f32_kernel(double a, const double* __restrict__ x, floa
     y64[i] = widen(v);
   }
 }
-// y = a*x + b*y
 // y += x
 __global__ void add_kernel(double* __restrict__ y, const double* __restrict__ x, int64_t n) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     y[i] += x[i];
 }
 
+// y = a*x + b*y
 __global__ void axpby_kernel(double a, const double* __restrict__ x, double b, double* __restrict__ y, int64_t n) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     y[i] = a * x[i] + b * y[i];

@@ -763,7 +763,6 @@ struct SweepParams {
   const int64_t* __restrict__ unit_base;  // [n_dir + 1]
   const Real* __restrict__ vals;
   const Real* __restrict__ xrow;          // periodic inflow rows: [unit][chunk][row][KV]
-  const int64_t* __restrict__ x_base;
   const Real* __restrict__ mfp;    // [m_pad]
   const Real* __restrict__ tco;    // [n_dir * m_pad]
   const Real* __restrict__ sig;    // [n_dir * m_pad * ds]
@@ -810,37 +809,24 @@ __device__ __forceinline__ double word_real<double>(const int32_t* r, int word) 
   return __hiloint2double(r[word + 1], r[word]);
 }
 
-// num / den.  FP32: hardware reciprocal.  FP64: an FP32 reciprocal seed r (relative error e <= 2^-21)
+// num / den by an FP32 reciprocal seed r (relative error e <= 2^-21)
 // and one residual correction of the quotient (Markstein's method), t = num r, q = t + (num - den t) r,
 // with relative error e^2 <= 2^-42 (~2e-13): three FP64 operations instead of the five of a fully
 // refined reciprocal, on GB300's narrow FP64 pipe, which bounds the FP64 sweep.
-__device__ __forceinline__ float quot(float num, float den) { return num * __fdividef(1.0f, den); }
 __device__ __forceinline__ double quot(double num, double den) {
   const double r = (double)__fdividef(1.0f, (float)den);
   const double t = num * r;
   return fma(fma(-den, t, num), r, t);
 }
 
-// 16-byte vectors of the ring: 4 floats or 2 doubles per lane.
-template <typename Real> struct V16;
-template <> struct V16<float> { static constexpr int K = 4; };
-template <> struct V16<double> { static constexpr int K = 2; };
-
+// 16-byte vectors: 4 floats or 2 doubles.
 template <int K>
 __device__ __forceinline__ void vload(const float* p, float (&x)[K]) {
-  if constexpr (K % 4 == 0) {
+  static_assert(K % 4 == 0, "whole vectors");
 #pragma unroll
-    for (int i = 0; i < K; i += 4) {
-      const float4 v = *reinterpret_cast<const float4*>(p + i);
-      x[i] = v.x; x[i + 1] = v.y; x[i + 2] = v.z; x[i + 3] = v.w;
-    }
-  } else {                 // 2 FP32 MFPs per lane: 8-byte rows
-    static_assert(K % 2 == 0, "an even number of FP32 MFPs per lane");
-#pragma unroll
-    for (int i = 0; i < K; i += 2) {
-      const float2 v = *reinterpret_cast<const float2*>(p + i);
-      x[i] = v.x; x[i + 1] = v.y;
-    }
+  for (int i = 0; i < K; i += 4) {
+    const float4 v = *reinterpret_cast<const float4*>(p + i);
+    x[i] = v.x; x[i + 1] = v.y; x[i + 2] = v.z; x[i + 3] = v.w;
   }
 }
 template <int K>
@@ -853,13 +839,9 @@ __device__ __forceinline__ void vload(const double* p, double (&x)[K]) {
 }
 template <int K>
 __device__ __forceinline__ void vstore(float* p, const float (&x)[K]) {
-  if constexpr (K % 4 == 0) {
+  static_assert(K % 4 == 0, "whole vectors");
 #pragma unroll
-    for (int i = 0; i < K; i += 4) *reinterpret_cast<float4*>(p + i) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
-  } else {
-#pragma unroll
-    for (int i = 0; i < K; i += 2) *reinterpret_cast<float2*>(p + i) = make_float2(x[i], x[i + 1]);
-  }
+  for (int i = 0; i < K; i += 4) *reinterpret_cast<float4*>(p + i) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
 }
 template <int K>
 __device__ __forceinline__ void vstore(double* p, const double (&x)[K]) {
@@ -867,39 +849,37 @@ __device__ __forceinline__ void vstore(double* p, const double (&x)[K]) {
   for (int i = 0; i < K; i += 2) *reinterpret_cast<double2*>(p + i) = make_double2(x[i], x[i + 1]);
 }
 
-// Lane `lane`'s KV of a ring row's MC MFPs, by the row's byte offset: a 16-byte row, or a 32-byte row of which
-// bit 4 of the offset says which half comes first (the lane's offset in the row is added without carry).
-template <int MC, int KV, typename Real>
-__device__ __forceinline__ void row_load(const unsigned char* ring, unsigned off, int lane, Real (&x)[KV]) {
+// A ring row's KV MFPs by the row's byte offset: 16 bytes, or 32 of which bit 4 of the offset says which half comes
+// first.
+template <int KV, typename Real>
+__device__ __forceinline__ void row_load(const unsigned char* ring, unsigned off, Real (&x)[KV]) {
   constexpr int H = 16 / (int)sizeof(Real);
-  static_assert(MC == H || MC == 2 * H, "one or two 16-byte vectors per row");
-  const unsigned o = MC == KV ? off : off ^ (unsigned)(lane * KV * (int)sizeof(Real));
-  if constexpr (KV <= H) {
-    vload(reinterpret_cast<const Real*>(ring + o), x);
+  static_assert(KV == H || KV == 2 * H, "one or two 16-byte vectors per row");
+  if constexpr (KV == H) {
+    vload(reinterpret_cast<const Real*>(ring + off), x);
   } else {
     Real a[H];
-    vload(reinterpret_cast<const Real*>(ring + o), a);
+    vload(reinterpret_cast<const Real*>(ring + off), a);
 #pragma unroll
     for (int i = 0; i < H; ++i) x[i] = a[i];
-    vload(reinterpret_cast<const Real*>(ring + (o ^ 16u)), a);
+    vload(reinterpret_cast<const Real*>(ring + (off ^ 16u)), a);
 #pragma unroll
     for (int i = 0; i < H; ++i) x[H + i] = a[i];
   }
 }
-template <int MC, int KV, typename Real>
-__device__ __forceinline__ void row_store(unsigned char* ring, unsigned off, int lane, const Real (&x)[KV]) {
+template <int KV, typename Real>
+__device__ __forceinline__ void row_store(unsigned char* ring, unsigned off, const Real (&x)[KV]) {
   constexpr int H = 16 / (int)sizeof(Real);
-  const unsigned o = MC == KV ? off : off ^ (unsigned)(lane * KV * (int)sizeof(Real));
-  if constexpr (KV <= H) {
-    vstore(reinterpret_cast<Real*>(ring + o), x);
+  if constexpr (KV == H) {
+    vstore(reinterpret_cast<Real*>(ring + off), x);
   } else {
     Real a[H];
 #pragma unroll
     for (int i = 0; i < H; ++i) a[i] = x[i];
-    vstore(reinterpret_cast<Real*>(ring + o), a);
+    vstore(reinterpret_cast<Real*>(ring + off), a);
 #pragma unroll
     for (int i = 0; i < H; ++i) a[i] = x[H + i];
-    vstore(reinterpret_cast<Real*>(ring + (o ^ 16u)), a);
+    vstore(reinterpret_cast<Real*>(ring + (off ^ 16u)), a);
   }
 }
 
@@ -922,7 +902,7 @@ __device__ __forceinline__ void wall_outputs(const SweepParams<Real>& p, const u
                                              const unsigned char* ring, const Real* s_sig, double* dT_out, int chunk) {
   const int4 ent = reinterpret_cast<const int4*>(wb)[i];
   Real T[MC];
-  row_load<MC, MC>(ring, (unsigned)ent.x, 0, T);
+  row_load(ring, (unsigned)ent.x, T);
   if constexpr (DF) {
 #pragma unroll
     for (int j = 0; j < MC; ++j) T[j] = dpack_value(T[j]);
@@ -1165,10 +1145,10 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
     // read together: while the row loads are in flight the issuer refills the stage of unit u - 1
     Real v0[KV], v1[KV], v2[NF > 2 ? KV : 1], v3[NF > 3 ? KV : 1];
     auto rows = [&]() {
-      row_load<MC, KV>(ring, ((unsigned)r[1] >> 12) & 0xFFFF0u, 0, v0);
-      row_load<MC, KV>(ring, ((unsigned)r[2] << 4) & 0xFFFF0u, 0, v1);
-      if constexpr (NF > 2) row_load<MC, KV>(ring, ((unsigned)r[2] >> 12) & 0xFFFF0u, 0, v2);
-      if constexpr (NF > 3) row_load<MC, KV>(ring, ((unsigned)r[3] << 4) & 0xFFFF0u, 0, v3);
+      row_load(ring, ((unsigned)r[1] >> 12) & 0xFFFF0u, v0);
+      row_load(ring, ((unsigned)r[2] << 4) & 0xFFFF0u, v1);
+      if constexpr (NF > 2) row_load(ring, ((unsigned)r[2] >> 12) & 0xFFFF0u, v2);
+      if constexpr (NF > 3) row_load(ring, ((unsigned)r[3] << 4) & 0xFFFF0u, v3);
     };
     if (el < n_el) rows();
     if (fail <= u) {
@@ -1229,7 +1209,7 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
         j0 = ((double)ja.h.x + (double)ja.h.y) + ((double)ja.l.x + (double)ja.l.y);
         j1 = ((double)jb.h.x + (double)jb.h.y) + ((double)jb.l.x + (double)jb.l.y);
         j2 = ((double)jc.h.x + (double)jc.h.y) + ((double)jc.l.x + (double)jc.l.y);
-        row_store<MC, KV>(ring, so, 0, Tp);
+        row_store(ring, so, Tp);
         // real values for the stored fields below
         const bool need = p.Xs != nullptr || p.Xd != nullptr;
 #pragma unroll
@@ -1253,7 +1233,7 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
           T[j] = t2.x;
           T[j + 1] = t2.y;
         }
-        row_store<MC, KV>(ring, so, 0, T);
+        row_store(ring, so, T);
         // sum over the chunk's MFPs, even and odd ones apart, in MFP order
         auto wsum = [&](auto weight) -> float {
           float2 acc = make_float2(0.0f, 0.0f);
@@ -1299,7 +1279,7 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
           }
         }
       }
-      if constexpr (!DF && sizeof(Real) == 8) row_store<MC, KV>(ring, so, 0, T);
+      if constexpr (!DF && sizeof(Real) == 8) row_store(ring, so, T);
       if (FINAL && p.Xs != nullptr) {
 #pragma unroll
         for (int j = 0; j < KV; ++j)
@@ -2152,13 +2132,14 @@ obte_status check_device_error(obte_plan plan) {
 
 // ---- sweep on library-owned static scratch ---------------------------------------------
 //
-// obte_bte_sweep keeps its per-sweep scratch (the (b, p) values the sweep kernel streams by
-// TMA, and the device error word) in buffers the plan allocates on first use.  Some callers
+// obte_bte_sweep keeps its per-sweep scratch (the (b, p) values the sweep kernel streams by TMA, the periodic inflow
+// rows and the device error word) in buffers the plan allocates on first use.  Some callers
 // cannot allocate device memory when they sweep: a host framework that has reserved nearly
 // all of the GPU's memory for its own pool (cudaMalloc then fails or forces that pool to give
 // memory back), or a latency-bound loop in which cudaMalloc / cudaFree would synchronise the
 // device and stall work on other streams.  obte_bte_sweep_static runs the same two kernels
-// with that scratch in the fixed array below instead, and allocates nothing.
+// with the values and the error word in the fixed array below instead and the inflow rows that came with the plan's
+// tables, and allocates nothing.
 //
 // The array is a file-scope __device__ variable: every GPU that loads this library holds
 // kStaticScratchBytes of it until the process exits.  Its name in host code is only a
@@ -2167,7 +2148,7 @@ obte_status check_device_error(obte_plan plan) {
 // the first call on that device.  Layout: [0, 256) device error word, [256, ...) the values.
 // All calls share the array, and it keeps the previous call's contents; each call clears
 // the error word before its kernels run, and the values are written in full by
-// sweep_values_kernel before the sweep kernel reads them.
+// sweep_prep_kernel before the sweep kernel reads them.
 namespace obte {
 
 static constexpr size_t kStaticScratchBytes = (size_t)8 << 20;
