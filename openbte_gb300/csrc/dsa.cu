@@ -364,7 +364,7 @@ obte_status dsa_add(obte_plan plan, const double* in, const double* base, double
   f.bar = {count + op.turn, plan->err.as<int>(),
            plan->test_barrier_polls > 0 ? plan->test_barrier_polls : kBarrierPolls, plan->test_barrier_skip};
   f.count_next = count + (op.turn ^ 1);
-  OBTE_CUDA(phase_launch(ps, dsa_kernel<ClusterBarrier>, dsa_kernel<GridBarrier>, f, 0, plan->stream));
+  OBTE_CUDA(phase_launch(ps, ps.cluster ? dsa_kernel<ClusterBarrier> : dsa_kernel<GridBarrier>, f, 0, 0, plan->stream));
   op.turn ^= 1;                   // a launch that failed has cleared nothing: its counter is still the next one
   count_launch();
   return OBTE_OK;

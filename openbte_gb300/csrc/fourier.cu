@@ -34,10 +34,14 @@ __device__ __forceinline__ double root(double s) { return sqrt(s < 0 ? 0.0 : s);
 
 // Blocks of a solve: as many as its rows fill, 104 to a block: the barrier is cheaper with fewer blocks, and the other SMs
 // are left to other streams (8,000 triangles: 77 blocks 3.55 ms, 152 3.7, 39 3.95); at least a quarter of the SMs
-// (2,000 triangles: 20 blocks 3.9 ms, 38 3.45).
+// (2,000 triangles: 20 blocks 3.9 ms, 38 3.45).  Above two rows to a thread of every SM's block, half an SM to a block
+// instead of a third: 100,000 tetrahedra 58 and 68 ms, 200,000 triangles 11.1 and 13.4 ms, while below the gain is less
+// than the room is worth (60,000 triangles 6.8 and 7.3 ms, but beside them 101 and 129 solves of 8,000 x 60 x 48 a second).
 PhaseShape fourier_shape(int64_t n, int num_sms) {
   PhaseShape s = phase_shape(n, num_sms);
-  if (!s.cluster) s.blocks = (int)std::min<int64_t>(num_sms, std::max<int64_t>(num_sms / 4, (n + 103) / 104));
+  if (s.cluster) return s;
+  s.blocks = (int)std::min<int64_t>(num_sms, std::max<int64_t>(num_sms / 4, (n + 103) / 104));
+  if (n > 2 * (int64_t)GridBarrier::kThreads * num_sms) s.threads = WideGridBarrier::kThreads;
   return s;
 }
 
@@ -591,9 +595,13 @@ extern "C" obte_status obte_fourier_solve(obte_fourier_plan P, const obte_fourie
   const PhaseShape shape = fourier_shape(n, P->ctx->num_sms);
   // shared memory for a block's part of the matrices (an eighth more, as rows differ), as far as it may have
   const int64_t bytes = (int64_t)(P->val.bytes + P->ci.bytes + P->rp.bytes) + (P->amg ? amg_bytes(*P->amg) : 0);
-  f.smem = (int)std::min<int64_t>(shape.cluster ? ClusterBarrier::kSmem : GridBarrier::kSmem,
-                                  (bytes / shape.blocks * 9 / 8 + 2048 + 127) & ~(int64_t)127);
-  OBTE_CUDA(phase_launch(shape, fourier_kernel<ClusterBarrier>, fourier_kernel<GridBarrier>, f, f.smem, st));
+  const bool wide = shape.threads == WideGridBarrier::kThreads;
+  const int most = shape.cluster ? ClusterBarrier::kSmem : wide ? WideGridBarrier::kSmem : GridBarrier::kSmem;
+  f.smem = (int)std::min<int64_t>(most, (bytes / shape.blocks * 9 / 8 + 2048 + 127) & ~(int64_t)127);
+  OBTE_CUDA(phase_launch(shape, shape.cluster ? fourier_kernel<ClusterBarrier>
+                                : wide        ? fourier_kernel<WideGridBarrier>
+                                              : fourier_kernel<GridBarrier>,
+                         f, f.smem, most, st));
   count_launch();
   double kappa = 0;
   std::vector<double> kh(std::max<int64_t>(P->nc, 1));

@@ -47,13 +47,14 @@ struct ClusterBarrier {
 // Barrier over the blocks of a cooperative launch: the counter grows by the number of blocks per
 // barrier.  The wait is bounded; when it gives up (on any block) the error word is set and wait() is false in
 // every thread of that block, whose caller returns; the other blocks run into their own bounds.
-struct GridBarrier {
-  static constexpr int kThreads = 256, kBlocks = 3, kSmem = 69 * 1024;
+template <int THREADS, int BLOCKS, int SMEM>
+struct GridBarrierOf {
+  static constexpr int kThreads = THREADS, kBlocks = BLOCKS, kSmem = SMEM;
   unsigned* count;
   int* err;
   int polls;
   unsigned target = 0, skip;                 // skip: the target at which this block does not arrive, 0: none
-  __device__ GridBarrier(const BarrierParams& p)
+  __device__ GridBarrierOf(const BarrierParams& p)
       : count(p.count), err(p.err), polls(p.polls), skip(blockIdx.x == 0 ? (unsigned)(p.skip + 1) * gridDim.x : 0) {}
   __device__ bool wait() {
     __shared__ int ok;
@@ -74,6 +75,9 @@ struct GridBarrier {
     return ok != 0;
   }
 };
+
+using GridBarrier = GridBarrierOf<256, 3, 69 * 1024>;          // a third of an SM to a block
+using WideGridBarrier = GridBarrierOf<512, 2, 104 * 1024>;     // half
 
 // Sum over the block's first `count` slots in a fixed order, valid in thread 0: the thread of slot s passes its
 // value with slot = s, the others a negative slot; red: one double per thread.  A warp's FP64 operation holds its quarter
@@ -340,22 +344,20 @@ struct PhaseShape {
 // x 60 x 48 beside one that repeats Fourier solves of 60,000 went from 189 to 6 a second (129 now; with
 // Fourier solves of 4-5 us launches 138, beside a fifth of the Fourier solves), four streams of Fourier solves of 8,000
 // from 492 a second to 274 (1,075 now), of 60,000 from 234 to 162 (357 now).  Alone, Fourier solves of
-// 60,000 triangles take 7.3 ms for the 6.3 of a whole-SM block (half an SM 7.1, a quarter 8.2), of 8,000 3.55 for 3.7.
+// 60,000 triangles take 7.3 ms for the 6.2 of a whole-SM block (half an SM 6.8, a quarter 8.2), of 8,000 3.55 for 3.7.
 constexpr int64_t kClusterElems = 1536;
 inline PhaseShape phase_shape(int64_t n, int num_sms) {
   if (n <= kClusterElems) return {8, ClusterBarrier::kThreads, true};
   return {num_sms, GridBarrier::kThreads, false};
 }
-// Launch kern<ClusterBarrier> or kern<GridBarrier> by the shape.
+// Launch a kernel over the shape's blocks, `smem` of `max_smem` bytes of shared memory to each.
 template <typename Params>
-cudaError_t phase_launch(const PhaseShape& ps, void (*clustered)(Params), void (*coop)(Params), const Params& p,
-                         int smem, cudaStream_t st) {
-  void (*kern)(Params) = ps.cluster ? clustered : coop;
-  if (smem > 0) {
+cudaError_t phase_launch(const PhaseShape& ps, void (*kern)(Params), const Params& p, int smem, int max_smem,
+                         cudaStream_t st) {
+  if (max_smem > 0) {
     // the limit is the kernel's, shared by every plan and thread: always the largest, so that no launch lowers it
     // under another's
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               ps.cluster ? ClusterBarrier::kSmem : GridBarrier::kSmem);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
     if (e != cudaSuccess) return e;
   }
   cudaLaunchConfig_t cfg = {};

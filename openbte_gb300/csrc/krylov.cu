@@ -621,7 +621,7 @@ struct Solver {
     int blocks = f.groups * f.sp;
     if (blocks <= 8) {
       while (blocks & (blocks - 1)) ++blocks;            // blocks above groups * sp only wait
-      OBTE_CUDA(phase_launch({blocks, VT, true}, arnoldi_kernel<Real>, arnoldi_kernel<Real>, f, 0, st));
+      OBTE_CUDA(phase_launch({blocks, VT, true}, arnoldi_kernel<Real>, f, 0, 0, st));
       count_launch();
     } else {
       arnoldi_phase_kernel<Real, 0><<<blocks, VT, 0, st>>>(f);
