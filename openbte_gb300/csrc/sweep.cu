@@ -1456,6 +1456,14 @@ static bool wide64(int64_t ctas, int resident, int sms) {
   return resident >= 4 && std::ceil(waves) <= 1.3 * waves;
 }
 
+// The units of the base layout and their counts.
+struct BaseUnits {
+  Units un;
+  std::vector<int64_t> unit_base;
+  std::vector<int32_t> cnt;
+  UnitStats st;
+};
+
 // A plan's launch shape and the units it is for.
 struct Shaped {
   Units un;
@@ -1471,8 +1479,8 @@ struct Shaped {
 // resident CTA (60,000) 1,159 and 1,422; units of 96, 128 and 192 elements on the 60k benchmark cell 1,549, 1,430 and
 // 1,649 us (5, 5 and 4 CTAs an SM).
 template <typename Real>
-static void shape_units(const Schedule& s, const DeviceShape& dev, const Units& base, const UnitStats& base_stats, int KV,
-                        int threads, int final_threads, Shaped& r) {
+static void shape_units(const Schedule& s, const DeviceShape& dev, const BaseUnits& base, int KV, int threads,
+                        int final_threads, Shaped& r) {
   int widest = 0;
   for (int q = 0; q < s.n_dir; ++q) {
     const int32_t* lp = s.lev_ptr.data() + s.lev_off[q];
@@ -1485,7 +1493,7 @@ static void shape_units(const Schedule& s, const DeviceShape& dev, const Units& 
   shape.KV = KV;
   shape.threads = threads;
   shape.final_threads = final_threads;
-  UnitStats st = base_stats;
+  UnitStats st = base.st;
   auto layout = [&](const UnitStats& e, int nbuf) { return make_layout<Real>(s, e, shape, nbuf); };
   auto steps = [&](int cap) {
     int64_t c = 0;
@@ -1512,11 +1520,16 @@ static void shape_units(const Schedule& s, const DeviceShape& dev, const Units& 
   }
   if (const char* e = std::getenv("OBTE_SWEEP_UNIT")) cap = std::max(32, std::min(kMaxUnit, std::atoi(e)));
   auto build = [&]() {
-    if (cap == kBaseUnit) r.un = base;
-    else build_units(s, cap, r.un);
+    build_units(s, cap, r.un);
     st = count_units(s, r.un, sizeof(Real), r.unit_base, r.cnt);
   };
-  build();
+  if (cap == kBaseUnit) {
+    r.un = base.un;
+    r.unit_base = base.unit_base;
+    r.cnt = base.cnt;
+  } else {
+    build();
+  }
   // smaller units while two stages do not fit a CTA
   while (layout(st, 2).smem > dev.smem && cap > 32) {
     cap /= 2;
@@ -1538,11 +1551,11 @@ static void shape_units(const Schedule& s, const DeviceShape& dev, const Units& 
 // width of the levels.  A front too wide for that is tried with narrow rows, then with units of 32 elements and as
 // many threads, whose stages are a quarter.
 template <typename Real>
-static obte_status choose_layout(const Schedule& s, const DeviceShape& dev, Units& base, Shaped& out) {
+static obte_status choose_layout(const Schedule& s, const DeviceShape& dev, BaseUnits& base, Shaped& out) {
   constexpr int kNarrow = 16 / (int)sizeof(Real), kWide = 2 * kNarrow;
-  build_units(s, kBaseUnit, base);
-  const UnitStats st = count_units(s, base, sizeof(Real), out.unit_base, out.cnt);
-  if (st.bad_wo) {
+  build_units(s, kBaseUnit, base.un);
+  base.st = count_units(s, base.un, sizeof(Real), base.unit_base, base.cnt);
+  if (base.st.bad_wo) {
     set_error("wall re-emission entries are not in sweep order");
     return OBTE_ERR_BAD_ARG;
   }
@@ -1556,7 +1569,7 @@ static obte_status choose_layout(const Schedule& s, const DeviceShape& dev, Unit
   }
   auto attempt = [&](int KV, int thr, int final_thr) {
     out.fits = false;
-    shape_units<Real>(s, dev, base, st, KV, thr, final_thr, out);
+    shape_units<Real>(s, dev, base, KV, thr, final_thr, out);
     return out.fits;
   };
   const char* kv_env = std::getenv("OBTE_SWEEP_KV");
@@ -1564,7 +1577,7 @@ static obte_status choose_layout(const Schedule& s, const DeviceShape& dev, Unit
   if (forced == kNarrow || forced == kWide) {
     if (attempt(forced, threads, kMaxThreads)) return OBTE_OK;
   } else if constexpr (sizeof(Real) == 4) {
-    if (frozen_mc32(s, st) == kWide && attempt(kWide, threads, kMaxThreads)) return OBTE_OK;
+    if (frozen_mc32(s, base.st) == kWide && attempt(kWide, threads, kMaxThreads)) return OBTE_OK;
   } else if (s.n_up == 2) {
     const int64_t ctas = (int64_t)s.n_dir * ((s.n_mfp + kWide - 1) / kWide);
     if (ctas >= 3 * dev.sms && attempt(kWide, threads, kMaxThreads) && wide64(ctas, resident<Real>(out.lay), dev.sms))
@@ -1584,9 +1597,9 @@ static obte_status upload_tables(obte_plan plan, DevSchedule& d) {
   Packed pk;
   {
     PhaseTimer tp("pack");
-    Units base;
+    BaseUnits base;
     OBTE_TRY(choose_layout<Real>(s, {(size_t)plan->ctx->smem_optin, plan->ctx->num_sms}, base, sh));
-    OBTE_TRY(pack<Real>(s, sh.un, base, sh.unit_base, sh.cnt, sh.lay, pk));
+    OBTE_TRY(pack<Real>(s, sh.un, base.un, sh.unit_base, sh.cnt, sh.lay, pk));
     OBTE_TRY(upload(d.unit_base, sh.unit_base, st));
     d.n_units = sh.unit_base[s.n_dir];
   }
@@ -1803,9 +1816,9 @@ static obte_status tables_digest_impl(const Schedule& s, uint64_t* digest) {
   Packed pk;
   {
     PhaseTimer tp("pack");
-    Units base;
+    BaseUnits base;
     OBTE_TRY(choose_layout<Real>(s, DeviceShape(), base, sh));
-    OBTE_TRY(pack<Real>(s, sh.un, base, sh.unit_base, sh.cnt, sh.lay, pk));
+    OBTE_TRY(pack<Real>(s, sh.un, base.un, sh.unit_base, sh.cnt, sh.lay, pk));
   }
   const Units& un = sh.un;
   const std::vector<int64_t>& unit_base = sh.unit_base;
