@@ -58,8 +58,8 @@ static constexpr int kMaxUnit = 1023;     // of any layout (counts of a header h
 //             output block << 16
 //   header 1: of unit u + nbuf: record block (kBlkUnit bytes) and value (16 bytes) sources, their sizes (16-byte units,
 //             block | values << 16), its first bank row among all units' rows
-//   outputs:  periodic sources (int2: source slot, row; padded to 16 B), wall / contact entries (int4: row,
-//             count | first of the unit's wall entries << 3 | wall entries of the unit << 16, contact entry, first
+//   outputs:  periodic sources (int2: source slot, row; padded to 16 B), wall / contact entries (int4: row | entry
+//             in the second order of the contact sums << 20, count | first of the unit's wall entries << 3 | wall entries of the unit << 16, contact entry, first
 //             wall entry overall; those with a contact entry first, in the order of their sums), wall entries (4 reals: area vector / volume, 1 / (-sum_mq min(sigma . w, 0))),
 //             their wall indices
 __host__ __device__ constexpr int rec_words(int real_bytes, int nf) {
@@ -289,15 +289,18 @@ struct Packed {
   int64_t n_pf = 0;
 };
 
-// The place of each contact entry of direction q in the sums K and S of an output pass, by entry (relative to the
+// The places of each contact entry of direction q in the sums K and S of an output pass, by entry (relative to the
 // direction's first).  The sums are in the sweep's precision, so their order is part of the result: unit by unit
-// of the base layout, in a unit the 32-element groups with fewer contact elements first (of equal ones the later
-// group), elements of a group in order.  That is the order in which one FP32 shared-memory atomic per element and MFP
-// arrives most often from a CTA with one element of a base unit to a thread: on 8,000 triangles x 60 x 48 at least
-// 2,876 of 2,880 sums have these bits (2,858 in position order; two runs of the atomics agree on as many), while
-// sums in FP64 would be 1e-7 off.  Beside it the atomics cost time: the resident solve of 60,000 triangles x 100 x 96
-// went from 46.1 to 45.0 ms without them, 8,000 x 60 x 48 from 11.95 to 11.83 ms.
-static void contact_order(const Schedule& s, const Units& base, int q, std::vector<int32_t>& place) {
+// of the base layout, in a unit the 32-element groups with fewer contact elements first, elements of a group in order;
+// of groups with equally many the later one first (`first`) or the earlier one first (`second`): K and S of an FP32
+// pass are the means of the two sums.  That is how one FP32 shared-memory atomic per element and MFP arrives from a CTA with one
+// element of a base unit to a thread: a group with fewer of them is through first, and which of two equal ones is, is
+// left to chance.  On 8,000 triangles x 60 x 48 at least 2,876 of 2,880 sums of such atomics have these bits in one of the
+// orders (2,858 in position order); their mean is 0.6e-9 to 1.1e-9 off K of a run of the atomics, two runs
+// 0.5e-9 to 1.5e-9 off each other, and sums in FP64 1e-7.  The atomics also cost time: the resident solve of 60,000
+// triangles x 100 x 96 went from 46.1 to 45.0 ms without them, 8,000 x 60 x 48 from 11.95 to 11.83 ms.
+static void contact_order(const Schedule& s, const Units& base, int q, std::vector<int32_t>& first,
+                          std::vector<int32_t>& second) {
   struct Entry { int32_t unit, count, group, pos; };
   std::vector<Entry> e;
   const int32_t* up = base.ptr.data() + base.off[q];
@@ -309,15 +312,19 @@ static void contact_order(const Schedule& s, const Units& base, int q, std::vect
     for (size_t k = a; k < b; ++k) e[k].count = (int32_t)(b - a);
   }
   std::vector<int32_t> ord(e.size());
-  std::iota(ord.begin(), ord.end(), 0);
-  std::sort(ord.begin(), ord.end(), [&](int32_t i, int32_t j) {
-    const Entry &x = e[i], &y = e[j];
-    if (x.unit != y.unit) return x.unit < y.unit;
-    if (x.count != y.count) return x.count < y.count;
-    return x.group != y.group ? x.group > y.group : x.pos < y.pos;
-  });
-  place.resize(e.size());
-  for (size_t k = 0; k < ord.size(); ++k) place[ord[k]] = (int32_t)k;
+  auto places = [&](bool late, std::vector<int32_t>& place) {
+    std::iota(ord.begin(), ord.end(), 0);
+    std::sort(ord.begin(), ord.end(), [&](int32_t i, int32_t j) {
+      const Entry &x = e[i], &y = e[j];
+      if (x.unit != y.unit) return x.unit < y.unit;
+      if (x.count != y.count) return x.count < y.count;
+      return x.group != y.group ? (x.group > y.group) == late : x.pos < y.pos;
+    });
+    place.resize(e.size());
+    for (size_t k = 0; k < ord.size(); ++k) place[ord[k]] = (int32_t)k;
+  };
+  places(true, first);
+  places(false, second);
 }
 
 // base: the units of the base layout
@@ -406,10 +413,12 @@ static obte_status pack(const Schedule& s, const Units& un, const Units& base, c
     int64_t nsp = spec_base[q];
     const int32_t* up = un.ptr.data() + un.off[q];
     int32_t wo_run = s.wo_off[q];          // first wall entry of the unit
-    std::vector<int32_t> place;            // of the direction's contact entries in their sums
-    contact_order(s, base, q, place);
+    std::vector<int32_t> place, place2;    // of the direction's contact entries in their sums
+    contact_order(s, base, q, place, place2);
     size_t ce = 0;                         // contact entries before the element
-    std::vector<std::pair<int32_t, std::array<int32_t, 4>>> entries;   // the unit's wall / contact entries
+    struct Out { int32_t first, second, w[4]; };
+    std::vector<Out> entries;              // the unit's wall / contact entries
+    std::vector<int32_t> ranked;
     for (int u = 0; u < un.n[q]; ++u) {
       const int64_t gu = unit_base[q] + u;
       const int n_el = up[u + 1] - up[u], npf = cnt[4 * gu], nwo = cnt[4 * gu + 1], nx = cnt[4 * gu + 2],
@@ -498,7 +507,7 @@ static obte_status pack(const Schedule& s, const Units& un, const Units& base, c
         r[3] = field(row_in[3]);
         if (s.wout[it] != 0 || s.contact[it] >= 0) {
           const bool contact = s.contact[it] >= 0;
-          entries.push_back({contact ? place[ce] : INT_MAX,
+          entries.push_back({contact ? place[ce] : INT_MAX, contact ? place2[ce] : INT_MAX,
                              {field(so) << 4,
                               (s.wout[it] ? (((s.wout[it] >> 3) - wo_run) << 3) | (s.wout[it] & 7) : 0) | (nwo << 16),
                               s.contact[it], s.wout[it] >> 3}});
@@ -525,9 +534,15 @@ static obte_status pack(const Schedule& s, const Units& un, const Units& base, c
         std::memcpy(&r[COEF + s.n_up * CSTEP], &dv, sizeof(Real));
         for (int wd = COEF + (s.n_up + 1) * CSTEP; wd < W; ++wd) r[wd] = 0;   // padding to 16 bytes
       }
-      // contact entries in the order of their sums, then the others
-      std::stable_sort(entries.begin(), entries.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
-      for (const auto& e : entries) wo = std::copy(e.second.begin(), e.second.end(), wo);
+      // contact entries in the first order of their sums, then the others; with the i-th, the one that is i-th in the
+      // second order
+      std::stable_sort(entries.begin(), entries.end(), [](const Out& a, const Out& b) { return a.first < b.first; });
+      ranked.resize(n_contact);
+      std::iota(ranked.begin(), ranked.end(), 0);
+      std::sort(ranked.begin(), ranked.end(),
+                [&](int32_t a, int32_t b) { return entries[a].second < entries[b].second; });
+      for (int i = 0; i < n_contact; ++i) entries[i].w[0] |= ranked[i] << 20;
+      for (const Out& e : entries) wo = std::copy(e.w, e.w + 4, wo);
       head[2] |= n_contact << 20;
       wo_run += nwo;
     }
@@ -902,7 +917,7 @@ __device__ __forceinline__ void wall_outputs(const SweepParams<Real>& p, const u
                                              const unsigned char* ring, const Real* s_sig, double* dT_out, int chunk) {
   const int4 ent = reinterpret_cast<const int4*>(wb)[i];
   Real T[MC];
-  row_load(ring, (unsigned)ent.x, T);
+  row_load(ring, (unsigned)ent.x & 0xFFFF0u, T);
   if constexpr (DF) {
 #pragma unroll
     for (int j = 0; j < MC; ++j) T[j] = dpack_value(T[j]);
@@ -1062,7 +1077,8 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
   int4 hd = make_int4(0, 0, 0, 0);
   // final pass: kappa and suppression sums of the direction, MFP `cj` in this thread (a warp before the issuer's)
   const int cj = nthr >= 64 ? tid - (nthr - 64) : tid;
-  Real ksum = 0, ssum = 0;
+  constexpr bool kTwoOrders = sizeof(Real) == 4;   // in FP64 the order is below any tolerance
+  Real ksum = 0, ssum = 0, ksum2 = 0, ssum2 = 0;
   // MFP j of the row at byte offset `off`
   auto row_value = [&](unsigned off, int j) -> Real {
     constexpr int H = 16 / (int)sizeof(Real);
@@ -1070,21 +1086,21 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
     if constexpr (DF) return dpack_value(v);
     else return v;
   };
-  // The unit's part of the contact sums in its entries' order (contact_order): products rounded, then added one by
-  // one, loads four entries ahead.  One thread per MFP instead of one shared-memory atomic per element and MFP:
-  // the sums are the same in every pass and whatever the threads and stages.
-  auto contacts = [&](const int4* ent, int count) {
+  // The unit's part of the contact sums in one of the two orders of its entries (contact_order): products rounded, then
+  // added one by one, loads four entries ahead.  One thread per MFP: the sums are the same in every pass and
+  // whatever the threads and stages.
+  auto contacts = [&](const int4* ent, int count, bool second, Real& ks, Real& ss) {
     for (int i0 = 0; i0 < count; i0 += 4) {
       Real kv[4], sv[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         kv[k] = sv[k] = Real(0);
         if (i0 + k < count) {
-          const int4 e = ent[i0 + k];
-          const Real T = row_value((unsigned)e.x, cj);
+          const int4 e = ent[second ? (int)((unsigned)ent[i0 + k].x >> 20) : i0 + k];
+          const Real T = row_value((unsigned)e.x & 0xFFFF0u, cj);
           kv[k] = mul_rn(p.kcoef[(int64_t)e.z * p.m_pad + m0 + cj], T);
           sv[k] = mul_rn(p.scoef[e.z], T);
-          if (p.det) {
+          if (p.det && !second) {
             p.kpart[(int64_t)e.z * p.m_pad + m0 + cj] = kv[k];
             p.spart[(int64_t)e.z * p.m_pad + m0 + cj] = sv[k];
           }
@@ -1092,8 +1108,8 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        ksum += kv[k];
-        ssum += sv[k];
+        ks += kv[k];
+        ss += sv[k];
       }
     }
   };
@@ -1118,7 +1134,11 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
         wall_outputs<Real, MC, DF>(p, wb, nw, i, ring, s_sig, dT_out, chunk);
       }
       if constexpr (FINAL) {
-        if (cj >= 0 && cj < mc) contacts(reinterpret_cast<const int4*>(wb), counts >> 20);
+        if (cj >= 0 && cj < mc) {
+          contacts(reinterpret_cast<const int4*>(wb), counts >> 20, false, ksum, ssum);
+          if constexpr (kTwoOrders)
+            if (!p.det) contacts(reinterpret_cast<const int4*>(wb), counts >> 20, true, ksum2, ssum2);
+        }
       }
     }
   };
@@ -1324,8 +1344,8 @@ __global__ void __launch_bounds__(kMaxThreads, SweepMinBlocks<Real, KV>::v)
   }
   if (counts) outputs(smem + p.out0 + oi * p.out, counts);
   if (FINAL && !p.det && cj >= 0 && cj < mc) {
-    p.K[(int64_t)(m0 + cj) * p.n_dir + q] = (double)ksum;
-    p.S_out[(int64_t)(m0 + cj) * p.n_dir + q] = (double)ssum;
+    p.K[(int64_t)(m0 + cj) * p.n_dir + q] = kTwoOrders ? 0.5 * ((double)ksum + (double)ksum2) : (double)ksum;
+    p.S_out[(int64_t)(m0 + cj) * p.n_dir + q] = kTwoOrders ? 0.5 * ((double)ssum + (double)ssum2) : (double)ssum;
   }
 }
 

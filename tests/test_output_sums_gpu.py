@@ -2,8 +2,9 @@
 
 An FP32 output pass adds kcoef T and scoef T of a direction's contact elements in FP32, so their order is part of
 the result: by units of 128 elements of a level (fewer where more than 48 cut inflow faces or 64 elements with
-outputs would come together), in a unit the groups of 32 elements with fewer contact elements first (of
-equal ones the later group), elements of a group in order.  The sums are restated here in numpy from the stored
+outputs would come together), in a unit the groups of 32 elements with fewer contact elements first, elements of a
+group in order; K and S are the means of the sums with the later and with the earlier of equal groups first.  The sums
+are restated here in numpy from the stored
 temperatures of the same pass; one FP32 rounding in another place is 6e-8 of a sum, so 1e-12 holds the order.
 Repeated passes and other threads, stages and (larger) units give the same bits; units below 128 elements
 cut the groups, and agree to FP32 rounding only: n terms of one sign, n 6e-8 at most, 1e-5 for a few hundred.
@@ -64,7 +65,7 @@ def _units(lp, order, n_cut, special):
 
 
 def _sums(geo, mat, bcs, ek, plan, T):
-    """K and S [n_mfp, n_dir] in FP32 as the pass adds them, the constant of K and the shifts of both per offset."""
+    """K and S [n_mfp, n_dir] from FP32 sums as the pass adds them, the constant of K and the shifts of both per offset."""
     row, nb, k, cut = sweep_order.directed_faces(geo)
     dirs = np.asarray(mat.vmfp)
     walls = np.asarray(geo.side_physical_regions["Boundary"])
@@ -91,7 +92,7 @@ def _sums(geo, mat, bcs, ek, plan, T):
     total = sum(len(f) for f, _ in free)
     pf = 48 if 100 * sum(o[0] for _, o in free) <= total else none
     sx = 64 if 100 * sum(o[1] for _, o in free) <= total else none
-    K, S = np.zeros((n_mfp, n_dir), np.float32), np.zeros((n_mfp, n_dir), np.float32)
+    K, S = np.zeros((2, n_mfp, n_dir), np.float32), np.zeros((2, n_mfp, n_dir), np.float32)
     const, kshift, sshift = np.zeros((n_mfp, n_dir)), np.zeros((n_mfp, n_dir)), np.zeros(n_dir)
     for q, (order, lp, u) in enumerate(data):
         first = np.array(u(pf, sx)[0])
@@ -111,12 +112,14 @@ def _sums(geo, mat, bcs, ek, plan, T):
         group = (pos - first[unit]) // 32
         tag = unit * 8 + group
         count = np.bincount(tag, minlength=tag.max() + 1)[tag]
-        for p in pos[np.lexsort((pos, -group, count, unit))]:
-            e = order[p]
-            K[:, q] = K[:, q] + (kc[e] * ek.normalization).astype(np.float32) * T[q, e]
-            S[:, q] = S[:, q] + np.float32(sc[e] * ek.normalization) * T[q, e]
+        for o, ties in enumerate((-group, group)):
+            for p in pos[np.lexsort((pos, ties, count, unit))]:
+                e = order[p]
+                K[o, :, q] = K[o, :, q] + (kc[e] * ek.normalization).astype(np.float32) * T[q, e]
+                S[o, :, q] = S[o, :, q] + np.float32(sc[e] * ek.normalization) * T[q, e]
         kshift[:, q] = (kc * ek.normalization).sum(axis=0)
         sshift[q] = sc.sum() * ek.normalization
+    K, S = K.astype(np.float64).mean(axis=0), S.astype(np.float64).mean(axis=0)
     return K, S, const * ek.normalization * bcs.periodic[ek.contact], kshift, sshift
 
 
