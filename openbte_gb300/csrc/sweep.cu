@@ -1469,12 +1469,13 @@ static int frozen_mc32(const Schedule& s, const UnitStats& base) {
 // us, 20,000 x 100 x 96 (2,400, 4) 2,754 and 2,594, 60,000 x 100 x 96 (2,400, 4) 6,554 and 6,008, x 100 x 48 (1,200, 4) 3,421
 // and 3,119; with 1.03 and 1.18 waves 60,000 x 52 x 48 (624, 4) 2,003 and 2,295, 20,000 x 60 x 48 (720, 4) 958 and
 // 1,181; with three to an SM 40,000 x 100 x 96 5,075 and 5,151, with two 180,000 x 60 x 48 5,830 and 6,843; in half a
-// wave 2,000 x 30 x 48 (384, 5) 146 and 194.  (The line is for a sweep alone: with four streams at once, whose CTAs fill
+// wave 2,000 x 30 x 48 (384, 5) 146 and 194; in 1.37 waves an output pass of 128^2 squares x 50 x 64 (832, 4) 3,513 and
+// 3,280.  (The line is for a sweep alone: with four streams at once, whose CTAs fill
 // each other's waves, four to a CTA were 3 to 20 % faster at each of nine sizes, 20,000 x 60 x 48 among them.)  Only with
 // two inflow rows do they fit the registers (8,000 tetrahedra x 30 x 128 704 and 718).
 static bool wide64(int64_t ctas, int resident, int sms) {
   const double waves = (double)ctas / ((double)std::max(resident, 1) * sms);
-  return resident >= 4 && std::ceil(waves) <= 1.3 * waves;
+  return resident >= 4 && std::ceil(waves) <= 1.6 * waves;
 }
 
 // The units of the base layout and their counts.
