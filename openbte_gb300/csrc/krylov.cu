@@ -123,6 +123,12 @@ struct ArnoldiParams {
   double* col;                               // h (+ h2) [k], |w|, second pass ran, the plan's error word
   const int* err;
 };
+// The error word goes with the column, from a warp of the last block: in block 0, which forms the column, its load and
+// store lengthened the last phase from 8.5 to 13.7 us.
+template <typename Real>
+__device__ __forceinline__ void arnoldi_error(const ArnoldiParams<Real>& P) {
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == VT - 1) P.col[P.k + 2] = *P.err != 0 ? 1.0 : 0.0;
+}
 
 template <typename Real>
 __device__ __forceinline__ void arnoldi_dots(const ArnoldiParams<Real>& P, bool first, int kk, Real* buf) {
@@ -331,7 +337,6 @@ __device__ __forceinline__ void arnoldi_finish(const ArnoldiParams<Real>& P, con
     if (blockIdx.x == 0) {
       P.col[k] = hn;
       P.col[k + 1] = two ? 1.0 : 0.0;
-      P.col[k + 2] = (double)*P.err;
     }
   }
   if (blockIdx.x == 0)
@@ -358,6 +363,7 @@ __global__ void __launch_bounds__(VT, 2) arnoldi_kernel(const __grid_constant__ 
   __shared__ double sc;
   ClusterBarrier bar(BarrierParams{});
   const int k = P.k;
+  arnoldi_error(P);
   arnoldi_dots(P, true, k + 1, buf);
   bar.wait();
   arnoldi_sums(P, k + 1, h);
@@ -403,6 +409,7 @@ __global__ void __launch_bounds__(VT, 2) arnoldi_phase_kernel(const __grid_const
   } else {
     __shared__ double red[VT];
     __shared__ double sc;
+    arnoldi_error(P);
     const bool two = *P.two != 0;
     double s = 0;
     grid_sum(P.s_part + (two ? P.groups : 0), P.groups, red, [&](double v) { return s = v; });
