@@ -158,12 +158,22 @@ __global__ void __launch_bounds__(Bar::kThreads, Bar::kBlocks == 1 ? 1 : 4) dsa_
   if (!bar.wait()) return;
   if (P.project) mu = mean(P.part + segments);
   const int64_t n = P.n, xoff = P.n + P.nd, t = (int64_t)blockIdx.x * nthr + tid, stride = (int64_t)nb * nthr;
-  for (int64_t i = t; i < P.nu; i += stride) {
-    const int64_t x = i - xoff;
-    int64_t c = i;
-    if (x >= 0) c = P.xcell[P.nu < ((int64_t)1 << 31) ? (int64_t)((unsigned)x / (unsigned)P.n_mfp) : x / P.n_mfp];
-    else if (i >= n) c = P.wcell[i - n];
-    P.out[i] = P.base[i] + (P.d[c] - mu);
+  // four entries of a thread at a time, their loads (element, correction) before any store: the state is larger than
+  // the elements by the walls and the inflow, and a block has few threads
+  for (int64_t i0 = t; i0 < P.nu; i0 += 4 * stride) {
+    double v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int64_t i = i0 + k * stride, x = i - xoff;
+      if (i >= P.nu) continue;
+      int64_t c = i;
+      if (x >= 0) c = P.xcell[P.nu < ((int64_t)1 << 31) ? (int64_t)((unsigned)x / (unsigned)P.n_mfp) : x / P.n_mfp];
+      else if (i >= n) c = P.wcell[i - n];
+      v[k] = P.base[i] + (P.d[c] - mu);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i0 + k * stride < P.nu) P.out[i0 + k * stride] = v[k];
   }
 }
 
