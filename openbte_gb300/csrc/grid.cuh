@@ -335,8 +335,8 @@ struct PhaseShape {
   bool cluster;
 };
 // A cluster's barrier is the cheaper one, but its 8 SMs have a twentieth of the FP64 rate.  Fourier solves of 2D
-// cells, cluster against grid: 600 elements 2.75 and 3.76 ms, 1,100 3.45 and 3.96, 2,000 4.24 and 3.42, 8,000
-// 5.96 and 3.55; of a 3D one with 2,000, 17.6 and 15.6.
+// cells, cluster against grid: 600 elements 2.73 and 3.35 ms, 1,100 3.31 and 3.59, 1,500 3.97 and 3.95, 2,000 4.09 and
+// 3.46, 8,000 4.88 and 3.61; of a 3D one with 2,000, 16.8 and 15.5.
 //
 // A cooperative launch waits until all its blocks fit and then holds their room for the whole solve, while other
 // streams' kernels wait for theirs.  So a block takes no more than a third of an SM: 256 threads of 80 registers
