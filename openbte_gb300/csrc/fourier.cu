@@ -303,25 +303,32 @@ __global__ void __launch_bounds__(Bar::kThreads, Bar::kBlocks) fourier_kernel(co
   }
 }
 
-// diffusive kappa terms per contact side (objects.py:152-170)
-__global__ void contact_kernel(int64_t nc, const int32_t* __restrict__ e1, const int32_t* __restrict__ e2,
-                               const double* __restrict__ coef, double t2const, const double* __restrict__ T,
-                               double* __restrict__ out) {
-  for (int64_t k = (int64_t)blockIdx.x * FT + threadIdx.x; k < nc; k += (int64_t)gridDim.x * FT) {
-    const double t2 = e2[k] >= 0 ? T[e2[k]] + t2const : t2const;
-    out[k] = (T[e1[k]] - t2) * coef[k];
+// After the solve: diffusive kappa terms per contact side (objects.py:152-170), the solve's counts and error word, all
+// into page-locked host memory, and J = -kappa . grad.  (Copied from the device they waited in the copy engine's queue
+// for the solve, and other streams' copies behind them: a sweep beside two streams of Fourier solves, 0.08 ms alone, took
+// half a solve.)
+struct OutputParams {
+  int64_t n, nc;
+  int dim;
+  const int32_t *e1, *e2;
+  const double *coef, *T, *kap, *grad, *sc;
+  double t2const;
+  double *J, *words, *terms;
+};
+__global__ void __launch_bounds__(FT) fourier_outputs_kernel(const __grid_constant__ OutputParams P) {
+  const int64_t t0 = (int64_t)blockIdx.x * FT + threadIdx.x, stride = (int64_t)gridDim.x * FT;
+  if (t0 < 4) P.words[t0] = P.sc[t0];
+  for (int64_t k = t0; k < P.nc; k += stride) {
+    const double t2 = P.e2[k] >= 0 ? P.T[P.e2[k]] + P.t2const : P.t2const;
+    P.terms[k] = (P.T[P.e1[k]] - t2) * P.coef[k];
   }
-}
-
-// J = -kappa . grad
-__global__ void flux_kernel(int64_t n, int dim, const double* __restrict__ kap, const double* __restrict__ grad,
-                            double* __restrict__ J) {
-  for (int64_t c = (int64_t)blockIdx.x * FT + threadIdx.x; c < n; c += (int64_t)gridDim.x * FT)
-    for (int a = 0; a < dim; ++a) {
-      double s = 0;
-      for (int b = 0; b < dim; ++b) s += kap[a * dim + b] * grad[c * dim + b];
-      J[c * dim + a] = -s;
-    }
+  if (P.J)
+    for (int64_t c = t0; c < P.n; c += stride)
+      for (int a = 0; a < P.dim; ++a) {
+        double s = 0;
+        for (int b = 0; b < P.dim; ++b) s += P.kap[a * P.dim + b] * P.grad[c * P.dim + b];
+        P.J[c * P.dim + a] = -s;
+      }
 }
 
 }  // namespace
@@ -337,8 +344,8 @@ struct obte_fourier_plan_s {
   obte::DevBuf rp, ci, val, dinv, vol, B, colpin, g_nb, g_off, g_mixed, gw, s_i, s_j, s_w, s_vnon, c_ptr, c_side,
       k_e1, k_e2, k_coef, kap;
   // work
-  obte::DevBuf C, r, z, p, Ap, part, sc, grad, kout;
-  obte::HostBuf hout;               // the two counts of a solve and the error word, read back
+  obte::DevBuf C, r, z, p, Ap, part, sc, grad;
+  obte::HostBuf hout;               // the two counts of a solve, its error word and kappa terms, written by the device
   int test_skip = -1, test_polls = 0;   // obte_fourier_plan_test_barrier_timeout
   // smoothed-aggregation AMG V-cycle as the CG preconditioner (null: Jacobi)
   obte::AmgPtr amg;
@@ -530,7 +537,6 @@ extern "C" obte_status obte_fourier_plan_create(obte_context ctx, const obte_fou
   up(P->C.alloc(vb)); up(P->r.alloc(2 * vb)); up(P->z.alloc(vb)); up(P->p.alloc(2 * vb));
   up(P->Ap.alloc(vb)); up(P->part.alloc(7 * sizeof(double) * (size_t)fourier_shape(n, ctx->num_sms).blocks));
   up(P->sc.alloc(4 * sizeof(double))); up(P->grad.alloc(vb * dim));
-  up(P->kout.alloc((size_t)std::max<int64_t>(P->nc, 1) * 8));
   // OBTE_FOURIER_JACOBI=1 keeps the diagonal preconditioner (same solution, ~40x more CG iterations)
   const char* jac = std::getenv("OBTE_FOURIER_JACOBI");
   if (s0 == OBTE_OK && !(jac && std::atoi(jac) != 0))
@@ -569,7 +575,7 @@ extern "C" obte_status obte_fourier_solve(obte_fourier_plan P, const obte_fourie
   const double rtol = opts->rtol > 0 ? opts->rtol : 1e-8;
   const double cg_rtol = opts->cg_rtol > 0 ? opts->cg_rtol : 1e-13;
   const int cg_max = opts->cg_max_iter > 0 ? opts->cg_max_iter : 20000;
-  if (!P->hout.p) OBTE_TRY(P->hout.alloc(4 * sizeof(double)));
+  if (!P->hout.p) OBTE_TRY(P->hout.alloc((size_t)(4 + P->nc) * sizeof(double)));
   FourierParams f = {};
   f.n = n;
   f.A = CsrDev{n, P->rp.as<int32_t>(), P->ci.as<int32_t>(), P->val.as<double>()};
@@ -603,27 +609,23 @@ extern "C" obte_status obte_fourier_solve(obte_fourier_plan P, const obte_fourie
                                               : fourier_kernel<GridBarrier>,
                          f, f.smem, most, st));
   count_launch();
-  double kappa = 0;
-  std::vector<double> kh(std::max<int64_t>(P->nc, 1));
-  if (P->nc > 0) {
-    contact_kernel<<<nb, FT, 0, st>>>(P->nc, P->k_e1.as<int32_t>(), P->k_e2.as<int32_t>(), P->k_coef.as<double>(),
-                                      P->contact_t2, T, P->kout.as<double>());
-    count_launch();
-    OBTE_CUDA(cudaMemcpyAsync(kh.data(), P->kout.p, P->nc * 8, cudaMemcpyDeviceToHost, st));
-  }
-  if (J) {
-    flux_kernel<<<nb, FT, 0, st>>>(n, P->dim, P->kap.as<double>(), P->grad.as<double>(), J);
-    count_launch();
-  }
-  OBTE_CUDA(cudaGetLastError());
   double* h = P->hout.as<double>();
-  OBTE_CUDA(cudaMemcpyAsync(h, P->sc.p, 4 * sizeof(double), cudaMemcpyDeviceToHost, st));
+  OutputParams o = {};
+  o.n = n; o.nc = P->nc; o.dim = P->dim;
+  o.e1 = P->k_e1.as<int32_t>(); o.e2 = P->k_e2.as<int32_t>(); o.coef = P->k_coef.as<double>();
+  o.T = T; o.kap = P->kap.as<double>(); o.grad = P->grad.as<double>(); o.sc = P->sc.as<double>();
+  o.t2const = P->contact_t2;
+  o.J = J; o.words = h; o.terms = h + 4;
+  fourier_outputs_kernel<<<nb, FT, 0, st>>>(o);
+  count_launch();
+  OBTE_CUDA(cudaGetLastError());
   OBTE_CUDA(cudaStreamSynchronize(st));
   if (reinterpret_cast<int*>(h + 3)[0] != 0) {
     set_error("a device-side wait timed out in the Fourier kernel");
     return OBTE_ERR_DEVICE_TIMEOUT;
   }
-  for (int64_t k = 0; k < P->nc; ++k) kappa += kh[k];
+  double kappa = 0;
+  for (int64_t k = 0; k < P->nc; ++k) kappa += h[4 + k];
   if (info) {
     info->kappa = kappa;
     info->n_iter = (int32_t)h[0];
